@@ -41,6 +41,9 @@ struct Linear {
   // FP8 mode: the same matrix as e4m3 = round(w / wscale), wscale = max|w| / 448
   void* w8 = nullptr;
   float wscale = 1.0f;
+  // fp32 mode: w holds three bf16 planes of N * K elements (split3.cuh), the operand of
+  // launch_gemm_split; only the skinny conditioning layers keep fp32 values
+  bool split = false;
   bool w8_stale = false;  // w was rewritten after w8 was formed: requantise at the next finalize
 };
 
@@ -68,8 +71,9 @@ struct Workspace {
   int B = 0, Tc = 0, Tx = 0;
   // f32
   float *temb, *th, *tout, *ph, *y, *mod, *c, *x, *pooled_f32;
-  // activation-dtype buffers (bf16, or f32 in the exact mode)
+  // activation buffers: bf16, or in the fp32 mode the three bf16 planes a GEMM reads (q, k, v: fp32)
   void *cap_in, *patches, *h_c, *h_x, *h_x2, *qkv, *qkv2, *o_c, *o_x, *o_x2, *hid_x, *hid_c;
+  float* o_f32 = nullptr;  // fp32 mode: attention output before it is split
   bf16* y_bf = nullptr;  // conditioning vector as a GEMM operand
   void* a8 = nullptr;    // FP8 mode: e4m3 copy of the current GEMM's left operand
   void* attn_scratch = nullptr;  // partial results of key-split attention launches (small batches, long sequences)
@@ -122,9 +126,11 @@ int dev_alloc(sd3_model* m, void** p, size_t bytes) {
   return ST_OK;
 }
 
-// weight given as (in, out) of dtype -> packed (out, in) at dst (model precision)
-int pack_linear_weight(sd3_model* m, const void* src, int dtype, int in_f, int out_f, void* dst,
+// weight given as (in, out) of dtype -> packed (out, in) at dst (model precision, or three planes)
+int pack_linear_weight(sd3_model* m, const void* src, int dtype, int in_f, int out_f, void* dst, bool split,
                        cudaStream_t st) {
+  if (split)
+    return launch_transpose_split3(src, dtype == SD3_DTYPE_F32, static_cast<bf16*>(dst), in_f, out_f, st);
   return launch_transpose(src, dtype == SD3_DTYPE_F32, dst, m->f32, in_f, out_f, st);
 }
 
@@ -250,7 +256,7 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
     if (e != cudaSuccess) return check_cuda(e, "cudaFree(workspace)");
   }
   const sd3_config& c = m->cfg;
-  const size_t E = m->E, F = m->F, T = static_cast<size_t>(Tc) + Tx, ab = m->wbytes();
+  const size_t E = m->E, F = m->F, T = static_cast<size_t>(Tc) + Tx, ab = m->f32 ? 6 : 2, qb = m->f32 ? 4 : 2;
   const size_t nB = B, nTc = static_cast<size_t>(B) * Tc, nTx = static_cast<size_t>(B) * Tx;
   struct Item { void** p; size_t bytes; };
   std::vector<Item> items = {
@@ -262,9 +268,10 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
       {&w.cap_in, nTc * static_cast<size_t>(c.captions_dim > 0 ? c.captions_dim : 1) * ab},
       {&w.patches, nTx * static_cast<size_t>(m->Kp > 0 ? m->Kp : 1) * ab},
       {&w.h_c, nTc * E * ab}, {&w.h_x, nTx * E * ab}, {&w.h_x2, nTx * E * ab},
-      {&w.qkv, nB * T * 3 * E * ab}, {&w.qkv2, nTx * 3 * E * ab},
+      {&w.qkv, nB * T * 3 * E * qb}, {&w.qkv2, nTx * 3 * E * qb},
       {&w.o_c, nTc * E * ab}, {&w.o_x, nTx * E * ab}, {&w.o_x2, nTx * E * ab},
       {&w.hid_x, nTx * F * ab}, {&w.hid_c, nTc * F * ab},
+      {(void**)&w.o_f32, m->f32 ? nB * T * E * 4 : 16},
       {&w.a8, m->fp8 ? (nTx > nTc ? nTx : nTc) * F : 16},
       {&w.attn_scratch, 16},
   };
@@ -294,6 +301,19 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
   return ST_OK;
 }
 
+// fp32 mode: A is three bf16 planes of M * K elements
+SplitGemmProblem split_problem(const Linear& L, const void* A, int M, const GemmEpilogue& e) {
+  SplitGemmProblem p;
+  p.A = static_cast<const bf16*>(A);
+  p.a_plane = static_cast<long>(M) * L.K;
+  p.W = static_cast<const bf16*>(L.w);
+  p.w_plane = static_cast<long>(L.N) * L.K;
+  p.M = M;
+  p.epi = e;
+  if (!p.epi.bias) p.epi.bias = L.b;
+  return p;
+}
+
 // a_e4m3: A already holds e4m3 bytes (FP8 mode: written by ln_modulate, the GELU
 // epilogue or a conversion pass)
 int run_linear(sd3_model* m, const Linear& L, const void* A, int M, const GemmEpilogue& e,
@@ -304,9 +324,7 @@ int run_linear(sd3_model* m, const Linear& L, const void* A, int M, const GemmEp
   }
   GemmEpilogue ee = e;
   if (!ee.bias) ee.bias = L.b;
-  if (m->f32)
-    return launch_gemm_f32(static_cast<const float*>(A), L.K, static_cast<const float*>(L.w), L.K,
-                           M, L.N, L.K, ee, st);
+  if (m->f32) return launch_gemm_split(split_problem(L, A, M, ee), nullptr, L.N, L.K, m->status, st);
   if (m->fp8 && L.w8) {
     // e4m3 x e4m3: the bf16 operand is converted as is (scale 1: LayerNorm
     // outputs, attention outputs and GELU outputs sit well inside e4m3's range and
@@ -334,6 +352,10 @@ int run_linear_pair(sd3_model* m, const Linear& La, const void* Aa, int Ma, cons
   const bool fp8a = m->fp8 && La.w8 && a8a, fp8b = m->fp8 && Lb.w8 && a8b;
   const bool plain_a = !(m->fp8 && La.w8) && !a8a, plain_b = !(m->fp8 && Lb.w8) && !a8b;
   const bool same_kind = (fp8a && fp8b) || (plain_a && plain_b);
+  if (m->f32 && La.w && Lb.w && La.N == Lb.N && La.K == Lb.K) {
+    const SplitGemmProblem b = split_problem(Lb, Ab, Mb, eb);
+    return launch_gemm_split(split_problem(La, Aa, Ma, ea), &b, La.N, La.K, m->status, st);
+  }
   if (m->f32 || !La.w || !Lb.w || La.N != Lb.N || La.K != Lb.K || !same_kind) {
     int rc = run_linear(m, La, Aa, Ma, ea, st, a8a);
     if (rc) return rc;
@@ -348,33 +370,44 @@ int run_linear_pair(sd3_model* m, const Linear& La, const void* Aa, int Ma, cons
   return launch_gemm_grouped(pa, pb, fp8a ? OPERAND_E4M3 : OPERAND_BF16, La.N, La.K, m->status, st);
 }
 
-// QKV projection of `T_in` tokens per sample into rows [row_off, row_off+T_in)
-// of each sample of the packed (B, T_total, 3E) buffer, q/k RMSNorm included.
-int run_qkv(sd3_model* m, const Linear& L, const void* h, void* qkv, int B, int T_in, int T_total,
-            int row_off, const float* wq, const float* wk, cudaStream_t st, bool h_e4m3 = false) {
-  const int E = m->E;
-  const bool norm = m->cfg.use_qk_norm && (wq || wk);
-  const bool fused = !m->f32 && m->D == 64;
+GemmEpilogue qkv_epilogue(sd3_model* m, void* qkv, int T_in, int T_total, int row_off, const float* wq,
+                          const float* wk) {
   GemmEpilogue e;
   e.mode = EPI_QKV_NORM;
   e.out = qkv;
   e.out_f32 = m->f32;
-  e.ldo = 3L * E;
+  e.ldo = 3L * m->E;
   e.rows_in = T_in; e.rows_out = T_total; e.row_off = row_off;
-  e.wq = wq; e.wk = wk; e.qk_cols = 2 * E; e.eps = 1e-6f;
-  e.do_norm = (fused && norm) ? 1 : 0;
-  if (!fused) e.qk_cols = 0;
-  int rc = run_linear(m, L, h, B * T_in, e, st, h_e4m3);
-  if (rc || fused || !norm) return rc;
-  const size_t ab = m->wbytes();
+  e.wq = wq; e.wk = wk; e.eps = 1e-6f;
+  e.qk_cols = m->D == 64 ? 2 * m->E : 0;  // fused for head_dim 64, run_qk_norm otherwise
+  e.do_norm = (m->D == 64 && m->cfg.use_qk_norm && (wq || wk)) ? 1 : 0;
+  return e;
+}
+
+// q/k RMSNorm of rows [row_off, row_off + T_in) of each sample of the packed (B, T_total, 3E) buffer, for
+// the head sizes whose norm is not fused into the QKV GEMM
+int run_qk_norm(sd3_model* m, void* qkv, int B, int T_in, int T_total, int row_off, const float* wq,
+                const float* wk, cudaStream_t st) {
+  const int E = m->E;
+  const size_t eb = m->f32 ? 4 : 2;
   for (int b = 0; b < B; ++b) {
-    char* rows = static_cast<char*>(qkv) + (static_cast<size_t>(b) * T_total + row_off) * 3 * E * ab;
-    rc = launch_rmsnorm_heads(rows, m->f32, 3L * E, T_in, 0, m->NH, m->D, wq, 1e-6f, st);
+    char* rows = static_cast<char*>(qkv) + (static_cast<size_t>(b) * T_total + row_off) * 3 * E * eb;
+    int rc = launch_rmsnorm_heads(rows, m->f32, 3L * E, T_in, 0, m->NH, m->D, wq, 1e-6f, st);
     if (rc) return rc;
     rc = launch_rmsnorm_heads(rows, m->f32, 3L * E, T_in, E, m->NH, m->D, wk, 1e-6f, st);
     if (rc) return rc;
   }
   return ST_OK;
+}
+
+// QKV projection of `T_in` tokens per sample into rows [row_off, row_off+T_in)
+// of each sample of the packed (B, T_total, 3E) buffer, q/k RMSNorm included.
+int run_qkv(sd3_model* m, const Linear& L, const void* h, void* qkv, int B, int T_in, int T_total,
+            int row_off, const float* wq, const float* wk, cudaStream_t st, bool h_e4m3 = false) {
+  const bool norm = m->cfg.use_qk_norm && (wq || wk);
+  int rc = run_linear(m, L, h, B * T_in, qkv_epilogue(m, qkv, T_in, T_total, row_off, wq, wk), st, h_e4m3);
+  if (rc || m->D == 64 || !norm) return rc;
+  return run_qk_norm(m, qkv, B, T_in, T_total, row_off, wq, wk, st);
 }
 
 // out_e4m3 (FP8 mode, head_dim 64 only): the outputs feed FP8 out-projections
@@ -391,44 +424,20 @@ int run_attention(sd3_model* m, const void* qkv, int B, int T, int Tc, void* o_c
     set_last_error("e4m3 attention output needs head_dim 64");
     return ST_UNSUPPORTED;
   }
-  const size_t ab = m->wbytes();
-  const char* q = static_cast<const char*>(qkv);
-  return launch_attention_simt(q, q + m->E * ab, q + 2 * m->E * ab, 3L * m->E, m->f32, B, T, m->NH,
-                               m->D, Tc, o_c, o_x, m->E, m->f32, scale, st);
-}
-
-int run_gate_resid(sd3_model* m, const Linear& L, const void* A, int B, int Tseg, const float* gate,
-                   long mod_stride, float* resid, cudaStream_t st, bool a_e4m3 = false) {
-  GemmEpilogue e;
-  e.mode = EPI_GATE_RESID;
-  e.out = resid; e.resid = resid; e.out_f32 = 1; e.ldo = L.N;
-  e.gate = gate; e.gate_stride = mod_stride;
-  e.rows_in = Tseg; e.rows_out = Tseg; e.row_off = 0;
-  return run_linear(m, L, A, B * Tseg, e, st, a_e4m3);
-}
-
-// hid_e4m3 (out): whether the hidden activations were written as e4m3
-int run_mlp1(sd3_model* m, const Linear& L, const Linear& next, const void* A, int M, void* hid,
-             cudaStream_t st, bool a_e4m3, bool* hid_e4m3) {
-  GemmEpilogue e;
-  e.mode = EPI_BIAS_GELU;
-  e.out = hid; e.out_f32 = m->f32; e.ldo = L.N;
-  *hid_e4m3 = m->fp8 && L.w8 && next.w8 && L.N % 64 == 0;
-  e.out_e4m3 = *hid_e4m3 ? 1 : 0;
-  return run_linear(m, L, A, M, e, st, a_e4m3);
-}
-
-GemmEpilogue qkv_epilogue(sd3_model* m, void* qkv, int T_in, int T_total, int row_off, const float* wq,
-                          const float* wk) {
-  GemmEpilogue e;
-  e.mode = EPI_QKV_NORM;
-  e.out = qkv;
-  e.out_f32 = 0;
-  e.ldo = 3L * m->E;
-  e.rows_in = T_in; e.rows_out = T_total; e.row_off = row_off;
-  e.wq = wq; e.wk = wk; e.qk_cols = 2 * m->E; e.eps = 1e-6f;
-  e.do_norm = (m->cfg.use_qk_norm && (wq || wk)) ? 1 : 0;
-  return e;
+  if (m->f32) {
+    // fp32 outputs: the context rows' block first, then the image rows'; each is split into its planes
+    const float* q = static_cast<const float*>(qkv);
+    const long E = m->E, nc = static_cast<long>(B) * Tc * E, nx = static_cast<long>(B) * (T - Tc) * E;
+    float* of = m->ws.o_f32;
+    int rc = launch_attention_simt(q, q + E, q + 2 * E, 3 * E, 1, B, T, m->NH, m->D, Tc, o_c ? of : nullptr, of + nc, E,
+                                   1, scale, st);
+    if (!rc && o_c && nc > 0) rc = launch_split3(of, 1, static_cast<bf16*>(o_c), nc, st);
+    if (!rc) rc = launch_split3(of + nc, 1, static_cast<bf16*>(o_x), nx, st);
+    return rc;
+  }
+  const bf16* q = static_cast<const bf16*>(qkv);
+  return launch_attention_simt(q, q + m->E, q + 2 * m->E, 3L * m->E, 0, B, T, m->NH, m->D, Tc, o_c, o_x, m->E, 0, scale,
+                               st);
 }
 
 GemmEpilogue gate_epilogue(const Linear& L, int Tseg, const float* gate, long mod_stride, float* resid) {
@@ -438,6 +447,23 @@ GemmEpilogue gate_epilogue(const Linear& L, int Tseg, const float* gate, long mo
   e.gate = gate; e.gate_stride = mod_stride;
   e.rows_in = Tseg; e.rows_out = Tseg; e.row_off = 0;
   return e;
+}
+
+int run_gate_resid(sd3_model* m, const Linear& L, const void* A, int B, int Tseg, const float* gate,
+                   long mod_stride, float* resid, cudaStream_t st, bool a_e4m3 = false) {
+  return run_linear(m, L, A, B * Tseg, gate_epilogue(L, Tseg, gate, mod_stride, resid), st, a_e4m3);
+}
+
+// hid_e4m3 (out): whether the hidden activations were written as e4m3
+int run_mlp1(sd3_model* m, const Linear& L, const Linear& next, const void* A, int M, void* hid,
+             cudaStream_t st, bool a_e4m3, bool* hid_e4m3) {
+  GemmEpilogue e;
+  e.mode = EPI_BIAS_GELU;
+  e.out = hid; e.out_f32 = 0; e.ldo = L.N;
+  e.out_plane = m->f32 ? static_cast<long>(M) * L.N : 0;
+  *hid_e4m3 = m->fp8 && L.w8 && next.w8 && L.N % 64 == 0;
+  e.out_e4m3 = *hid_e4m3 ? 1 : 0;
+  return run_linear(m, L, A, M, e, st, a_e4m3);
 }
 
 int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, const float* mod,
@@ -464,7 +490,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   // that GEMM (and, for the dual output, its twin) has e4m3 weights.
   const bool c8a = m->fp8 && L.c_qkv.w8, x8a = m->fp8 && L.x_qkv.w8 && (!L.dual || L.d_qkv.w8);
   const bool c8m = m->fp8 && L.c_mlp1.w8, x8m = m->fp8 && L.x_mlp1.w8;
-  auto ln_out = [&](bool e4m3) { return m->f32 ? 1 : (e4m3 ? 2 : 0); };
+  auto ln_out = [&](bool e4m3) { return m->f32 ? 3 : (e4m3 ? 2 : 0); };
   // pre-attention LayerNorm + modulate
   SD3_TRY(launch_ln_modulate(c, B, Tc, E, 1e-6f, c_shift_a, c_scale_a, w.h_c, nullptr, nullptr,
                              nullptr, ms, ln_out(c8a), st));
@@ -475,13 +501,13 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     SD3_TRY(launch_ln_modulate(x, B, Tx, E, 1e-6f, x_shift_a, x_scale_a, w.h_x, nullptr, nullptr,
                                nullptr, ms, ln_out(x8a), st));
   // QKV (context rows first, then image rows) and joint attention
-  // the tensor-core path (bf16 / FP8 modes, head_dim 64): image and context GEMMs of a kind share a launch
-  const bool grouped = !m->f32 && m->D == 64;
+  // image and context GEMMs of a kind share a launch (bf16 / FP8 modes: with head_dim 64)
+  const bool grouped = m->f32 || m->D == 64;
   // q pre-scaled by softmax_scale * log2(e) through its norm weight (both streams or neither)
   const bool pre_j = L.c_wq_s != nullptr && L.x_wq_s != nullptr;
   const float* c_wq = pre_j ? L.c_wq_s : L.c_wq;
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
-  if (grouped) {
+  if (m->D == 64) {
     SD3_TRY(run_linear_pair(m, L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, Tx, T, Tc, x_wq, L.x_wk), x8a,
                             L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, Tc, T, 0, c_wq, L.c_wk), c8a, st));
   } else {
@@ -519,6 +545,10 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     GemmEpilogue ex, ec;
     ex.mode = EPI_BIAS_GELU; ex.out = w.hid_x; ex.out_f32 = 0; ex.ldo = L.x_mlp1.N; ex.out_e4m3 = hx8 ? 1 : 0;
     ec.mode = EPI_BIAS_GELU; ec.out = w.hid_c; ec.out_f32 = 0; ec.ldo = L.c_mlp1.N; ec.out_e4m3 = hc8 ? 1 : 0;
+    if (m->f32) {
+      ex.out_plane = static_cast<long>(B) * Tx * L.x_mlp1.N;
+      ec.out_plane = static_cast<long>(B) * Tc * L.c_mlp1.N;
+    }
     SD3_TRY(run_linear_pair(m, L.x_mlp1, w.h_x, B * Tx, ex, x8m, L.c_mlp1, w.h_c, B * Tc, ec, c8m, st));
     SD3_TRY(run_linear_pair(m, L.x_mlp2, w.hid_x, B * Tx, gate_epilogue(L.x_mlp2, Tx, x_gate_m, ms, x), hx8,
                             L.c_mlp2, w.hid_c, B * Tc, gate_epilogue(L.c_mlp2, Tc, c_gate_m, ms, c), hc8, st));
@@ -696,6 +726,13 @@ int sd3_model_create(const sd3_config* cfg, sd3_model** out) {
     L.c_mod_off = off; off += static_cast<long>(L.c_chunks) * m->E;
     L.x_mod_off = off; off += static_cast<long>(L.x_chunks) * m->E;
   }
+  if (m->f32) {
+    for (LayerW& L : m->layers)
+      for (Linear* p : {&L.c_qkv, &L.c_out, &L.c_mlp1, &L.c_mlp2, &L.x_qkv, &L.x_out, &L.x_mlp1, &L.x_mlp2, &L.d_qkv,
+                        &L.d_out})
+        p->split = true;
+    m->cap.split = m->patch.split = m->fin.split = true;
+  }
   m->fin_mod_off = off;
   if (!cfg->block_only) off += 2L * m->E;
   m->ada_total = off;
@@ -770,14 +807,16 @@ int sd3_model_set_param(sd3_model* m, const char* name, const void* dev_ptr, int
     if (s.ada_off >= 0) {
       dst = static_cast<char*>(m->ada_w) + static_cast<size_t>(s.ada_off) * m->E * m->wbytes();
     } else {
-      if (!s.lin->w) rc = dev_alloc(m, &s.lin->w, static_cast<size_t>(numel) * m->wbytes());
+      if (!s.lin->w) rc = dev_alloc(m, &s.lin->w, static_cast<size_t>(numel) * (s.lin->split ? 6 : m->wbytes()));
       dst = s.lin->w;
       s.lin->N = s.N;
       s.lin->K = s.K;
       if (s.lin->w8) s.lin->w8_stale = true;
     }
     if (!rc) {
-      if (s.conv) {
+      if (s.conv && s.lin->split) {
+        rc = launch_split3(dev_ptr, dtype == SD3_DTYPE_F32, static_cast<bf16*>(dst), numel, st);
+      } else if (s.conv) {
         if ((dtype == SD3_DTYPE_F32) == m->f32)
           rc = check_cuda(cudaMemcpyAsync(dst, dev_ptr, numel * m->wbytes(),
                                           cudaMemcpyDeviceToDevice, st), "conv weight copy");
@@ -788,7 +827,7 @@ int sd3_model_set_param(sd3_model* m, const char* name, const void* dev_ptr, int
           rc = launch_cast_bf16_to_f32(static_cast<const bf16*>(dev_ptr), static_cast<float*>(dst),
                                        numel, st);
       } else {
-        rc = pack_linear_weight(m, dev_ptr, dtype, s.K, s.N, dst, st);
+        rc = pack_linear_weight(m, dev_ptr, dtype, s.K, s.N, dst, s.lin && s.lin->split, st);
       }
     }
   }
@@ -932,9 +971,11 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   {
     const void* cap_in = captions;
     const long n = static_cast<long>(B) * Tc * c.captions_dim;
-    if (io_f32 != m->f32) {
-      if (io_f32) SD3_TRY(launch_cast_f32_to_bf16(static_cast<const float*>(captions), static_cast<bf16*>(w.cap_in), n, st));
-      else SD3_TRY(launch_cast_bf16_to_f32(static_cast<const bf16*>(captions), static_cast<float*>(w.cap_in), n, st));
+    if (m->f32) {
+      SD3_TRY(launch_split3(captions, io_f32, static_cast<bf16*>(w.cap_in), n, st));
+      cap_in = w.cap_in;
+    } else if (io_f32) {
+      SD3_TRY(launch_cast_f32_to_bf16(static_cast<const float*>(captions), static_cast<bf16*>(w.cap_in), n, st));
       cap_in = w.cap_in;
     }
     GemmEpilogue e;
@@ -943,7 +984,7 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   }
   // image stream x = patch conv + bias + position table
   {
-    SD3_TRY(launch_patchify(latent, io_f32, w.patches, m->f32, B, c.in_channels, H, W, p, st));
+    SD3_TRY(launch_patchify(latent, io_f32, w.patches, m->f32 ? 3 : 0, B, c.in_channels, H, W, p, st));
     GemmEpilogue e;
     e.mode = EPI_ADD_TABLE; e.out = w.x; e.out_f32 = 1; e.ldo = E;
     e.rows_in = Tx; e.rows_out = Tx; e.table = m->pos_store;
@@ -955,7 +996,7 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   {
     const float* fm = w.mod + m->fin_mod_off;
     SD3_TRY(launch_ln_modulate(w.x, B, Tx, E, 1e-5f, fm + E, fm, w.h_x, nullptr, nullptr, nullptr,
-                               m->ada_total, m->f32, st));
+                               m->ada_total, m->f32 ? 3 : 0, st));
     GemmEpilogue e;
     e.mode = EPI_UNPATCHIFY; e.out = out; e.out_f32 = io_f32; e.ldo = m->Nout;
     e.rows_in = Tx; e.rows_out = Tx;

@@ -1,0 +1,515 @@
+// fp32 GEMM on the tcgen05 tensor cores: every fp32 operand is held as three
+// bf16 planes that add up to it exactly (x = h + m + l, 8 + 8 + 8 mantissa
+// bits, each plane rounded to nearest), and
+//
+//   a w  =  ah wh + (ah wm + am wh) + (am wm + ah wl + al wh)
+//
+// is formed by six bf16 MMAs with fp32 accumulation.  The three products left
+// out (am wl, al wm, al wl) are below 2^-25 of |a w|, under the rounding of an
+// fp32 product.
+//
+//   acc[m, n] = sum_k A[m, k] * W[n, k]     A: 3 planes of (M, K), W: 3 planes of (N, K)
+//
+// The tensor core's accumulation does not round to nearest, so a sum over all of
+// K in TMEM would drift (one-sided) by more than a chain of FFMAs does.  Each
+// 32-wide K block therefore gets a TMEM accumulator of its own, in which the
+// small products are added first and the two ah wh steps last; the epilogue
+// warps fetch it and add it to fp32 registers (round to nearest, K / 32
+// additions instead of K).  Measured against 64-bit sums the result is closer
+// than the FFMA kernel's.
+//
+// One CTA per SM walks 128 x BN tiles (persistent): warp 0 streams the planes
+// with TMA (3-D boxes of 32 K x rows x 3 planes, 64-byte swizzle), one thread of
+// warp 1 issues 12 MMAs per K block, the epilogue warps add up the blocks and
+// run the fused epilogue.  The TMEM accumulators rotate (512 / BN of them, at
+// most four), so the adds run under the MMAs of the following blocks.
+// What bounds it: the tensor pipe (six MMAs per K step); a 32-wide K block of a
+// 128 x 256 tile is 1536 cycles of MMA for 72 KiB of operands.
+//
+// Measured against the FFMA kernel it replaced in the fp32 models: one dual block of 256 + 77
+// tokens 4.74 -> 2.79 ms, the 24-block model at 512 x 512 (1024 + 333 tokens) 754 -> 668 ms, all
+// of the difference in the GEMMs.
+#include <cuda.h>
+#include <mutex>
+
+#include "gemm_epilogue.cuh"
+#include "kernels.h"
+#include "ptx.cuh"
+#include "split3.cuh"
+
+namespace sd3 {
+
+int encode_tmap_3d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t d0, uint64_t d1, uint64_t d2,
+                   uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2,
+                   int swizzle_bytes = 128);
+int device_sm_count();
+
+namespace {
+
+using gemm_detail::GemmArgs;
+using gemm_detail::map_row;
+using gemm_detail::RowMap;
+using gemm_detail::st_global_32B;
+
+constexpr int S_BM = 128;
+constexpr int S_KB = 32;               // K elements per block (64-byte rows)
+constexpr int S_KBYTES = 2 * S_KB;
+constexpr int S_A_PLANE = S_BM * S_KBYTES;  // 8 KiB
+
+template <int BN>
+struct SplitCfg {
+  static constexpr int W_PLANE = BN * S_KBYTES;
+  static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);       // 72 / 48 / 36 KiB
+  static constexpr int STAGES = BN == 256 ? 3 : (BN == 128 ? 4 : 6);  // 216 / 192 / 216 KiB
+  static constexpr int NBUF = BN == 256 ? 2 : 4;                      // TMEM accumulators
+  static constexpr int TMEM_COLS = NBUF * BN;
+  static constexpr int EPI_WARPS = BN == 64 ? 4 : 8;
+  static constexpr int CPW = BN == 256 ? 128 : 64;  // accumulator columns per epilogue thread
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
+};
+
+// K-major operand, 64-byte swizzle: rows of 64 B, groups of eight rows 512 B apart
+__device__ __forceinline__ uint64_t make_smem_desc_sw64(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
+  d |= static_cast<uint64_t>(1) << 16;
+  d |= static_cast<uint64_t>(512 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(4) << 61;
+  return d;
+}
+
+__device__ __forceinline__ float gelu_tanh_exact(float x) {
+  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
+  return 0.5f * x * (1.0f + tanhf(u));
+}
+
+// eight consecutive fp32 outputs / eight outputs as three planes (16-byte stores)
+__device__ __forceinline__ void store8_f32(float* p, const float* v) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+// Fused epilogue of 64 consecutive accumulator columns of output row m; the row exists.
+template <int EPI, int OUT>  // OUT: 0 bf16 (unpatchify only), 1 fp32, 2 three bf16 planes
+__device__ __forceinline__ void split_epilogue_64(float* v, const RowMap& rm, int n_base, const GemmArgs& g) {
+  const GemmEpilogue& e = g.epi;
+  const int N = g.N;
+  if (n_base >= N) return;
+  if (e.bias) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (n_base + 4 * i < N) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(e.bias + n_base) + i);
+        v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
+      }
+    }
+  }
+  if constexpr (EPI == EPI_QKV_NORM) {
+    if (e.do_norm && n_base < e.qk_cols) {  // head_dim 64: these columns are one head
+      const float* w = (n_base < (e.qk_cols >> 1)) ? e.wq : e.wk;
+      float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+      for (int j = 0; j < 64; j += 4) {
+        s0 = fmaf(v[j], v[j], s0);
+        s1 = fmaf(v[j + 1], v[j + 1], s1);
+        s2 = fmaf(v[j + 2], v[j + 2], s2);
+        s3 = fmaf(v[j + 3], v[j + 3], s3);
+      }
+      const float r = rsqrtf(((s0 + s1) + (s2 + s3)) * (1.0f / 64.0f) + e.eps);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float4 t = w ? __ldg(reinterpret_cast<const float4*>(w) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        v[4 * i] = v[4 * i] * r * t.x;
+        v[4 * i + 1] = v[4 * i + 1] * r * t.y;
+        v[4 * i + 2] = v[4 * i + 2] * r * t.z;
+        v[4 * i + 3] = v[4 * i + 3] * r * t.w;
+      }
+    }
+  }
+  if constexpr (EPI == EPI_BIAS_GELU) {
+#pragma unroll
+    for (int j = 0; j < 64; ++j) v[j] = gelu_tanh_exact(v[j]);
+  }
+  if constexpr (EPI == EPI_ADD_TABLE) {
+    const float4* t4 = reinterpret_cast<const float4*>(e.table + static_cast<long>(rm.t_in) * N + n_base);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (n_base + 4 * i < N) {
+        const float4 t = __ldg(t4 + i);
+        v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
+      }
+    }
+  }
+  if constexpr (EPI == EPI_UNPATCHIFY) {
+    // m = (b, r, s) over the patch grid; n = ph * (p * C) + pw * C + c
+    const int p = e.up_patch, C = e.up_cin;
+    const int s = rm.t_in % e.up_w, r = rm.t_in / e.up_w;
+    const long Wpix = static_cast<long>(e.up_w) * p, Hpix = static_cast<long>(e.up_h) * p;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      const int n = n_base + j;
+      if (n < N) {
+        const int c = n % C, pw = (n / C) % p, ph = n / (C * p);
+        const long idx = ((static_cast<long>(rm.b) * C + c) * Hpix + (r * p + ph)) * Wpix + (s * p + pw);
+        if constexpr (OUT == 1)
+          static_cast<float*>(e.out)[idx] = v[j];
+        else
+          static_cast<bf16*>(e.out)[idx] = __float2bfloat16(v[j]);
+      }
+    }
+    return;
+  }
+  const long base = rm.orow * e.ldo + n_base;
+  if constexpr (EPI == EPI_GATE_RESID) {
+    const float4* g4 = reinterpret_cast<const float4*>(e.gate + static_cast<long>(rm.b) * e.gate_stride + n_base);
+    const float4* r4 = reinterpret_cast<const float4*>(e.resid + base);  // also written here: ordinary loads
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (n_base + 4 * i < N) {
+        const float4 t = __ldg(g4 + i), x = r4[i];
+        v[4 * i] = x.x + t.x * v[4 * i];
+        v[4 * i + 1] = x.y + t.y * v[4 * i + 1];
+        v[4 * i + 2] = x.z + t.z * v[4 * i + 2];
+        v[4 * i + 3] = x.w + t.w * v[4 * i + 3];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int n = n_base + 16 * i;
+    float* o = v + 16 * i;
+    if constexpr (OUT == 1) {
+      float* p = static_cast<float*>(e.out) + base + 16 * i;
+      if (g.wide_store && n + 16 <= N) {
+#pragma unroll
+        for (int h = 0; h < 16; h += 8)
+          st_global_32B(p + h, __float_as_uint(o[h]), __float_as_uint(o[h + 1]), __float_as_uint(o[h + 2]),
+                        __float_as_uint(o[h + 3]), __float_as_uint(o[h + 4]), __float_as_uint(o[h + 5]),
+                        __float_as_uint(o[h + 6]), __float_as_uint(o[h + 7]));
+      } else {
+        if (n < N) store8_f32(p, o);
+        if (n + 8 < N) store8_f32(p + 8, o + 8);
+      }
+    } else {
+      uint32_t u[3][8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) split3_x2(o[2 * j], o[2 * j + 1], u[0][j], u[1][j], u[2][j]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        bf16* p = static_cast<bf16*>(e.out) + q * e.out_plane + base + 16 * i;
+        if (g.wide_store && n + 16 <= N) {
+          st_global_32B(p, u[q][0], u[q][1], u[q][2], u[q][3], u[q][4], u[q][5], u[q][6], u[q][7]);
+        } else {
+          if (n < N) reinterpret_cast<uint4*>(p)[0] = make_uint4(u[q][0], u[q][1], u[q][2], u[q][3]);
+          if (n + 8 < N) reinterpret_cast<uint4*>(p)[1] = make_uint4(u[q][4], u[q][5], u[q][6], u[q][7]);
+        }
+      }
+    }
+  }
+}
+
+// One problem of a (possibly grouped) launch
+struct SplitProblem {
+  CUtensorMap tmA, tmW;
+  GemmArgs g;
+};
+
+template <int BN, int EPI, int OUT>
+__global__ void __launch_bounds__(SplitCfg<BN>::THREADS, 1)
+gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_constant__ SplitProblem p1,
+                          const int tiles0, const int tiles1) {
+  using Cfg = SplitCfg<BN>;
+  constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, CPW = Cfg::CPW;
+  constexpr uint32_t IDESC = make_idesc(1, 1, S_BM, BN, 0, 0);
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tfull_bar = empty_bar + STAGES;
+  uint64_t* tempty_bar = tfull_bar + NBUF;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + NBUF);
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int a = 0; a < NBUF; ++a) {
+      mbar_init(&tfull_bar[a], 1);
+      mbar_init(&tempty_bar[a], Cfg::EPI_WARPS);
+    }
+    *s_abort = 0;
+    fence_barrier_init();
+    prefetch_tmap(&p0.tmA);
+    prefetch_tmap(&p0.tmW);
+    if (tiles1 > 0) {
+      prefetch_tmap(&p1.tmA);
+      prefetch_tmap(&p1.tmW);
+    }
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const WaitCtx wc{s_abort, p0.g.status};
+  const int num_tiles = tiles0 + tiles1;
+  const int KB = p0.g.k_blocks;  // the same K for both problems
+
+  if (warp == 0 && lane == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      const bool second = tile >= tiles0;
+      const SplitProblem& pp = second ? p1 : p0;
+      const int lt = second ? tile - tiles0 : tile;
+      const int m0 = (lt / pp.g.tiles_n) * S_BM, n0 = (lt % pp.g.tiles_n) * BN;
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+        uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
+        mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
+        tma_load_3d(sa, &pp.tmA, &full_bar[stage], kb * S_KB, m0, 0);
+        tma_load_3d(sa + 3 * S_A_PLANE, &pp.tmW, &full_bar[stage], kb * S_KB, n0, 0);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1 && lane == 0) {
+    // ------------------------------ MMA issuer --------------------------------
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, bphase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait(&tempty_bar[buf], bphase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BN);
+        const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+        const uint64_t a0 = make_smem_desc_sw64(a_addr);
+        const uint64_t w0 = make_smem_desc_sw64(a_addr + 3 * S_A_PLANE);
+        constexpr uint64_t AP = S_A_PLANE >> 4, WP = Cfg::W_PLANE >> 4;
+        // (A plane, W plane), smallest products first
+        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            mma_f16_ss(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
+        mma_commit(&empty_bar[stage]);
+        mma_commit(&tfull_bar[buf]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++buf == NBUF) { buf = 0; bphase ^= 1; }
+      }
+    }
+  } else if (warp >= 2) {
+    // ------------------------------ accumulation + epilogue -------------------
+    const int quad = warp & 3;
+    const int half = (warp - 2) >> 2;
+    const int row = quad * 32 + lane;
+    int buf = 0;
+    uint32_t bphase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      const bool second = tile >= tiles0;
+      const GemmArgs& g = second ? p1.g : p0.g;
+      const int lt = second ? tile - tiles0 : tile;
+      const int m = (lt / g.tiles_n) * S_BM + row;
+      const int n0 = (lt % g.tiles_n) * BN + half * CPW;
+      float acc[CPW];
+#pragma unroll
+      for (int j = 0; j < CPW; ++j) acc[j] = 0.f;
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait_warp(&tfull_bar[buf], bphase, wc, DEV_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
+                               static_cast<uint32_t>(buf * BN + half * CPW);
+#pragma unroll
+        for (int s = 0; s < CPW / 32; ++s) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_row + s * 32, r);
+          tmem_wait_ld();
+          if (s == CPW / 32 - 1) {  // everything is in registers: the accumulator may be reused
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[s * 32 + j] += __uint_as_float(r[j]);
+        }
+        if (++buf == NBUF) { buf = 0; bphase ^= 1; }
+      }
+      if (!ok) break;
+      if (m < g.M) {
+        const RowMap rm = map_row(m, g.epi);
+#pragma unroll
+        for (int c = 0; c < CPW; c += 64) split_epilogue_64<EPI, OUT>(acc + c, rm, n0 + c, g);
+      }
+      __syncwarp();
+    }
+  }
+
+  // ------------------------------ teardown ------------------------------------
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*s_abort) drain_after_abort();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+template <int BN, int EPI, int OUT>
+int launch_split_inst(const SplitProblem& p0, const SplitProblem& p1, int tiles0, int tiles1, cudaStream_t stream) {
+  using Cfg = SplitCfg<BN>;
+  auto kern = gemm_split_tcgen05_kernel<BN, EPI, OUT>;
+  static std::mutex attr_mutex;
+  static bool attr_done[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64) {
+    std::lock_guard<std::mutex> lock(attr_mutex);
+    if (!attr_done[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+      if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_split)");
+      attr_done[dev] = true;
+    }
+  }
+  const int tiles = tiles0 + tiles1, sms = device_sm_count();
+  kern<<<tiles < sms ? tiles : sms, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(p0, p1, tiles0, tiles1);
+  return after_launch("gemm_split_tcgen05_kernel");
+}
+
+template <int EPI, int OUT>
+int launch_split_width(int bn, const SplitProblem& p0, const SplitProblem& p1, int t0, int t1, cudaStream_t st) {
+  if (bn == 256) return launch_split_inst<256, EPI, OUT>(p0, p1, t0, t1, st);
+  if (bn == 128) return launch_split_inst<128, EPI, OUT>(p0, p1, t0, t1, st);
+  return launch_split_inst<64, EPI, OUT>(p0, p1, t0, t1, st);
+}
+
+int validate_split(const SplitGemmProblem& q, int N, int K) {
+  const GemmEpilogue& e = q.epi;
+  if (!q.A || !q.W || !e.out || q.M <= 0 || N <= 0 || K <= 0 || K % 8 || N % 8 || q.a_plane % 8 || q.w_plane % 8 ||
+      (reinterpret_cast<uintptr_t>(q.A) & 15) || (reinterpret_cast<uintptr_t>(q.W) & 15) || e.alpha != 1.0f) {
+    set_last_error("gemm_split: invalid argument (M %d N %d K %d)", q.M, N, K);
+    return ST_INVALID_ARG;
+  }
+  const bool planes = e.out_plane > 0;
+  if (e.mode != EPI_UNPATCHIFY &&
+      ((reinterpret_cast<uintptr_t>(e.out) & 15) || e.ldo % 8 || e.out_plane % 8 || (!planes && !e.out_f32))) {
+    set_last_error("gemm_split: output must be fp32 or bf16 planes, 16-byte aligned");
+    return ST_INVALID_ARG;
+  }
+  if (planes && e.mode != EPI_BIAS_GELU && e.mode != EPI_QKV_NORM) {
+    set_last_error("gemm_split: no plane output for epilogue mode %d", e.mode);
+    return ST_UNSUPPORTED;
+  }
+  if (e.mode == EPI_QKV_NORM && (e.do_norm && e.qk_cols % 128 != 0)) {
+    set_last_error("gemm_split: fused q/k norm needs head_dim 64");
+    return ST_INVALID_ARG;
+  }
+  if (e.mode == EPI_GATE_RESID && (!e.gate || !e.resid || e.gate_stride % 4)) {
+    set_last_error("gemm_split: gate/residual epilogue needs gate and resid pointers");
+    return ST_INVALID_ARG;
+  }
+  if (e.mode == EPI_ADD_TABLE && (!e.table || e.rows_in <= 0)) {
+    set_last_error("gemm_split: table epilogue needs table and rows_in");
+    return ST_INVALID_ARG;
+  }
+  return ST_OK;
+}
+
+int build_split(SplitProblem* pp, const SplitGemmProblem& q, int N, int K, int bn, int* dev_status) {
+  GemmArgs& g = pp->g;
+  g.M = q.M; g.N = N; g.K = K;
+  g.k_blocks = (K + S_KB - 1) / S_KB;
+  g.tiles_m = (q.M + S_BM - 1) / S_BM;
+  g.tiles_n = (N + bn - 1) / bn;
+  g.epi = q.epi;
+  g.status = dev_status;
+  g.tma_store = 0;
+  const long esz = q.epi.out_plane > 0 ? 2 : 4;
+  g.wide_store = (q.epi.ldo * esz) % 32 == 0 && (q.epi.out_plane * 2) % 32 == 0 &&
+                 (reinterpret_cast<uintptr_t>(q.epi.out) & 31) == 0;
+  int rc = encode_tmap_3d(&pp->tmA, q.A, 2, K, q.M, 3, static_cast<uint64_t>(K) * 2, q.a_plane * 2, S_KB, S_BM, 3,
+                          S_KBYTES);
+  if (rc) return rc;
+  return encode_tmap_3d(&pp->tmW, q.W, 2, K, N, 3, static_cast<uint64_t>(K) * 2, q.w_plane * 2, S_KB, bn, 3, S_KBYTES);
+}
+
+// The tile width with the least (waves over the SMs) x (time of a K block of a tile).  A K block
+// is 12 MMAs of 128 / 64 cycles at BN = 256 / 128 and of about 50 at BN = 64 (an MMA is issue-bound
+// below 64 columns' worth of math).
+int choose_split_width(long rows_tiles, int N) {
+  const long sms = device_sm_count();
+  int best = 256;
+  long best_cost = 0;
+  const int bn[3] = {256, 128, 64}, cost[3] = {128, 66, 50};
+  for (int i = 0; i < 3; ++i) {
+    const long tiles = rows_tiles * ((N + bn[i] - 1) / bn[i]);
+    const long c = (tiles + sms - 1) / sms * cost[i];
+    if (i == 0 || c < best_cost) { best = bn[i]; best_cost = c; }
+  }
+  return best;
+}
+
+}  // namespace
+
+int launch_gemm_split(const SplitGemmProblem& a, const SplitGemmProblem* b, int N, int K, int* dev_status,
+                      cudaStream_t stream) {
+  int rc = validate_split(a, N, K);
+  if (rc) return rc;
+  if (b) {
+    rc = validate_split(*b, N, K);
+    if (rc) return rc;
+    if (b->epi.mode != a.epi.mode || (b->epi.out_plane > 0) != (a.epi.out_plane > 0) || b->epi.out_f32 != a.epi.out_f32) {
+      set_last_error("gemm_split: grouped problems need the same epilogue kind");
+      return ST_INVALID_ARG;
+    }
+  }
+  const int bn = choose_split_width((a.M + S_BM - 1) / S_BM + (b ? (b->M + S_BM - 1) / S_BM : 0), N);
+  SplitProblem p0, p1;
+  rc = build_split(&p0, a, N, K, bn, dev_status);
+  if (rc) return rc;
+  int t1 = 0;
+  if (b) {
+    rc = build_split(&p1, *b, N, K, bn, dev_status);
+    if (rc) return rc;
+    t1 = p1.g.tiles_m * p1.g.tiles_n;
+  } else {
+    p1 = p0;
+  }
+  const int t0 = p0.g.tiles_m * p0.g.tiles_n;
+  const bool planes = a.epi.out_plane > 0;
+  switch (a.epi.mode) {
+    case EPI_BIAS: return launch_split_width<EPI_BIAS, 1>(bn, p0, p1, t0, t1, stream);
+    case EPI_BIAS_GELU:
+      if (planes) return launch_split_width<EPI_BIAS_GELU, 2>(bn, p0, p1, t0, t1, stream);
+      break;
+    case EPI_QKV_NORM:
+      return planes ? launch_split_width<EPI_QKV_NORM, 2>(bn, p0, p1, t0, t1, stream)
+                    : launch_split_width<EPI_QKV_NORM, 1>(bn, p0, p1, t0, t1, stream);
+    case EPI_GATE_RESID: return launch_split_width<EPI_GATE_RESID, 1>(bn, p0, p1, t0, t1, stream);
+    case EPI_ADD_TABLE: return launch_split_width<EPI_ADD_TABLE, 1>(bn, p0, p1, t0, t1, stream);
+    case EPI_UNPATCHIFY:
+      return a.epi.out_f32 ? launch_split_width<EPI_UNPATCHIFY, 1>(bn, p0, p1, t0, t1, stream)
+                           : launch_split_width<EPI_UNPATCHIFY, 0>(bn, p0, p1, t0, t1, stream);
+    default: break;
+  }
+  set_last_error("gemm_split: unsupported epilogue mode %d", a.epi.mode);
+  return ST_UNSUPPORTED;
+}
+
+}  // namespace sd3

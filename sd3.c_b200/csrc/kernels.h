@@ -47,6 +47,8 @@ struct GemmEpilogue {
   int out_f32 = 0;              // 0: bf16 output, 1: fp32 output
   int out_e4m3 = 0;             // with out_f32 == 0: one e4m3 byte per element (N % 64 == 0), the
                                 // operand of a following FP8 GEMM; BIAS and BIAS_GELU modes only
+  long out_plane = 0;           // > 0 (gemm_split): the output is three bf16 planes that add up to the
+                                // fp32 value, out_plane elements apart (split3.cuh)
   long ldo = 0;                 // output leading dimension in elements
   // Row remap: GEMM row m belongs to sample b = m / rows_in and is written to
   // output row b * rows_out + row_off + (m % rows_in).  rows_in = 0 means no remap.
@@ -99,6 +101,20 @@ struct GemmProblem {
 int launch_gemm_grouped(const GemmProblem& a, const GemmProblem& b, int operand_dtype, int N, int K,
                         int* dev_status, cudaStream_t stream);
 
+// fp32 GEMM on the tensor cores: A and W are three bf16 planes each (split3.cuh), a_plane / w_plane
+// elements apart, rows of K elements; the result has fp32 accuracy.  One or two problems (b may be
+// null) of the same N, K and epilogue kind as one launch.  K % 8 == 0, N % 8 == 0.
+struct SplitGemmProblem {
+  const bf16* A = nullptr;
+  long a_plane = 0;
+  const bf16* W = nullptr;
+  long w_plane = 0;
+  int M = 0;
+  GemmEpilogue epi;
+};
+int launch_gemm_split(const SplitGemmProblem& a, const SplitGemmProblem* b, int N, int K, int* dev_status,
+                      cudaStream_t stream);
+
 // ----------------------------------------------------------------------------
 // Flash-style attention on tcgen05 (head_dim 64, bf16, non-causal).
 // qkv: (B, T, 3*E) bf16 with q | k | v column blocks, head h at columns h*64.
@@ -127,8 +143,8 @@ int launch_attention_simt(const void* q, const void* k, const void* v, long ld, 
 // Memory-bound kernels
 // ----------------------------------------------------------------------------
 // LayerNorm (no affine) + up to two modulations:  out_i = LN(x) * (1 + scale_i[b]) + shift_i[b]
-// x: (B*T, E) fp32.  shift/scale: [b * mod_stride + e].  out: bf16 (out_f32 = 0), fp32 (1) or
-// e4m3 converted as is (2).
+// x: (B*T, E) fp32.  shift/scale: [b * mod_stride + e].  out: bf16 (out_f32 = 0), fp32 (1),
+// e4m3 converted as is (2) or three bf16 planes of B*T*E elements (3, split3.cuh).
 int launch_ln_modulate(const float* x, int B, int T, int E, float eps, const float* shift1,
                        const float* scale1, void* out1, const float* shift2, const float* scale2,
                        void* out2, long mod_stride, int out_f32, cudaStream_t stream);
@@ -147,7 +163,8 @@ int launch_sinusoidal(const float* t, float* out, int B, int dim, cudaStream_t s
 int launch_pos_table(float* table, int h, int w, int E, int pmax, int base_size,
                      cudaStream_t stream);
 
-// latent (B, C, H, W) fp32/bf16 -> patches (B*h*w, C*p*p) bf16 or fp32, k = c*p*p + ph*p + pw
+// latent (B, C, H, W) fp32/bf16 -> patches (B*h*w, C*p*p), k = c*p*p + ph*p + pw: bf16 (out_f32 = 0),
+// fp32 (1) or three bf16 planes of B*C*H*W elements (3)
 int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int B, int C, int H,
                     int W, int p, cudaStream_t stream);
 
@@ -166,6 +183,10 @@ int launch_cast_bf16_to_f32(const bf16* in, float* out, long n, cudaStream_t str
 // in: (R, C) row-major of in dtype -> out: (C, R) row-major of out dtype
 int launch_transpose(const void* in, int in_f32, void* out, int out_f32, int R, int C,
                      cudaStream_t stream);
+// in (fp32 or bf16) -> three bf16 planes that add up to it, n elements apart; n % 4 == 0
+int launch_split3(const void* in, int in_f32, bf16* out, long n, cudaStream_t stream);
+// in: (R, C) row-major -> three bf16 planes of (C, R), R * C elements apart
+int launch_transpose_split3(const void* in, int in_f32, bf16* out, int R, int C, cudaStream_t stream);
 // per-head RMSNorm in place on rows of width ncols_total; heads of width D
 // starting at column col0, nheads of them; x fp32 or bf16
 int launch_rmsnorm_heads(void* x, int x_f32, long ld, long rows, int col0, int nheads, int D,

@@ -14,6 +14,7 @@
 // (modules.cpp:1037-1117); rmsnorm_key_query_kernel2 (cuda/dit.cu:384-447).
 #include "kernels.h"
 #include "ptx.cuh"
+#include "split3.cuh"
 
 namespace sd3 {
 
@@ -24,7 +25,8 @@ namespace {
 // ----------------------------------------------------------------------------
 // LayerNorm + modulate.  One warp per row, the row lives in registers.
 // ----------------------------------------------------------------------------
-// OUT: 0 bf16, 1 fp32, 2 e4m3 (operand of an FP8 GEMM, converted as is)
+// OUT: 0 bf16, 1 fp32, 2 e4m3 (operand of an FP8 GEMM, converted as is), 3 three bf16 planes of
+// rows * E elements (operand of a split fp32 GEMM)
 //
 // A CTA of 8 warps owns 8 * rpw consecutive rows (rpw per warp, at most 8; fewer
 // for small inputs so that the grid still covers the GPU).  The
@@ -36,9 +38,21 @@ namespace {
 constexpr int LN_MAX_ROWS_PER_WARP = 8;
 constexpr int LN_WARPS = 8;
 
+// four consecutive values as three bf16 planes
+__device__ __forceinline__ void store4_split(bf16* p, long plane, const float4& o) {
+  uint2 h, m, l;
+  split3_x2(o.x, o.y, h.x, m.x, l.x);
+  split3_x2(o.z, o.w, h.y, m.y, l.y);
+  *reinterpret_cast<uint2*>(p) = h;
+  *reinterpret_cast<uint2*>(p + plane) = m;
+  *reinterpret_cast<uint2*>(p + 2 * plane) = l;
+}
+
 template <int OUT>
-__device__ __forceinline__ void ln_store4(void* out, long row, int E, int i, const float4& o) {
-  if constexpr (OUT == 1) {
+__device__ __forceinline__ void ln_store4(void* out, long row, long rows, int E, int i, const float4& o) {
+  if constexpr (OUT == 3) {
+    store4_split(static_cast<bf16*>(out) + row * E + 4 * i, rows * E, o);
+  } else if constexpr (OUT == 1) {
     reinterpret_cast<float4*>(static_cast<float*>(out) + row * E)[i] = o;
   } else if constexpr (OUT == 2) {
     reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(out) + row * E)[i] = pack_e4m3x4(o.x, o.y, o.z, o.w);
@@ -133,7 +147,7 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
           o.y = fmaf(n.y, s.y, h.y);
           o.z = fmaf(n.z, s.z, h.z);
           o.w = fmaf(n.w, s.w, h.w);
-          ln_store4<OUT>(out1, row, E, i, o);
+          ln_store4<OUT>(out1, row, rows, E, i, o);
         }
         if constexpr (DUAL) {
           float4 s, h;
@@ -149,7 +163,7 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
           o.y = fmaf(n.y, s.y, h.y);
           o.z = fmaf(n.z, s.z, h.z);
           o.w = fmaf(n.w, s.w, h.w);
-          ln_store4<OUT>(out2, row, E, i, o);
+          ln_store4<OUT>(out2, row, rows, E, i, o);
         }
       }
     }
@@ -173,6 +187,8 @@ int launch_ln_inst(const float* x, long rows, int T, int E, float eps, const flo
     if (dual) SD3_LN_LAUNCH(1, true); else SD3_LN_LAUNCH(1, false);
   } else if (out_f32 == 2) {
     if (dual) SD3_LN_LAUNCH(2, true); else SD3_LN_LAUNCH(2, false);
+  } else if (out_f32 == 3) {
+    if (dual) SD3_LN_LAUNCH(3, true); else SD3_LN_LAUNCH(3, false);
   } else {
     if (dual) SD3_LN_LAUNCH(0, true); else SD3_LN_LAUNCH(0, false);
   }
@@ -336,7 +352,7 @@ template <> __device__ __forceinline__ bf16 convert_elem<float, bf16>(float v) {
 template <> __device__ __forceinline__ float convert_elem<bf16, float>(bf16 v) { return __bfloat162float(v); }
 template <> __device__ __forceinline__ bf16 convert_elem<bf16, bf16>(bf16 v) { return v; }
 
-template <typename IT, typename OT>
+template <typename IT, typename OT, bool SPLIT = false>
 __global__ void patchify_kernel(const IT* __restrict__ latent, OT* __restrict__ out, int B, int C,
                                 int H, int W, int p) {
   const int hp = H / p, wp = W / p;
@@ -351,7 +367,16 @@ __global__ void patchify_kernel(const IT* __restrict__ latent, OT* __restrict__ 
   const int b = static_cast<int>(tok / (static_cast<long>(wp) * hp));
   const int pw = k % p, ph = (k / p) % p, c = k / (p * p);
   const long src = ((static_cast<long>(b) * C + c) * H + (r * p + ph)) * W + (s * p + pw);
-  out[idx] = convert_elem<IT, OT>(latent[src]);
+  if constexpr (SPLIT) {
+    uint32_t h, m, l;
+    split3_x2(convert_elem<IT, float>(latent[src]), 0.f, h, m, l);
+    unsigned short* o = reinterpret_cast<unsigned short*>(out) + idx;
+    o[0] = static_cast<unsigned short>(h);
+    o[total] = static_cast<unsigned short>(m);
+    o[2 * total] = static_cast<unsigned short>(l);
+  } else {
+    out[idx] = convert_elem<IT, OT>(latent[src]);
+  }
 }
 
 template <typename IT, typename OT>
@@ -375,6 +400,48 @@ __global__ void transpose_kernel(const IT* __restrict__ in, OT* __restrict__ out
     const int c = c0 + j, r = r0 + threadIdx.x;
     if (r < R && c < C)
       out[static_cast<long>(c) * R + r] = convert_elem<float, OT>(tile[threadIdx.x][j]);
+  }
+}
+
+template <typename IT>
+__global__ void split3_kernel(const IT* __restrict__ in, bf16* __restrict__ out, long n) {
+  long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+  const long stride = static_cast<long>(gridDim.x) * blockDim.x * 4;
+  for (; i < n; i += stride) {
+    float4 f;
+    if constexpr (sizeof(IT) == 4) {
+      f = *reinterpret_cast<const float4*>(in + i);
+    } else {
+      const uint2 u = *reinterpret_cast<const uint2*>(in + i);
+      f = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                      __uint_as_float(u.y & 0xffff0000u));
+    }
+    store4_split(out + i, n, f);
+  }
+}
+
+// 64 rows x 32 columns per CTA: reads rows of 128 bytes, writes rows of 64 bf16 per plane
+template <typename IT>
+__global__ void transpose_split3_kernel(const IT* __restrict__ in, bf16* __restrict__ out, int R, int C) {
+  __shared__ float tile[64][33];
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 64;
+  const long plane = static_cast<long>(R) * C;
+  for (int j = threadIdx.y; j < 64; j += blockDim.y) {
+    const int r = r0 + j, c = c0 + threadIdx.x;
+    tile[j][threadIdx.x] = (r < R && c < C) ? convert_elem<IT, float>(in[static_cast<long>(r) * C + c]) : 0.f;
+  }
+  __syncthreads();
+  const int r = r0 + 2 * threadIdx.x;  // R is even
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    const int c = c0 + j;
+    if (r < R && c < C) {
+      uint32_t h, m, l;
+      split3_x2(tile[2 * threadIdx.x][j], tile[2 * threadIdx.x + 1][j], h, m, l);
+      bf16* o = out + static_cast<long>(c) * R + r;
+      *reinterpret_cast<uint32_t*>(o) = h;
+      *reinterpret_cast<uint32_t*>(o + plane) = m;
+      *reinterpret_cast<uint32_t*>(o + 2 * plane) = l;
+    }
   }
 }
 
@@ -485,7 +552,11 @@ int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int 
   }
   const long total = static_cast<long>(B) * C * H * W;
   const unsigned grid = static_cast<unsigned>((total + 255) / 256);
-  if (in_f32 && out_f32)
+  if (in_f32 && out_f32 == 3)
+    patchify_kernel<float, bf16, true><<<grid, 256, 0, stream>>>((const float*)latent, (bf16*)out, B, C, H, W, p);
+  else if (out_f32 == 3)
+    patchify_kernel<bf16, bf16, true><<<grid, 256, 0, stream>>>((const bf16*)latent, (bf16*)out, B, C, H, W, p);
+  else if (in_f32 && out_f32)
     patchify_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)latent, (float*)out, B, C, H, W, p);
   else if (in_f32)
     patchify_kernel<float, bf16><<<grid, 256, 0, stream>>>((const float*)latent, (bf16*)out, B, C, H, W, p);
@@ -608,6 +679,34 @@ int launch_transpose(const void* in, int in_f32, void* out, int out_f32, int R, 
   else
     transpose_kernel<bf16, bf16><<<grid, block, 0, stream>>>((const bf16*)in, (bf16*)out, R, C);
   return after_launch("transpose_kernel");
+}
+
+int launch_split3(const void* in, int in_f32, bf16* out, long n, cudaStream_t stream) {
+  if (!in || !out || n <= 0 || n % 4 || (reinterpret_cast<uintptr_t>(in) & (in_f32 ? 15 : 7)) ||
+      (reinterpret_cast<uintptr_t>(out) & 7)) {
+    set_last_error("split3: need n %% 4 == 0 and aligned pointers (n %ld)", n);
+    return ST_INVALID_ARG;
+  }
+  const long blocks = (n / 4 + 255) / 256, most = device_sm_count() * 16L;
+  const unsigned grid = static_cast<unsigned>(blocks < most ? blocks : most);
+  if (in_f32)
+    split3_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(in), out, n);
+  else
+    split3_kernel<bf16><<<grid, 256, 0, stream>>>(static_cast<const bf16*>(in), out, n);
+  return after_launch("split3_kernel");
+}
+
+int launch_transpose_split3(const void* in, int in_f32, bf16* out, int R, int C, cudaStream_t stream) {
+  if (!in || !out || R <= 0 || C <= 0 || R % 2 || (static_cast<long>(R) * C) % 2) {
+    set_last_error("transpose_split3: invalid argument (R %d must be even)", R);
+    return ST_INVALID_ARG;
+  }
+  const dim3 grid((C + 31) / 32, (R + 63) / 64), block(32, 8);
+  if (in_f32)
+    transpose_split3_kernel<float><<<grid, block, 0, stream>>>(static_cast<const float*>(in), out, R, C);
+  else
+    transpose_split3_kernel<bf16><<<grid, block, 0, stream>>>(static_cast<const bf16*>(in), out, R, C);
+  return after_launch("transpose_split3_kernel");
 }
 
 int launch_rmsnorm_heads(void* x, int x_f32, long ld, long rows, int col0, int nheads, int D,

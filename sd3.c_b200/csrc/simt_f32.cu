@@ -1,8 +1,8 @@
 // Exact-fp32 SIMT kernels: a shared-memory tiled FFMA GEMM with the same fused
 // epilogues as the tcgen05 GEMM, and a generic attention kernel for any head
-// size up to 128.  They serve the fp32 parity mode (fp32 tensors in, results
-// within 1e-4 of the fp32 PyTorch modules) and shapes the tensor-core kernels
-// do not cover (head_dim != 64).  Speed is secondary here; the arithmetic is
+// size up to 128.  They serve the operator-level fp32 entry points, the attention
+// of fp32 models and head sizes the tensor-core kernels do not cover (the fp32
+// models' GEMMs are gemm_split.cu's).  Speed is secondary here; the arithmetic is
 // plain fp32 FMA with fp32 accumulation.
 //
 // Reference counterparts: linear / partial_linear (modules.cpp:475-511) and

@@ -1,0 +1,45 @@
+"""The fp32 mode's blocks against the oracle in float64, at the sizes where the tensor-core kernels
+behind it (fp32 operands as three bf16 planes) can go wrong: partial row and column tiles, every tile
+width, ragged and single key tiles, remainders of the 32-wide K blocks, unfused head sizes.
+
+Tolerance: a block output passes through on the order of a thousand fp32 roundings (four chained
+GEMMs of K / 32 additions, LayerNorm sums, softmax), a random walk of 2^-24 steps: sqrt(1000) * 2^-24
+= 1.9e-6 relative to the result."""
+import pytest
+import torch
+
+from oracle import mmdit_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,NH,B,Tx,Tc,dual,last", [
+    (64, 1, 1, 1, 1, True, False),         # one token per stream
+    (64, 1, 2, 63, 65, True, False),       # samples straddle a row tile
+    (128, 2, 3, 128, 1, False, False),     # exact key tile + 1
+    (192, 3, 1, 255, 130, True, False),    # ragged last key tile, N not a multiple of 256
+    (192, 3, 2, 129, 77, False, True),     # last block: no context output
+    (72, 3, 2, 40, 24, True, False),       # head_dim 24: unfused norm, K with a remainder of 8
+    (128, 4, 1, 130, 33, True, False),     # head_dim 32
+    (1536, 24, 1, 256, 77, True, False),   # narrow tiles
+    (1536, 24, 1, 1024, 333, True, False), # 128-wide tiles
+    (1536, 24, 4, 1000, 154, False, False),# 256-wide tiles
+])
+def test_block_fp32_against_float64(sd3, E, NH, B, Tx, Tc, dual, last):
+    gen = torch.Generator().manual_seed(E + 7 * Tx + Tc)
+    p = O.random_params(O.block_param_shapes(E, 4, E // NH, dual, last, True), seed=Tx, std=0.02 * (1536 / E) ** 0.5,
+                        bias_std=0.02, norm_std=0.3)
+    x, c = torch.randn(B, Tx, E, generator=gen), torch.randn(B, Tc, E, generator=gen)
+    y = torch.nn.functional.silu(torch.randn(B, E, generator=gen))
+    p64 = {k: v.double().cuda() for k, v in p.items()}
+    c_ref, x_ref = O.dit_block(x.double().cuda(), c.double().cuda(), y.double().cuda(), p64, NH, dual, True, last)
+    m = sd3.Model(1, [0] if dual else [], 0, 0, 0, E, NH, 4, 0, 0, 0, True, sd3.PRECISION_F32,
+                  last_discards_context=last, block_only=True)
+    m.load({k: v.cuda() for k, v in p.items()}, prefix="transformer.0.")
+    xx, cc = x.cuda(), c.cuda()
+    m.block_forward(0, y.cuda(), cc, xx)
+    torch.cuda.synchronize()
+    assert sd3.device_status() == 0
+    m.close()
+    for got, ref in ((xx, x_ref),) + (() if last else ((cc, c_ref),)):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 2e-6
