@@ -71,9 +71,10 @@ struct Workspace {
   int B = 0, Tc = 0, Tx = 0;
   // f32
   float *temb, *th, *tout, *ph, *y, *mod, *c, *x, *pooled_f32;
-  // activation buffers: bf16, or in the fp32 mode the three bf16 planes a GEMM reads (q, k, v: fp32)
+  // activation buffers: bf16, or in the fp32 mode the three bf16 planes a GEMM or the
+  // attention reads (head sizes other than 64: q, k, v as fp32)
   void *cap_in, *patches, *h_c, *h_x, *h_x2, *qkv, *qkv2, *o_c, *o_x, *o_x2, *hid_x, *hid_c;
-  float* o_f32 = nullptr;  // fp32 mode: attention output before it is split
+  float* o_f32 = nullptr;  // fp32 mode, head sizes other than 64: attention output before it is split
   bf16* y_bf = nullptr;  // conditioning vector as a GEMM operand
   void* a8 = nullptr;    // FP8 mode: e4m3 copy of the current GEMM's left operand
   void* attn_scratch = nullptr;  // partial results of key-split attention launches (small batches, long sequences)
@@ -256,7 +257,8 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
     if (e != cudaSuccess) return check_cuda(e, "cudaFree(workspace)");
   }
   const sd3_config& c = m->cfg;
-  const size_t E = m->E, F = m->F, T = static_cast<size_t>(Tc) + Tx, ab = m->f32 ? 6 : 2, qb = m->f32 ? 4 : 2;
+  const size_t E = m->E, F = m->F, T = static_cast<size_t>(Tc) + Tx, ab = m->f32 ? 6 : 2,
+               qb = m->f32 && m->D != 64 ? 4 : ab;
   const size_t nB = B, nTc = static_cast<size_t>(B) * Tc, nTx = static_cast<size_t>(B) * Tx;
   struct Item { void** p; size_t bytes; };
   std::vector<Item> items = {
@@ -271,7 +273,7 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
       {&w.qkv, nB * T * 3 * E * qb}, {&w.qkv2, nTx * 3 * E * qb},
       {&w.o_c, nTc * E * ab}, {&w.o_x, nTx * E * ab}, {&w.o_x2, nTx * E * ab},
       {&w.hid_x, nTx * F * ab}, {&w.hid_c, nTc * F * ab},
-      {(void**)&w.o_f32, m->f32 ? nB * T * E * 4 : 16},
+      {(void**)&w.o_f32, m->f32 && m->D != 64 ? nB * T * E * 4 : 16},
       {&w.a8, m->fp8 ? (nTx > nTc ? nTx : nTc) * F : 16},
       {&w.attn_scratch, 16},
   };
@@ -370,12 +372,14 @@ int run_linear_pair(sd3_model* m, const Linear& La, const void* Aa, int Ma, cons
   return launch_gemm_grouped(pa, pb, fp8a ? OPERAND_E4M3 : OPERAND_BF16, La.N, La.K, m->status, st);
 }
 
-GemmEpilogue qkv_epilogue(sd3_model* m, void* qkv, int T_in, int T_total, int row_off, const float* wq,
+GemmEpilogue qkv_epilogue(sd3_model* m, void* qkv, int B, int T_in, int T_total, int row_off, const float* wq,
                           const float* wk) {
   GemmEpilogue e;
   e.mode = EPI_QKV_NORM;
   e.out = qkv;
-  e.out_f32 = m->f32;
+  const bool planes = m->f32 && m->D == 64;  // q, k, v as the planes attention_split reads
+  e.out_f32 = m->f32 && !planes;
+  e.out_plane = planes ? static_cast<long>(B) * T_total * 3 * m->E : 0;
   e.ldo = 3L * m->E;
   e.rows_in = T_in; e.rows_out = T_total; e.row_off = row_off;
   e.wq = wq; e.wk = wk; e.eps = 1e-6f;
@@ -405,7 +409,7 @@ int run_qk_norm(sd3_model* m, void* qkv, int B, int T_in, int T_total, int row_o
 int run_qkv(sd3_model* m, const Linear& L, const void* h, void* qkv, int B, int T_in, int T_total,
             int row_off, const float* wq, const float* wk, cudaStream_t st, bool h_e4m3 = false) {
   const bool norm = m->cfg.use_qk_norm && (wq || wk);
-  int rc = run_linear(m, L, h, B * T_in, qkv_epilogue(m, qkv, T_in, T_total, row_off, wq, wk), st, h_e4m3);
+  int rc = run_linear(m, L, h, B * T_in, qkv_epilogue(m, qkv, B, T_in, T_total, row_off, wq, wk), st, h_e4m3);
   if (rc || m->D == 64 || !norm) return rc;
   return run_qk_norm(m, qkv, B, T_in, T_total, row_off, wq, wk, st);
 }
@@ -424,6 +428,9 @@ int run_attention(sd3_model* m, const void* qkv, int B, int T, int Tc, void* o_c
     set_last_error("e4m3 attention output needs head_dim 64");
     return ST_UNSUPPORTED;
   }
+  if (m->f32 && m->D == 64)
+    return launch_attention_split(static_cast<const bf16*>(qkv), B, T, m->NH, Tc, static_cast<bf16*>(o_c),
+                                  static_cast<bf16*>(o_x), scale, m->status, st);
   if (m->f32) {
     // fp32 outputs: the context rows' block first, then the image rows'; each is split into its planes
     const float* q = static_cast<const float*>(qkv);
@@ -508,8 +515,8 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const float* c_wq = pre_j ? L.c_wq_s : L.c_wq;
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
   if (m->D == 64) {
-    SD3_TRY(run_linear_pair(m, L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, Tx, T, Tc, x_wq, L.x_wk), x8a,
-                            L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, Tc, T, 0, c_wq, L.c_wk), c8a, st));
+    SD3_TRY(run_linear_pair(m, L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk), x8a,
+                            L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, B, Tc, T, 0, c_wq, L.c_wk), c8a, st));
   } else {
     SD3_TRY(run_qkv(m, L.c_qkv, w.h_c, w.qkv, B, Tc, T, 0, c_wq, L.c_wk, st, c8a));
     SD3_TRY(run_qkv(m, L.x_qkv, w.h_x, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk, st, x8a));

@@ -132,6 +132,12 @@ int launch_attention_bf16(const bf16* qkv, int B, int T, int NH, int Tc, bf16* o
                           void* scratch = nullptr, size_t scratch_bytes = 0, float score_bound = 0.0f);
 size_t attention_scratch_bytes(int B, int T, int NH);
 
+// fp32 attention for head_dim 64 on the tensor cores.  qkv: three bf16 planes (split3.cuh) of
+// (B, T, 3E), B * T * 3E elements apart; outputs split by rows like above, as three planes of
+// B * Tc * E (out_c, may be null) and B * (T - Tc) * E (out_x) elements.
+int launch_attention_split(const bf16* qkv, int B, int T, int NH, int Tc, bf16* out_c, bf16* out_x, float scale,
+                           int* dev_status, cudaStream_t stream);
+
 // Generic SIMT attention (any head_dim <= 128, fp32 or bf16 in, fp32 math).
 // q: row (b*T + t) at base + row*ld + h*D; k, v: row (b*L + j) at base + row*ldk + h*D
 // (L keys per sample; L <= 0 means L = T, ldk <= 0 means ldk = ld).  out rows split like above.

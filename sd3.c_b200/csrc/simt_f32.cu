@@ -1,8 +1,7 @@
 // Exact-fp32 SIMT kernels: a shared-memory tiled FFMA GEMM with the same fused
 // epilogues as the tcgen05 GEMM, and a generic attention kernel for any head
-// size up to 128.  They serve the operator-level fp32 entry points, the attention
-// of fp32 models and head sizes the tensor-core kernels do not cover (the fp32
-// models' GEMMs are gemm_split.cu's).  Speed is secondary here; the arithmetic is
+// size up to 128.  They serve the operator-level fp32 entry points and head sizes
+// the tensor-core kernels do not cover (fp32 models: gemm_split.cu, attention_split.cu).  Speed is secondary here; the arithmetic is
 // plain fp32 FMA with fp32 accumulation.
 //
 // Reference counterparts: linear / partial_linear (modules.cpp:475-511) and
