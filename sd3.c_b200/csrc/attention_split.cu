@@ -116,6 +116,8 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm, const Spl
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_dep_wait();
+  grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, a.status};
 
@@ -359,7 +361,8 @@ int launch_attention_split(const bf16* qkv, int B, int T, int NH, int Tc, bf16* 
   a.out_x = out_x;
   a.c = scale * 1.4426950408889634f;
   a.status = dev_status;
-  attention_split_tcgen05_kernel<<<dim3((T + AS_BM - 1) / AS_BM, NH, B), AS_THREADS, AS_SMEM_BYTES, stream>>>(tm, a);
+  launch_dependent(attention_split_tcgen05_kernel, dim3((T + AS_BM - 1) / AS_BM, NH, B), AS_THREADS, AS_SMEM_BYTES, stream,
+                   tm, a);
   return after_launch("attention_split_tcgen05_kernel");
 }
 

@@ -307,6 +307,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmQKV, const AttnAr
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_dep_wait();
+  grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, a.status};
 
@@ -551,6 +553,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmQKV, const AttnAr
 // token) row, two output columns per lane; rows go to the context / image outputs like in
 // the attention kernel's own epilogue.
 __global__ void __launch_bounds__(256) attention_merge_kernel(const AttnArgs a) {
+  grid_dep_wait();
+  grid_dep_launch();
   const long row = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long rows = static_cast<long>(a.B) * a.NH * a.T;
@@ -682,15 +686,15 @@ int launch_attention_bf16(const bf16* qkv, int B, int T, int NH, int Tc, bf16* o
   const dim3 grid(qtiles * a.kv_split, NH, B);
   const float bound_log2 = score_bound * fabsf(a.scale_log2e);
   if (score_bound > 0.0f && bound_log2 <= AT_BOUND_MAX && unit)
-    attention_tcgen05_kernel<true, true><<<grid, AT_THREADS, AT_SMEM_BYTES, stream>>>(tm, a);
+    launch_dependent(attention_tcgen05_kernel<true, true>, grid, AT_THREADS, AT_SMEM_BYTES, stream, tm, a);
   else if (score_bound > 0.0f && bound_log2 <= AT_BOUND_MAX)
-    attention_tcgen05_kernel<true, false><<<grid, AT_THREADS, AT_SMEM_BYTES, stream>>>(tm, a);
+    launch_dependent(attention_tcgen05_kernel<true, false>, grid, AT_THREADS, AT_SMEM_BYTES, stream, tm, a);
   else
-    attention_tcgen05_kernel<false, false><<<grid, AT_THREADS, AT_SMEM_BYTES, stream>>>(tm, a);
+    launch_dependent(attention_tcgen05_kernel<false, false>, grid, AT_THREADS, AT_SMEM_BYTES, stream, tm, a);
   int lrc = after_launch("attention_tcgen05_kernel");
   if (lrc || a.kv_split == 1) return lrc;
   const long warps = static_cast<long>(B) * NH * T;
-  attention_merge_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(a);
+  launch_dependent(attention_merge_kernel, static_cast<unsigned>((warps + 7) / 8), 256, 0, stream, a);
   return after_launch("attention_merge_kernel");
 }
 

@@ -131,6 +131,8 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote signal
   tc_fence_after_sync();
+  grid_dep_wait();
+  grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
 
@@ -297,7 +299,7 @@ int launch_pair_inst(const PairProblem& p0, const PairProblem& p1, int tiles0, i
   const int tiles = tiles0 + tiles1;
   const int max_pairs = device_sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  kern<<<2 * pairs, P_THREADS, SMEM, stream>>>(p0, p1, tiles0, tiles1);
+  launch_dependent(kern, 2 * pairs, P_THREADS, SMEM, stream, p0, p1, tiles0, tiles1);
   return after_launch("gemm_pair_tcgen05_kernel");
 }
 

@@ -262,6 +262,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_dep_wait();
+  grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
   const int num_tiles = tiles0 + tiles1;
@@ -388,7 +390,7 @@ int launch_split_inst(const SplitProblem& p0, const SplitProblem& p1, int tiles0
     }
   }
   const int tiles = tiles0 + tiles1, sms = device_sm_count();
-  kern<<<tiles < sms ? tiles : sms, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(p0, p1, tiles0, tiles1);
+  launch_dependent(kern, tiles < sms ? tiles : sms, Cfg::THREADS, Cfg::SMEM_BYTES, stream, p0, p1, tiles0, tiles1);
   return after_launch("gemm_split_tcgen05_kernel");
 }
 

@@ -92,6 +92,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_dep_wait();
+  grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, g.status};
 
@@ -302,7 +304,7 @@ int launch_inst(const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs& 
   }
   const int tiles = g.tiles_m * g.tiles_n;
   const int grid = tiles < device_sm_count() ? tiles : device_sm_count();
-  kern<<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(tmA, tmW, g);
+  launch_dependent(kern, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, tmA, tmW, g);
   return after_launch("gemm_tcgen05_kernel");
 }
 

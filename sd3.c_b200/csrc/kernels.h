@@ -26,6 +26,27 @@ int check_cuda(cudaError_t e, const char* what);
 int after_launch(const char* kernel_name);
 long launch_count(int reset);
 
+// Launches a kernel that may begin while its predecessor in the stream drains (programmatic
+// dependent launch).  Every kernel launched this way runs grid_dep_wait() (ptx.cuh) in all threads
+// before it touches global memory that another kernel writes or reads, and only then
+// grid_dep_launch(): a kernel that has started therefore has every kernel but its immediate
+// predecessor complete, and its own loads and stores come after that one completed as well.
+template <typename... Params, typename... Args>
+inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             Args&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // an error is picked up by after_launch
+}
+
 // ----------------------------------------------------------------------------
 // tcgen05 GEMM:  acc[m, n] = sum_k A[m, k] * W[n, k]   (A: M x K row-major,
 // W: N x K row-major, i.e. both operands K-major), fp32 accumulation in TMEM,

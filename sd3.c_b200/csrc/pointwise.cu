@@ -71,6 +71,8 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
                    void* __restrict__ out1, const float* __restrict__ shift2,
                    const float* __restrict__ scale2, void* __restrict__ out2, long mod_stride,
                    int rpw) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ float4 ln_smem[];  // [1 + scale1 | shift1 | 1 + scale2 | shift2], E floats each
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = E >> 2;
@@ -181,7 +183,7 @@ int launch_ln_inst(const float* x, long rows, int T, int E, float eps, const flo
   const bool dual = out2 != nullptr;
   const size_t smem = static_cast<size_t>(E) * 4 * (dual ? 4 : 2);
 #define SD3_LN_LAUNCH(F32, DUALV)                                                              \
-  ln_modulate_kernel<MAXV, F32, DUALV><<<grid, LN_WARPS * 32, smem, stream>>>(                   \
+  launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream,      \
       x, rows, T, E, eps, shift1, scale1, out1, shift2, scale2, out2, mod_stride, rpw)
   if (out_f32 == 1) {
     if (dual) SD3_LN_LAUNCH(1, true); else SD3_LN_LAUNCH(1, false);
@@ -253,6 +255,8 @@ __global__ void __launch_bounds__(128)
 skinny_linear_kernel(const float* __restrict__ in, long ld_in, const WT* __restrict__ W,
                      const float* __restrict__ bias, const float* __restrict__ add, long ld_add,
                      float* __restrict__ out, long ld_out, int B, int N, int K, int act_out) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long n0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + warp) * R;
   if (n0 >= N) return;
@@ -313,6 +317,8 @@ skinny_linear_kernel(const float* __restrict__ in, long ld_in, const WT* __restr
 
 __global__ void sinusoidal_kernel(const float* __restrict__ t, float* __restrict__ out, int B,
                                   int dim) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int half = dim / 2;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * half) return;
@@ -355,6 +361,8 @@ template <> __device__ __forceinline__ bf16 convert_elem<bf16, bf16>(bf16 v) { r
 template <typename IT, typename OT, bool SPLIT = false>
 __global__ void patchify_kernel(const IT* __restrict__ latent, OT* __restrict__ out, int B, int C,
                                 int H, int W, int p) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int hp = H / p, wp = W / p;
   const int Kp = C * p * p;
   const long total = static_cast<long>(B) * hp * wp * Kp;
@@ -381,6 +389,8 @@ __global__ void patchify_kernel(const IT* __restrict__ latent, OT* __restrict__ 
 
 template <typename IT, typename OT>
 __global__ void cast_kernel(const IT* __restrict__ in, OT* __restrict__ out, long n) {
+  grid_dep_wait();
+  grid_dep_launch();
   long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long stride = static_cast<long>(gridDim.x) * blockDim.x;
   for (; i < n; i += stride) out[i] = convert_elem<IT, OT>(in[i]);
@@ -405,6 +415,8 @@ __global__ void transpose_kernel(const IT* __restrict__ in, OT* __restrict__ out
 
 template <typename IT>
 __global__ void split3_kernel(const IT* __restrict__ in, bf16* __restrict__ out, long n) {
+  grid_dep_wait();
+  grid_dep_launch();
   long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   const long stride = static_cast<long>(gridDim.x) * blockDim.x * 4;
   for (; i < n; i += stride) {
@@ -448,6 +460,8 @@ __global__ void transpose_split3_kernel(const IT* __restrict__ in, bf16* __restr
 template <typename XT>
 __global__ void rmsnorm_heads_kernel(XT* __restrict__ x, long ld, long rows, int col0, int nheads,
                                      int D, const float* __restrict__ w, float eps) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long unit = static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + warp;
   if (unit >= rows * nheads) return;
@@ -510,13 +524,13 @@ int launch_skinny_linear(const float* in, long ld_in, const void* W, int w_f32, 
     constexpr int R = 4;
     const long warps = (static_cast<long>(N) + R - 1) / R;
     const unsigned grid = static_cast<unsigned>((warps + WPB - 1) / WPB);
-    skinny_linear_kernel<float, R, BC, 2><<<grid, WPB * 32, 0, stream>>>(
+    launch_dependent(skinny_linear_kernel<float, R, BC, 2>, grid, WPB * 32, 0, stream,
         in, ld_in, static_cast<const float*>(W), bias, add, ld_add, out, ld_out, B, N, K, act_out);
   } else {
     constexpr int R = 8;
     const long warps = (static_cast<long>(N) + R - 1) / R;
     const unsigned grid = static_cast<unsigned>((warps + WPB - 1) / WPB);
-    skinny_linear_kernel<bf16, R, BC, 2><<<grid, WPB * 32, 0, stream>>>(
+    launch_dependent(skinny_linear_kernel<bf16, R, BC, 2>, grid, WPB * 32, 0, stream,
         in, ld_in, static_cast<const bf16*>(W), bias, add, ld_add, out, ld_out, B, N, K, act_out);
   }
   return after_launch("skinny_linear_kernel");
@@ -528,7 +542,7 @@ int launch_sinusoidal(const float* t, float* out, int B, int dim, cudaStream_t s
     return ST_INVALID_ARG;
   }
   const int n = B * (dim / 2);
-  sinusoidal_kernel<<<(n + 127) / 128, 128, 0, stream>>>(t, out, B, dim);
+  launch_dependent(sinusoidal_kernel, (n + 127) / 128, 128, 0, stream, t, out, B, dim);
   return after_launch("sinusoidal_kernel");
 }
 
@@ -553,17 +567,17 @@ int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int 
   const long total = static_cast<long>(B) * C * H * W;
   const unsigned grid = static_cast<unsigned>((total + 255) / 256);
   if (in_f32 && out_f32 == 3)
-    patchify_kernel<float, bf16, true><<<grid, 256, 0, stream>>>((const float*)latent, (bf16*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<float, bf16, true>, grid, 256, 0, stream, (const float*)latent, (bf16*)out, B, C, H, W, p);
   else if (out_f32 == 3)
-    patchify_kernel<bf16, bf16, true><<<grid, 256, 0, stream>>>((const bf16*)latent, (bf16*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<bf16, bf16, true>, grid, 256, 0, stream, (const bf16*)latent, (bf16*)out, B, C, H, W, p);
   else if (in_f32 && out_f32)
-    patchify_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)latent, (float*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<float, float>, grid, 256, 0, stream, (const float*)latent, (float*)out, B, C, H, W, p);
   else if (in_f32)
-    patchify_kernel<float, bf16><<<grid, 256, 0, stream>>>((const float*)latent, (bf16*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<float, bf16>, grid, 256, 0, stream, (const float*)latent, (bf16*)out, B, C, H, W, p);
   else if (out_f32)
-    patchify_kernel<bf16, float><<<grid, 256, 0, stream>>>((const bf16*)latent, (float*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<bf16, float>, grid, 256, 0, stream, (const bf16*)latent, (float*)out, B, C, H, W, p);
   else
-    patchify_kernel<bf16, bf16><<<grid, 256, 0, stream>>>((const bf16*)latent, (bf16*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<bf16, bf16>, grid, 256, 0, stream, (const bf16*)latent, (bf16*)out, B, C, H, W, p);
   return after_launch("patchify_kernel");
 }
 
@@ -576,6 +590,8 @@ namespace {
 template <typename TI>
 __global__ void quantize_e4m3_kernel(const TI* __restrict__ in, uint8_t* __restrict__ out, long n,
                                      float inv_scale) {
+  grid_dep_wait();
+  grid_dep_launch();
   // four elements per thread per step (n is a multiple of 4)
   long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   const long stride = static_cast<long>(gridDim.x) * blockDim.x * 4;
@@ -623,10 +639,10 @@ int launch_quantize_e4m3(const void* in, int in_f32, void* out, long n, float in
   const long blocks = (n / 4 + 255) / 256;
   const unsigned grid = static_cast<unsigned>(blocks < device_sm_count() * 16 ? blocks : device_sm_count() * 16);
   if (in_f32)
-    quantize_e4m3_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(in),
+    launch_dependent(quantize_e4m3_kernel<float>, grid, 256, 0, stream, static_cast<const float*>(in),
                                                           static_cast<uint8_t*>(out), n, inv_scale);
   else
-    quantize_e4m3_kernel<bf16><<<grid, 256, 0, stream>>>(static_cast<const bf16*>(in),
+    launch_dependent(quantize_e4m3_kernel<bf16>, grid, 256, 0, stream, static_cast<const bf16*>(in),
                                                          static_cast<uint8_t*>(out), n, inv_scale);
   return after_launch("quantize_e4m3_kernel");
 }
@@ -652,14 +668,14 @@ int launch_absmax(const void* in, int in_f32, long n, float* out, cudaStream_t s
 int launch_cast_f32_to_bf16(const float* in, bf16* out, long n, cudaStream_t stream) {
   if (n <= 0) return ST_OK;
   const unsigned grid = static_cast<unsigned>(n / 256 + 1 < device_sm_count() * 16 ? n / 256 + 1 : device_sm_count() * 16);
-  cast_kernel<float, bf16><<<grid, 256, 0, stream>>>(in, out, n);
+  launch_dependent(cast_kernel<float, bf16>, grid, 256, 0, stream, in, out, n);
   return after_launch("cast_kernel");
 }
 
 int launch_cast_bf16_to_f32(const bf16* in, float* out, long n, cudaStream_t stream) {
   if (n <= 0) return ST_OK;
   const unsigned grid = static_cast<unsigned>(n / 256 + 1 < device_sm_count() * 16 ? n / 256 + 1 : device_sm_count() * 16);
-  cast_kernel<bf16, float><<<grid, 256, 0, stream>>>(in, out, n);
+  launch_dependent(cast_kernel<bf16, float>, grid, 256, 0, stream, in, out, n);
   return after_launch("cast_kernel");
 }
 
@@ -690,9 +706,9 @@ int launch_split3(const void* in, int in_f32, bf16* out, long n, cudaStream_t st
   const long blocks = (n / 4 + 255) / 256, most = device_sm_count() * 16L;
   const unsigned grid = static_cast<unsigned>(blocks < most ? blocks : most);
   if (in_f32)
-    split3_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(in), out, n);
+    launch_dependent(split3_kernel<float>, grid, 256, 0, stream, static_cast<const float*>(in), out, n);
   else
-    split3_kernel<bf16><<<grid, 256, 0, stream>>>(static_cast<const bf16*>(in), out, n);
+    launch_dependent(split3_kernel<bf16>, grid, 256, 0, stream, static_cast<const bf16*>(in), out, n);
   return after_launch("split3_kernel");
 }
 
@@ -718,9 +734,9 @@ int launch_rmsnorm_heads(void* x, int x_f32, long ld, long rows, int col0, int n
   const long units = rows * nheads;
   const unsigned grid = static_cast<unsigned>((units + 7) / 8);
   if (x_f32)
-    rmsnorm_heads_kernel<float><<<grid, 256, 0, stream>>>((float*)x, ld, rows, col0, nheads, D, w, eps);
+    launch_dependent(rmsnorm_heads_kernel<float>, grid, 256, 0, stream, (float*)x, ld, rows, col0, nheads, D, w, eps);
   else
-    rmsnorm_heads_kernel<bf16><<<grid, 256, 0, stream>>>((bf16*)x, ld, rows, col0, nheads, D, w, eps);
+    launch_dependent(rmsnorm_heads_kernel<bf16>, grid, 256, 0, stream, (bf16*)x, ld, rows, col0, nheads, D, w, eps);
   return after_launch("rmsnorm_heads_kernel");
 }
 

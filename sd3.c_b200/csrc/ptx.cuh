@@ -113,6 +113,12 @@ __device__ __forceinline__ uint32_t mbar_test_wait(uint64_t* bar, uint32_t parit
   return ok;
 }
 
+// Programmatic dependent launch: wait until the preceding kernel of the stream is complete and its
+// writes are visible / allow the following kernel to be scheduled.  Both do nothing in a launch
+// without the attribute.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Shared by all roles of a CTA: the abort flag in shared memory and the
 // status word in global memory.
 struct WaitCtx {
