@@ -325,8 +325,8 @@ int sd3_layernorm_modulate(const float* x, int B, int T, int E, float eps, const
     set_last_error("sd3_layernorm_modulate: bad out_dtype %d", out_dtype);
     return SD3_ERR_INVALID_ARG;
   }
-  return launch_ln_modulate(x, B, T, E, eps, shift1, scale1, out1, shift2, scale2, out2,
-                            mod_stride, out_dtype == SD3_DTYPE_F32, S(stream));
+  const LnProblem p = {x, B, T, shift1, scale1, out1, shift2, scale2, out2};
+  return launch_ln_modulate(p, nullptr, E, eps, mod_stride, out_dtype == SD3_DTYPE_F32, S(stream));
 }
 
 int sd3_skinny_linear(const float* in, long ld_in, const void* w, int w_dtype, const float* bias,

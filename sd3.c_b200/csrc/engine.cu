@@ -10,12 +10,12 @@
 // the caller's stream, nothing synchronises.
 //
 // Per block the launch sequence is
-//   LN+modulate(c) | LN+modulate(x) (both modulations of a dual block at once)
+//   LN+modulate(x), LN+modulate(c) in one launch (both modulations of a dual block at once)
 //   QKV GEMM(c), QKV GEMM(x)  -> packed (B, Tc+Tx, 3E), RMSNorm fused, context rows first
 //   joint attention           -> o_c, o_x
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
 //   [dual] QKV GEMM(x2), attention over image tokens, out-proj GEMM with gate2
-//   LN+modulate(x), MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual); same for c
+//   LN+modulate(x), (c); MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual), each for x and c at once
 #include <math.h>
 #include <algorithm>
 #include <cmath>
@@ -473,6 +473,13 @@ int run_mlp1(sd3_model* m, const Linear& L, const Linear& next, const void* A, i
   return run_linear(m, L, A, M, e, st, a_e4m3);
 }
 
+// the LayerNorms of the image and the context rows as one launch where both write the same type
+int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st) {
+  if (!pc || out_x == out_c) return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
+  int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st);
+  return rc ? rc : launch_ln_modulate(px, nullptr, E, 1e-6f, ms, out_x, st);
+}
+
 int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, const float* mod,
                long ms, cudaStream_t st) {
   const LayerW& L = m->layers[l];
@@ -499,14 +506,12 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const bool c8m = m->fp8 && L.c_mlp1.w8, x8m = m->fp8 && L.x_mlp1.w8;
   auto ln_out = [&](bool e4m3) { return m->f32 ? 3 : (e4m3 ? 2 : 0); };
   // pre-attention LayerNorm + modulate
-  SD3_TRY(launch_ln_modulate(c, B, Tc, E, 1e-6f, c_shift_a, c_scale_a, w.h_c, nullptr, nullptr,
-                             nullptr, ms, ln_out(c8a), st));
-  if (L.dual)
-    SD3_TRY(launch_ln_modulate(x, B, Tx, E, 1e-6f, x_shift_a, x_scale_a, w.h_x, x_shift_2, x_scale_2,
-                               w.h_x2, ms, ln_out(x8a), st));
-  else
-    SD3_TRY(launch_ln_modulate(x, B, Tx, E, 1e-6f, x_shift_a, x_scale_a, w.h_x, nullptr, nullptr,
-                               nullptr, ms, ln_out(x8a), st));
+  {
+    LnProblem px = {x, B, Tx, x_shift_a, x_scale_a, w.h_x, nullptr, nullptr, nullptr};
+    if (L.dual) { px.shift2 = x_shift_2; px.scale2 = x_scale_2; px.out2 = w.h_x2; }
+    const LnProblem pc = {c, B, Tc, c_shift_a, c_scale_a, w.h_c, nullptr, nullptr, nullptr};
+    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st));
+  }
   // QKV (context rows first, then image rows) and joint attention
   // image and context GEMMs of a kind share a launch (bf16 / FP8 modes: with head_dim 64)
   const bool grouped = m->f32 || m->D == 64;
@@ -541,11 +546,11 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   }
   // MLPs of both streams: LayerNorm + modulate each, then the two first linears (GELU-tanh) and
   // the two second linears (gate + residual), each pair as one grouped launch
-  SD3_TRY(launch_ln_modulate(x, B, Tx, E, 1e-6f, x_shift_m, x_scale_m, w.h_x, nullptr, nullptr,
-                             nullptr, ms, ln_out(x8m), st));
-  if (!L.last)
-    SD3_TRY(launch_ln_modulate(c, B, Tc, E, 1e-6f, c_shift_m, c_scale_m, w.h_c, nullptr, nullptr,
-                               nullptr, ms, ln_out(c8m), st));
+  {
+    const LnProblem px = {x, B, Tx, x_shift_m, x_scale_m, w.h_x, nullptr, nullptr, nullptr};
+    const LnProblem pc = {c, B, Tc, c_shift_m, c_scale_m, w.h_c, nullptr, nullptr, nullptr};
+    SD3_TRY(run_ln_pair(px, ln_out(x8m), L.last ? nullptr : &pc, ln_out(c8m), E, ms, st));
+  }
   if (grouped && !L.last) {
     const bool hx8 = m->fp8 && L.x_mlp1.w8 && L.x_mlp2.w8 && L.x_mlp1.N % 64 == 0;
     const bool hc8 = m->fp8 && L.c_mlp1.w8 && L.c_mlp2.w8 && L.c_mlp1.N % 64 == 0;
@@ -1002,8 +1007,8 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   // final layer: LN(eps 1e-5) * (1 + scale) + shift with chunks (scale, shift), linear, unpatchify
   {
     const float* fm = w.mod + m->fin_mod_off;
-    SD3_TRY(launch_ln_modulate(w.x, B, Tx, E, 1e-5f, fm + E, fm, w.h_x, nullptr, nullptr, nullptr,
-                               m->ada_total, m->f32 ? 3 : 0, st));
+    const LnProblem px = {w.x, B, Tx, fm + E, fm, w.h_x, nullptr, nullptr, nullptr};
+    SD3_TRY(launch_ln_modulate(px, nullptr, E, 1e-5f, m->ada_total, m->f32 ? 3 : 0, st));
     GemmEpilogue e;
     e.mode = EPI_UNPATCHIFY; e.out = out; e.out_f32 = io_f32; e.ldo = m->Nout;
     e.rows_in = Tx; e.rows_out = Tx;

@@ -31,6 +31,8 @@ long launch_count(int reset);
 // before it touches global memory that another kernel writes or reads, and only then
 // grid_dep_launch(): a kernel that has started therefore has every kernel but its immediate
 // predecessor complete, and its own loads and stores come after that one completed as well.
+// Measured on the forward of one image: 256x256 4131 -> 3520 us, 512x512 5090 -> 4553 us, 1024x1024
+// 14.22 -> 13.97 ms; unchanged at batch 8 and under graph replay.
 template <typename... Params, typename... Args>
 inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                              Args&&... args) {
@@ -171,10 +173,18 @@ int launch_attention_simt(const void* q, const void* k, const void* v, long ld, 
 // ----------------------------------------------------------------------------
 // LayerNorm (no affine) + up to two modulations:  out_i = LN(x) * (1 + scale_i[b]) + shift_i[b]
 // x: (B*T, E) fp32.  shift/scale: [b * mod_stride + e].  out: bf16 (out_f32 = 0), fp32 (1),
-// e4m3 converted as is (2) or three bf16 planes of B*T*E elements (3, split3.cuh).
-int launch_ln_modulate(const float* x, int B, int T, int E, float eps, const float* shift1,
-                       const float* scale1, void* out1, const float* shift2, const float* scale2,
-                       void* out2, long mod_stride, int out_f32, cudaStream_t stream);
+// e4m3 converted as is (2) or three bf16 planes of B*T*E elements (3, split3.cuh).  One or two
+// problems (b may be null) as one launch.
+struct LnProblem {
+  const float* x = nullptr;
+  int B = 0, T = 0;
+  const float *shift1 = nullptr, *scale1 = nullptr;
+  void* out1 = nullptr;
+  const float *shift2 = nullptr, *scale2 = nullptr;  // second modulation (out2 null: none)
+  void* out2 = nullptr;
+};
+int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
+                       cudaStream_t stream);
 
 // Skinny linear for M = B <= 64 rows:  out[b, n] = act_out(sum_k in[b,k] W[n,k] + bias[n] + add[b,n])
 // W is (N, K) row-major, bf16 or fp32 (w_f32).  act: 0 none, 1 SiLU.

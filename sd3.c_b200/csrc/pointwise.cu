@@ -35,6 +35,13 @@ namespace {
 // global memory for every row (12 KB per 6 KB row, all L1 hits) cost a quarter
 // of the kernel's bandwidth.  Rows of another sample (a CTA that straddles a
 // sample boundary) read theirs from global memory.
+//
+// One launch takes one or two problems (the image and the context rows of a block,
+// whose LayerNorms stand next to each other everywhere): at small sizes the kernel
+// is one chain of latencies (launch, row, two reductions, store; 7 us for 256 rows),
+// and two of them in a row cost twice that.  The first row is requested before the
+// barrier behind the staging.  Measured (whole forward, one image): 256x256 3510 -> 3326 us,
+// 1024x1024 14.18 -> 13.96 ms.  Three CTAs per SM for the plane output, whose splits need the registers.
 constexpr int LN_MAX_ROWS_PER_WARP = 8;
 constexpr int LN_WARPS = 8;
 
@@ -65,54 +72,56 @@ __device__ __forceinline__ void ln_store4(void* out, long row, long rows, int E,
 }
 
 template <int MAXV, int OUT, bool DUAL>
-__global__ void __launch_bounds__(LN_WARPS * 32, 4)
-ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float eps,
-                   const float* __restrict__ shift1, const float* __restrict__ scale1,
-                   void* __restrict__ out1, const float* __restrict__ shift2,
-                   const float* __restrict__ scale2, void* __restrict__ out2, long mod_stride,
+__global__ void __launch_bounds__(LN_WARPS * 32, OUT == 3 ? 3 : 4)
+ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a, int E, float eps, long mod_stride,
                    int rpw) {
+  extern __shared__ float4 ln_smem[];  // [1 + scale1 | shift1 | 1 + scale2 | shift2], E floats each
   grid_dep_wait();
   grid_dep_launch();
-  extern __shared__ float4 ln_smem[];  // [1 + scale1 | shift1 | 1 + scale2 | shift2], E floats each
+  const bool second = blockIdx.x >= grid_a;
+  const LnProblem& p = second ? pb : pa;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = E >> 2;
-  const long row0 = static_cast<long>(blockIdx.x) * (LN_WARPS * rpw);
+  const int T = p.T;
+  const long rows = static_cast<long>(p.B) * T;
+  const bool dual = DUAL && p.out2 != nullptr;
+  const long row0 = static_cast<long>(second ? blockIdx.x - grid_a : blockIdx.x) * (LN_WARPS * rpw);
   const int b_cta = static_cast<int>(row0 / T);
   float4* s_sc1 = ln_smem;
   float4* s_sh1 = ln_smem + nvec;
   float4* s_sc2 = ln_smem + 2 * nvec;
   float4* s_sh2 = ln_smem + 3 * nvec;
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    float4 s = __ldg(reinterpret_cast<const float4*>(scale1 + b_cta * mod_stride) + i);
+    float4 s = __ldg(reinterpret_cast<const float4*>(p.scale1 + b_cta * mod_stride) + i);
     s.x += 1.f; s.y += 1.f; s.z += 1.f; s.w += 1.f;
     s_sc1[i] = s;
-    s_sh1[i] = __ldg(reinterpret_cast<const float4*>(shift1 + b_cta * mod_stride) + i);
-    if constexpr (DUAL) {
-      float4 s2 = __ldg(reinterpret_cast<const float4*>(scale2 + b_cta * mod_stride) + i);
+    s_sh1[i] = __ldg(reinterpret_cast<const float4*>(p.shift1 + b_cta * mod_stride) + i);
+    if (dual) {
+      float4 s2 = __ldg(reinterpret_cast<const float4*>(p.scale2 + b_cta * mod_stride) + i);
       s2.x += 1.f; s2.y += 1.f; s2.z += 1.f; s2.w += 1.f;
       s_sc2[i] = s2;
-      s_sh2[i] = __ldg(reinterpret_cast<const float4*>(shift2 + b_cta * mod_stride) + i);
+      s_sh2[i] = __ldg(reinterpret_cast<const float4*>(p.shift2 + b_cta * mod_stride) + i);
     }
   }
-  __syncthreads();
 #pragma unroll 1
   for (int rw = 0; rw < rpw; ++rw) {
     const long row = row0 + static_cast<long>(rw) * LN_WARPS + warp;  // warps interleave rows
-    if (row >= rows) break;
-    const int b = static_cast<int>(row / T);
-    const float4* xr = reinterpret_cast<const float4*>(x + row * E);
+    const bool live = row < rows;
+    const float4* xr = reinterpret_cast<const float4*>(p.x + row * E);
     float4 v[MAXV];
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
       const int i = lane + 32 * j;
-      if (i < nvec) {
+      if (live && i < nvec) {
         v[j] = xr[i];
         sum += (v[j].x + v[j].y) + (v[j].z + v[j].w);
       } else {
         v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
+    if (rw == 0) __syncthreads();  // the staged vectors are complete; the first row was requested before
+    if (!live) break;
     const float mean = warp_sum(sum) / static_cast<float>(E);
     float sq = 0.f;
 #pragma unroll
@@ -123,6 +132,7 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
         sq += (a * a + bq * bq) + (c * c + d * d);
       }
     }
+    const int b = static_cast<int>(row / T);
     const float rstd = rsqrtf(warp_sum(sq) / static_cast<float>(E) + eps);
     const bool cached = b == b_cta;  // warp-uniform
     const long moff = static_cast<long>(b) * mod_stride;  // used by rows of another sample only
@@ -140,8 +150,8 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
           if (cached) {
             s = s_sc1[i]; h = s_sh1[i];
           } else {
-            s = __ldg(reinterpret_cast<const float4*>(scale1 + moff) + i);
-            h = __ldg(reinterpret_cast<const float4*>(shift1 + moff) + i);
+            s = __ldg(reinterpret_cast<const float4*>(p.scale1 + moff) + i);
+            h = __ldg(reinterpret_cast<const float4*>(p.shift1 + moff) + i);
             s.x += 1.f; s.y += 1.f; s.z += 1.f; s.w += 1.f;
           }
           float4 o;
@@ -149,15 +159,15 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
           o.y = fmaf(n.y, s.y, h.y);
           o.z = fmaf(n.z, s.z, h.z);
           o.w = fmaf(n.w, s.w, h.w);
-          ln_store4<OUT>(out1, row, rows, E, i, o);
+          ln_store4<OUT>(p.out1, row, rows, E, i, o);
         }
-        if constexpr (DUAL) {
+        if (dual) {
           float4 s, h;
           if (cached) {
             s = s_sc2[i]; h = s_sh2[i];
           } else {
-            s = __ldg(reinterpret_cast<const float4*>(scale2 + moff) + i);
-            h = __ldg(reinterpret_cast<const float4*>(shift2 + moff) + i);
+            s = __ldg(reinterpret_cast<const float4*>(p.scale2 + moff) + i);
+            h = __ldg(reinterpret_cast<const float4*>(p.shift2 + moff) + i);
             s.x += 1.f; s.y += 1.f; s.z += 1.f; s.w += 1.f;
           }
           float4 o;
@@ -165,7 +175,7 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
           o.y = fmaf(n.y, s.y, h.y);
           o.z = fmaf(n.z, s.z, h.z);
           o.w = fmaf(n.w, s.w, h.w);
-          ln_store4<OUT>(out2, row, rows, E, i, o);
+          ln_store4<OUT>(p.out2, row, rows, E, i, o);
         }
       }
     }
@@ -173,18 +183,20 @@ ln_modulate_kernel(const float* __restrict__ x, long rows, int T, int E, float e
 }
 
 template <int MAXV>
-int launch_ln_inst(const float* x, long rows, int T, int E, float eps, const float* shift1,
-                   const float* scale1, void* out1, const float* shift2, const float* scale2,
-                   void* out2, long mod_stride, int out_f32, cudaStream_t stream) {
+int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
+                   cudaStream_t stream) {
+  const long rows_a = static_cast<long>(a.B) * a.T, rows_b = b ? static_cast<long>(b->B) * b->T : 0;
   // rows per warp: as many as keeps at least two CTAs per SM busy
   int rpw = LN_MAX_ROWS_PER_WARP;
-  while (rpw > 1 && (rows + LN_WARPS * rpw - 1) / (LN_WARPS * rpw) < 2L * device_sm_count()) rpw >>= 1;
-  const unsigned grid = static_cast<unsigned>((rows + LN_WARPS * rpw - 1) / (LN_WARPS * rpw));
-  const bool dual = out2 != nullptr;
+  auto ctas = [&](long rows) { return (rows + LN_WARPS * rpw - 1) / (LN_WARPS * rpw); };
+  while (rpw > 1 && ctas(rows_a) + ctas(rows_b) < 2L * device_sm_count()) rpw >>= 1;
+  const unsigned grid_a = static_cast<unsigned>(ctas(rows_a)), grid = grid_a + static_cast<unsigned>(ctas(rows_b));
+  const bool dual = a.out2 != nullptr || (b && b->out2 != nullptr);
   const size_t smem = static_cast<size_t>(E) * 4 * (dual ? 4 : 2);
-#define SD3_LN_LAUNCH(F32, DUALV)                                                              \
-  launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream,      \
-      x, rows, T, E, eps, shift1, scale1, out1, shift2, scale2, out2, mod_stride, rpw)
+  const LnProblem pb = b ? *b : a;
+#define SD3_LN_LAUNCH(F32, DUALV)                                                                                    \
+  launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, E, eps,   \
+                   mod_stride, rpw)
   if (out_f32 == 1) {
     if (dual) SD3_LN_LAUNCH(1, true); else SD3_LN_LAUNCH(1, false);
   } else if (out_f32 == 2) {
@@ -482,24 +494,23 @@ __global__ void rmsnorm_heads_kernel(XT* __restrict__ x, long ld, long rows, int
 
 }  // namespace
 
-int launch_ln_modulate(const float* x, int B, int T, int E, float eps, const float* shift1,
-                       const float* scale1, void* out1, const float* shift2, const float* scale2,
-                       void* out2, long mod_stride, int out_f32, cudaStream_t stream) {
-  if (!x || !out1 || !shift1 || !scale1 || B <= 0 || T <= 0 || E <= 0 || (E & 3) ||
-      (mod_stride & 3)) {
-    set_last_error("ln_modulate: invalid argument (E %d must be a multiple of 4)", E);
-    return ST_INVALID_ARG;
+int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
+                       cudaStream_t stream) {
+  for (const LnProblem* p : {&a, b}) {
+    if (!p) continue;
+    if (!p->x || !p->out1 || !p->shift1 || !p->scale1 || p->B <= 0 || p->T <= 0 || E <= 0 || (E & 3) ||
+        (mod_stride & 3)) {
+      set_last_error("ln_modulate: invalid argument (E %d must be a multiple of 4)", E);
+      return ST_INVALID_ARG;
+    }
+    if (p->out2 && (!p->shift2 || !p->scale2)) {
+      set_last_error("ln_modulate: second output needs its own shift/scale");
+      return ST_INVALID_ARG;
+    }
   }
-  if (out2 && (!shift2 || !scale2)) {
-    set_last_error("ln_modulate: second output needs its own shift/scale");
-    return ST_INVALID_ARG;
-  }
-  const long rows = static_cast<long>(B) * T;
   const int nvec = E / 4;
-#define SD3_LN_CASE(MV)                                                                         \
-  if (nvec <= 32 * MV)                                                                          \
-    return launch_ln_inst<MV>(x, rows, T, E, eps, shift1, scale1, out1, shift2, scale2, out2,    \
-                              mod_stride, out_f32, stream)
+#define SD3_LN_CASE(MV) \
+  if (nvec <= 32 * MV) return launch_ln_inst<MV>(a, b, E, eps, mod_stride, out_f32, stream)
   SD3_LN_CASE(2);
   SD3_LN_CASE(6);
   SD3_LN_CASE(12);
