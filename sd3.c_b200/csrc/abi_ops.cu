@@ -11,13 +11,13 @@ namespace sd3 {
 // the process.  Kernels write a DEV_TIMEOUT_* code there when a wait runs out.
 int* static_status_word_if_resolved();
 
-int* device_status_word() {
+int* device_status_word(bool create) {
   static int* words[64] = {nullptr};
   static std::mutex mu;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> lock(mu);
-  if (!words[dev]) {
+  if (!words[dev] && create) {
     int* p = nullptr;
     if (cudaMalloc(&p, sizeof(int)) != cudaSuccess) return nullptr;
     if (cudaMemset(p, 0, sizeof(int)) != cudaSuccess) {
@@ -35,6 +35,11 @@ using namespace sd3;
 
 namespace {
 inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
+// for operators that used not to need a status word: a first use under stream capture must not allocate
+inline int* status_word_for(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return device_status_word(cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone);
+}
 inline bool dtype_ok(int d) { return d == SD3_DTYPE_F32 || d == SD3_DTYPE_BF16; }
 }  // namespace
 
@@ -337,7 +342,7 @@ int sd3_skinny_linear(const float* in, long ld_in, const void* w, int w_dtype, c
     return SD3_ERR_INVALID_ARG;
   }
   return launch_skinny_linear(in, ld_in, w, w_dtype == SD3_DTYPE_F32, bias, add, ld_add, out,
-                              ld_out, B, N, K, act, S(stream));
+                              ld_out, B, N, K, act, status_word_for(S(stream)), S(stream));
 }
 
 int sd3_sinusoidal_embedding(const float* t, float* out, int B, int dim, void* stream) {

@@ -30,8 +30,6 @@
 
 namespace sd3 {
 
-int* device_status_word();
-
 namespace {
 
 struct Linear {
@@ -864,6 +862,10 @@ int sd3_model_finalize(sd3_model* m, int* missing) {
     set_last_error("%d required parameter(s) missing, first: %s", n, first.c_str());
     return SD3_ERR_NOT_READY;
   }
+  if (!m->finalized) {  // the kernels take the packed weights as settled (launch_skinny_linear: w_static)
+    int rc = check_cuda(cudaDeviceSynchronize(), "parameter copies");
+    if (rc) return rc;
+  }
   if (m->fp8 && !m->finalized) {
     int rc = quantize_block_weights(m);
     if (rc) return rc;
@@ -905,7 +907,7 @@ int sd3_block_forward(sd3_model* m, int layer, const float* y, float* c, float* 
   rc = launch_skinny_linear(y, m->E,
                             static_cast<char*>(m->ada_w) + static_cast<size_t>(lo) * m->E * m->wbytes(),
                             m->f32, m->ada_b + lo, nullptr, 0, m->ws.mod + lo, m->ada_total, B,
-                            static_cast<int>(n), m->E, 0, st);
+                            static_cast<int>(n), m->E, 0, m->status, st, true);
   if (rc) return rc;
   return block_body(m, layer, c, x, B, Tc, Tx, m->ws.mod, m->ada_total, st);
 }
@@ -956,10 +958,14 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
     pooled32 = w.pooled_f32;
   }
   SD3_TRY(launch_sinusoidal(timesteps, w.temb, B, 256, st));
-  SD3_TRY(launch_skinny_linear(w.temb, 256, m->t1.w, m->f32, m->t1.b, nullptr, 0, w.th, E, B, E, 256, 1, st));
-  SD3_TRY(launch_skinny_linear(w.th, E, m->t2.w, m->f32, m->t2.b, nullptr, 0, w.tout, E, B, E, E, 0, st));
-  SD3_TRY(launch_skinny_linear(pooled32, c.pooled_dim, m->p1.w, m->f32, m->p1.b, nullptr, 0, w.ph, E, B, E, c.pooled_dim, 1, st));
-  SD3_TRY(launch_skinny_linear(w.ph, E, m->p2.w, m->f32, m->p2.b, w.tout, E, w.y, E, B, E, E, 1, st));
+  SD3_TRY(launch_skinny_linear(w.temb, 256, m->t1.w, m->f32, m->t1.b, nullptr, 0, w.th, E, B, E, 256, 1,
+                               m->status, st, true));
+  SD3_TRY(launch_skinny_linear(w.th, E, m->t2.w, m->f32, m->t2.b, nullptr, 0, w.tout, E, B, E, E, 0,
+                               m->status, st, true));
+  SD3_TRY(launch_skinny_linear(pooled32, c.pooled_dim, m->p1.w, m->f32, m->p1.b, nullptr, 0, w.ph, E, B, E, c.pooled_dim, 1,
+                               m->status, st, true));
+  SD3_TRY(launch_skinny_linear(w.ph, E, m->p2.w, m->f32, m->p2.b, w.tout, E, w.y, E, B, E, E, 1,
+                               m->status, st, true));
   // every AdaLN vector of every block and of the final layer in one launch
   if (!m->f32 && m->ada_total % 64 == 0 && E % 64 == 0) {
     // As a tensor-core GEMM with M = batch: out (B, ada_total) = y W^T + b.  Only B
@@ -977,7 +983,7 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
                         m->status, st));
   } else {
     SD3_TRY(launch_skinny_linear(w.y, E, m->ada_w, m->f32, m->ada_b, nullptr, 0, w.mod, m->ada_total, B,
-                                 static_cast<int>(m->ada_total), E, 0, st));
+                                 static_cast<int>(m->ada_total), E, 0, m->status, st, true));
   }
   // context stream c = captions W + b
   {

@@ -25,6 +25,8 @@ const char* get_last_error();
 int check_cuda(cudaError_t e, const char* what);
 int after_launch(const char* kernel_name);
 long launch_count(int reset);
+// The device's status word (null if it cannot be had); create: allocate it on first use.
+int* device_status_word(bool create = true);
 
 // Launches a kernel that may begin while its predecessor in the stream drains (programmatic
 // dependent launch).  Every kernel launched this way runs grid_dep_wait() (ptx.cuh) in all threads
@@ -187,10 +189,11 @@ int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps,
                        cudaStream_t stream);
 
 // Skinny linear for M = B <= 64 rows:  out[b, n] = act_out(sum_k in[b,k] W[n,k] + bias[n] + add[b,n])
-// W is (N, K) row-major, bf16 or fp32 (w_f32).  act: 0 none, 1 SiLU.
+// W is (N, K) row-major, bf16 or fp32 (w_f32).  act: 0 none, 1 SiLU.  w_static: no kernel that may
+// still be running when this one is launched writes W.
 int launch_skinny_linear(const float* in, long ld_in, const void* W, int w_f32, const float* bias,
                          const float* add, long ld_add, float* out, long ld_out, int B, int N,
-                         int K, int act_out, cudaStream_t stream);
+                         int K, int act_out, int* dev_status, cudaStream_t stream, bool w_static = false);
 
 // emb[b, i] = cos(t_b f_i), emb[b, half + i] = sin(t_b f_i), f_i = exp(-ln(1e4) i / half)
 int launch_sinusoidal(const float* t, float* out, int B, int dim, cudaStream_t stream);

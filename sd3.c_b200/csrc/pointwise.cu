@@ -1,6 +1,5 @@
 // HBM-bound kernels of the denoiser forward: LayerNorm + AdaLN modulation,
-// the skinny (M = batch) linears that produce the conditioning vector and all
-// AdaLN modulation vectors, timestep / position embeddings, patch gathering,
+// timestep / position embeddings, patch gathering,
 // casts and transposes for weight packing, and a stand-alone per-head RMSNorm.
 // All of them are coalesced, 128-bit vectorised and warp-shuffle reduced.
 //
@@ -210,123 +209,6 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   return after_launch("ln_modulate_kernel");
 }
 
-// ----------------------------------------------------------------------------
-// Skinny linear: each warp owns R output columns and a chunk of BC samples.
-// ----------------------------------------------------------------------------
-__device__ __forceinline__ void load_w8(const bf16* p, float (&w)[8]) {
-  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = __bfloat1622float2(h[j]);
-    w[2 * j] = f.x;
-    w[2 * j + 1] = f.y;
-  }
-}
-__device__ __forceinline__ void load_w8(const float* p, float (&w)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-  const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-  w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-}
-
-// raw 8-element weight chunk kept in registers until it is needed
-template <typename WT> struct WChunk;
-template <> struct WChunk<bf16> {
-  uint4 u;
-  __device__ __forceinline__ void load(const bf16* p) { u = __ldg(reinterpret_cast<const uint4*>(p)); }
-  __device__ __forceinline__ void zero() { u = make_uint4(0, 0, 0, 0); }
-  __device__ __forceinline__ void get(float (&w)[8]) const {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(h[j]);
-      w[2 * j] = f.x;
-      w[2 * j + 1] = f.y;
-    }
-  }
-};
-template <> struct WChunk<float> {
-  float4 a, b;
-  __device__ __forceinline__ void load(const float* p) {
-    a = __ldg(reinterpret_cast<const float4*>(p));
-    b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  }
-  __device__ __forceinline__ void zero() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ void get(float (&w)[8]) const {
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-  }
-};
-
-// Each warp owns R output columns and walks K in slabs of KU * 256 elements;
-// all weight loads of a slab are issued before any of them is consumed, so a
-// warp keeps R * KU * 512 bytes of weight reads in flight.
-template <typename WT, int R, int BC, int KU>
-__global__ void __launch_bounds__(128)
-skinny_linear_kernel(const float* __restrict__ in, long ld_in, const WT* __restrict__ W,
-                     const float* __restrict__ bias, const float* __restrict__ add, long ld_add,
-                     float* __restrict__ out, long ld_out, int B, int N, int K, int act_out) {
-  grid_dep_wait();
-  grid_dep_launch();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long n0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + warp) * R;
-  if (n0 >= N) return;
-  for (int b0 = 0; b0 < B; b0 += BC) {
-    float acc[R][BC];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int b = 0; b < BC; ++b) acc[r][b] = 0.f;
-    for (int kb = 0; kb < K; kb += 256 * KU) {
-      WChunk<WT> wc[R][KU];
-#pragma unroll
-      for (int u = 0; u < KU; ++u) {
-        const int k = kb + u * 256 + lane * 8;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (k < K && n0 + r < N) wc[r][u].load(W + (n0 + r) * static_cast<long>(K) + k);
-          else wc[r][u].zero();
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < KU; ++u) {
-        const int k = kb + u * 256 + lane * 8;
-        if (k < K) {
-          float w[R][8];
-#pragma unroll
-          for (int r = 0; r < R; ++r) wc[r][u].get(w[r]);
-#pragma unroll
-          for (int b = 0; b < BC; ++b) {
-            if (b0 + b < B) {
-              float xv[8];
-              load_w8(in + (b0 + b) * ld_in + k, xv);
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[r][b] = fmaf(xv[j], w[r][j], acc[r][b]);
-              }
-            }
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-#pragma unroll
-      for (int b = 0; b < BC; ++b) {
-        const float s = warp_sum(acc[r][b]);
-        if (lane == 0 && n0 + r < N && b0 + b < B) {
-          float o = s + (bias ? bias[n0 + r] : 0.f);
-          if (add) o += add[(b0 + b) * ld_add + n0 + r];
-          if (act_out == 1) o = o / (1.f + expf(-o));
-          out[(b0 + b) * ld_out + n0 + r] = o;
-        }
-      }
-    }
-  }
-}
-
 __global__ void sinusoidal_kernel(const float* __restrict__ t, float* __restrict__ out, int B,
                                   int dim) {
   grid_dep_wait();
@@ -519,32 +401,6 @@ int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps,
 #undef SD3_LN_CASE
   set_last_error("ln_modulate: E %d too large (max 4096)", E);
   return ST_UNSUPPORTED;
-}
-
-int launch_skinny_linear(const float* in, long ld_in, const void* W, int w_f32, const float* bias,
-                         const float* add, long ld_add, float* out, long ld_out, int B, int N,
-                         int K, int act_out, cudaStream_t stream) {
-  if (!in || !W || !out || B <= 0 || N <= 0 || K <= 0 || (K & 7) || (ld_in & 3)) {
-    set_last_error("skinny_linear: invalid argument (K %d must be a multiple of 8)", K);
-    return ST_INVALID_ARG;
-  }
-  // R output columns per warp: every activation chunk read from L1 is reused R
-  // times, so larger R keeps the L1 traffic per weight byte low.
-  constexpr int BC = 8, WPB = 4;
-  if (w_f32) {
-    constexpr int R = 4;
-    const long warps = (static_cast<long>(N) + R - 1) / R;
-    const unsigned grid = static_cast<unsigned>((warps + WPB - 1) / WPB);
-    launch_dependent(skinny_linear_kernel<float, R, BC, 2>, grid, WPB * 32, 0, stream,
-        in, ld_in, static_cast<const float*>(W), bias, add, ld_add, out, ld_out, B, N, K, act_out);
-  } else {
-    constexpr int R = 8;
-    const long warps = (static_cast<long>(N) + R - 1) / R;
-    const unsigned grid = static_cast<unsigned>((warps + WPB - 1) / WPB);
-    launch_dependent(skinny_linear_kernel<bf16, R, BC, 2>, grid, WPB * 32, 0, stream,
-        in, ld_in, static_cast<const bf16*>(W), bias, add, ld_add, out, ld_out, B, N, K, act_out);
-  }
-  return after_launch("skinny_linear_kernel");
 }
 
 int launch_sinusoidal(const float* t, float* out, int B, int dim, cudaStream_t stream) {

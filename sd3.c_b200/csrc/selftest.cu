@@ -11,8 +11,6 @@
 #include "ptx.cuh"
 
 namespace sd3 {
-int* device_status_word();
-
 namespace {
 
 __global__ void __launch_bounds__(64, 1) wait_timeout_kernel(int* status, unsigned long long limit_ns) {
