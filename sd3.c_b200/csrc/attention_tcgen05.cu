@@ -64,7 +64,7 @@ namespace sd3 {
 int device_sm_count();
 int encode_tmap_3d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t d0, uint64_t d1,
                    uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0,
-                   uint32_t box1, uint32_t box2, int swizzle_bytes = 128);
+                   uint32_t box1, uint32_t box2);
 
 namespace {
 

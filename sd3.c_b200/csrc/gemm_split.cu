@@ -5,30 +5,35 @@
 //   a w  =  ah wh + (ah wm + am wh) + (am wm + ah wl + al wh)
 //
 // is formed by six bf16 MMAs with fp32 accumulation.  The three products left
-// out (am wl, al wm, al wl) are below 2^-25 of |a w|, under the rounding of an
-// fp32 product.
+// out (am wl, al wm, al wl) are together at most 2^-24 of |a w|, the rounding of
+// one fp32 product.
 //
 //   acc[m, n] = sum_k A[m, k] * W[n, k]     A: 3 planes of (M, K), W: 3 planes of (N, K)
 //
 // The tensor core's accumulation does not round to nearest, so a sum over all of
 // K in TMEM would drift (one-sided) by more than a chain of FFMAs does.  Each
-// 32-wide K block therefore gets a TMEM accumulator of its own, in which the
-// small products are added first and the two ah wh steps last; the epilogue
-// warps fetch it and add it to fp32 registers (round to nearest, K / 32
+// 64-wide K block therefore gets a TMEM accumulator of its own, in which the
+// small products are added first and the four ah wh steps last; the epilogue
+// warps fetch it and add it to fp32 registers (round to nearest, K / 64
 // additions instead of K).  Measured against 64-bit sums the result is closer
 // than the FFMA kernel's.
 //
-// One CTA per SM walks 128 x BN tiles (persistent): warp 0 streams the planes
-// with TMA (3-D boxes of 32 K x rows x 3 planes, 64-byte swizzle), one thread of
-// warp 1 issues 12 MMAs per K block, the epilogue warps add up the blocks and
-// run the fused epilogue.  The TMEM accumulators rotate (512 / BN of them, at
-// most four), so the adds run under the MMAs of the following blocks.
-// What bounds it: the tensor pipe (six MMAs per K step); a 32-wide K block of a
-// 128 x 256 tile is 1536 cycles of MMA for 72 KiB of operands.
+// Two CTAs (a cluster on neighbouring SMs) share a 256 x PBN tile with
+// tcgen05.mma.cta_group::2 and walk tiles persistently: each CTA's warp 0 streams the
+// planes of its 128 rows of A and its half of W with TMA (3-D boxes of 64 K x rows
+// x 3 planes), two threads of the even CTA issue the 24 MMAs of every K block (blocks in turn: a
+// block has its own accumulator, so the threads need no order between them and the
+// barrier work of one runs under the MMAs of the other), the epilogue warps of both add
+// up the blocks and run the fused epilogue.  The accumulators rotate (512 / PBN of them,
+// at most four), so the adds run under the MMAs of the following blocks.
 //
-// Measured against the FFMA kernel it replaced in the fp32 models: one dual block of 256 + 77
-// tokens 4.74 -> 2.79 ms, the 24-block model at 512 x 512 (1024 + 333 tokens) 754 -> 668 ms, all
-// of the difference in the GEMMs.
+// What bounds it: the tensor pipe (six MMAs per K step) and the operand loads: a K
+// block of a 256 x 256 tile is 3072 cycles of MMA for 96 KiB per CTA, of a 256 x 128
+// tile 1536 for 72 KiB.  A one-CTA version with 128 x 256 tiles and 32-wide K blocks
+// (64-byte rows, half of W's bytes more per MMA) kept the tensor pipe 38 % busy.
+//
+// Measured, 24-block model at 512 x 512 (1024 + 333 tokens): 19.26 (one-CTA tiles) -> 17.57 ms; the FFMA
+// kernel and the SIMT attention took 754 ms.  One dual block of 256 + 77 tokens 454 -> 411 us.
 #include <cuda.h>
 #include <mutex>
 
@@ -40,8 +45,7 @@
 namespace sd3 {
 
 int encode_tmap_3d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t d0, uint64_t d1, uint64_t d2,
-                   uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2,
-                   int swizzle_bytes = 128);
+                   uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2);
 int device_sm_count();
 
 namespace {
@@ -51,34 +55,24 @@ using gemm_detail::map_row;
 using gemm_detail::RowMap;
 using gemm_detail::st_global_32B;
 
-constexpr int S_BM = 128;
-constexpr int S_KB = 32;               // K elements per block (64-byte rows)
-constexpr int S_KBYTES = 2 * S_KB;
-constexpr int S_A_PLANE = S_BM * S_KBYTES;  // 8 KiB
+constexpr int S_BM = 128;              // rows of A per CTA (256 per pair)
+constexpr int S_KB = 64;               // K elements per block (128-byte rows)
+constexpr int S_A_PLANE = S_BM * 128;  // 16 KiB
 
-template <int BN>
+template <int PBN>
 struct SplitCfg {
-  static constexpr int W_PLANE = BN * S_KBYTES;
-  static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);       // 72 / 48 / 36 KiB
-  static constexpr int STAGES = BN == 256 ? 3 : (BN == 128 ? 4 : 6);  // 216 / 192 / 216 KiB
-  static constexpr int NBUF = BN == 256 ? 2 : 4;                      // TMEM accumulators
-  static constexpr int TMEM_COLS = NBUF * BN;
-  static constexpr int EPI_WARPS = BN == 64 ? 4 : 8;
-  static constexpr int CPW = BN == 256 ? 128 : 64;  // accumulator columns per epilogue thread
-  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int W_ROWS = PBN / 2;  // rows of W per CTA
+  static constexpr int W_PLANE = W_ROWS * 128;
+  static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);  // 96 / 72 / 60 KiB
+  static constexpr int STAGES = PBN == 256 ? 2 : 3;              // 192 / 216 / 180 KiB
+  static constexpr int NBUF = PBN == 256 ? 2 : 4;                // TMEM accumulators
+  static constexpr int TMEM_COLS = NBUF * PBN;
+  static constexpr int EPI_WARPS = PBN == 64 ? 4 : 8;
+  static constexpr int CPW = PBN == 256 ? 128 : 64;  // accumulator columns per epilogue thread
+  static constexpr int MMA2_WARP = 2 + EPI_WARPS;    // second MMA-issuing warp
+  static constexpr int THREADS = 32 * (3 + EPI_WARPS);
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
 };
-
-// K-major operand, 64-byte swizzle: rows of 64 B, groups of eight rows 512 B apart
-__device__ __forceinline__ uint64_t make_smem_desc_sw64(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
-  d |= static_cast<uint64_t>(1) << 16;
-  d |= static_cast<uint64_t>(512 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(4) << 61;
-  return d;
-}
 
 __device__ __forceinline__ float gelu_tanh_exact(float x) {
   const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
@@ -216,13 +210,13 @@ struct SplitProblem {
   GemmArgs g;
 };
 
-template <int BN, int EPI, int OUT>
-__global__ void __launch_bounds__(SplitCfg<BN>::THREADS, 1)
+template <int PBN, int EPI, int OUT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SplitCfg<PBN>::THREADS, 1)
 gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_constant__ SplitProblem p1,
                           const int tiles0, const int tiles1) {
-  using Cfg = SplitCfg<BN>;
+  using Cfg = SplitCfg<PBN>;
   constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, CPW = Cfg::CPW;
-  constexpr uint32_t IDESC = make_idesc(1, 1, S_BM, BN, 0, 0);
+  constexpr uint32_t IDESC = make_idesc(1, 1, 2 * S_BM, PBN, 0, 0);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -236,15 +230,18 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();  // 0 = leader
+  const int pair = blockIdx.x >> 1;
+  const int num_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      mbar_init(&full_bar[s], 1);   // leader's expect_tx arrival; bytes of both CTAs
+      mbar_init(&empty_bar[s], 1);  // one multicast commit per use
     }
     for (int a = 0; a < NBUF; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], Cfg::EPI_WARPS);
+      mbar_init(&tempty_bar[a], 2 * Cfg::EPI_WARPS);  // epilogue warps of both CTAs (leader's copy is used)
     }
     *s_abort = 0;
     fence_barrier_init();
@@ -256,80 +253,90 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     }
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
+    tmem_relinquish_pair();
   }
   tc_fence_before_sync();
   __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers are initialised before any remote signal
   tc_fence_after_sync();
   grid_dep_wait();
   grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
-  const int num_tiles = tiles0 + tiles1;
-  const int KB = p0.g.k_blocks;  // the same K for both problems
+  const int num_tiles = tiles0 + tiles1;  // tiles of 256 x PBN: the first problem's, then the second's
+  const int KB = p0.g.k_blocks;           // the same K for both problems
 
   if (warp == 0 && lane == 0) {
-    // ------------------------------ TMA producer ------------------------------
+    // ------------------------------ TMA producer (both CTAs) ------------------
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const bool second = tile >= tiles0;
       const SplitProblem& pp = second ? p1 : p0;
       const int lt = second ? tile - tiles0 : tile;
-      const int m0 = (lt / pp.g.tiles_n) * S_BM, n0 = (lt % pp.g.tiles_n) * BN;
+      const int m0 = (lt / pp.g.tiles_n) * (2 * S_BM) + static_cast<int>(rank) * S_BM;
+      const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS;
       for (int kb = 0; kb < KB; ++kb) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
         uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
-        mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
-        tma_load_3d(sa, &pp.tmA, &full_bar[stage], kb * S_KB, m0, 0);
-        tma_load_3d(sa + 3 * S_A_PLANE, &pp.tmW, &full_bar[stage], kb * S_KB, n0, 0);
+        // all bytes of the stage (both CTAs) are credited to the leader's barrier
+        const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+        if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
+        tma_load_3d_pair(sa, &pp.tmA, bar, kb * S_KB, m0, 0);
+        tma_load_3d_pair(sa + 3 * S_A_PLANE, &pp.tmW, bar, kb * S_KB, n0, 0);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ------------------------------ MMA issuer --------------------------------
-    int stage = 0, buf = 0;
-    uint32_t phase = 0, bphase = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      for (int kb = 0; kb < KB; ++kb) {
-        if (!mbar_wait(&tempty_bar[buf], bphase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-        if (!mbar_wait(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BN);
-        const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
-        const uint64_t a0 = make_smem_desc_sw64(a_addr);
-        const uint64_t w0 = make_smem_desc_sw64(a_addr + 3 * S_A_PLANE);
-        constexpr uint64_t AP = S_A_PLANE >> 4, WP = Cfg::W_PLANE >> 4;
-        // (A plane, W plane), smallest products first
-        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
+  } else if ((warp == 1 || warp == Cfg::MMA2_WARP) && lane == 0) {
+    // ------------------------------ MMA issuers (leader only) -----------------
+    if (rank == 0) {
+      const int me = warp == 1 ? 0 : 1;
+      int stage = 0, buf = 0, turn = 0;
+      uint32_t phase = 0, bphase = 0;
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+        for (int kb = 0; kb < KB; ++kb) {
+          if (turn == me) {
+            if (!mbar_wait(&tempty_bar[buf], bphase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+            if (!mbar_wait(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * PBN);
+            const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+            const uint64_t a0 = make_smem_desc_sw128(a_addr, 16, 1024);
+            const uint64_t w0 = make_smem_desc_sw128(a_addr + 3 * S_A_PLANE, 16, 1024);
+            constexpr uint64_t AP = S_A_PLANE >> 4, WP = Cfg::W_PLANE >> 4;
+            // (A plane, W plane), smallest products first
+            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-        for (int q = 0; q < 6; ++q)
+            for (int q = 0; q < 6; ++q)
 #pragma unroll
-          for (int k = 0; k < 2; ++k)
-            mma_f16_ss(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
-        mma_commit(&empty_bar[stage]);
-        mma_commit(&tfull_bar[buf]);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        if (++buf == NBUF) { buf = 0; bphase ^= 1; }
+              for (int k = 0; k < S_KB / 16; ++k)
+                mma_f16_ss_pair(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
+            mma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+            mma_commit_pair(&tfull_bar[buf], 3);    // block sum ready in both CTAs
+          }
+          turn ^= 1;
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++buf == NBUF) { buf = 0; bphase ^= 1; }
+        }
       }
     }
-  } else if (warp >= 2) {
-    // ------------------------------ accumulation + epilogue -------------------
+  } else if (warp >= 2 && warp < 2 + Cfg::EPI_WARPS) {
+    // ------------------------------ accumulation + epilogue (both CTAs) -------
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
-    const int row = quad * 32 + lane;
+    const int row = static_cast<int>(rank) * S_BM + quad * 32 + lane;
     int buf = 0;
     uint32_t bphase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       const bool second = tile >= tiles0;
       const GemmArgs& g = second ? p1.g : p0.g;
       const int lt = second ? tile - tiles0 : tile;
-      const int m = (lt / g.tiles_n) * S_BM + row;
-      const int n0 = (lt % g.tiles_n) * BN + half * CPW;
+      const int m = (lt / g.tiles_n) * (2 * S_BM) + row;
+      const int n0 = (lt % g.tiles_n) * PBN + half * CPW;
       float acc[CPW];
 #pragma unroll
       for (int j = 0; j < CPW; ++j) acc[j] = 0.f;
@@ -337,7 +344,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
         if (!mbar_wait_warp(&tfull_bar[buf], bphase, wc, DEV_TIMEOUT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
-                               static_cast<uint32_t>(buf * BN + half * CPW);
+                               static_cast<uint32_t>(buf * PBN + half * CPW);
 #pragma unroll
         for (int s = 0; s < CPW / 32; ++s) {
           uint32_t r[32];
@@ -346,7 +353,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
           if (s == CPW / 32 - 1) {  // everything is in registers: the accumulator may be reused
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), 0));
           }
 #pragma unroll
           for (int j = 0; j < 32; ++j) acc[s * 32 + j] += __uint_as_float(r[j]);
@@ -367,16 +374,17 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   tc_fence_before_sync();
   __syncthreads();
   if (*s_abort) drain_after_abort();
+  cluster_sync_all();  // no remote arrival or multicast commit may target an exited CTA
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
   }
 }
 
-template <int BN, int EPI, int OUT>
+template <int PBN, int EPI, int OUT>
 int launch_split_inst(const SplitProblem& p0, const SplitProblem& p1, int tiles0, int tiles1, cudaStream_t stream) {
-  using Cfg = SplitCfg<BN>;
-  auto kern = gemm_split_tcgen05_kernel<BN, EPI, OUT>;
+  using Cfg = SplitCfg<PBN>;
+  auto kern = gemm_split_tcgen05_kernel<PBN, EPI, OUT>;
   static std::mutex attr_mutex;
   static bool attr_done[64] = {false};
   int dev = 0;
@@ -389,8 +397,8 @@ int launch_split_inst(const SplitProblem& p0, const SplitProblem& p1, int tiles0
       attr_done[dev] = true;
     }
   }
-  const int tiles = tiles0 + tiles1, sms = device_sm_count();
-  launch_dependent(kern, tiles < sms ? tiles : sms, Cfg::THREADS, Cfg::SMEM_BYTES, stream, p0, p1, tiles0, tiles1);
+  const int tiles = tiles0 + tiles1, most = device_sm_count() / 2;
+  launch_dependent(kern, 2 * (tiles < most ? tiles : most), Cfg::THREADS, Cfg::SMEM_BYTES, stream, p0, p1, tiles0, tiles1);
   return after_launch("gemm_split_tcgen05_kernel");
 }
 
@@ -437,7 +445,7 @@ int build_split(SplitProblem* pp, const SplitGemmProblem& q, int N, int K, int b
   GemmArgs& g = pp->g;
   g.M = q.M; g.N = N; g.K = K;
   g.k_blocks = (K + S_KB - 1) / S_KB;
-  g.tiles_m = (q.M + S_BM - 1) / S_BM;
+  g.tiles_m = (q.M + 2 * S_BM - 1) / (2 * S_BM);
   g.tiles_n = (N + bn - 1) / bn;
   g.epi = q.epi;
   g.status = dev_status;
@@ -445,23 +453,21 @@ int build_split(SplitProblem* pp, const SplitGemmProblem& q, int N, int K, int b
   const long esz = q.epi.out_plane > 0 ? 2 : 4;
   g.wide_store = (q.epi.ldo * esz) % 32 == 0 && (q.epi.out_plane * 2) % 32 == 0 &&
                  (reinterpret_cast<uintptr_t>(q.epi.out) & 31) == 0;
-  int rc = encode_tmap_3d(&pp->tmA, q.A, 2, K, q.M, 3, static_cast<uint64_t>(K) * 2, q.a_plane * 2, S_KB, S_BM, 3,
-                          S_KBYTES);
+  int rc = encode_tmap_3d(&pp->tmA, q.A, 2, K, q.M, 3, static_cast<uint64_t>(K) * 2, q.a_plane * 2, S_KB, S_BM, 3);
   if (rc) return rc;
-  return encode_tmap_3d(&pp->tmW, q.W, 2, K, N, 3, static_cast<uint64_t>(K) * 2, q.w_plane * 2, S_KB, bn, 3, S_KBYTES);
+  return encode_tmap_3d(&pp->tmW, q.W, 2, K, N, 3, static_cast<uint64_t>(K) * 2, q.w_plane * 2, S_KB, bn / 2, 3);
 }
 
-// The tile width with the least (waves over the SMs) x (time of a K block of a tile).  A K block
-// is 12 MMAs of 128 / 64 cycles at BN = 256 / 128 and of about 50 at BN = 64 (an MMA is issue-bound
-// below 64 columns' worth of math).
-int choose_split_width(long rows_tiles, int N) {
-  const long sms = device_sm_count();
+// The tile width with the least (waves over the CTA pairs) x (time of a K block of a tile).  The
+// costs are in units of 24 cycles: 24 MMAs of 128 / 64 cycles, and at PBN = 64 the 480 rows of TMA per CTA.
+int choose_split_width(long row_tiles, int N) {
+  const long pairs = device_sm_count() / 2 > 0 ? device_sm_count() / 2 : 1;
   int best = 256;
   long best_cost = 0;
-  const int bn[3] = {256, 128, 64}, cost[3] = {128, 66, 50};
+  const int bn[3] = {256, 128, 64}, cost[3] = {128, 68, 52};
   for (int i = 0; i < 3; ++i) {
-    const long tiles = rows_tiles * ((N + bn[i] - 1) / bn[i]);
-    const long c = (tiles + sms - 1) / sms * cost[i];
+    const long tiles = row_tiles * ((N + bn[i] - 1) / bn[i]);
+    const long c = (tiles + pairs - 1) / pairs * cost[i];
     if (i == 0 || c < best_cost) { best = bn[i]; best_cost = c; }
   }
   return best;
@@ -481,7 +487,7 @@ int launch_gemm_split(const SplitGemmProblem& a, const SplitGemmProblem* b, int 
       return ST_INVALID_ARG;
     }
   }
-  const int bn = choose_split_width((a.M + S_BM - 1) / S_BM + (b ? (b->M + S_BM - 1) / S_BM : 0), N);
+  const int bn = choose_split_width((a.M + 255) / 256 + (b ? (b->M + 255) / 256 : 0), N);
   SplitProblem p0, p1;
   rc = build_split(&p0, a, N, K, bn, dev_status);
   if (rc) return rc;

@@ -217,7 +217,7 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
 
 }  // namespace
 
-// 2-D / 3-D tiled tensor maps with 128-byte (3-D: or 64-byte) swizzle, also used by attention.
+// 2-D / 3-D tiled tensor maps with 128-byte swizzle (also used by attention).
 int encode_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t inner,
                    uint64_t outer, uint64_t ld_bytes, uint32_t box_inner, uint32_t box_outer) {
   auto fn = get_encode_fn();
@@ -246,7 +246,7 @@ int encode_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t 
 
 int encode_tmap_3d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t d0, uint64_t d1,
                    uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0,
-                   uint32_t box1, uint32_t box2, int swizzle_bytes) {
+                   uint32_t box1, uint32_t box2) {
   auto fn = get_encode_fn();
   if (!fn) {
     set_last_error("cuTensorMapEncodeTiled entry point not available");
@@ -259,7 +259,7 @@ int encode_tmap_3d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t 
   CUtensorMapDataType dt =
       elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   CUresult r = fn(map, dt, 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_last_error("cuTensorMapEncodeTiled(3d) failed: %d", (int)r);
