@@ -175,7 +175,7 @@ int sd3_linear_pair(const void* x0, const void* w0, const float* bias0, void* ou
     p[i].epi.out_f32 = out_dtype == SD3_DTYPE_F32;
     p[i].epi.ldo = N;
   }
-  return launch_gemm_grouped(p[0], p[1], OPERAND_BF16, N, K, device_status_word(), S(stream));
+  return launch_gemm_grouped(p, 2, OPERAND_BF16, N, K, device_status_word(), S(stream));
 }
 
 int sd3_linear_gate_residual_pair(const void* x0, const void* w0, const float* bias0, const float* gate0,
@@ -209,7 +209,7 @@ int sd3_linear_gate_residual_pair(const void* x0, const void* w0, const float* b
     e.rows_out = rps[i];
     e.row_off = 0;
   }
-  return launch_gemm_grouped(p[0], p[1], OPERAND_BF16, N, K, device_status_word(), S(stream));
+  return launch_gemm_grouped(p, 2, OPERAND_BF16, N, K, device_status_word(), S(stream));
 }
 
 int sd3_qkv_project(const void* x, const void* w, const float* bias, const float* wq,

@@ -11,10 +11,11 @@
 //
 // Per block the launch sequence is
 //   LN+modulate(x), LN+modulate(c) in one launch (both modulations of a dual block at once)
-//   QKV GEMM(c), QKV GEMM(x)  -> packed (B, Tc+Tx, 3E), RMSNorm fused, context rows first
+//   QKV GEMM(x), (c)         -> packed (B, Tc+Tx, 3E), RMSNorm fused, context rows first; a dual block's
+//                               second QKV GEMM(x) rides in the same launch
 //   joint attention           -> o_c, o_x
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
-//   [dual] QKV GEMM(x2), attention over image tokens, out-proj GEMM with gate2
+//   [dual] attention over image tokens, out-proj GEMM with gate2
 //   LN+modulate(x), (c); MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual), each for x and c at once
 #include <math.h>
 #include <algorithm>
@@ -324,7 +325,10 @@ int run_linear(sd3_model* m, const Linear& L, const void* A, int M, const GemmEp
   }
   GemmEpilogue ee = e;
   if (!ee.bias) ee.bias = L.b;
-  if (m->f32) return launch_gemm_split(split_problem(L, A, M, ee), nullptr, L.N, L.K, m->status, st);
+  if (m->f32) {
+    const SplitGemmProblem p = split_problem(L, A, M, ee);
+    return launch_gemm_split(&p, 1, L.N, L.K, m->status, st);
+  }
   if (m->fp8 && L.w8) {
     // e4m3 x e4m3: the bf16 operand is converted as is (scale 1: LayerNorm
     // outputs, attention outputs and GELU outputs sit well inside e4m3's range and
@@ -345,29 +349,52 @@ int run_linear(sd3_model* m, const Linear& L, const void* A, int M, const GemmEp
   return launch_gemm(A, L.K, L.w, L.K, OPERAND_BF16, M, L.N, L.K, ee, m->status, st);
 }
 
-// Two linears of the same shape class (the image-stream GEMM and its context-stream twin) as
-// one grouped launch where the tensor-core path takes both; otherwise one after the other.
+struct LinearCall {
+  const Linear* L = nullptr;
+  const void* A = nullptr;
+  int M = 0;
+  GemmEpilogue epi;
+  bool a_e4m3 = false;
+};
+
+// One to three linears of the same shape class (the image-stream GEMM, its context-stream twin, the
+// second QKV projection of a dual block) as one grouped launch where the tensor-core path takes
+// them; otherwise one after the other.
+int run_linear_group(sd3_model* m, const LinearCall* c, int n, cudaStream_t st) {
+  const int N = c[0].L->N, K = c[0].L->K;
+  bool same = true, all8 = true, none8 = true;
+  for (int i = 0; i < n; ++i) {
+    const Linear& L = *c[i].L;
+    same = same && L.w && L.N == N && L.K == K;
+    all8 = all8 && m->fp8 && L.w8 && c[i].a_e4m3;
+    none8 = none8 && !(m->fp8 && L.w8) && !c[i].a_e4m3;
+  }
+  if (m->f32 && same) {
+    SplitGemmProblem p[3];
+    for (int i = 0; i < n; ++i) p[i] = split_problem(*c[i].L, c[i].A, c[i].M, c[i].epi);
+    return launch_gemm_split(p, n, N, K, m->status, st);
+  }
+  if (m->f32 || !same || !(all8 || none8)) {
+    for (int i = 0; i < n; ++i) {
+      int rc = run_linear(m, *c[i].L, c[i].A, c[i].M, c[i].epi, st, c[i].a_e4m3);
+      if (rc) return rc;
+    }
+    return ST_OK;
+  }
+  GemmProblem p[3];
+  for (int i = 0; i < n; ++i) {
+    const Linear& L = *c[i].L;
+    p[i].A = c[i].A; p[i].lda = K; p[i].W = all8 ? L.w8 : L.w; p[i].ldw = K; p[i].M = c[i].M; p[i].epi = c[i].epi;
+    if (!p[i].epi.bias) p[i].epi.bias = L.b;
+    if (all8) p[i].epi.alpha = L.wscale;
+  }
+  return launch_gemm_grouped(p, n, all8 ? OPERAND_E4M3 : OPERAND_BF16, N, K, m->status, st);
+}
+
 int run_linear_pair(sd3_model* m, const Linear& La, const void* Aa, int Ma, const GemmEpilogue& ea, bool a8a,
                     const Linear& Lb, const void* Ab, int Mb, const GemmEpilogue& eb, bool a8b, cudaStream_t st) {
-  const bool fp8a = m->fp8 && La.w8 && a8a, fp8b = m->fp8 && Lb.w8 && a8b;
-  const bool plain_a = !(m->fp8 && La.w8) && !a8a, plain_b = !(m->fp8 && Lb.w8) && !a8b;
-  const bool same_kind = (fp8a && fp8b) || (plain_a && plain_b);
-  if (m->f32 && La.w && Lb.w && La.N == Lb.N && La.K == Lb.K) {
-    const SplitGemmProblem b = split_problem(Lb, Ab, Mb, eb);
-    return launch_gemm_split(split_problem(La, Aa, Ma, ea), &b, La.N, La.K, m->status, st);
-  }
-  if (m->f32 || !La.w || !Lb.w || La.N != Lb.N || La.K != Lb.K || !same_kind) {
-    int rc = run_linear(m, La, Aa, Ma, ea, st, a8a);
-    if (rc) return rc;
-    return run_linear(m, Lb, Ab, Mb, eb, st, a8b);
-  }
-  GemmProblem pa, pb;
-  pa.A = Aa; pa.lda = La.K; pa.W = fp8a ? La.w8 : La.w; pa.ldw = La.K; pa.M = Ma; pa.epi = ea;
-  pb.A = Ab; pb.lda = Lb.K; pb.W = fp8b ? Lb.w8 : Lb.w; pb.ldw = Lb.K; pb.M = Mb; pb.epi = eb;
-  if (!pa.epi.bias) pa.epi.bias = La.b;
-  if (!pb.epi.bias) pb.epi.bias = Lb.b;
-  if (fp8a) { pa.epi.alpha = La.wscale; pb.epi.alpha = Lb.wscale; }
-  return launch_gemm_grouped(pa, pb, fp8a ? OPERAND_E4M3 : OPERAND_BF16, La.N, La.K, m->status, st);
+  const LinearCall c[2] = {{&La, Aa, Ma, ea, a8a}, {&Lb, Ab, Mb, eb, a8b}};
+  return run_linear_group(m, c, 2, st);
 }
 
 GemmEpilogue qkv_epilogue(sd3_model* m, void* qkv, int B, int T_in, int T_total, int row_off, const float* wq,
@@ -517,9 +544,15 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const bool pre_j = L.c_wq_s != nullptr && L.x_wq_s != nullptr;
   const float* c_wq = pre_j ? L.c_wq_s : L.c_wq;
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
+  const bool pre_d = L.d_wq_s != nullptr;
+  const float* d_wq = pre_d ? L.d_wq_s : L.d_wq;
   if (m->D == 64) {
-    SD3_TRY(run_linear_pair(m, L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk), x8a,
-                            L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, B, Tc, T, 0, c_wq, L.c_wk), c8a, st));
+    // the image rows' two projections (a dual block's second one included) and the context rows'
+    const LinearCall qkv[3] = {
+        {&L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk), x8a},
+        {&L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, B, Tc, T, 0, c_wq, L.c_wk), c8a},
+        {&L.d_qkv, w.h_x2, B * Tx, qkv_epilogue(m, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk), x8a}};
+    SD3_TRY(run_linear_group(m, qkv, L.dual ? 3 : 2, st));
   } else {
     SD3_TRY(run_qkv(m, L.c_qkv, w.h_c, w.qkv, B, Tc, T, 0, c_wq, L.c_wk, st, c8a));
     SD3_TRY(run_qkv(m, L.x_qkv, w.h_x, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk, st, x8a));
@@ -536,8 +569,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     SD3_TRY(run_gate_resid(m, L.x_out, w.o_x, B, Tx, x_gate_a, ms, x, st, o8));
   }
   if (L.dual) {
-    const bool pre_d = L.d_wq_s != nullptr;
-    SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, pre_d ? L.d_wq_s : L.d_wq, L.d_wk, st, x8a));
+    if (m->D != 64) SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
     const bool o8d = m->fp8 && m->D == 64 && L.d_out.w8;
     SD3_TRY(run_attention(m, w.qkv2, B, Tx, 0, nullptr, w.o_x2, st, o8d, L.dual_bound, pre_d));
     SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));

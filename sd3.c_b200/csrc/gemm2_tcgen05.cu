@@ -1,11 +1,13 @@
 // CTA-pair variant of the tcgen05 GEMM: two CTAs (a cluster of two on
 // neighbouring SMs) cooperate on 256 x 256 (or, for problems of less than half a
 // wave of those, 256 x 128) output tiles with
-// tcgen05.mma.cta_group::2.  One launch can carry TWO problems of the same
-// shape class (same N, K and epilogue: the image-stream GEMM of a block and its
-// small context-stream twin); the persistent tile loop runs the first problem's
-// tiles and then the second's, so the small one rides in the tail of the large
-// one instead of being a launch of its own that fills less than a wave.
+// tcgen05.mma.cta_group::2.  One launch can carry up to THREE problems of the same
+// shape class (same N, K and epilogue: the image-stream GEMM of a block, its
+// small context-stream twin and, for QKV, the second projection of a dual block);
+// the persistent tile loop runs one problem's tiles after the other's, so the small
+// ones ride in the tail of the large one instead of being launches of their own
+// that fill less than a wave (the third problem: forward of one 256x256 image 3284 -> 3133 us, 512x512
+// 4467 -> 4407 us, 1024x1024 unchanged).
 //
 //   acc[m, n] = sum_k A[m, k] * W[n, k]        A: (M, K) K-major, W: (N, K) K-major
 //
@@ -77,7 +79,8 @@ struct PairProblem {
 template <int EPI, bool OUT_F32, bool FP8, int PBN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_constant__ PairProblem p1,
-                         const int tiles0, const int tiles1) {
+                         const __grid_constant__ PairProblem p2, const int end0, const int end1,
+                         const int num_tiles) {
   // M = 256 across the pair; operands bf16, or e4m3 (128 K-elements per 128-byte stage row,
   // 32 per instruction: the byte arithmetic of the stages is the same)
   constexpr uint32_t IDESC = FP8 ? make_idesc(0, 0, 2 * P_BM, PBN, 0, 0) : make_idesc(1, 1, 2 * P_BM, PBN, 0, 0);
@@ -118,9 +121,13 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     fence_barrier_init();
     prefetch_tmap(&p0.tmA);
     prefetch_tmap(&p0.tmW);
-    if (tiles1 > 0) {
+    if (end1 > end0) {
       prefetch_tmap(&p1.tmA);
       prefetch_tmap(&p1.tmW);
+    }
+    if (num_tiles > end1) {
+      prefetch_tmap(&p2.tmA);
+      prefetch_tmap(&p2.tmW);
     }
   }
   if (warp == 1) {
@@ -136,9 +143,9 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
 
-  const int num_tiles = tiles0 + tiles1;  // tiles of 256 x PBN: the first problem's, then the second's
+  // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
   constexpr int NSLOT = P_STAGES / 2;     // slots of two stages
-  const int KB = p0.g.k_blocks;        // the same K for both problems
+  const int KB = p0.g.k_blocks;        // the same K for all problems
   const int KS = (KB + 1) / 2;         // slots per tile (the last may hold one stage)
 
   if (warp == 0 && lane == 0) {
@@ -147,9 +154,8 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-      const bool second = tile >= tiles0;
-      const PairProblem& pp = second ? p1 : p0;
-      const int lt = second ? tile - tiles0 : tile;
+      const PairProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
+      const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
       const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF;
       for (int ks = 0; ks < KS; ++ks) {
@@ -240,10 +246,9 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
-      const bool second = tile >= tiles0;
-      const PairProblem& pp = second ? p1 : p0;
+      const PairProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
       const GemmArgs& g = pp.g;
-      const int lt = second ? tile - tiles0 : tile;
+      const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / g.tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
       const int n0 = (lt % g.tiles_n) * PBN;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
@@ -281,7 +286,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
 }
 
 template <int EPI, bool OUT_F32, bool FP8, int PBN>
-int launch_pair_inst(const PairProblem& p0, const PairProblem& p1, int tiles0, int tiles1, cudaStream_t stream) {
+int launch_pair_inst(const PairProblem* p, const int* end, cudaStream_t stream) {
   auto kern = gemm_pair_tcgen05_kernel<EPI, OUT_F32, FP8, PBN>;
   constexpr int SMEM = pair_smem_bytes(EPI, OUT_F32, PBN);
   static std::mutex attr_mutex;
@@ -296,23 +301,22 @@ int launch_pair_inst(const PairProblem& p0, const PairProblem& p1, int tiles0, i
       attr_done[dev] = true;
     }
   }
-  const int tiles = tiles0 + tiles1;
+  const int tiles = end[2];
   const int max_pairs = device_sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_dependent(kern, 2 * pairs, P_THREADS, SMEM, stream, p0, p1, tiles0, tiles1);
+  launch_dependent(kern, 2 * pairs, P_THREADS, SMEM, stream, p[0], p[1], p[2], end[0], end[1], tiles);
   return after_launch("gemm_pair_tcgen05_kernel");
 }
 
 // the block GEMM epilogues exist for both tile widths, the others for 256 only
 template <int EPI, bool OUT_F32, bool FP8>
-int launch_pair_width(int pbn, const PairProblem& p0, const PairProblem& p1, int tiles0, int tiles1,
-                      cudaStream_t stream) {
+int launch_pair_width(int pbn, const PairProblem* p, const int* end, cudaStream_t stream) {
   constexpr bool narrow_built = (EPI == EPI_GATE_RESID && OUT_F32) ||
                                 (!OUT_F32 && (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_QKV_NORM));
   if constexpr (narrow_built) {
-    if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p0, p1, tiles0, tiles1, stream);
+    if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p, end, stream);
   }
-  return launch_pair_inst<EPI, OUT_F32, FP8, 256>(p0, p1, tiles0, tiles1, stream);
+  return launch_pair_inst<EPI, OUT_F32, FP8, 256>(p, end, stream);
 }
 
 bool narrow_tiles_built(const GemmEpilogue& epi) {
@@ -400,35 +404,39 @@ bool gemm_pair_supported(int operand_dtype, int M, int N, int K, const GemmEpilo
   return operand_dtype == OPERAND_BF16;
 }
 
-// One or two problems (b may be null) of the same N, K, operand type and epilogue kind.
-int launch_gemm_pair(const GemmProblem& a, const GemmProblem* b, int operand_dtype, int N, int K,
-                     int* dev_status, cudaStream_t stream) {
+// One to three problems of the same N, K, operand type and epilogue kind.
+int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
+                     cudaStream_t stream) {
   const bool fp8 = operand_dtype == OPERAND_E4M3;
-  if (b && (b->epi.mode != a.epi.mode || b->epi.out_f32 != a.epi.out_f32)) {
-    set_last_error("gemm_pair: grouped problems need the same epilogue kind");
-    return ST_INVALID_ARG;
+  const GemmProblem& a = q[0];
+  long tiles256 = 0;
+  for (int i = 0; i < n; ++i) {
+    if (q[i].epi.mode != a.epi.mode || q[i].epi.out_f32 != a.epi.out_f32) {
+      set_last_error("gemm_pair: grouped problems need the same epilogue kind");
+      return ST_INVALID_ARG;
+    }
+    tiles256 += static_cast<long>((q[i].M + 255) / 256) * (N / 256);
   }
-  const long tiles256 = static_cast<long>((a.M + 255) / 256 + (b ? (b->M + 255) / 256 : 0)) * (N / 256);
   const int pbn = choose_tile_width(tiles256, a.epi);
-  PairProblem p0, p1;
-  int rc = build_problem(&p0, a, operand_dtype, N, K, pbn, dev_status);
-  if (rc) return rc;
-  int tiles1 = 0;
-  if (b) {
-    rc = build_problem(&p1, *b, operand_dtype, N, K, pbn, dev_status);
-    if (rc) return rc;
-    tiles1 = p1.g.tiles_m * p1.g.tiles_n;
-  } else {
-    p1 = p0;
+  PairProblem p[3];
+  int end[3] = {0, 0, 0}, tiles = 0;
+  for (int i = 0; i < 3; ++i) {
+    if (i < n) {
+      int rc = build_problem(&p[i], q[i], operand_dtype, N, K, pbn, dev_status);
+      if (rc) return rc;
+      tiles += p[i].g.tiles_m * p[i].g.tiles_n;
+    } else {
+      p[i] = p[0];  // no tiles
+    }
+    end[i] = tiles;
   }
-  const int tiles0 = p0.g.tiles_m * p0.g.tiles_n;
   const bool f32 = a.epi.out_f32 != 0;
   if (fp8) {
     switch (a.epi.mode) {
-      case EPI_BIAS: return launch_pair_width<EPI_BIAS, false, true>(pbn, p0, p1, tiles0, tiles1, stream);
-      case EPI_BIAS_GELU: return launch_pair_width<EPI_BIAS_GELU, false, true>(pbn, p0, p1, tiles0, tiles1, stream);
-      case EPI_QKV_NORM: return launch_pair_width<EPI_QKV_NORM, false, true>(pbn, p0, p1, tiles0, tiles1, stream);
-      case EPI_GATE_RESID: return launch_pair_width<EPI_GATE_RESID, true, true>(pbn, p0, p1, tiles0, tiles1, stream);
+      case EPI_BIAS: return launch_pair_width<EPI_BIAS, false, true>(pbn, p, end, stream);
+      case EPI_BIAS_GELU: return launch_pair_width<EPI_BIAS_GELU, false, true>(pbn, p, end, stream);
+      case EPI_QKV_NORM: return launch_pair_width<EPI_QKV_NORM, false, true>(pbn, p, end, stream);
+      case EPI_GATE_RESID: return launch_pair_width<EPI_GATE_RESID, true, true>(pbn, p, end, stream);
       default: break;
     }
     set_last_error("gemm_pair: no e4m3 instantiation for epilogue mode %d", a.epi.mode);
@@ -436,20 +444,20 @@ int launch_gemm_pair(const GemmProblem& a, const GemmProblem* b, int operand_dty
   }
   switch (a.epi.mode) {
     case EPI_BIAS:
-      return f32 ? launch_pair_width<EPI_BIAS, true, false>(pbn, p0, p1, tiles0, tiles1, stream)
-                 : launch_pair_width<EPI_BIAS, false, false>(pbn, p0, p1, tiles0, tiles1, stream);
+      return f32 ? launch_pair_width<EPI_BIAS, true, false>(pbn, p, end, stream)
+                 : launch_pair_width<EPI_BIAS, false, false>(pbn, p, end, stream);
     case EPI_BIAS_GELU:
-      return f32 ? launch_pair_width<EPI_BIAS_GELU, true, false>(pbn, p0, p1, tiles0, tiles1, stream)
-                 : launch_pair_width<EPI_BIAS_GELU, false, false>(pbn, p0, p1, tiles0, tiles1, stream);
+      return f32 ? launch_pair_width<EPI_BIAS_GELU, true, false>(pbn, p, end, stream)
+                 : launch_pair_width<EPI_BIAS_GELU, false, false>(pbn, p, end, stream);
     case EPI_GATE_RESID:
       if (!f32) break;
-      return launch_pair_width<EPI_GATE_RESID, true, false>(pbn, p0, p1, tiles0, tiles1, stream);
+      return launch_pair_width<EPI_GATE_RESID, true, false>(pbn, p, end, stream);
     case EPI_QKV_NORM:
-      return f32 ? launch_pair_width<EPI_QKV_NORM, true, false>(pbn, p0, p1, tiles0, tiles1, stream)
-                 : launch_pair_width<EPI_QKV_NORM, false, false>(pbn, p0, p1, tiles0, tiles1, stream);
+      return f32 ? launch_pair_width<EPI_QKV_NORM, true, false>(pbn, p, end, stream)
+                 : launch_pair_width<EPI_QKV_NORM, false, false>(pbn, p, end, stream);
     case EPI_ADD_TABLE:
       if (!f32) break;
-      return launch_pair_width<EPI_ADD_TABLE, true, false>(pbn, p0, p1, tiles0, tiles1, stream);
+      return launch_pair_width<EPI_ADD_TABLE, true, false>(pbn, p, end, stream);
     default:
       break;
   }

@@ -213,7 +213,8 @@ struct SplitProblem {
 template <int PBN, int EPI, int OUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SplitCfg<PBN>::THREADS, 1)
 gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_constant__ SplitProblem p1,
-                          const int tiles0, const int tiles1) {
+                          const __grid_constant__ SplitProblem p2, const int end0, const int end1,
+                          const int num_tiles) {
   using Cfg = SplitCfg<PBN>;
   constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, CPW = Cfg::CPW;
   constexpr uint32_t IDESC = make_idesc(1, 1, 2 * S_BM, PBN, 0, 0);
@@ -247,9 +248,13 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     fence_barrier_init();
     prefetch_tmap(&p0.tmA);
     prefetch_tmap(&p0.tmW);
-    if (tiles1 > 0) {
+    if (end1 > end0) {
       prefetch_tmap(&p1.tmA);
       prefetch_tmap(&p1.tmW);
+    }
+    if (num_tiles > end1) {
+      prefetch_tmap(&p2.tmA);
+      prefetch_tmap(&p2.tmW);
     }
   }
   if (warp == 1) {
@@ -264,8 +269,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
-  const int num_tiles = tiles0 + tiles1;  // tiles of 256 x PBN: the first problem's, then the second's
-  const int KB = p0.g.k_blocks;           // the same K for both problems
+  // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
+  const int KB = p0.g.k_blocks;           // the same K for all problems
 
   if (warp == 0 && lane == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------
@@ -273,9 +278,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-      const bool second = tile >= tiles0;
-      const SplitProblem& pp = second ? p1 : p0;
-      const int lt = second ? tile - tiles0 : tile;
+      const SplitProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
+      const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * S_BM) + static_cast<int>(rank) * S_BM;
       const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS;
       for (int kb = 0; kb < KB; ++kb) {
@@ -332,9 +336,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     uint32_t bphase = 0;
     bool ok = true;
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
-      const bool second = tile >= tiles0;
-      const GemmArgs& g = second ? p1.g : p0.g;
-      const int lt = second ? tile - tiles0 : tile;
+      const GemmArgs& g = tile < end0 ? p0.g : tile < end1 ? p1.g : p2.g;
+      const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m = (lt / g.tiles_n) * (2 * S_BM) + row;
       const int n0 = (lt % g.tiles_n) * PBN + half * CPW;
       float acc[CPW];
@@ -382,7 +385,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
 }
 
 template <int PBN, int EPI, int OUT>
-int launch_split_inst(const SplitProblem& p0, const SplitProblem& p1, int tiles0, int tiles1, cudaStream_t stream) {
+int launch_split_inst(const SplitProblem* p, const int* end, cudaStream_t stream) {
   using Cfg = SplitCfg<PBN>;
   auto kern = gemm_split_tcgen05_kernel<PBN, EPI, OUT>;
   static std::mutex attr_mutex;
@@ -397,16 +400,17 @@ int launch_split_inst(const SplitProblem& p0, const SplitProblem& p1, int tiles0
       attr_done[dev] = true;
     }
   }
-  const int tiles = tiles0 + tiles1, most = device_sm_count() / 2;
-  launch_dependent(kern, 2 * (tiles < most ? tiles : most), Cfg::THREADS, Cfg::SMEM_BYTES, stream, p0, p1, tiles0, tiles1);
+  const int tiles = end[2], most = device_sm_count() / 2;
+  launch_dependent(kern, 2 * (tiles < most ? tiles : most), Cfg::THREADS, Cfg::SMEM_BYTES, stream,
+                   p[0], p[1], p[2], end[0], end[1], tiles);
   return after_launch("gemm_split_tcgen05_kernel");
 }
 
 template <int EPI, int OUT>
-int launch_split_width(int bn, const SplitProblem& p0, const SplitProblem& p1, int t0, int t1, cudaStream_t st) {
-  if (bn == 256) return launch_split_inst<256, EPI, OUT>(p0, p1, t0, t1, st);
-  if (bn == 128) return launch_split_inst<128, EPI, OUT>(p0, p1, t0, t1, st);
-  return launch_split_inst<64, EPI, OUT>(p0, p1, t0, t1, st);
+int launch_split_width(int bn, const SplitProblem* p, const int* end, cudaStream_t st) {
+  if (bn == 256) return launch_split_inst<256, EPI, OUT>(p, end, st);
+  if (bn == 128) return launch_split_inst<128, EPI, OUT>(p, end, st);
+  return launch_split_inst<64, EPI, OUT>(p, end, st);
 }
 
 int validate_split(const SplitGemmProblem& q, int N, int K) {
@@ -475,45 +479,50 @@ int choose_split_width(long row_tiles, int N) {
 
 }  // namespace
 
-int launch_gemm_split(const SplitGemmProblem& a, const SplitGemmProblem* b, int N, int K, int* dev_status,
-                      cudaStream_t stream) {
-  int rc = validate_split(a, N, K);
-  if (rc) return rc;
-  if (b) {
-    rc = validate_split(*b, N, K);
+int launch_gemm_split(const SplitGemmProblem* q, int n, int N, int K, int* dev_status, cudaStream_t stream) {
+  if (n < 1 || n > 3) {
+    set_last_error("gemm_split: one to three problems (got %d)", n);
+    return ST_INVALID_ARG;
+  }
+  const SplitGemmProblem& a = q[0];
+  long row_tiles = 0;
+  for (int i = 0; i < n; ++i) {
+    int rc = validate_split(q[i], N, K);
     if (rc) return rc;
-    if (b->epi.mode != a.epi.mode || (b->epi.out_plane > 0) != (a.epi.out_plane > 0) || b->epi.out_f32 != a.epi.out_f32) {
+    if (q[i].epi.mode != a.epi.mode || (q[i].epi.out_plane > 0) != (a.epi.out_plane > 0) ||
+        q[i].epi.out_f32 != a.epi.out_f32) {
       set_last_error("gemm_split: grouped problems need the same epilogue kind");
       return ST_INVALID_ARG;
     }
+    row_tiles += (q[i].M + 2 * S_BM - 1) / (2 * S_BM);
   }
-  const int bn = choose_split_width((a.M + 255) / 256 + (b ? (b->M + 255) / 256 : 0), N);
-  SplitProblem p0, p1;
-  rc = build_split(&p0, a, N, K, bn, dev_status);
-  if (rc) return rc;
-  int t1 = 0;
-  if (b) {
-    rc = build_split(&p1, *b, N, K, bn, dev_status);
-    if (rc) return rc;
-    t1 = p1.g.tiles_m * p1.g.tiles_n;
-  } else {
-    p1 = p0;
+  const int bn = choose_split_width(row_tiles, N);
+  SplitProblem p[3];
+  int end[3] = {0, 0, 0}, tiles = 0;
+  for (int i = 0; i < 3; ++i) {
+    if (i < n) {
+      int rc = build_split(&p[i], q[i], N, K, bn, dev_status);
+      if (rc) return rc;
+      tiles += p[i].g.tiles_m * p[i].g.tiles_n;
+    } else {
+      p[i] = p[0];  // no tiles
+    }
+    end[i] = tiles;
   }
-  const int t0 = p0.g.tiles_m * p0.g.tiles_n;
   const bool planes = a.epi.out_plane > 0;
   switch (a.epi.mode) {
-    case EPI_BIAS: return launch_split_width<EPI_BIAS, 1>(bn, p0, p1, t0, t1, stream);
+    case EPI_BIAS: return launch_split_width<EPI_BIAS, 1>(bn, p, end, stream);
     case EPI_BIAS_GELU:
-      if (planes) return launch_split_width<EPI_BIAS_GELU, 2>(bn, p0, p1, t0, t1, stream);
+      if (planes) return launch_split_width<EPI_BIAS_GELU, 2>(bn, p, end, stream);
       break;
     case EPI_QKV_NORM:
-      return planes ? launch_split_width<EPI_QKV_NORM, 2>(bn, p0, p1, t0, t1, stream)
-                    : launch_split_width<EPI_QKV_NORM, 1>(bn, p0, p1, t0, t1, stream);
-    case EPI_GATE_RESID: return launch_split_width<EPI_GATE_RESID, 1>(bn, p0, p1, t0, t1, stream);
-    case EPI_ADD_TABLE: return launch_split_width<EPI_ADD_TABLE, 1>(bn, p0, p1, t0, t1, stream);
+      return planes ? launch_split_width<EPI_QKV_NORM, 2>(bn, p, end, stream)
+                    : launch_split_width<EPI_QKV_NORM, 1>(bn, p, end, stream);
+    case EPI_GATE_RESID: return launch_split_width<EPI_GATE_RESID, 1>(bn, p, end, stream);
+    case EPI_ADD_TABLE: return launch_split_width<EPI_ADD_TABLE, 1>(bn, p, end, stream);
     case EPI_UNPATCHIFY:
-      return a.epi.out_f32 ? launch_split_width<EPI_UNPATCHIFY, 1>(bn, p0, p1, t0, t1, stream)
-                           : launch_split_width<EPI_UNPATCHIFY, 0>(bn, p0, p1, t0, t1, stream);
+      return a.epi.out_f32 ? launch_split_width<EPI_UNPATCHIFY, 1>(bn, p, end, stream)
+                           : launch_split_width<EPI_UNPATCHIFY, 0>(bn, p, end, stream);
     default: break;
   }
   set_last_error("gemm_split: unsupported epilogue mode %d", a.epi.mode);

@@ -341,8 +341,8 @@ int dispatch_epi(const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs&
 }  // namespace
 
 bool gemm_pair_supported(int operand_dtype, int M, int N, int K, const GemmEpilogue& epi);
-int launch_gemm_pair(const GemmProblem& a, const GemmProblem* b, int operand_dtype, int N, int K,
-                     int* dev_status, cudaStream_t stream);
+int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
+                     cudaStream_t stream);
 
 namespace {
 // argument checks shared by the single and the grouped launch
@@ -392,18 +392,33 @@ int validate_gemm(const void* A, long lda, const void* W, long ldw, int operand_
 }
 }  // namespace
 
-int launch_gemm_grouped(const GemmProblem& a, const GemmProblem& b, int operand_dtype, int N, int K,
-                        int* dev_status, cudaStream_t stream) {
-  int rc = validate_gemm(a.A, a.lda, a.W, a.ldw, operand_dtype, a.M, N, K, a.epi);
-  if (rc) return rc;
-  rc = validate_gemm(b.A, b.lda, b.W, b.ldw, operand_dtype, b.M, N, K, b.epi);
-  if (rc) return rc;
-  if (a.epi.mode == b.epi.mode && a.epi.out_f32 == b.epi.out_f32 &&
-      gemm_pair_supported(operand_dtype, a.M, N, K, a.epi) && gemm_pair_supported(operand_dtype, b.M, N, K, b.epi))
-    return launch_gemm_pair(a, &b, operand_dtype, N, K, dev_status, stream);
-  rc = launch_gemm(a.A, a.lda, a.W, a.ldw, operand_dtype, a.M, N, K, a.epi, dev_status, stream);
-  if (rc) return rc;
-  return launch_gemm(b.A, b.lda, b.W, b.ldw, operand_dtype, b.M, N, K, b.epi, dev_status, stream);
+int launch_gemm_grouped(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
+                        cudaStream_t stream) {
+  if (n < 1 || n > 3) {
+    set_last_error("gemm_grouped: one to three problems (got %d)", n);
+    return ST_INVALID_ARG;
+  }
+  GemmProblem paired[3];
+  int np = 0;
+  for (int i = 0; i < n; ++i) {
+    int rc = validate_gemm(q[i].A, q[i].lda, q[i].W, q[i].ldw, operand_dtype, q[i].M, N, K, q[i].epi);
+    if (rc) return rc;
+    if (q[i].epi.mode == q[0].epi.mode && q[i].epi.out_f32 == q[0].epi.out_f32 &&
+        gemm_pair_supported(operand_dtype, q[i].M, N, K, q[i].epi))
+      paired[np++] = q[i];
+  }
+  if (np > 0) {
+    int rc = launch_gemm_pair(paired, np, operand_dtype, N, K, dev_status, stream);
+    if (rc) return rc;
+  }
+  for (int i = 0; i < n; ++i) {
+    if (q[i].epi.mode == q[0].epi.mode && q[i].epi.out_f32 == q[0].epi.out_f32 &&
+        gemm_pair_supported(operand_dtype, q[i].M, N, K, q[i].epi))
+      continue;
+    int rc = launch_gemm(q[i].A, q[i].lda, q[i].W, q[i].ldw, operand_dtype, q[i].M, N, K, q[i].epi, dev_status, stream);
+    if (rc) return rc;
+  }
+  return ST_OK;
 }
 
 int launch_gemm(const void* A, long lda, const void* W, long ldw, int operand_dtype, int M, int N,
@@ -415,7 +430,7 @@ int launch_gemm(const void* A, long lda, const void* W, long ldw, int operand_dt
   if (gemm_pair_supported(operand_dtype, M, N, K, epi)) {
     GemmProblem q;
     q.A = A; q.lda = lda; q.W = W; q.ldw = ldw; q.M = M; q.epi = epi;
-    return launch_gemm_pair(q, nullptr, operand_dtype, N, K, dev_status, stream);
+    return launch_gemm_pair(&q, 1, operand_dtype, N, K, dev_status, stream);
   }
 
   const int BN = (N >= 256 && N % 256 == 0) ? 256 : (N > 64 ? 128 : 64);

@@ -120,15 +120,16 @@ struct GemmProblem {
   int M = 0;
   GemmEpilogue epi;
 };
-// Two GEMMs of the same N, K, operand type and epilogue kind as ONE launch when the CTA-pair
-// kernel covers both (the second problem's tiles run in the tail of the first's); otherwise
-// two launches.  Used for the image-stream GEMM of a block and its small context-stream twin.
-int launch_gemm_grouped(const GemmProblem& a, const GemmProblem& b, int operand_dtype, int N, int K,
-                        int* dev_status, cudaStream_t stream);
+// One to three GEMMs of the same N, K, operand type and epilogue kind.  Those the CTA-pair kernel
+// covers share ONE launch (one problem's tiles run in the tail of the other's), the others get
+// their own.  Used for the image-stream GEMM of a block, its small context-stream twin and the
+// second QKV projection of a dual block.
+int launch_gemm_grouped(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
+                        cudaStream_t stream);
 
 // fp32 GEMM on the tensor cores: A and W are three bf16 planes each (split3.cuh), a_plane / w_plane
-// elements apart, rows of K elements; the result has fp32 accuracy.  One or two problems (b may be
-// null) of the same N, K and epilogue kind as one launch.  K % 8 == 0, N % 8 == 0.
+// elements apart, rows of K elements; the result has fp32 accuracy.  One to three problems of the
+// same N, K and epilogue kind as one launch.  K % 8 == 0, N % 8 == 0.
 struct SplitGemmProblem {
   const bf16* A = nullptr;
   long a_plane = 0;
@@ -137,8 +138,7 @@ struct SplitGemmProblem {
   int M = 0;
   GemmEpilogue epi;
 };
-int launch_gemm_split(const SplitGemmProblem& a, const SplitGemmProblem* b, int N, int K, int* dev_status,
-                      cudaStream_t stream);
+int launch_gemm_split(const SplitGemmProblem* q, int n, int N, int K, int* dev_status, cudaStream_t stream);
 
 // ----------------------------------------------------------------------------
 // Flash-style attention on tcgen05 (head_dim 64, bf16, non-causal).
