@@ -69,7 +69,13 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 }
 
 __global__ void __launch_bounds__(AS_THREADS, 1)
-attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm, const SplitAttnArgs a) {
+attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
+                               const __grid_constant__ SplitAttnArgs a0, const __grid_constant__ SplitAttnArgs a1,
+                               const int grid0) {
+  // grid.x: the query tiles of the first attention, then those of the second (the image-only one of a dual block)
+  const bool second = static_cast<int>(blockIdx.x) >= grid0;
+  const CUtensorMap& tm = second ? tm1 : tm0;
+  const SplitAttnArgs& a = second ? a1 : a0;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -89,7 +95,7 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm, const Spl
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * AS_BM, h = blockIdx.y, b = blockIdx.z;
+  const int q0 = (static_cast<int>(blockIdx.x) - (second ? grid0 : 0)) * AS_BM, h = blockIdx.y, b = blockIdx.z;
   const int T = a.T, nkv = (T + AS_BN - 1) / AS_BN;
 
   if (threadIdx.x == 0) {
@@ -325,22 +331,12 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm, const Spl
 
 }  // namespace
 
-int launch_attention_split(const bf16* qkv, int B, int T, int NH, int Tc, bf16* out_c, bf16* out_x, float scale,
-                           int* dev_status, cudaStream_t stream) {
-  if (!qkv || !out_x || B <= 0 || T <= 0 || NH <= 0 || Tc < 0 || Tc > T || (reinterpret_cast<uintptr_t>(qkv) & 15) ||
-      (reinterpret_cast<uintptr_t>(out_x) & 15) || (reinterpret_cast<uintptr_t>(out_c) & 15)) {
-    set_last_error("attention_split: invalid argument (B %d T %d NH %d Tc %d)", B, T, NH, Tc);
-    return ST_INVALID_ARG;
-  }
-  if (B > 65535 || NH > 65535) {
-    set_last_error("attention_split: B and NH must each be <= 65535");
+int launch_attention_split(const AttnProblem* p, int n, int B, int NH, int* dev_status, cudaStream_t stream) {
+  if (n < 1 || n > 2 || B > 65535 || NH > 65535) {
+    set_last_error("attention_split: one or two problems, B and NH at most 65535 each");
     return ST_UNSUPPORTED;
   }
   const int E = NH * AS_D;
-  CUtensorMap tm;
-  int rc = encode_tmap_3d(&tm, qkv, 2, 3ull * E, (uint64_t)T, 3ull * B, 3ull * E * 2, (uint64_t)T * 3ull * E * 2, AS_D,
-                          64, 1);
-  if (rc) return rc;
   static std::mutex attr_mutex;
   static bool attr_done[64] = {false};
   int dev = 0;
@@ -354,14 +350,29 @@ int launch_attention_split(const bf16* qkv, int B, int T, int NH, int Tc, bf16* 
       attr_done[dev] = true;
     }
   }
-  SplitAttnArgs a;
-  a.B = B; a.T = T; a.NH = NH; a.Tc = Tc; a.E = E;
-  a.out_c = out_c;
-  a.out_x = out_x;
-  a.c = scale * 1.4426950408889634f;
-  a.status = dev_status;
-  launch_dependent(attention_split_tcgen05_kernel, dim3((T + AS_BM - 1) / AS_BM, NH, B), AS_THREADS, AS_SMEM_BYTES, stream,
-                   tm, a);
+  CUtensorMap tm[2];
+  SplitAttnArgs a[2];
+  int grid[2] = {0, 0};
+  for (int i = 0; i < n; ++i) {
+    const AttnProblem& q = p[i];
+    if (!q.qkv || !q.out_x || B <= 0 || q.T <= 0 || NH <= 0 || q.Tc < 0 || q.Tc > q.T ||
+        (reinterpret_cast<uintptr_t>(q.qkv) & 15) || (reinterpret_cast<uintptr_t>(q.out_x) & 15) ||
+        (reinterpret_cast<uintptr_t>(q.out_c) & 15)) {
+      set_last_error("attention_split: invalid argument (B %d T %d NH %d Tc %d)", B, q.T, NH, q.Tc);
+      return ST_INVALID_ARG;
+    }
+    int rc = encode_tmap_3d(&tm[i], q.qkv, 2, 3ull * E, (uint64_t)q.T, 3ull * B, 3ull * E * 2,
+                            (uint64_t)q.T * 3ull * E * 2, AS_D, 64, 1);
+    if (rc) return rc;
+    a[i].B = B; a[i].T = q.T; a[i].NH = NH; a[i].Tc = q.Tc; a[i].E = E;
+    a[i].out_c = q.out_c;
+    a[i].out_x = q.out_x;
+    a[i].c = q.scale * 1.4426950408889634f;
+    a[i].status = dev_status;
+    grid[i] = (q.T + AS_BM - 1) / AS_BM;
+  }
+  launch_dependent(attention_split_tcgen05_kernel, dim3(grid[0] + grid[1], NH, B), AS_THREADS, AS_SMEM_BYTES, stream,
+                   tm[0], tm[n - 1], a[0], a[n - 1], grid[0]);
   return after_launch("attention_split_tcgen05_kernel");
 }
 

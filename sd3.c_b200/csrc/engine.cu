@@ -13,9 +13,9 @@
 //   LN+modulate(x), LN+modulate(c) in one launch (both modulations of a dual block at once)
 //   QKV GEMM(x), (c)         -> packed (B, Tc+Tx, 3E), RMSNorm fused, context rows first; a dual block's
 //                               second QKV GEMM(x) rides in the same launch
-//   joint attention           -> o_c, o_x
+//   joint attention          -> o_c, o_x; a dual block's attention over the image tokens in the same launch
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
-//   [dual] attention over image tokens, out-proj GEMM with gate2
+//   [dual] out-proj GEMM with gate2
 //   LN+modulate(x), (c); MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual), each for x and c at once
 #include <math.h>
 #include <algorithm>
@@ -440,22 +440,17 @@ int run_qkv(sd3_model* m, const Linear& L, const void* h, void* qkv, int B, int 
 }
 
 // out_e4m3 (FP8 mode, head_dim 64 only): the outputs feed FP8 out-projections
-int run_attention(sd3_model* m, const void* qkv, int B, int T, int Tc, void* o_c, void* o_x,
-                  cudaStream_t st, bool out_e4m3 = false, float score_bound = 0.f, bool prescaled = false) {
-  // prescaled: q already carries scale * log2(e) (only set up for the bf16 kernel)
-  const float scale = prescaled ? 0.0f : 1.0f / sqrtf(static_cast<float>(m->D));
-  if (!m->f32 && m->D == 64)
-    return launch_attention_bf16(static_cast<const bf16*>(qkv), B, T, m->NH, Tc,
-                                 static_cast<bf16*>(o_c), static_cast<bf16*>(o_x), scale, m->status,
-                                 st, out_e4m3 ? 1 : 0, m->ws.attn_scratch_bytes ? m->ws.attn_scratch : nullptr,
-                                 m->ws.attn_scratch_bytes, score_bound);
-  if (out_e4m3) {
-    set_last_error("e4m3 attention output needs head_dim 64");
-    return ST_UNSUPPORTED;
-  }
-  if (m->f32 && m->D == 64)
-    return launch_attention_split(static_cast<const bf16*>(qkv), B, T, m->NH, Tc, static_cast<bf16*>(o_c),
-                                  static_cast<bf16*>(o_x), scale, m->status, st);
+struct AttnCall {
+  const void* qkv;
+  int T, Tc;
+  void *o_c, *o_x;
+  bool out_e4m3;
+  float score_bound;
+  bool prescaled;  // q already carries scale * log2(e) (only set up for the bf16 kernel)
+};
+
+int run_attention_simt(sd3_model* m, const void* qkv, int B, int T, int Tc, void* o_c, void* o_x, cudaStream_t st) {
+  const float scale = 1.0f / sqrtf(static_cast<float>(m->D));
   if (m->f32) {
     // fp32 outputs: the context rows' block first, then the image rows'; each is split into its planes
     const float* q = static_cast<const float*>(qkv);
@@ -470,6 +465,29 @@ int run_attention(sd3_model* m, const void* qkv, int B, int T, int Tc, void* o_c
   const bf16* q = static_cast<const bf16*>(qkv);
   return launch_attention_simt(q, q + m->E, q + 2 * m->E, 3L * m->E, 0, B, T, m->NH, m->D, Tc, o_c, o_x, m->E, 0, scale,
                                st);
+}
+
+// one or two attentions over the same samples (joint, image-only), as one launch where that pays
+int run_attention(sd3_model* m, const AttnCall* c, int n, int B, cudaStream_t st) {
+  if (m->D == 64) {
+    AttnProblem p[2];
+    for (int i = 0; i < n; ++i)
+      p[i] = {static_cast<const bf16*>(c[i].qkv), c[i].T, c[i].Tc, static_cast<bf16*>(c[i].o_c),
+              static_cast<bf16*>(c[i].o_x), c[i].prescaled ? 0.0f : 1.0f / sqrtf(static_cast<float>(m->D)),
+              c[i].out_e4m3 ? 1 : 0, m->ws.attn_scratch_bytes ? m->ws.attn_scratch : nullptr,
+              m->ws.attn_scratch_bytes, c[i].score_bound};
+    return m->f32 ? launch_attention_split(p, n, B, m->NH, m->status, st)
+                  : launch_attention_group(p, n, B, m->NH, m->status, st);
+  }
+  for (int i = 0; i < n; ++i) {
+    if (c[i].out_e4m3) {
+      set_last_error("e4m3 attention output needs head_dim 64");
+      return ST_UNSUPPORTED;
+    }
+    int rc = run_attention_simt(m, c[i].qkv, B, c[i].T, c[i].Tc, c[i].o_c, c[i].o_x, st);
+    if (rc) return rc;
+  }
+  return ST_OK;
 }
 
 GemmEpilogue gate_epilogue(const Linear& L, int Tseg, const float* gate, long mod_stride, float* resid) {
@@ -560,7 +578,11 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   // FP8 mode: both out-projections of the joint attention must take e4m3 for the
   // kernel to write it (one flag for both outputs)
   const bool o8 = m->fp8 && m->D == 64 && L.x_out.w8 && (L.last || L.c_out.w8);
-  SD3_TRY(run_attention(m, w.qkv, B, T, Tc, L.last ? nullptr : w.o_c, w.o_x, st, o8, L.joint_bound, pre_j));
+  const bool o8d = m->fp8 && m->D == 64 && L.d_out.w8;
+  if (m->D != 64 && L.dual) SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
+  const AttnCall att[2] = {{w.qkv, T, Tc, L.last ? nullptr : w.o_c, w.o_x, o8, L.joint_bound, pre_j},
+                           {w.qkv2, Tx, 0, nullptr, w.o_x2, o8d, L.dual_bound, pre_d}};
+  SD3_TRY(run_attention(m, att, L.dual ? 2 : 1, B, st));
   if (grouped && !L.last) {
     SD3_TRY(run_linear_pair(m, L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8,
                             L.c_out, w.o_c, B * Tc, gate_epilogue(L.c_out, Tc, c_gate_a, ms, c), o8, st));
@@ -568,12 +590,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     if (!L.last) SD3_TRY(run_gate_resid(m, L.c_out, w.o_c, B, Tc, c_gate_a, ms, c, st, o8));
     SD3_TRY(run_gate_resid(m, L.x_out, w.o_x, B, Tx, x_gate_a, ms, x, st, o8));
   }
-  if (L.dual) {
-    if (m->D != 64) SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
-    const bool o8d = m->fp8 && m->D == 64 && L.d_out.w8;
-    SD3_TRY(run_attention(m, w.qkv2, B, Tx, 0, nullptr, w.o_x2, st, o8d, L.dual_bound, pre_d));
-    SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
-  }
+  if (L.dual) SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
   // MLPs of both streams: LayerNorm + modulate each, then the two first linears (GELU-tanh) and
   // the two second linears (gate + residual), each pair as one grouped launch
   {

@@ -156,12 +156,25 @@ int launch_attention_bf16(const bf16* qkv, int B, int T, int NH, int Tc, bf16* o
                           float scale, int* dev_status, cudaStream_t stream, int out_e4m3 = 0,
                           void* scratch = nullptr, size_t scratch_bytes = 0, float score_bound = 0.0f);
 size_t attention_scratch_bytes(int B, int T, int NH);
+// One or two attentions of the same B and NH (the joint and the image-only one of a dual block) as
+// one launch where both run the same instantiation: at small sizes neither fills the GPU alone.
+struct AttnProblem {
+  const bf16* qkv;
+  int T, Tc;
+  bf16 *out_c, *out_x;
+  float scale;
+  int out_e4m3;
+  void* scratch;
+  size_t scratch_bytes;
+  float score_bound;
+};
+int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_status, cudaStream_t stream);
 
 // fp32 attention for head_dim 64 on the tensor cores.  qkv: three bf16 planes (split3.cuh) of
 // (B, T, 3E), B * T * 3E elements apart; outputs split by rows like above, as three planes of
 // B * Tc * E (out_c, may be null) and B * (T - Tc) * E (out_x) elements.
-int launch_attention_split(const bf16* qkv, int B, int T, int NH, int Tc, bf16* out_c, bf16* out_x, float scale,
-                           int* dev_status, cudaStream_t stream);
+// One or two problems as one launch (of AttnProblem: qkv, T, Tc, out_c, out_x and scale).
+int launch_attention_split(const AttnProblem* p, int n, int B, int NH, int* dev_status, cudaStream_t stream);
 
 // Generic SIMT attention (any head_dim <= 128, fp32 or bf16 in, fp32 math).
 // q: row (b*T + t) at base + row*ld + h*D; k, v: row (b*L + j) at base + row*ldk + h*D
