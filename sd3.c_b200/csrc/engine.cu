@@ -311,6 +311,7 @@ SplitGemmProblem split_problem(const Linear& L, const void* A, int M, const Gemm
   p.w_plane = static_cast<long>(L.N) * L.K;
   p.M = M;
   p.epi = e;
+  p.epi.w_static = 1;
   if (!p.epi.bias) p.epi.bias = L.b;
   return p;
 }
@@ -324,6 +325,7 @@ int run_linear(sd3_model* m, const Linear& L, const void* A, int M, const GemmEp
     return ST_NOT_READY;
   }
   GemmEpilogue ee = e;
+  ee.w_static = 1;  // written by set_param only, which sd3_model_finalize waits for
   if (!ee.bias) ee.bias = L.b;
   if (m->f32) {
     const SplitGemmProblem p = split_problem(L, A, M, ee);
@@ -385,6 +387,7 @@ int run_linear_group(sd3_model* m, const LinearCall* c, int n, cudaStream_t st) 
   for (int i = 0; i < n; ++i) {
     const Linear& L = *c[i].L;
     p[i].A = c[i].A; p[i].lda = K; p[i].W = all8 ? L.w8 : L.w; p[i].ldw = K; p[i].M = c[i].M; p[i].epi = c[i].epi;
+    p[i].epi.w_static = 1;
     if (!p[i].epi.bias) p[i].epi.bias = L.b;
     if (all8) p[i].epi.alpha = L.wscale;
   }

@@ -138,8 +138,10 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote signal
   tc_fence_after_sync();
-  grid_dep_wait();
-  grid_dep_launch();
+  if (warp != 0) {  // the TMA producer waits after its first weight tiles
+    grid_dep_wait();
+    grid_dep_launch();
+  }
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
 
@@ -153,25 +155,43 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    constexpr int KEL = FP8 ? P_KBYTES : P_KBYTES / 2;  // K elements per stage
+    auto expect_slot = [&](int st, int ks) {
+      // all bytes of the slot (both CTAs) are credited to the leader's barrier
+      if (rank == 0) mbar_expect_tx(&full_bar[st], (KB - 2 * ks < 2 ? KB - 2 * ks : 2) * 2 * P_STAGE_BYTES);
+    };
+    auto load_w = [&](const PairProblem& pp, int st, int ks, int n0) {
+      const uint32_t bar = map_to_cta(smem_u32(&full_bar[st]), 0);
+      for (int hs = 0; hs < (KB - 2 * ks < 2 ? KB - 2 * ks : 2); ++hs)
+        tma_load_2d_pair(smem + (2 * st + hs) * P_STAGE_BYTES + P_A_BYTES, &pp.tmW, bar, (2 * ks + hs) * KEL, n0);
+    };
+    int pre = 0;  // slots of the first tile whose weights are under way before the wait
+    if (p0.g.epi.w_static) {
+      const PairProblem& pp = pair < end0 ? p0 : pair < end1 ? p1 : p2;
+      const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
+      for (; pre < NSLOT && pre < KS; ++pre) {
+        expect_slot(pre, pre);
+        load_w(pp, pre, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF);
+      }
+    }
+    grid_dep_wait();
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const PairProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
       const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF;
       for (int ks = 0; ks < KS; ++ks) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-        {
-          const int nk = KB - 2 * ks < 2 ? KB - 2 * ks : 2;  // stages of this slot that carry data
-          // all bytes of the slot (both CTAs) are credited to the leader's barrier
-          const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], nk * 2 * P_STAGE_BYTES);
-          constexpr int KEL = FP8 ? P_KBYTES : P_KBYTES / 2;  // K elements per stage
-          for (int hs = 0; hs < nk; ++hs) {
-            uint8_t* sa = smem + (2 * stage + hs) * P_STAGE_BYTES;
-            tma_load_2d_pair(sa, &pp.tmA, bar, (2 * ks + hs) * KEL, m0);
-            tma_load_2d_pair(sa + P_A_BYTES, &pp.tmW, bar, (2 * ks + hs) * KEL, n0);
-          }
+        if (pre > 0) {
+          --pre;
+        } else {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+          expect_slot(stage, ks);
+          load_w(pp, stage, ks, n0);
         }
+        const int nk = KB - 2 * ks < 2 ? KB - 2 * ks : 2;  // stages of this slot that carry data
+        const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+        for (int hs = 0; hs < nk; ++hs)
+          tma_load_2d_pair(smem + (2 * stage + hs) * P_STAGE_BYTES, &pp.tmA, bar, (2 * ks + hs) * KEL, m0);
         if (++stage == NSLOT) { stage = 0; phase ^= 1; }
       }
     }

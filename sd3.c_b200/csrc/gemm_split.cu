@@ -265,8 +265,10 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote signal
   tc_fence_after_sync();
-  grid_dep_wait();
-  grid_dep_launch();
+  if (warp != 0) {  // the TMA producer waits after its first weight tiles
+    grid_dep_wait();
+    grid_dep_launch();
+  }
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
   // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
@@ -277,19 +279,34 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    // the weights of a stage; all its bytes (both CTAs) are credited to the leader's barrier
+    auto load_w = [&](const SplitProblem& pp, int st, int kb, int n0) {
+      if (rank == 0) mbar_expect_tx(&full_bar[st], 2 * Cfg::STAGE_BYTES);
+      tma_load_3d_pair(smem + st * Cfg::STAGE_BYTES + 3 * S_A_PLANE, &pp.tmW, map_to_cta(smem_u32(&full_bar[st]), 0),
+                       kb * S_KB, n0, 0);
+    };
+    int pre = 0;  // stages of the first tile whose weights are under way before the wait
+    if (p0.g.epi.w_static) {
+      const SplitProblem& pp = pair < end0 ? p0 : pair < end1 ? p1 : p2;
+      const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
+      for (; pre < STAGES && pre < KB; ++pre)
+        load_w(pp, pre, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS);
+    }
+    grid_dep_wait();
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const SplitProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * S_BM) + static_cast<int>(rank) * S_BM;
       const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS;
       for (int kb = 0; kb < KB; ++kb) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-        uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
-        // all bytes of the stage (both CTAs) are credited to the leader's barrier
-        const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-        if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
-        tma_load_3d_pair(sa, &pp.tmA, bar, kb * S_KB, m0, 0);
-        tma_load_3d_pair(sa + 3 * S_A_PLANE, &pp.tmW, bar, kb * S_KB, n0, 0);
+        if (pre > 0) {
+          --pre;
+        } else {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+          load_w(pp, stage, kb, n0);
+        }
+        tma_load_3d_pair(smem + stage * Cfg::STAGE_BYTES, &pp.tmA, map_to_cta(smem_u32(&full_bar[stage]), 0),
+                         kb * S_KB, m0, 0);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
