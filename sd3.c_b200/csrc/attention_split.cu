@@ -5,8 +5,8 @@
 //
 // One CTA owns 128 queries of one (sample, head).  Warp 0 streams the planes of
 // K (two 128-key stages) and V (two 64-key halves) with TMA; one thread of
-// warp 1 issues the MMAs; four softmax warps own one query row per thread
-// (TMEM lane == row).  Per 128 keys:
+// warp 1 issues the MMAs; eight softmax warps own half the keys of a query row
+// per thread (TMEM lane == row).  Per 128 keys:
 //   S = Q K^T   24 MMAs of N = 128, smallest products first;
 //   P           = 2^((S - m) c) in registers, split and written to TMEM planes;
 //   acc = P V   three MMAs per 16 keys: Ph x [Vh Vm Vl] (N = 192), Pm x [Vh Vm]
@@ -17,14 +17,19 @@
 //   O = (O + acc) 2^((m_old - m_new) c) in registers, round to nearest: the tensor core's own
 //               accumulation truncates and is only used within one tile.
 // The score buffer is emptied into registers at once, so the scores of tile j + 1
-// run under the exponentials of tile j, and the exponentials of tile j + 1 under
-// the products of tile j.
+// run under the exponentials of tile j, and the exponentials and splits of tile
+// j + 1 under the products of tile j; what stands between two tiles' products is
+// the addition of acc and the store of P.
+// Two warps share a row (keys 0..63 and 64..127 of a tile, 32 of the 64 output
+// columns each; they exchange the tile's maximum through shared memory): one warp
+// per scheduler with a whole row in registers ran 2500 unrolled instructions a
+// tile, more than the instruction cache holds, at 0.3 instructions per cycle (8500 cycles a tile).
 // What bounds it: the tensor pipe, 1536 + 1680 cycles per 128 x 128 tile pair.
 //
-// Measured against attention_simt_kernel (one warp per query, uncoalesced key rows), which it
+// Measured against attention_simt_kernel (one warp per query, uncoalesced key rows), which this
 // replaces for fp32 models with head_dim 64: one dual block of 256 + 77 tokens 2.79 -> 0.49 ms, the
-// 24-block model at 512 x 512 668 -> 19.1 ms.  Error of that block's branches against float64: 3.8e-7
-// (FFMA GEMMs and SIMT attention: 1.6e-6).
+// 24-block model at 512 x 512 668 -> 19.1 ms; the second warp per row: 17.53 -> 16.79 ms.  Error of
+// that block's branches against float64: 3.4e-7 (FFMA GEMMs and SIMT attention: 1.6e-6).
 #include <cuda.h>
 #include <mutex>
 
@@ -43,11 +48,12 @@ constexpr int AS_BM = 128, AS_BN = 128, AS_D = 64;
 constexpr int AS_PLANE = AS_BN * AS_D * 2;   // 16 KiB: one plane of 128 rows
 constexpr int AS_HPLANE = AS_PLANE / 2;      // one plane of 64 rows
 constexpr int AS_TILE = 3 * AS_PLANE;        // Q, one K stage, both V halves
-constexpr int AS_THREADS = 192;
+constexpr int AS_THREADS = 64 + 8 * 32;
 constexpr int AS_S_COL = 0;    // scores: 128 fp32 columns
 constexpr int AS_P_COL = 128;  // P: three planes of 64 columns (bf16 pairs)
 constexpr int AS_O_COL = 320;  // P V of one tile: three blocks of 64 fp32 columns
-constexpr int AS_SMEM_BYTES = 4 * AS_TILE + 256 + 1024;  // Q, two K stages, V
+constexpr int AS_XCHG_BYTES = 2 * 2 * AS_BM * 4;  // row maxima: [tile parity][half][row]
+constexpr int AS_SMEM_BYTES = 4 * AS_TILE + AS_XCHG_BYTES + 256 + 1024;  // Q, two K stages, V
 
 struct SplitAttnArgs {
   int B, T, NH, Tc, E;
@@ -82,16 +88,18 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
   uint8_t* q_smem = smem;                 // [plane][128 rows][128 B]
   uint8_t* k_smem = smem + AS_TILE;       // [stage][plane][128 rows][128 B]
   uint8_t* v_smem = smem + 3 * AS_TILE;   // [half][plane][64 rows][128 B]
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + 4 * AS_TILE);
+  float* s_max = reinterpret_cast<float*>(smem + 4 * AS_TILE);
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + 4 * AS_TILE + AS_XCHG_BYTES);
   uint64_t* k_full = q_full + 1;    // 2
   uint64_t* k_empty = k_full + 2;   // 2
   uint64_t* v_full = k_empty + 2;   // 2
   uint64_t* v_empty = v_full + 2;   // 2
   uint64_t* s_full = v_empty + 2;   // scores of a tile complete
-  uint64_t* s_free = s_full + 1;    // scores are in registers (4 arrivals)
-  uint64_t* p_ready = s_free + 1;   // P of a tile is in TMEM and acc has been read (4 arrivals)
+  uint64_t* s_free = s_full + 1;    // scores are in registers (8 arrivals)
+  uint64_t* p_ready = s_free + 1;   // P of a tile is in TMEM and acc has been read (8 arrivals)
   uint64_t* pv_done = p_ready + 1;  // products of a tile complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
+  uint64_t* xchg = pv_done + 1;     // 4: both warps of a row quadrant have written their maxima
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xchg + 4);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,9 +115,10 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
       mbar_init(&v_empty[s], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(s_free, 4);
-    mbar_init(p_ready, 4);
+    mbar_init(s_free, 8);
+    mbar_init(p_ready, 8);
     mbar_init(pv_done, 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&xchg[i], 2);
     *s_abort = 0;
     fence_barrier_init();
     prefetch_tmap(&tm);
@@ -208,17 +217,19 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
   } else {
     // ------------------------------ softmax + output --------------------------
     const int quad = warp & 3, row = quad * 32 + lane;
+    const int half = (warp - 2) >> 2;  // keys 64 * half .. + 63 of a tile, output columns 32 * half .. + 31
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    const uint32_t s_tmem = lane_base + AS_S_COL, p_tmem = lane_base + AS_P_COL, o_tmem = lane_base + AS_O_COL;
+    const uint32_t s_tmem = lane_base + AS_S_COL + 64 * half, p_tmem = lane_base + AS_P_COL + 32 * half,
+                   o_tmem = lane_base + AS_O_COL + 32 * half;
     const float c = a.c;
     float m = -INFINITY, l = 0.f;
-    float o[AS_D];
+    float o[32];
 #pragma unroll
-    for (int i = 0; i < AS_D; ++i) o[i] = 0.f;
+    for (int i = 0; i < 32; ++i) o[i] = 0.f;
     // o += the finished products of a tile
     auto add_acc = [&]() {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < 2; ++g) {
         uint32_t a0[16], a1[16], a2[16];
         tmem_ld_32x32b_x16(o_tmem + 16 * g, a0);
         tmem_ld_32x32b_x16(o_tmem + 64 + 16 * g, a1);
@@ -229,45 +240,61 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
           o[16 * g + i] += __uint_as_float(a0[i]) + (__uint_as_float(a1[i]) + __uint_as_float(a2[i]));
       }
     };
+    // this row's value of the other half's thread (slot: alternating buffers, see below)
+    auto exchange = [&](int n, float v, float& other) -> bool {
+      float* buf = s_max + (n & 1) * 2 * AS_BM;
+      buf[half * AS_BM + row] = v;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&xchg[quad]);  // release: the warp's writes before it are visible to the waiter
+      if (!mbar_wait_warp(&xchg[quad], n & 1, wc, DEV_TIMEOUT_ATTN_S)) return false;
+      __syncwarp();
+      // a slot is written again two exchanges later, after this warp's next arrival
+      other = buf[(half ^ 1) * AS_BM + row];
+      return true;
+    };
     bool ok = true;
     for (int j = 0; j < nkv; ++j) {
       if (!mbar_wait_warp(s_full, j & 1, wc, DEV_TIMEOUT_ATTN_S)) { ok = false; break; }
       tc_fence_after_sync();
-      uint32_t r[4][32];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) tmem_ld_32x32b_x32(s_tmem + 32 * q, r[q]);
+      uint32_t r[2][32];
+      tmem_ld_32x32b_x32(s_tmem, r[0]);
+      tmem_ld_32x32b_x32(s_tmem + 32, r[1]);
       tmem_wait_ld();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free);
-      if (j * AS_BN + AS_BN > T) {  // keys >= T do not exist
+      const int key0 = j * AS_BN + 64 * half;
+      if (key0 + 64 > T) {  // keys >= T do not exist
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 2; ++q)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (j * AS_BN + 32 * q + i >= T) r[q][i] = 0xff800000u;
+            if (key0 + 32 * q + i >= T) r[q][i] = 0xff800000u;
       }
       float mx[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        mx[q] = fmaxf(__uint_as_float(r[q][0]), __uint_as_float(r[q][1]));
+        const uint32_t* v = &r[q >> 1][(q & 1) * 16];
+        mx[q] = fmaxf(__uint_as_float(v[0]), __uint_as_float(v[1]));
 #pragma unroll
-        for (int i = 2; i < 32; i += 2) mx[q] = fmax3(mx[q], __uint_as_float(r[q][i]), __uint_as_float(r[q][i + 1]));
+        for (int i = 2; i < 16; i += 2) mx[q] = fmax3(mx[q], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
       }
-      const float m_new = fmax3(fmax3(m, mx[0], mx[1]), mx[2], mx[3]);
+      const float own = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]);
+      float other;
+      if (!exchange(j, own, other)) { ok = false; break; }
+      const float m_new = fmax3(m, own, other);
       const float alpha = ex2_f32((m - m_new) * c);
       m = m_new;
-      float sum[4];
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t ph[32], pm[32], pl[32];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        sum[q] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          // the difference is exact near the maximum, where its error would count
-          const float p = ex2_f32((__uint_as_float(r[q][i]) - m_new) * c);
-          sum[q] += p;
-          r[q][i] = __float_as_uint(p);
-        }
+      for (int i = 0; i < 32; ++i) {
+        // the difference is exact near the maximum, where its error would count
+        const float p0 = ex2_f32((__uint_as_float(r[i >> 4][(2 * i) & 31]) - m_new) * c);
+        const float p1 = ex2_f32((__uint_as_float(r[i >> 4][(2 * i + 1) & 31]) - m_new) * c);
+        sum[i & 1] += p0;
+        sum[2 + (i & 1)] += p1;
+        split3_x2(p0, p1, ph[i], pm[i], pl[i]);
       }
       l = fmaf(l, alpha, (sum[0] + sum[1]) + (sum[2] + sum[3]));
       if (j >= 1) {
@@ -275,24 +302,18 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
         tc_fence_after_sync();
         add_acc();
 #pragma unroll
-        for (int i = 0; i < AS_D; ++i) o[i] *= alpha;
+        for (int i = 0; i < 32; ++i) o[i] *= alpha;
       }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t ph[16], pm[16], pl[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          split3_x2(__uint_as_float(r[q][2 * i]), __uint_as_float(r[q][2 * i + 1]), ph[i], pm[i], pl[i]);
-        tmem_st_32x32b_x16(p_tmem + 16 * q, ph);
-        tmem_st_32x32b_x16(p_tmem + 64 + 16 * q, pm);
-        tmem_st_32x32b_x16(p_tmem + 128 + 16 * q, pl);
-      }
+      tmem_st_32x32b_x32(p_tmem, ph);
+      tmem_st_32x32b_x32(p_tmem + 64, pm);
+      tmem_st_32x32b_x32(p_tmem + 128, pl);
       tmem_wait_st();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_ready);
     }
-    if (ok && mbar_wait_warp(pv_done, (nkv - 1) & 1, wc, DEV_TIMEOUT_ATTN_O)) {
+    float l_other = 0.f;
+    if (ok && exchange(nkv, l, l_other) && mbar_wait_warp(pv_done, (nkv - 1) & 1, wc, DEV_TIMEOUT_ATTN_O)) {
       tc_fence_after_sync();
       add_acc();
       const int t = q0 + row;
@@ -301,10 +322,10 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
       if (t < T && out) {
         const int rows = ctx ? a.Tc : T - a.Tc;
         const long plane = static_cast<long>(a.B) * rows * a.E;
-        bf16* dst = out + (static_cast<long>(b) * rows + (ctx ? t : t - a.Tc)) * a.E + h * AS_D;
-        const float inv = 1.0f / l;
+        bf16* dst = out + (static_cast<long>(b) * rows + (ctx ? t : t - a.Tc)) * a.E + h * AS_D + 32 * half;
+        const float inv = 1.0f / (half ? l_other + l : l + l_other);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
           uint4 uh, um, ul;
           const float* v = o + 8 * i;
           split3_x2(v[0] * inv, v[1] * inv, uh.x, um.x, ul.x);
