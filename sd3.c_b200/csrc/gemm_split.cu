@@ -27,6 +27,12 @@
 // up the blocks and run the fused epilogue.  The accumulators rotate (512 / PBN of them,
 // at most four), so the adds run under the MMAs of the following blocks.
 //
+// K split: where one wave of tiles leaves half of the SMs without work, two CTA pairs
+// (a cluster of four) share a tile, each takes half of K, and the second pair hands
+// its sums to the first through distributed shared memory (the operand ring, idle
+// by then) before the epilogue: a fixed order, no scratch memory, no second kernel.
+// One dual block of 256 + 77 tokens 381 -> 337 us.
+//
 // What bounds it: the tensor pipe (six MMAs per K step) and the operand loads: a K
 // block of a 256 x 256 tile is 3072 cycles of MMA for 96 KiB per CTA, of a 256 x 128
 // tile 1536 for 72 KiB.  A one-CTA version with 128 x 256 tiles and 32-wide K blocks
@@ -210,8 +216,8 @@ struct SplitProblem {
   GemmArgs g;
 };
 
-template <int PBN, int EPI, int OUT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SplitCfg<PBN>::THREADS, 1)
+template <int PBN, int EPI, int OUT, int KSPLIT>
+__global__ void __cluster_dims__(2 * KSPLIT, 1, 1) __launch_bounds__(SplitCfg<PBN>::THREADS, 1)
 gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_constant__ SplitProblem p1,
                           const __grid_constant__ SplitProblem p2, const int end0, const int end1,
                           const int num_tiles) {
@@ -231,9 +237,12 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();  // 0 = leader
-  const int pair = blockIdx.x >> 1;
-  const int num_pairs = gridDim.x >> 1;
+  const uint32_t part = cluster_ctarank() >> 1;  // share of K (KSPLIT == 2)
+  const uint32_t rank = cluster_ctarank() & 1;   // CTA of the pair, 0 = leader
+  const uint32_t leader = cluster_ctarank() & ~1u;
+  const uint16_t pair_mask = static_cast<uint16_t>(3u << leader);
+  const int pair = blockIdx.x / (2 * KSPLIT);  // index of the pair (cluster) among those that walk the tiles
+  const int num_pairs = gridDim.x / (2 * KSPLIT);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -272,7 +281,10 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx wc{s_abort, p0.g.status};
   // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
-  const int KB = p0.g.k_blocks;           // the same K for all problems
+  // K blocks of this pair (the same K for all problems)
+  const int kb0 = KSPLIT == 2 && part == 1 ? (p0.g.k_blocks + 1) / 2 : 0;
+  const int KB = (KSPLIT == 2 && part == 0 ? (p0.g.k_blocks + 1) / 2 : p0.g.k_blocks) - kb0;
+  float acc[CPW];  // running sums of an epilogue thread
 
   if (warp == 0 && lane == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------
@@ -282,8 +294,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     // the weights of a stage; all its bytes (both CTAs) are credited to the leader's barrier
     auto load_w = [&](const SplitProblem& pp, int st, int kb, int n0) {
       if (rank == 0) mbar_expect_tx(&full_bar[st], 2 * Cfg::STAGE_BYTES);
-      tma_load_3d_pair(smem + st * Cfg::STAGE_BYTES + 3 * S_A_PLANE, &pp.tmW, map_to_cta(smem_u32(&full_bar[st]), 0),
-                       kb * S_KB, n0, 0);
+      tma_load_3d_pair(smem + st * Cfg::STAGE_BYTES + 3 * S_A_PLANE, &pp.tmW, map_to_cta(smem_u32(&full_bar[st]), leader),
+                       (kb0 + kb) * S_KB, n0, 0);
     };
     int pre = 0;  // stages of the first tile whose weights are under way before the wait
     if (p0.g.epi.w_static) {
@@ -305,8 +317,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
           load_w(pp, stage, kb, n0);
         }
-        tma_load_3d_pair(smem + stage * Cfg::STAGE_BYTES, &pp.tmA, map_to_cta(smem_u32(&full_bar[stage]), 0),
-                         kb * S_KB, m0, 0);
+        tma_load_3d_pair(smem + stage * Cfg::STAGE_BYTES, &pp.tmA, map_to_cta(smem_u32(&full_bar[stage]), leader),
+                         (kb0 + kb) * S_KB, m0, 0);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
@@ -335,8 +347,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
 #pragma unroll
               for (int k = 0; k < S_KB / 16; ++k)
                 mma_f16_ss_pair(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
-            mma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
-            mma_commit_pair(&tfull_bar[buf], 3);    // block sum ready in both CTAs
+            mma_commit_pair(&empty_bar[stage], pair_mask);  // frees the stage in both CTAs
+            mma_commit_pair(&tfull_bar[buf], pair_mask);    // block sum ready in both CTAs
           }
           turn ^= 1;
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -357,7 +369,6 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m = (lt / g.tiles_n) * (2 * S_BM) + row;
       const int n0 = (lt % g.tiles_n) * PBN + half * CPW;
-      float acc[CPW];
 #pragma unroll
       for (int j = 0; j < CPW; ++j) acc[j] = 0.f;
       for (int kb = 0; kb < KB; ++kb) {
@@ -373,7 +384,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
           if (s == CPW / 32 - 1) {  // everything is in registers: the accumulator may be reused
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), 0));
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), leader));
           }
 #pragma unroll
           for (int j = 0; j < 32; ++j) acc[s * 32 + j] += __uint_as_float(r[j]);
@@ -381,6 +392,40 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
         if (++buf == NBUF) { buf = 0; bphase ^= 1; }
       }
       if (!ok) break;
+      if (KSPLIT == 1 && m < g.M) {
+        const RowMap rm = map_row(m, g.epi);
+#pragma unroll
+        for (int c = 0; c < CPW; c += 64) split_epilogue_64<EPI, OUT>(acc + c, rm, n0 + c, g);
+      }
+      __syncwarp();
+    }
+  }
+
+  if constexpr (KSPLIT == 2) {
+    // One tile per cluster.  The second pair's sums go to the first pair's CTA of the same rank, 16
+    // bytes per lane and store: [epilogue warp][4-column group][lane].
+    const int ew = warp - 2;
+    const bool epi_warp = warp >= 2 && warp < 2 + Cfg::EPI_WARPS;
+    __syncwarp();
+    cluster_sync_all();  // every MMA of both pairs is complete: the first pair's ring is idle
+    if (part == 1 && epi_warp) {
+      const uint32_t dst = map_to_cta(smem_u32(smem), rank) + static_cast<uint32_t>((ew * (CPW / 4) * 32 + lane) * 16);
+#pragma unroll
+      for (int i = 0; i < CPW / 4; ++i)
+        st_cluster_v4(dst + i * 512, acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+    }
+    cluster_sync_all();  // release / acquire: the sums are visible to the first pair
+    if (part == 0 && epi_warp) {
+      const float4* src = reinterpret_cast<const float4*>(smem) + ew * (CPW / 4) * 32 + lane;
+#pragma unroll
+      for (int i = 0; i < CPW / 4; ++i) {
+        const float4 t = src[i * 32];
+        acc[4 * i] += t.x; acc[4 * i + 1] += t.y; acc[4 * i + 2] += t.z; acc[4 * i + 3] += t.w;
+      }
+      const GemmArgs& g = pair < end0 ? p0.g : pair < end1 ? p1.g : p2.g;
+      const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
+      const int m = (lt / g.tiles_n) * (2 * S_BM) + static_cast<int>(rank) * S_BM + (warp & 3) * 32 + lane;
+      const int n0 = (lt % g.tiles_n) * PBN + (ew >> 2) * CPW;
       if (m < g.M) {
         const RowMap rm = map_row(m, g.epi);
 #pragma unroll
@@ -401,10 +446,10 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   }
 }
 
-template <int PBN, int EPI, int OUT>
+template <int PBN, int EPI, int OUT, int KSPLIT>
 int launch_split_inst(const SplitProblem* p, const int* end, cudaStream_t stream) {
   using Cfg = SplitCfg<PBN>;
-  auto kern = gemm_split_tcgen05_kernel<PBN, EPI, OUT>;
+  auto kern = gemm_split_tcgen05_kernel<PBN, EPI, OUT, KSPLIT>;
   static std::mutex attr_mutex;
   static bool attr_done[64] = {false};
   int dev = 0;
@@ -418,16 +463,23 @@ int launch_split_inst(const SplitProblem* p, const int* end, cudaStream_t stream
     }
   }
   const int tiles = end[2], most = device_sm_count() / 2;
-  launch_dependent(kern, 2 * (tiles < most ? tiles : most), Cfg::THREADS, Cfg::SMEM_BYTES, stream,
+  launch_dependent(kern, 2 * KSPLIT * (KSPLIT == 2 || tiles < most ? tiles : most), Cfg::THREADS, Cfg::SMEM_BYTES, stream,
                    p[0], p[1], p[2], end[0], end[1], tiles);
   return after_launch("gemm_split_tcgen05_kernel");
 }
 
 template <int EPI, int OUT>
-int launch_split_width(int bn, const SplitProblem* p, const int* end, cudaStream_t st) {
-  if (bn == 256) return launch_split_inst<256, EPI, OUT>(p, end, st);
-  if (bn == 128) return launch_split_inst<128, EPI, OUT>(p, end, st);
-  return launch_split_inst<64, EPI, OUT>(p, end, st);
+int launch_split_width(int bn, int ksplit, const SplitProblem* p, const int* end, cudaStream_t st) {
+  if constexpr (EPI == EPI_GATE_RESID) {  // the GEMMs with few tiles and a long K
+    if (ksplit == 2) {
+      if (bn == 256) return launch_split_inst<256, EPI, OUT, 2>(p, end, st);
+      if (bn == 128) return launch_split_inst<128, EPI, OUT, 2>(p, end, st);
+      return launch_split_inst<64, EPI, OUT, 2>(p, end, st);
+    }
+  }
+  if (bn == 256) return launch_split_inst<256, EPI, OUT, 1>(p, end, st);
+  if (bn == 128) return launch_split_inst<128, EPI, OUT, 1>(p, end, st);
+  return launch_split_inst<64, EPI, OUT, 1>(p, end, st);
 }
 
 int validate_split(const SplitGemmProblem& q, int N, int K) {
@@ -479,17 +531,50 @@ int build_split(SplitProblem* pp, const SplitGemmProblem& q, int N, int K, int b
   return encode_tmap_3d(&pp->tmW, q.W, 2, K, N, 3, static_cast<uint64_t>(K) * 2, q.w_plane * 2, S_KB, bn / 2, 3);
 }
 
-// The tile width with the least (waves over the CTA pairs) x (time of a K block of a tile).  The
-// costs are in units of 24 cycles: 24 MMAs of 128 / 64 cycles, and at PBN = 64 the 480 rows of TMA per CTA.
-int choose_split_width(long row_tiles, int N) {
+// How many clusters of four the device holds at once (a GPC whose SM count is not a multiple of four
+// leaves some without work), from the occupancy of the widest instantiation.
+long max_clusters_of_four() {
+  static std::mutex mu;
+  static int known[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  if (known[dev] == 0) {
+    using Cfg = SplitCfg<128>;
+    auto kern = gemm_split_tcgen05_kernel<128, EPI_GATE_RESID, 1, 2>;
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(4);
+    cfg.blockDim = dim3(Cfg::THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known[dev] = n > 0 ? n : -1;
+  }
+  return known[dev];
+}
+
+// The tile width (and, for the gate + residual GEMMs, whether two pairs share a tile's K) with the least
+// (waves over the CTA pairs) x (K blocks of a pair) x (time of a block).  In units of 24 cycles a
+// block is 24 MMAs of 128 / 64 cycles, and at PBN = 64 the 480 rows of TMA per CTA; handing the
+// sums over costs two cluster barriers and PBN / 2 KiB of distributed shared memory per CTA.
+int choose_split_width(long row_tiles, int N, int k_blocks, bool may_split, int* ksplit) {
   const long pairs = device_sm_count() / 2 > 0 ? device_sm_count() / 2 : 1;
   int best = 256;
   long best_cost = 0;
   const int bn[3] = {256, 128, 64}, cost[3] = {128, 68, 52};
+  *ksplit = 1;
   for (int i = 0; i < 3; ++i) {
     const long tiles = row_tiles * ((N + bn[i] - 1) / bn[i]);
-    const long c = (tiles + pairs - 1) / pairs * cost[i];
-    if (i == 0 || c < best_cost) { best = bn[i]; best_cost = c; }
+    const long c = (tiles + pairs - 1) / pairs * cost[i] * k_blocks;
+    if (i == 0 || c < best_cost) { best = bn[i]; best_cost = c; *ksplit = 1; }
+    if (may_split && k_blocks >= 2 && tiles <= max_clusters_of_four()) {
+      const long cs = (k_blocks + 1) / 2 * cost[i] + 125 + 2 * bn[i] / 3;
+      if (cs < best_cost) { best = bn[i]; best_cost = cs; *ksplit = 2; }
+    }
   }
   return best;
 }
@@ -513,7 +598,8 @@ int launch_gemm_split(const SplitGemmProblem* q, int n, int N, int K, int* dev_s
     }
     row_tiles += (q[i].M + 2 * S_BM - 1) / (2 * S_BM);
   }
-  const int bn = choose_split_width(row_tiles, N);
+  int ksplit = 1;
+  const int bn = choose_split_width(row_tiles, N, (K + S_KB - 1) / S_KB, a.epi.mode == EPI_GATE_RESID, &ksplit);
   SplitProblem p[3];
   int end[3] = {0, 0, 0}, tiles = 0;
   for (int i = 0; i < 3; ++i) {
@@ -528,18 +614,18 @@ int launch_gemm_split(const SplitGemmProblem* q, int n, int N, int K, int* dev_s
   }
   const bool planes = a.epi.out_plane > 0;
   switch (a.epi.mode) {
-    case EPI_BIAS: return launch_split_width<EPI_BIAS, 1>(bn, p, end, stream);
+    case EPI_BIAS: return launch_split_width<EPI_BIAS, 1>(bn, ksplit, p, end, stream);
     case EPI_BIAS_GELU:
-      if (planes) return launch_split_width<EPI_BIAS_GELU, 2>(bn, p, end, stream);
+      if (planes) return launch_split_width<EPI_BIAS_GELU, 2>(bn, ksplit, p, end, stream);
       break;
     case EPI_QKV_NORM:
-      return planes ? launch_split_width<EPI_QKV_NORM, 2>(bn, p, end, stream)
-                    : launch_split_width<EPI_QKV_NORM, 1>(bn, p, end, stream);
-    case EPI_GATE_RESID: return launch_split_width<EPI_GATE_RESID, 1>(bn, p, end, stream);
-    case EPI_ADD_TABLE: return launch_split_width<EPI_ADD_TABLE, 1>(bn, p, end, stream);
+      return planes ? launch_split_width<EPI_QKV_NORM, 2>(bn, ksplit, p, end, stream)
+                    : launch_split_width<EPI_QKV_NORM, 1>(bn, ksplit, p, end, stream);
+    case EPI_GATE_RESID: return launch_split_width<EPI_GATE_RESID, 1>(bn, ksplit, p, end, stream);
+    case EPI_ADD_TABLE: return launch_split_width<EPI_ADD_TABLE, 1>(bn, ksplit, p, end, stream);
     case EPI_UNPATCHIFY:
-      return a.epi.out_f32 ? launch_split_width<EPI_UNPATCHIFY, 1>(bn, p, end, stream)
-                           : launch_split_width<EPI_UNPATCHIFY, 0>(bn, p, end, stream);
+      return a.epi.out_f32 ? launch_split_width<EPI_UNPATCHIFY, 1>(bn, ksplit, p, end, stream)
+                           : launch_split_width<EPI_UNPATCHIFY, 0>(bn, ksplit, p, end, stream);
     default: break;
   }
   set_last_error("gemm_split: unsupported epilogue mode %d", a.epi.mode);
