@@ -416,9 +416,12 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, float a, fl
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(a), "f"(b), "f"(c), "f"(d)
                : "memory");
 }
+// Arrival on a barrier that may live in another CTA of the cluster, with the default (CTA) scope: it orders
+// reads of tensor memory (complete after tcgen05.wait::ld), not writes to memory.  With .release.cluster
+// every arrival waited for the warp's outstanding stores (a membar: the first stall reason of the
+// split GEMM, whose epilogue warps arrive once per K block).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar_addr)
-               : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar_addr) : "memory");
 }
 // TMA load whose completion bytes are credited to a barrier that may live in
 // the other CTA of the pair (bar is a shared::cluster address).
