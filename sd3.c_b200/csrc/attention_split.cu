@@ -8,7 +8,7 @@
 // warp 1 issues the MMAs; eight softmax warps own half the keys of a query row
 // per thread (TMEM lane == row).  Per 128 keys:
 //   S = Q K^T   24 MMAs of N = 128, smallest products first;
-//   P           = 2^((S - m) c) in registers, split and written to TMEM planes;
+//   P           = 2^(S c - m c) in registers, split and written to TMEM planes;
 //   acc = P V   three MMAs per 16 keys: Ph x [Vh Vm Vl] (N = 192), Pm x [Vh Vm]
 //               (N = 128), Pl x [Vh] (N = 64) into three column blocks that hold
 //               the products of size 1, 2^-8 and 2^-16 (V's planes lie side by
@@ -65,7 +65,7 @@ struct SplitAttnArgs {
 
 __device__ __forceinline__ float ex2_f32(float x) {
   float y;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));  // without ftz three more instructions
   return y;
 }
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
@@ -222,10 +222,12 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
     const uint32_t s_tmem = lane_base + AS_S_COL + 64 * half, p_tmem = lane_base + AS_P_COL + 32 * half,
                    o_tmem = lane_base + AS_O_COL + 32 * half;
     const float c = a.c;
-    float m = -INFINITY, l = 0.f;
-    float o[32];
+    // The exponentials refer to mc, the running maximum times c as rounded: 2^(s c - mc) has one rounding, and
+    // the rounding of mc is the same factor in every term of the row.
+    float m = -INFINITY, mc = -INFINITY, l = 0.f;
+    float2 o[16];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) o[i] = 0.f;
+    for (int i = 0; i < 16; ++i) o[i] = make_float2(0.f, 0.f);
     // o += the finished products of a tile
     auto add_acc = [&]() {
 #pragma unroll
@@ -236,8 +238,12 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
         tmem_ld_32x32b_x16(o_tmem + 128 + 16 * g, a2);
         tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          o[16 * g + i] += __uint_as_float(a0[i]) + (__uint_as_float(a1[i]) + __uint_as_float(a2[i]));
+        for (int i = 0; i < 8; ++i) {
+          auto pair = [&](const uint32_t (&v)[16]) {
+            return make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+          };
+          o[8 * g + i] = __fadd2_rn(o[8 * g + i], __fadd2_rn(pair(a0), __fadd2_rn(pair(a1), pair(a2))));
+        }
       }
     };
     // this row's value of the other half's thread (slot: alternating buffers, see below)
@@ -282,27 +288,29 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
       const float own = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]);
       float other;
       if (!exchange(j, own, other)) { ok = false; break; }
-      const float m_new = fmax3(m, own, other);
-      const float alpha = ex2_f32((m - m_new) * c);
-      m = m_new;
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      m = fmax3(m, own, other);
+      const float mc_new = m * c;
+      const float alpha = ex2_f32(mc - mc_new);
+      mc = mc_new;
+      const float2 c2 = make_float2(c, c), nm2 = make_float2(-mc, -mc);
+      float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t ph[32], pm[32], pl[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        // the difference is exact near the maximum, where its error would count
-        const float p0 = ex2_f32((__uint_as_float(r[i >> 4][(2 * i) & 31]) - m_new) * c);
-        const float p1 = ex2_f32((__uint_as_float(r[i >> 4][(2 * i + 1) & 31]) - m_new) * c);
-        sum[i & 1] += p0;
-        sum[2 + (i & 1)] += p1;
-        split3_x2(p0, p1, ph[i], pm[i], pl[i]);
+        float2 p = __ffma2_rn(make_float2(__uint_as_float(r[i >> 4][(2 * i) & 31]),
+                                          __uint_as_float(r[i >> 4][(2 * i + 1) & 31])), c2, nm2);
+        p.x = ex2_f32(p.x);
+        p.y = ex2_f32(p.y);
+        sum[i & 1] = __fadd2_rn(sum[i & 1], p);
+        split3_x2(p.x, p.y, ph[i], pm[i], pl[i]);
       }
-      l = fmaf(l, alpha, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+      l = fmaf(l, alpha, (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
       if (j >= 1) {
         if (!mbar_wait_warp(pv_done, (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_O)) { ok = false; break; }
         tc_fence_after_sync();
         add_acc();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] *= alpha;
+        for (int i = 0; i < 16; ++i) o[i] = __fmul2_rn(o[i], make_float2(alpha, alpha));
       }
       tmem_st_32x32b_x32(p_tmem, ph);
       tmem_st_32x32b_x32(p_tmem + 64, pm);
@@ -327,11 +335,11 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint4 uh, um, ul;
-          const float* v = o + 8 * i;
-          split3_x2(v[0] * inv, v[1] * inv, uh.x, um.x, ul.x);
-          split3_x2(v[2] * inv, v[3] * inv, uh.y, um.y, ul.y);
-          split3_x2(v[4] * inv, v[5] * inv, uh.z, um.z, ul.z);
-          split3_x2(v[6] * inv, v[7] * inv, uh.w, um.w, ul.w);
+          const float2* v = o + 4 * i;
+          split3_x2(v[0].x * inv, v[0].y * inv, uh.x, um.x, ul.x);
+          split3_x2(v[1].x * inv, v[1].y * inv, uh.y, um.y, ul.y);
+          split3_x2(v[2].x * inv, v[2].y * inv, uh.z, um.z, ul.z);
+          split3_x2(v[3].x * inv, v[3].y * inv, uh.w, um.w, ul.w);
           reinterpret_cast<uint4*>(dst)[i] = uh;
           reinterpret_cast<uint4*>(dst + plane)[i] = um;
           reinterpret_cast<uint4*>(dst + 2 * plane)[i] = ul;
