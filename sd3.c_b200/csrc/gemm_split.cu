@@ -80,9 +80,16 @@ struct SplitCfg {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
 };
 
-__device__ __forceinline__ float gelu_tanh_exact(float x) {
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  return 0.5f * x * (1.0f + tanhf(u));
+// 0.5 x (1 + tanh(u)) = x / (1 + e^(-2u)),  u = sqrt(2/pi) (x + 0.044715 x^3): no cancellation for
+// negative u, two MUFU operations where tanhf takes some thirty instructions (they stood between the
+// tiles: an epilogue thread has 128 of them)
+__device__ __forceinline__ float gelu_tanh_f32(float x) {
+  const float t = x * fmaf(x * x, -2.0f * 1.4426950408889634f * 0.7978845608028654f * 0.044715f,
+                           -2.0f * 1.4426950408889634f * 0.7978845608028654f);  // -2 u log2(e)
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return x * r;
 }
 
 // eight consecutive fp32 outputs / eight outputs as three planes (16-byte stores)
@@ -130,7 +137,7 @@ __device__ __forceinline__ void split_epilogue_64(float* v, const RowMap& rm, in
   }
   if constexpr (EPI == EPI_BIAS_GELU) {
 #pragma unroll
-    for (int j = 0; j < 64; ++j) v[j] = gelu_tanh_exact(v[j]);
+    for (int j = 0; j < 64; ++j) v[j] = gelu_tanh_f32(v[j]);
   }
   if constexpr (EPI == EPI_ADD_TABLE) {
     const float4* t4 = reinterpret_cast<const float4*>(e.table + static_cast<long>(rm.t_in) * N + n_base);
@@ -387,7 +394,12 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), leader));
           }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[s * 32 + j] += __uint_as_float(r[j]);
+          for (int j = 0; j < 32; j += 2) {
+            const float2 t = __fadd2_rn(make_float2(acc[s * 32 + j], acc[s * 32 + j + 1]),
+                                        make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])));
+            acc[s * 32 + j] = t.x;
+            acc[s * 32 + j + 1] = t.y;
+          }
         }
         if (++buf == NBUF) { buf = 0; bphase ^= 1; }
       }
