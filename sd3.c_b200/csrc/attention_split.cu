@@ -57,6 +57,7 @@ constexpr int AS_SMEM_BYTES = 4 * AS_TILE + AS_XCHG_BYTES + 256 + 1024;  // Q, t
 
 struct SplitAttnArgs {
   int B, T, NH, Tc, E;
+  int b0;       // sample of blockIdx.z == 0 (grids hold at most 65535 samples)
   bf16* out_c;  // three planes of B * Tc * E, or null
   bf16* out_x;  // three planes of B * (T - Tc) * E
   float c;      // softmax scale * log2(e)
@@ -103,7 +104,7 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = (static_cast<int>(blockIdx.x) - (second ? grid0 : 0)) * AS_BM, h = blockIdx.y, b = blockIdx.z;
+  const int q0 = (static_cast<int>(blockIdx.x) - (second ? grid0 : 0)) * AS_BM, h = blockIdx.y, b = a.b0 + blockIdx.z;
   const int T = a.T, nkv = (T + AS_BN - 1) / AS_BN;
 
   if (threadIdx.x == 0) {
@@ -361,8 +362,8 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
 }  // namespace
 
 int launch_attention_split(const AttnProblem* p, int n, int B, int NH, int* dev_status, cudaStream_t stream) {
-  if (n < 1 || n > 2 || B > 65535 || NH > 65535) {
-    set_last_error("attention_split: one or two problems, B and NH at most 65535 each");
+  if (n < 1 || n > 2 || NH > 65535) {
+    set_last_error("attention_split: one or two problems, NH at most 65535");
     return ST_UNSUPPORTED;
   }
   const int E = NH * AS_D;
@@ -400,9 +401,14 @@ int launch_attention_split(const AttnProblem* p, int n, int B, int NH, int* dev_
     a[i].status = dev_status;
     grid[i] = (q.T + AS_BM - 1) / AS_BM;
   }
-  launch_dependent(attention_split_tcgen05_kernel, dim3(grid[0] + grid[1], NH, B), AS_THREADS, AS_SMEM_BYTES, stream,
-                   tm[0], tm[n - 1], a[0], a[n - 1], grid[0]);
-  return after_launch("attention_split_tcgen05_kernel");
+  for (int b0 = 0; b0 < B; b0 += 65535) {
+    a[0].b0 = a[1].b0 = b0;
+    launch_dependent(attention_split_tcgen05_kernel, dim3(grid[0] + grid[1], NH, B - b0 < 65535 ? B - b0 : 65535),
+                     AS_THREADS, AS_SMEM_BYTES, stream, tm[0], tm[n - 1], a[0], a[n - 1], grid[0]);
+    int rc = after_launch("attention_split_tcgen05_kernel");
+    if (rc) return rc;
+  }
+  return ST_OK;
 }
 
 }  // namespace sd3

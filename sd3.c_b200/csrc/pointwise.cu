@@ -307,7 +307,8 @@ __global__ void transpose_kernel(const IT* __restrict__ in, OT* __restrict__ out
   }
 }
 
-template <typename IT>
+// VEC: in is aligned to four elements (a caller's captions need not be)
+template <typename IT, bool VEC>
 __global__ void split3_kernel(const IT* __restrict__ in, bf16* __restrict__ out, long n) {
   grid_dep_wait();
   grid_dep_launch();
@@ -315,7 +316,10 @@ __global__ void split3_kernel(const IT* __restrict__ in, bf16* __restrict__ out,
   const long stride = static_cast<long>(gridDim.x) * blockDim.x * 4;
   for (; i < n; i += stride) {
     float4 f;
-    if constexpr (sizeof(IT) == 4) {
+    if constexpr (!VEC) {
+      f = make_float4(convert_elem<IT, float>(in[i]), convert_elem<IT, float>(in[i + 1]),
+                      convert_elem<IT, float>(in[i + 2]), convert_elem<IT, float>(in[i + 3]));
+    } else if constexpr (sizeof(IT) == 4) {
       f = *reinterpret_cast<const float4*>(in + i);
     } else {
       const uint2 u = *reinterpret_cast<const uint2*>(in + i);
@@ -565,17 +569,19 @@ int launch_transpose(const void* in, int in_f32, void* out, int out_f32, int R, 
 }
 
 int launch_split3(const void* in, int in_f32, bf16* out, long n, cudaStream_t stream) {
-  if (!in || !out || n <= 0 || n % 4 || (reinterpret_cast<uintptr_t>(in) & (in_f32 ? 15 : 7)) ||
-      (reinterpret_cast<uintptr_t>(out) & 7)) {
-    set_last_error("split3: need n %% 4 == 0 and aligned pointers (n %ld)", n);
+  if (!in || !out || n <= 0 || n % 4 || (reinterpret_cast<uintptr_t>(out) & 7)) {
+    set_last_error("split3: need n %% 4 == 0 and an aligned output (n %ld)", n);
     return ST_INVALID_ARG;
   }
+  const bool vec = (reinterpret_cast<uintptr_t>(in) & (in_f32 ? 15 : 7)) == 0;
   const long blocks = (n / 4 + 255) / 256, most = device_sm_count() * 16L;
   const unsigned grid = static_cast<unsigned>(blocks < most ? blocks : most);
   if (in_f32)
-    launch_dependent(split3_kernel<float>, grid, 256, 0, stream, static_cast<const float*>(in), out, n);
+    launch_dependent(vec ? split3_kernel<float, true> : split3_kernel<float, false>, grid, 256, 0, stream,
+                     static_cast<const float*>(in), out, n);
   else
-    launch_dependent(split3_kernel<bf16>, grid, 256, 0, stream, static_cast<const bf16*>(in), out, n);
+    launch_dependent(vec ? split3_kernel<bf16, true> : split3_kernel<bf16, false>, grid, 256, 0, stream,
+                     static_cast<const bf16*>(in), out, n);
   return after_launch("split3_kernel");
 }
 

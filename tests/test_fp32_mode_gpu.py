@@ -43,3 +43,22 @@ def test_block_fp32_against_float64(sd3, E, NH, B, Tx, Tc, dual, last):
     m.close()
     for got, ref in ((xx, x_ref),) + (() if last else ((cc, c_ref),)):
         assert ((got.double() - ref).norm() / ref.norm()).item() < 2e-6
+
+
+def test_captions_at_any_address(sd3):
+    """Captions that start in the middle of a vector load give the bits of aligned ones (fp32 and bf16 tensors)."""
+    L, E, NH, P, C = 2, 64, 1, 64, 128
+    p = O.random_params(O.model_param_shapes(L, (0,), 16, E, P, C, 2, NH, 4), seed=1, std=0.1)
+    m = sd3.Model(L, (0,), P, C, 16, E, NH, 4, 2, 32, 16, True, sd3.PRECISION_F32)
+    m.load({k: v.cuda() for k, v in p.items()})
+    gen = torch.Generator().manual_seed(2)
+    for dtype in (torch.float32, torch.bfloat16):
+        pooled, caps = torch.randn(1, P, generator=gen).to(dtype).cuda(), torch.randn(1, 9, C, generator=gen).to(dtype).cuda()
+        lat, t = torch.randn(1, 16, 8, 8, generator=gen).to(dtype).cuda(), torch.tensor([500.0]).cuda()
+        odd = torch.empty(caps.numel() + 1, device="cuda", dtype=dtype)[1:].view_as(caps)
+        odd.copy_(caps)
+        assert odd.data_ptr() % 8 and odd.is_contiguous()
+        assert torch.equal(m.forward(pooled, caps, lat, t), m.forward(pooled, odd, lat, t))
+    torch.cuda.synchronize()
+    assert sd3.device_status() == 0
+    m.close()
