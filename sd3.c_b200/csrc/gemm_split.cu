@@ -24,8 +24,8 @@
 // x 3 planes), two threads of the even CTA issue the 24 MMAs of every K block (blocks in turn: a
 // block has its own accumulator, so the threads need no order between them and the
 // barrier work of one runs under the MMAs of the other), the epilogue warps of both add
-// up the blocks and run the fused epilogue.  The accumulators rotate (512 / PBN of them,
-// at most four), so the adds run under the MMAs of the following blocks.
+// up the blocks and run the fused epilogue.  Four accumulators rotate, so the adds run
+// under the MMAs of the following blocks.
 //
 // K split: where one wave of tiles leaves half of the SMs without work, two CTA pairs
 // (a cluster of four) share a tile, each takes half of K, and the second pair hands
@@ -34,12 +34,15 @@
 // One dual block of 256 + 77 tokens 381 -> 337 us.
 //
 // What bounds it: the tensor pipe (six MMAs per K step) and the operand loads: a K
-// block of a 256 x 256 tile is 3072 cycles of MMA for 96 KiB per CTA, of a 256 x 128
-// tile 1536 for 72 KiB.  A one-CTA version with 128 x 256 tiles and 32-wide K blocks
-// (64-byte rows, half of W's bytes more per MMA) kept the tensor pipe 38 % busy.
+// block of a 256 x 128 tile is 1536 cycles of MMA for 72 KiB per CTA and takes 1740 to 1800.  Not
+// kept: one-CTA tiles of 128 x 256 with 32-wide K blocks (64-byte rows, half of W's bytes more per
+// MMA: tensor pipe 38 % busy); 256 x 256 tiles (3072 cycles of MMA took 4060: two stages of
+// operands, two accumulators, and an epilogue of 128 columns per thread between tiles).
 //
-// Measured, 24-block model at 512 x 512 (1024 + 333 tokens): 19.26 (one-CTA tiles) -> 17.57 ms; the FFMA
-// kernel and the SIMT attention took 754 ms.  One dual block of 256 + 77 tokens 454 -> 411 us.
+// Measured, 24-block model at 512 x 512 (1024 + 333 tokens): one-CTA tiles 19.26, pairs 17.57, no cluster-scope
+// release in the accumulator's hand-back 16.8 -> 15.7 with the attention as it was then, GELU 15.5 -> 15.2,
+// 128-wide tiles only 15.3 -> 15.1 ms; the FFMA kernel and the SIMT attention took 754 ms.  One dual block of 256 + 77
+// tokens: 454, 411 (K split 381 -> 337), 338, 294 us; start 4740.
 #include <cuda.h>
 #include <mutex>
 
@@ -69,12 +72,12 @@ template <int PBN>
 struct SplitCfg {
   static constexpr int W_ROWS = PBN / 2;  // rows of W per CTA
   static constexpr int W_PLANE = W_ROWS * 128;
-  static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);  // 96 / 72 / 60 KiB
-  static constexpr int STAGES = PBN == 256 ? 2 : 3;              // 192 / 216 / 180 KiB
-  static constexpr int NBUF = PBN == 256 ? 2 : 4;                // TMEM accumulators
+  static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);  // 72 / 60 KiB
+  static constexpr int STAGES = 3;                               // 216 / 180 KiB
+  static constexpr int NBUF = 4;                                 // TMEM accumulators
   static constexpr int TMEM_COLS = NBUF * PBN;
   static constexpr int EPI_WARPS = PBN == 64 ? 4 : 8;
-  static constexpr int CPW = PBN == 256 ? 128 : 64;  // accumulator columns per epilogue thread
+  static constexpr int CPW = 64;                     // accumulator columns per epilogue thread
   static constexpr int MMA2_WARP = 2 + EPI_WARPS;    // second MMA-issuing warp
   static constexpr int THREADS = 32 * (3 + EPI_WARPS);
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
@@ -483,15 +486,10 @@ int launch_split_inst(const SplitProblem* p, const int* end, cudaStream_t stream
 template <int EPI, int OUT>
 int launch_split_width(int bn, int ksplit, const SplitProblem* p, const int* end, cudaStream_t st) {
   if constexpr (EPI == EPI_GATE_RESID) {  // the GEMMs with few tiles and a long K
-    if (ksplit == 2) {
-      if (bn == 256) return launch_split_inst<256, EPI, OUT, 2>(p, end, st);
-      if (bn == 128) return launch_split_inst<128, EPI, OUT, 2>(p, end, st);
-      return launch_split_inst<64, EPI, OUT, 2>(p, end, st);
-    }
+    if (ksplit == 2)
+      return bn == 128 ? launch_split_inst<128, EPI, OUT, 2>(p, end, st) : launch_split_inst<64, EPI, OUT, 2>(p, end, st);
   }
-  if (bn == 256) return launch_split_inst<256, EPI, OUT, 1>(p, end, st);
-  if (bn == 128) return launch_split_inst<128, EPI, OUT, 1>(p, end, st);
-  return launch_split_inst<64, EPI, OUT, 1>(p, end, st);
+  return bn == 128 ? launch_split_inst<128, EPI, OUT, 1>(p, end, st) : launch_split_inst<64, EPI, OUT, 1>(p, end, st);
 }
 
 int validate_split(const SplitGemmProblem& q, int N, int K) {
@@ -571,15 +569,16 @@ long max_clusters_of_four() {
 
 // The tile width (and, for the gate + residual GEMMs, whether two pairs share a tile's K) with the least
 // (waves over the CTA pairs) x (K blocks of a pair) x (time of a block).  In units of 24 cycles a
-// block is 24 MMAs of 128 / 64 cycles, and at PBN = 64 the 480 rows of TMA per CTA; handing the
-// sums over costs two cluster barriers and PBN / 2 KiB of distributed shared memory per CTA.
+// block takes 74 at PBN = 128 (measured: 24 MMAs of 64 cycles, a seventh on top) and 56 at PBN = 64 (480
+// rows of TMA per CTA); handing the sums over costs two cluster barriers and PBN / 2 KiB of
+// distributed shared memory per CTA.
 int choose_split_width(long row_tiles, int N, int k_blocks, bool may_split, int* ksplit) {
   const long pairs = device_sm_count() / 2 > 0 ? device_sm_count() / 2 : 1;
-  int best = 256;
+  int best = 128;
   long best_cost = 0;
-  const int bn[3] = {256, 128, 64}, cost[3] = {128, 68, 52};
+  const int bn[2] = {128, 64}, cost[2] = {74, 56};
   *ksplit = 1;
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < 2; ++i) {
     const long tiles = row_tiles * ((N + bn[i] - 1) / bn[i]);
     const long c = (tiles + pairs - 1) / pairs * cost[i] * k_blocks;
     if (i == 0 || c < best_cost) { best = bn[i]; best_cost = c; *ksplit = 1; }

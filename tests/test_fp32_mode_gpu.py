@@ -1,6 +1,6 @@
 """The fp32 mode's blocks against the oracle in float64, at the sizes where the tensor-core kernels
 behind it (fp32 operands as three bf16 planes) can go wrong: partial row and column tiles, every tile
-width, ragged and single key tiles, remainders of the 32-wide K blocks, unfused head sizes.
+width, ragged and single key tiles, remainders of the 64-wide K blocks, unfused head sizes.
 
 Tolerance: a block output passes through on the order of a thousand fp32 roundings (four chained
 GEMMs of K / 32 additions, LayerNorm sums, softmax), a random walk of 2^-24 steps: sqrt(1000) * 2^-24
@@ -21,9 +21,9 @@ pytestmark = pytest.mark.gpu
     (192, 3, 2, 129, 77, False, True),     # last block: no context output
     (72, 3, 2, 40, 24, True, False),       # head_dim 24: unfused norm, K with a remainder of 8
     (128, 4, 1, 130, 33, True, False),     # head_dim 32
-    (1536, 24, 1, 256, 77, True, False),   # narrow tiles
-    (1536, 24, 1, 1024, 333, True, False), # 128-wide tiles
-    (1536, 24, 4, 1000, 154, False, False),# 256-wide tiles
+    (1536, 24, 1, 256, 77, True, False),   # 64-wide tiles, K split
+    (1536, 24, 1, 1024, 333, True, False),  # 128-wide tiles
+    (1536, 24, 4, 1000, 154, False, False), 
 ])
 def test_block_fp32_against_float64(sd3, E, NH, B, Tx, Tc, dual, last):
     gen = torch.Generator().manual_seed(E + 7 * Tx + Tc)
