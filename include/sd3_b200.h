@@ -46,7 +46,7 @@ extern "C" {
 
 /* precision modes of a model */
 #define SD3_PRECISION_BF16 0 /* bf16 tensor-core operands, fp32 accumulation / residual streams */
-#define SD3_PRECISION_F32 1  /* exact fp32 arithmetic (parity mode for fp32 tensors) */
+#define SD3_PRECISION_F32 1  /* fp32 accuracy (parity mode for fp32 tensors; operands split into bf16 planes) */
 #define SD3_PRECISION_FP8 2  /* bf16 mode with the block GEMMs on e4m3 operands (one scale per weight matrix) */
 
 /* epilogues of sd3_linear */

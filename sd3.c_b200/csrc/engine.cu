@@ -10,10 +10,10 @@
 // the caller's stream, nothing synchronises.
 //
 // Per block the launch sequence is
-//   LN+modulate(x), LN+modulate(c) in one launch (both modulations of a dual block at once)
+//   LN+modulate(x), LN+modulate(c) (both modulations of a dual block at once; one launch up to MERGE_MAX_ROWS)
 //   QKV GEMM(x), (c)         -> packed (B, Tc+Tx, 3E), RMSNorm fused, context rows first; a dual block's
-//                               second QKV GEMM(x) rides in the same launch
-//   joint attention          -> o_c, o_x; a dual block's attention over the image tokens in the same launch
+//                               second QKV GEMM(x) rides in the same launch (up to MERGE_MAX_ROWS)
+//   joint attention          -> o_c, o_x; a dual block's attention over the image tokens too
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
 //   [dual] out-proj GEMM with gate2
 //   LN+modulate(x), (c); MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual), each for x and c at once
@@ -519,9 +519,17 @@ int run_mlp1(sd3_model* m, const Linear& L, const Linear& next, const void* A, i
   return run_linear(m, L, A, M, e, st, a_e4m3);
 }
 
-// the LayerNorms of the image and the context rows as one launch where both write the same type
+// Launches are merged (LayerNorms of both streams, the two QKV projections and the two attentions of a dual
+// block) up to this many rows.  Below, a kernel is little more than its latency; measured on the
+// forward (merged against separate): LayerNorms 256x256 5.6 %, 1024x1024 1.6 %, four 512x512 nothing; QKV 256x256
+// 4.8 %, 512x512 1.4 %, 1024x1024 0.2 %.  Above there is nothing to gain, and eight 1024x1024
+// images were 0.8 % slower with everything merged.
+constexpr long MERGE_MAX_ROWS = 16384;
+
+// the LayerNorms of the image and the context rows, as one launch where both write the same type
 int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st) {
-  if (!pc || out_x == out_c) return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
+  const long rows = static_cast<long>(px.B) * px.T + (pc ? static_cast<long>(pc->B) * pc->T : 0);
+  if (!pc || (out_x == out_c && rows <= MERGE_MAX_ROWS)) return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
   int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st);
   return rc ? rc : launch_ln_modulate(px, nullptr, E, 1e-6f, ms, out_x, st);
 }
@@ -565,6 +573,8 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const bool pre_j = L.c_wq_s != nullptr && L.x_wq_s != nullptr;
   const float* c_wq = pre_j ? L.c_wq_s : L.c_wq;
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
+  // a dual block's image-only attention beside the joint one, or after it
+  const bool together = L.dual && m->D == 64 && static_cast<long>(B) * (2L * Tx + Tc) <= MERGE_MAX_ROWS;
   const bool pre_d = L.d_wq_s != nullptr;
   const float* d_wq = pre_d ? L.d_wq_s : L.d_wq;
   if (m->D == 64) {
@@ -573,7 +583,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
         {&L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk), x8a},
         {&L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, B, Tc, T, 0, c_wq, L.c_wk), c8a},
         {&L.d_qkv, w.h_x2, B * Tx, qkv_epilogue(m, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk), x8a}};
-    SD3_TRY(run_linear_group(m, qkv, L.dual ? 3 : 2, st));
+    SD3_TRY(run_linear_group(m, qkv, together ? 3 : 2, st));
   } else {
     SD3_TRY(run_qkv(m, L.c_qkv, w.h_c, w.qkv, B, Tc, T, 0, c_wq, L.c_wk, st, c8a));
     SD3_TRY(run_qkv(m, L.x_qkv, w.h_x, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk, st, x8a));
@@ -582,10 +592,9 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   // kernel to write it (one flag for both outputs)
   const bool o8 = m->fp8 && m->D == 64 && L.x_out.w8 && (L.last || L.c_out.w8);
   const bool o8d = m->fp8 && m->D == 64 && L.d_out.w8;
-  if (m->D != 64 && L.dual) SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
   const AttnCall att[2] = {{w.qkv, T, Tc, L.last ? nullptr : w.o_c, w.o_x, o8, L.joint_bound, pre_j},
                            {w.qkv2, Tx, 0, nullptr, w.o_x2, o8d, L.dual_bound, pre_d}};
-  SD3_TRY(run_attention(m, att, L.dual ? 2 : 1, B, st));
+  SD3_TRY(run_attention(m, att, together ? 2 : 1, B, st));
   if (grouped && !L.last) {
     SD3_TRY(run_linear_pair(m, L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8,
                             L.c_out, w.o_c, B * Tc, gate_epilogue(L.c_out, Tc, c_gate_a, ms, c), o8, st));
@@ -593,7 +602,13 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     if (!L.last) SD3_TRY(run_gate_resid(m, L.c_out, w.o_c, B, Tc, c_gate_a, ms, c, st, o8));
     SD3_TRY(run_gate_resid(m, L.x_out, w.o_x, B, Tx, x_gate_a, ms, x, st, o8));
   }
-  if (L.dual) SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
+  if (L.dual) {
+    if (!together) {
+      SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
+      SD3_TRY(run_attention(m, att + 1, 1, B, st));
+    }
+    SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
+  }
   // MLPs of both streams: LayerNorm + modulate each, then the two first linears (GELU-tanh) and
   // the two second linears (gate + residual), each pair as one grouped launch
   {

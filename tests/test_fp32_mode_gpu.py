@@ -23,7 +23,7 @@ pytestmark = pytest.mark.gpu
     (128, 4, 1, 130, 33, True, False),     # head_dim 32
     (1536, 24, 1, 256, 77, True, False),   # 64-wide tiles, K split
     (1536, 24, 1, 1024, 333, True, False),  # 128-wide tiles
-    (1536, 24, 4, 1000, 154, False, False), 
+    (1536, 24, 4, 1000, 154, False, False),  # several waves of them
 ])
 def test_block_fp32_against_float64(sd3, E, NH, B, Tx, Tc, dual, last):
     gen = torch.Generator().manual_seed(E + 7 * Tx + Tc)
