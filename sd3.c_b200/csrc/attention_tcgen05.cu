@@ -256,12 +256,15 @@ __device__ __forceinline__ void exp2_pack(uint32_t (&r)[32], float c, float2& ac
 // UNIT (bounded mode only): the queries were multiplied by scale log2(e) where they were formed
 // (the engine folds the factor into the RMSNorm weight of q), so a score is its own exp2
 // argument: one packed multiply per pair of scores less (measured: 4 % of the kernel).
-template <bool BOUNDED, bool UNIT>
+// PAIR: the launch carries two attentions (a launch of one keeps its parameters at fixed places and some
+// registers fewer: 152 instead of 156 to 161).  With it and separate launches above 16384 rows,
+// eight 1024x1024 images take 96.17 ms against 96.03 before launches were merged, 2048x2048 99.64 against 99.68.
+template <bool BOUNDED, bool UNIT, bool PAIR>
 __global__ void __launch_bounds__(AT_THREADS, 2)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
                          const __grid_constant__ AttnArgs a0, const __grid_constant__ AttnArgs a1, const int grid0) {
   // grid.x: the CTAs of the first attention, then those of the second (the image-only one of a dual block)
-  const bool second = static_cast<int>(blockIdx.x) >= grid0;
+  const bool second = PAIR && static_cast<int>(blockIdx.x) >= grid0;
   const CUtensorMap& tmQKV = second ? tm1 : tm0;
   const AttnArgs& a = second ? a1 : a0;
   const int bx = second ? static_cast<int>(blockIdx.x) - grid0 : static_cast<int>(blockIdx.x);
@@ -645,14 +648,12 @@ int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_
   if (dev >= 0 && dev < 64) {
     std::lock_guard<std::mutex> lock(attr_mutex);
     if (!attr_done[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<false, false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM_BYTES);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(attention_tcgen05_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 AT_SMEM_BYTES);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(attention_tcgen05_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 AT_SMEM_BYTES);
+      cudaError_t e = cudaSuccess;
+      for (auto kern : {attention_tcgen05_kernel<false, false, false>, attention_tcgen05_kernel<true, false, false>,
+                        attention_tcgen05_kernel<true, true, false>, attention_tcgen05_kernel<false, false, true>,
+                        attention_tcgen05_kernel<true, false, true>, attention_tcgen05_kernel<true, true, true>})
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM_BYTES);
       if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(attention)");
       attr_done[dev] = true;
     }
@@ -706,15 +707,13 @@ int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_
   for (int i = 0; i < (merged ? 1 : n); ++i) {
     const int j = merged ? 1 : i;
     const dim3 g(merged ? grid[0] + grid[1] : grid[i], NH, B);
-    if (mode[i] == 2)
-      launch_dependent(attention_tcgen05_kernel<true, true>, g, AT_THREADS, AT_SMEM_BYTES, stream, tm[i], tm[j], a[i],
-                       a[j], grid[i]);
-    else if (mode[i] == 1)
-      launch_dependent(attention_tcgen05_kernel<true, false>, g, AT_THREADS, AT_SMEM_BYTES, stream, tm[i], tm[j], a[i],
-                       a[j], grid[i]);
-    else
-      launch_dependent(attention_tcgen05_kernel<false, false>, g, AT_THREADS, AT_SMEM_BYTES, stream, tm[i], tm[j],
-                       a[i], a[j], grid[i]);
+    auto kern = mode[i] == 2   ? (merged ? attention_tcgen05_kernel<true, true, true>
+                                         : attention_tcgen05_kernel<true, true, false>)
+                : mode[i] == 1 ? (merged ? attention_tcgen05_kernel<true, false, true>
+                                         : attention_tcgen05_kernel<true, false, false>)
+                               : (merged ? attention_tcgen05_kernel<false, false, true>
+                                         : attention_tcgen05_kernel<false, false, false>);
+    launch_dependent(kern, g, AT_THREADS, AT_SMEM_BYTES, stream, tm[i], tm[j], a[i], a[j], grid[i]);
     int rc = after_launch("attention_tcgen05_kernel");
     if (rc) return rc;
     if (a[i].kv_split > 1) {
