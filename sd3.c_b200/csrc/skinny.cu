@@ -10,7 +10,15 @@
 // takes, as they did in the kernel this replaced (weights straight into registers, loads
 // and arithmetic in turn).  Measured, before -> after, 1 / 8 samples: 502272 x 1536 fp32
 // 721 / 1389 -> 595 / 1285 us (5.2 / 2.4 TB/s of weights), 23040 x 1536 (one dual block) fp32 48 / 85 ->
-// 34 / 68 us, bf16 43 / 72 -> 22 / 54 us.  With eight samples the activations' shared-memory reads bound it.
+// 34 / 68 us, bf16 43 / 72 -> 22 / 57 us.  With eight samples the activations' shared-memory reads bound it.
+//
+// The order of a sum is part of the result: it decides the last bits of the conditioning vector, some of
+// which then round to the neighbouring bf16 and reach every block.  With bf16 weights lane l adds the
+// products of k = 256 i + 8 l + j in the order of i and j (16 bytes of a weight row per lane and step), then
+// the lanes are added pairwise, 16 apart first: the bits of the kernel that this one replaced.  With fp32 weights a lane
+// takes 4 consecutive elements, k = 128 i + 4 l + j, also 16 bytes; 8 would cost 595 -> 937 us on
+// 502272 x 1536 (two loads per row and step, shorter chunks), and the fp32 model's GEMMs
+// sum in another order than before in any case.
 //
 // R = 4 for matrices that give every SM work for several rounds, R = 1 for the
 // small ones (1536 rows: 192 CTAs instead of 48, the chain of K chunks is what they take).
@@ -35,6 +43,7 @@ constexpr int SK_CHUNK = 1536;                 // bytes of a weight row per stag
 template <typename WT, int R, int BC>
 struct SkinnyCfg {
   static constexpr int KC = SK_CHUNK / static_cast<int>(sizeof(WT));  // K elements per stage
+  static constexpr int VK = 16 / static_cast<int>(sizeof(WT));        // consecutive elements of K per lane and step
   static constexpr int ROWS = SK_WARPS * R;
   static constexpr int W_BYTES = ROWS * SK_CHUNK;
   static constexpr int X_BYTES = BC * KC * 4;
@@ -64,16 +73,19 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
 }
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-  const uint2 u = *reinterpret_cast<const uint2*>(p);
-  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
-                     __uint_as_float(u.y & 0xffff0000u));
+// elements 2 i and 2 i + 1 of the words of a packed weight vector as floats
+__device__ __forceinline__ float4 unpack4(uint32_t a, uint32_t b) {
+  return make_float4(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u), __uint_as_float(b << 16),
+                     __uint_as_float(b & 0xffff0000u));
+}
+__device__ __forceinline__ float dot4(const float4& x, const float4& w, float acc) {
+  return fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc))));
 }
 
 template <typename WT, int R, int BC>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_stream_kernel(const SkinnyArgs a) {
   using Cfg = SkinnyCfg<WT, R, BC>;
-  constexpr int KC = Cfg::KC, STAGES = Cfg::STAGES;
+  constexpr int KC = Cfg::KC, VK = Cfg::VK, STAGES = Cfg::STAGES;
   extern __shared__ __align__(128) uint8_t sk_smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(sk_smem + STAGES * Cfg::STAGE);
   uint64_t* empty = full + STAGES;
@@ -146,19 +158,32 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_stream_kernel(const Skin
           const uint8_t* st = sk_smem + s * Cfg::STAGE;
           const float* xs = reinterpret_cast<const float*>(st + Cfg::W_BYTES);
 #pragma unroll
-          for (int i = 0; i < KC / 128; ++i) {
-            const int k = 128 * i + 4 * lane;
+          for (int i = 0; i < KC / (32 * VK); ++i) {
+            const int k = 32 * VK * i + VK * lane;
             if (k < len) {  // K is a multiple of 8
-              float4 w[R];
+              uint4 w[R];
 #pragma unroll
               for (int r = 0; r < R; ++r)
-                w[r] = load4(reinterpret_cast<const WT*>(st + (warp * R + r) * SK_CHUNK) + k);
+                w[r] = *reinterpret_cast<const uint4*>(reinterpret_cast<const WT*>(st + (warp * R + r) * SK_CHUNK) + k);
 #pragma unroll
               for (int b = 0; b < BC; ++b) {
-                const float4 x = load4(xs + b * KC + k);
+                const float* xp = xs + b * KC + k;
+                if constexpr (VK == 4) {
+                  const float4 x = load4(xp);
 #pragma unroll
-                for (int r = 0; r < R; ++r)
-                  acc[r][b] = fmaf(x.w, w[r].w, fmaf(x.z, w[r].z, fmaf(x.y, w[r].y, fmaf(x.x, w[r].x, acc[r][b]))));
+                  for (int r = 0; r < R; ++r)
+                    acc[r][b] = dot4(x, make_float4(__uint_as_float(w[r].x), __uint_as_float(w[r].y),
+                                                    __uint_as_float(w[r].z), __uint_as_float(w[r].w)), acc[r][b]);
+                } else {
+                  // 32 bytes per lane: every other group of four lanes reads its halves in the opposite
+                  // order, so that eight lanes cover all banks
+                  const int swap = lane & 4;
+                  const float4 u = load4(xp + swap), v = load4(xp + 4 - swap);
+                  const float4 x0 = swap ? v : u, x1 = swap ? u : v;
+#pragma unroll
+                  for (int r = 0; r < R; ++r)
+                    acc[r][b] = dot4(x1, unpack4(w[r].z, w[r].w), dot4(x0, unpack4(w[r].x, w[r].y), acc[r][b]));
+                }
               }
             }
           }
