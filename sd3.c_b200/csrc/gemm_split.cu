@@ -21,11 +21,14 @@
 // Two CTAs (a cluster on neighbouring SMs) share a 256 x PBN tile with
 // tcgen05.mma.cta_group::2 and walk tiles persistently: each CTA's warp 0 streams the
 // planes of its 128 rows of A and its half of W with TMA (3-D boxes of 64 K x rows
-// x 3 planes), two threads of the even CTA issue the 24 MMAs of every K block (blocks in turn: a
-// block has its own accumulator, so the threads need no order between them and the
+// x 3 planes), two threads of the even CTA issue the 24 MMAs of every K block (blocks in turn, so the
 // barrier work of one runs under the MMAs of the other), the epilogue warps of both add
 // up the blocks and run the fused epilogue.  Four accumulators rotate, so the adds run
 // under the MMAs of the following blocks.
+//
+// A block has its own accumulator, so no order is needed between the MMAs of the two threads; but each
+// thread waits for its own blocks only, and the ring has three stages: the barriers that announce
+// landed operands are laid out by operand_ring.h so that a thread sees every phase of those it waits on.
 //
 // K split: where one wave of tiles leaves half of the SMs without work, two CTA pairs
 // (a cluster of four) share a tile, each takes half of K, and the second pair hands
@@ -48,6 +51,7 @@
 
 #include "gemm_epilogue.cuh"
 #include "kernels.h"
+#include "operand_ring.h"
 #include "ptx.cuh"
 #include "split3.cuh"
 
@@ -75,11 +79,15 @@ struct SplitCfg {
   static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);  // 72 / 60 KiB
   static constexpr int STAGES = 3;                               // 216 / 180 KiB
   static constexpr int NBUF = 4;                                 // TMEM accumulators
+  static_assert(NBUF % 2 == 0, "an accumulator belongs to one of the two MMA-issuing threads");
   static constexpr int TMEM_COLS = NBUF * PBN;
   static constexpr int EPI_WARPS = PBN == 64 ? 4 : 8;
   static constexpr int CPW = 64;                     // accumulator columns per epilogue thread
   static constexpr int MMA2_WARP = 2 + EPI_WARPS;    // second MMA-issuing warp
   static constexpr int THREADS = 32 * (3 + EPI_WARPS);
+  using Ring = OperandRing<STAGES, 2>;  // two MMA-issuing threads
+  static constexpr int BAR_BYTES = (Ring::FULL_BARS + STAGES + 2 * NBUF) * 8 + 8;  // barriers, TMEM address, abort flag
+  static_assert(BAR_BYTES <= 256, "barrier block");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
 };
 
@@ -232,6 +240,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
                           const __grid_constant__ SplitProblem p2, const int end0, const int end1,
                           const int num_tiles) {
   using Cfg = SplitCfg<PBN>;
+  using Ring = typename Cfg::Ring;
   constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, CPW = Cfg::CPW;
   constexpr uint32_t IDESC = make_idesc(1, 1, 2 * S_BM, PBN, 0, 0);
 
@@ -239,7 +248,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
-  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* empty_bar = full_bar + Ring::FULL_BARS;
   uint64_t* tfull_bar = empty_bar + STAGES;
   uint64_t* tempty_bar = tfull_bar + NBUF;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + NBUF);
@@ -255,10 +264,8 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   const int num_pairs = gridDim.x / (2 * KSPLIT);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);   // leader's expect_tx arrival; bytes of both CTAs
-      mbar_init(&empty_bar[s], 1);  // one multicast commit per use
-    }
+    for (int s = 0; s < Ring::FULL_BARS; ++s) mbar_init(&full_bar[s], 1);  // leader's expect_tx arrival; bytes of both CTAs
+    for (int s = 0; s < STAGES; ++s) mbar_init(&empty_bar[s], 1);          // one multicast commit per use
     for (int a = 0; a < NBUF; ++a) {
       mbar_init(&tfull_bar[a], 1);
       mbar_init(&tempty_bar[a], 2 * Cfg::EPI_WARPS);  // epilogue warps of both CTAs (leader's copy is used)
@@ -298,21 +305,21 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
 
   if (warp == 0 && lane == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------
-    int stage = 0;
-    uint32_t phase = 0;
+    Ring ring;
     bool ok = true;
     // the weights of a stage; all its bytes (both CTAs) are credited to the leader's barrier
-    auto load_w = [&](const SplitProblem& pp, int st, int kb, int n0) {
-      if (rank == 0) mbar_expect_tx(&full_bar[st], 2 * Cfg::STAGE_BYTES);
-      tma_load_3d_pair(smem + st * Cfg::STAGE_BYTES + 3 * S_A_PLANE, &pp.tmW, map_to_cta(smem_u32(&full_bar[st]), leader),
-                       (kb0 + kb) * S_KB, n0, 0);
+    auto load_w = [&](const SplitProblem& pp, const Ring& at, int kb, int n0) {
+      if (rank == 0) mbar_expect_tx(&full_bar[at.full], 2 * Cfg::STAGE_BYTES);
+      tma_load_3d_pair(smem + at.stage * Cfg::STAGE_BYTES + 3 * S_A_PLANE, &pp.tmW,
+                       map_to_cta(smem_u32(&full_bar[at.full]), leader), (kb0 + kb) * S_KB, n0, 0);
     };
     int pre = 0;  // stages of the first tile whose weights are under way before the wait
     if (p0.g.epi.w_static) {
       const SplitProblem& pp = pair < end0 ? p0 : pair < end1 ? p1 : p2;
       const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
-      for (; pre < STAGES && pre < KB; ++pre)
-        load_w(pp, pre, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS);
+      Ring at;
+      for (; pre < STAGES && pre < KB; ++pre, at.next())
+        load_w(pp, at, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS);
     }
     grid_dep_wait();
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -324,29 +331,30 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
         if (pre > 0) {
           --pre;
         } else {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-          load_w(pp, stage, kb, n0);
+          if (!mbar_wait(&empty_bar[ring.stage], ring.stage_parity ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+          load_w(pp, ring, kb, n0);
         }
-        tma_load_3d_pair(smem + stage * Cfg::STAGE_BYTES, &pp.tmA, map_to_cta(smem_u32(&full_bar[stage]), leader),
+        tma_load_3d_pair(smem + ring.stage * Cfg::STAGE_BYTES, &pp.tmA, map_to_cta(smem_u32(&full_bar[ring.full]), leader),
                          (kb0 + kb) * S_KB, m0, 0);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        ring.next();
       }
     }
   } else if ((warp == 1 || warp == Cfg::MMA2_WARP) && lane == 0) {
     // ------------------------------ MMA issuers (leader only) -----------------
     if (rank == 0) {
       const int me = warp == 1 ? 0 : 1;
-      int stage = 0, buf = 0, turn = 0;
-      uint32_t phase = 0, bphase = 0;
+      Ring ring;
+      int buf = 0;  // four accumulators: a thread sees every use of its two
+      uint32_t bphase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         for (int kb = 0; kb < KB; ++kb) {
-          if (turn == me) {
+          if (ring.turn == me) {
             if (!mbar_wait(&tempty_bar[buf], bphase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-            if (!mbar_wait(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
+            if (!mbar_wait(&full_bar[ring.full], ring.full_parity, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * PBN);
-            const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+            const uint32_t a_addr = smem_u32(smem + ring.stage * Cfg::STAGE_BYTES);
             const uint64_t a0 = make_smem_desc_sw128(a_addr, 16, 1024);
             const uint64_t w0 = make_smem_desc_sw128(a_addr + 3 * S_A_PLANE, 16, 1024);
             constexpr uint64_t AP = S_A_PLANE >> 4, WP = Cfg::W_PLANE >> 4;
@@ -357,11 +365,10 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
 #pragma unroll
               for (int k = 0; k < S_KB / 16; ++k)
                 mma_f16_ss_pair(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
-            mma_commit_pair(&empty_bar[stage], pair_mask);  // frees the stage in both CTAs
+            mma_commit_pair(&empty_bar[ring.stage], pair_mask);  // frees the stage in both CTAs
             mma_commit_pair(&tfull_bar[buf], pair_mask);    // block sum ready in both CTAs
           }
-          turn ^= 1;
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          ring.next();
           if (++buf == NBUF) { buf = 0; bphase ^= 1; }
         }
       }
