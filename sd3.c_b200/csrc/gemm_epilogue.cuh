@@ -92,24 +92,13 @@ __device__ __forceinline__ void store8(void* out, long idx, const float* o) {
   }
 }
 
-// `count` groups of 4 floats starting at p into dst (zeros past column N)
+// GROUPS groups of 4 floats starting at p into dst (zeros past column N, or without p)
 template <int GROUPS>
 __device__ __forceinline__ void load_f4_batch(const float* p, int n_base, int N, float (&dst)[GROUPS * 4]) {
 #pragma unroll
   for (int i = 0; i < GROUPS; ++i) {
     float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p != nullptr && n_base + i * 4 < N) t = __ldg(reinterpret_cast<const float4*>(p + n_base) + i);
-    dst[4 * i] = t.x; dst[4 * i + 1] = t.y; dst[4 * i + 2] = t.z; dst[4 * i + 3] = t.w;
-  }
-}
-
-// same, through ordinary (coherent) loads: for data this kernel also writes
-template <int GROUPS>
-__device__ __forceinline__ void load_f4_batch_rw(const float* p, int n_base, int N, float (&dst)[GROUPS * 4]) {
-#pragma unroll
-  for (int i = 0; i < GROUPS; ++i) {
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n_base + i * 4 < N) t = *(reinterpret_cast<const float4*>(p + n_base) + i);
+    if (p != nullptr && n_base + i * 4 < N) t = *(reinterpret_cast<const float4*>(p + n_base) + i);
     dst[4 * i] = t.x; dst[4 * i + 1] = t.y; dst[4 * i + 2] = t.z; dst[4 * i + 3] = t.w;
   }
 }
@@ -274,7 +263,7 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
     const int nw = n0 + half * COLS_PER_WARP;
     float rr[32], gg[32], bb[32];
     if (valid) {
-      load_f4_batch_rw<8>(res_row, nw, g.N, rr);
+      load_f4_batch<8>(res_row, nw, g.N, rr);
       load_f4_batch<8>(gate_row, nw, g.N, gg);
       load_f4_batch<8>(e.bias, nw, g.N, bb);
     }
@@ -291,7 +280,7 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
       for (int j = 0; j < 32; ++j)
         o[j] = fmaf(gg[j], fmaf(__uint_as_float(r[j]), e.alpha, bb[j]), rr[j]);
       if (sub + 1 < NSUB && valid) {  // next sub-chunk's parameters, in flight during the stores
-        load_f4_batch_rw<8>(res_row, n_base + 32, g.N, rr);
+        load_f4_batch<8>(res_row, n_base + 32, g.N, rr);
         load_f4_batch<8>(gate_row, n_base + 32, g.N, gg);
         load_f4_batch<8>(e.bias, n_base + 32, g.N, bb);
       }

@@ -119,7 +119,7 @@ __device__ __forceinline__ void split_epilogue_64(float* v, const RowMap& rm, in
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       if (n_base + 4 * i < N) {
-        const float4 t = __ldg(reinterpret_cast<const float4*>(e.bias + n_base) + i);
+        const float4 t = *(reinterpret_cast<const float4*>(e.bias + n_base) + i);
         v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
       }
     }
@@ -138,7 +138,7 @@ __device__ __forceinline__ void split_epilogue_64(float* v, const RowMap& rm, in
       const float r = rsqrtf(((s0 + s1) + (s2 + s3)) * (1.0f / 64.0f) + e.eps);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float4 t = w ? __ldg(reinterpret_cast<const float4*>(w) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 t = w ? *(reinterpret_cast<const float4*>(w) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
         v[4 * i] = v[4 * i] * r * t.x;
         v[4 * i + 1] = v[4 * i + 1] * r * t.y;
         v[4 * i + 2] = v[4 * i + 2] * r * t.z;
@@ -155,7 +155,7 @@ __device__ __forceinline__ void split_epilogue_64(float* v, const RowMap& rm, in
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       if (n_base + 4 * i < N) {
-        const float4 t = __ldg(t4 + i);
+        const float4 t = t4[i];
         v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
       }
     }
@@ -182,11 +182,11 @@ __device__ __forceinline__ void split_epilogue_64(float* v, const RowMap& rm, in
   const long base = rm.orow * e.ldo + n_base;
   if constexpr (EPI == EPI_GATE_RESID) {
     const float4* g4 = reinterpret_cast<const float4*>(e.gate + static_cast<long>(rm.b) * e.gate_stride + n_base);
-    const float4* r4 = reinterpret_cast<const float4*>(e.resid + base);  // also written here: ordinary loads
+    const float4* r4 = reinterpret_cast<const float4*>(e.resid + base);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       if (n_base + 4 * i < N) {
-        const float4 t = __ldg(g4 + i), x = r4[i];
+        const float4 t = g4[i], x = r4[i];
         v[4 * i] = x.x + t.x * v[4 * i];
         v[4 * i + 1] = x.y + t.y * v[4 * i + 1];
         v[4 * i + 2] = x.z + t.z * v[4 * i + 2];

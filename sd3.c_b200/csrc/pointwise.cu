@@ -91,15 +91,15 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
   float4* s_sc2 = ln_smem + 2 * nvec;
   float4* s_sh2 = ln_smem + 3 * nvec;
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    float4 s = __ldg(reinterpret_cast<const float4*>(p.scale1 + b_cta * mod_stride) + i);
+    float4 s = *(reinterpret_cast<const float4*>(p.scale1 + b_cta * mod_stride) + i);
     s.x += 1.f; s.y += 1.f; s.z += 1.f; s.w += 1.f;
     s_sc1[i] = s;
-    s_sh1[i] = __ldg(reinterpret_cast<const float4*>(p.shift1 + b_cta * mod_stride) + i);
+    s_sh1[i] = *(reinterpret_cast<const float4*>(p.shift1 + b_cta * mod_stride) + i);
     if (dual) {
-      float4 s2 = __ldg(reinterpret_cast<const float4*>(p.scale2 + b_cta * mod_stride) + i);
+      float4 s2 = *(reinterpret_cast<const float4*>(p.scale2 + b_cta * mod_stride) + i);
       s2.x += 1.f; s2.y += 1.f; s2.z += 1.f; s2.w += 1.f;
       s_sc2[i] = s2;
-      s_sh2[i] = __ldg(reinterpret_cast<const float4*>(p.shift2 + b_cta * mod_stride) + i);
+      s_sh2[i] = *(reinterpret_cast<const float4*>(p.shift2 + b_cta * mod_stride) + i);
     }
   }
 #pragma unroll 1
@@ -149,8 +149,8 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
           if (cached) {
             s = s_sc1[i]; h = s_sh1[i];
           } else {
-            s = __ldg(reinterpret_cast<const float4*>(p.scale1 + moff) + i);
-            h = __ldg(reinterpret_cast<const float4*>(p.shift1 + moff) + i);
+            s = *(reinterpret_cast<const float4*>(p.scale1 + moff) + i);
+            h = *(reinterpret_cast<const float4*>(p.shift1 + moff) + i);
             s.x += 1.f; s.y += 1.f; s.z += 1.f; s.w += 1.f;
           }
           float4 o;
@@ -165,8 +165,8 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
           if (cached) {
             s = s_sc2[i]; h = s_sh2[i];
           } else {
-            s = __ldg(reinterpret_cast<const float4*>(p.scale2 + moff) + i);
-            h = __ldg(reinterpret_cast<const float4*>(p.shift2 + moff) + i);
+            s = *(reinterpret_cast<const float4*>(p.scale2 + moff) + i);
+            h = *(reinterpret_cast<const float4*>(p.shift2 + moff) + i);
             s.x += 1.f; s.y += 1.f; s.z += 1.f; s.w += 1.f;
           }
           float4 o;
@@ -209,7 +209,7 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   return after_launch("ln_modulate_kernel");
 }
 
-__global__ void sinusoidal_kernel(const float* __restrict__ t, float* __restrict__ out, int B,
+__global__ void sinusoidal_kernel(const float* t, float* out, int B,
                                   int dim) {
   grid_dep_wait();
   grid_dep_launch();
@@ -253,7 +253,7 @@ template <> __device__ __forceinline__ float convert_elem<bf16, float>(bf16 v) {
 template <> __device__ __forceinline__ bf16 convert_elem<bf16, bf16>(bf16 v) { return v; }
 
 template <typename IT, typename OT, bool SPLIT = false>
-__global__ void patchify_kernel(const IT* __restrict__ latent, OT* __restrict__ out, int B, int C,
+__global__ void patchify_kernel(const IT* latent, OT* out, int B, int C,
                                 int H, int W, int p) {
   grid_dep_wait();
   grid_dep_launch();
@@ -282,7 +282,7 @@ __global__ void patchify_kernel(const IT* __restrict__ latent, OT* __restrict__ 
 }
 
 template <typename IT, typename OT>
-__global__ void cast_kernel(const IT* __restrict__ in, OT* __restrict__ out, long n) {
+__global__ void cast_kernel(const IT* in, OT* out, long n) {
   grid_dep_wait();
   grid_dep_launch();
   long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -309,7 +309,7 @@ __global__ void transpose_kernel(const IT* __restrict__ in, OT* __restrict__ out
 
 // VEC: in is aligned to four elements (a caller's captions need not be)
 template <typename IT, bool VEC>
-__global__ void split3_kernel(const IT* __restrict__ in, bf16* __restrict__ out, long n) {
+__global__ void split3_kernel(const IT* in, bf16* out, long n) {
   grid_dep_wait();
   grid_dep_launch();
   long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
@@ -356,8 +356,8 @@ __global__ void transpose_split3_kernel(const IT* __restrict__ in, bf16* __restr
 }
 
 template <typename XT>
-__global__ void rmsnorm_heads_kernel(XT* __restrict__ x, long ld, long rows, int col0, int nheads,
-                                     int D, const float* __restrict__ w, float eps) {
+__global__ void rmsnorm_heads_kernel(XT* x, long ld, long rows, int col0, int nheads,
+                                     int D, const float* w, float eps) {
   grid_dep_wait();
   grid_dep_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -459,7 +459,7 @@ int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int 
 namespace {
 
 template <typename TI>
-__global__ void quantize_e4m3_kernel(const TI* __restrict__ in, uint8_t* __restrict__ out, long n,
+__global__ void quantize_e4m3_kernel(const TI* in, uint8_t* out, long n,
                                      float inv_scale) {
   grid_dep_wait();
   grid_dep_launch();
