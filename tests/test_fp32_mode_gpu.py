@@ -72,6 +72,37 @@ def test_attention_sublayer_fp32_against_float64(sd3, E, NH, B, Tx, Tc):
     assert max(branch_errors(sd3, p, E, NH, x, c, y, True, False)) < TOLERANCE
 
 
+@pytest.mark.parametrize("what", ["activation", "weight", "infinite activation"])
+def test_values_above_bf16_range(sd3, what):
+    """The end of float32's range lies above bf16's (3.4028e38, 3.3895e38): such an operand of the second MLP linear
+    counts with its value, and an infinite one makes its row infinite with the signs of its weights."""
+    E, big = 64, 3.4e38
+    gen = torch.Generator().manual_seed(5)
+    p = O.random_params(O.block_param_shapes(E, 4, E, False, False, True), seed=5, std=0.1, bias_std=0.02, norm_std=0.3)
+    x, c = torch.randn(2, 65, E, generator=gen), torch.randn(2, 20, E, generator=gen)
+    y = torch.nn.functional.silu(torch.randn(2, E, generator=gen))
+    w1, b1, w2 = (p["latent_mlp." + k] for k in ("lin1.weight", "lin1.bias", "lin2.weight"))
+    w1[:, 0] = 0.0  # hidden channel 0 is gelu(b1[0])
+    b1[0] = {"activation": big, "weight": 1e-30, "infinite activation": float("inf")}[what]
+    if what == "activation":
+        w2[0] = 1e-30 * torch.randn(E, generator=gen)
+    if what == "weight":
+        w2[0] = big
+    if what != "infinite activation":
+        assert max(branch_errors(sd3, p, E, 1, x, c, y, False, False)) < TOLERANCE
+        return
+    m = sd3.Model(1, [], 0, 0, 0, E, 1, 4, 0, 0, 0, True, sd3.PRECISION_F32, last_discards_context=False,
+                  block_only=True)
+    m.load({k: v.cuda() for k, v in p.items()}, prefix="transformer.0.")
+    xx, cc = x.cuda(), c.cuda()
+    m.block_forward(0, y.cuda(), cc, xx)
+    torch.cuda.synchronize()
+    m.close()
+    ref = O.dit_block(x.double(), c.double(), y.double(), {k: v.double() for k, v in p.items()}, 1, False, True, False)
+    assert ref[1].isinf().all() and torch.equal(xx.cpu().double(), ref[1])
+    assert cc.isfinite().all()
+
+
 def test_captions_at_any_address(sd3):
     """Captions that start in the middle of a vector load give the bits of aligned ones (fp32 and bf16 tensors)."""
     L, E, NH, P, C = 2, 64, 1, 64, 128
