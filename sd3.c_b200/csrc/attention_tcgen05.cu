@@ -257,7 +257,7 @@ __device__ __forceinline__ void exp2_pack(uint32_t (&r)[32], float c, float2& ac
 // (the engine folds the factor into the RMSNorm weight of q), so a score is its own exp2
 // argument: one packed multiply per pair of scores less (measured: 4 % of the kernel).
 // PAIR: the launch carries two attentions (a launch of one keeps its parameters at fixed places and some
-// registers fewer: 152 instead of 156 to 161).  With it and separate launches above 16384 rows,
+// registers fewer: 152 instead of 156 to 161).  With it and separate launches above 16384 tokens,
 // eight 1024x1024 images take 96.17 ms against 96.03 before launches were merged, 2048x2048 99.64 against 99.68.
 template <bool BOUNDED, bool UNIT, bool PAIR>
 __global__ void __launch_bounds__(AT_THREADS, 2)

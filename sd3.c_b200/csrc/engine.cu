@@ -10,9 +10,9 @@
 // the caller's stream, nothing synchronises.
 //
 // Per block the launch sequence is
-//   LN+modulate(x), LN+modulate(c) (both modulations of a dual block at once; one launch up to MERGE_MAX_ROWS)
+//   LN+modulate(x), LN+modulate(c) (both modulations of a dual block at once; one launch up to MERGE_MAX_TOKENS)
 //   QKV GEMM(x), (c)         -> packed (B, Tc+Tx, 3E), RMSNorm fused, context rows first; a dual block's
-//                               second QKV GEMM(x) rides in the same launch (up to MERGE_MAX_ROWS)
+//                               second QKV GEMM(x) rides in the same launch (up to MERGE_MAX_TOKENS)
 //   joint attention          -> o_c, o_x; a dual block's attention over the image tokens too
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
 //   [dual] out-proj GEMM with gate2
@@ -520,16 +520,24 @@ int run_mlp1(sd3_model* m, const Linear& L, const Linear& next, const void* A, i
 }
 
 // Launches are merged (LayerNorms of both streams, the two QKV projections and the two attentions of a dual
-// block) up to this many rows.  Below, a kernel is little more than its latency; measured on the
-// forward (merged against separate): LayerNorms 256x256 5.6 %, 1024x1024 1.6 %, four 512x512 nothing; QKV 256x256
-// 4.8 %, 512x512 1.4 %, 1024x1024 0.2 %.  Above there is nothing to gain, and eight 1024x1024
-// images were 0.8 % slower with everything merged.
-constexpr long MERGE_MAX_ROWS = 16384;
+// block) up to this many tokens, image and context rows of all samples together.  The results are the same bits
+// either way.  Measured, everything merged against everything separate (tokens: change, in %):
+//   bf16 forward  589: -13, 1357: -6.7, 2714: -6.7, 4429: -4.0, 5428: -1.4, 8142: -4.0, 8858: -3.4, 13185: -1.0,
+//                 10856 (eight 512x512 images): +1.2 | 16717: -0.5, 17716: -1.4, 18740: -0.5, 26574: -0.7, 35432: 0
+//   dual block    fp32 333: -6.2, 4429: -4.7, 8858: -2.9, 13287: -2.1 | 17716: -0.2
+//                 FP8  333: -11, 4429: -4.9, 8858: -5.9, 13287: -0.7 | 17716: -1.8
+// Below the line all but one size gain; 18 sizes of 8702 to 16136 tokens against the LayerNorms alone merged: +0.04
+// to -2.4.  Above it the gains are small, and eight 768x768 images (19664) lose 2.0.
+constexpr long MERGE_MAX_TOKENS = 16384;
+
+bool merge_launches(int B, int Tc, int Tx) {
+  return static_cast<long>(B) * (static_cast<long>(Tc) + Tx) <= MERGE_MAX_TOKENS;
+}
 
 // the LayerNorms of the image and the context rows, as one launch where both write the same type
 int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st) {
-  const long rows = static_cast<long>(px.B) * px.T + (pc ? static_cast<long>(pc->B) * pc->T : 0);
-  if (!pc || (out_x == out_c && rows <= MERGE_MAX_ROWS)) return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
+  if (!pc || (out_x == out_c && merge_launches(px.B, pc->T, px.T)))
+    return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
   int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st);
   return rc ? rc : launch_ln_modulate(px, nullptr, E, 1e-6f, ms, out_x, st);
 }
@@ -574,7 +582,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const float* c_wq = pre_j ? L.c_wq_s : L.c_wq;
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
   // a dual block's image-only attention beside the joint one, or after it
-  const bool together = L.dual && m->D == 64 && static_cast<long>(B) * (2L * Tx + Tc) <= MERGE_MAX_ROWS;
+  const bool together = L.dual && m->D == 64 && merge_launches(B, Tc, Tx);
   const bool pre_d = L.d_wq_s != nullptr;
   const float* d_wq = pre_d ? L.d_wq_s : L.d_wq;
   if (m->D == 64) {

@@ -46,7 +46,7 @@ def branch_errors(sd3, p, E, NH, x, c, y, dual, last):
     (1536, 24, 1, 256, 77, True, False),   # 64-wide tiles, K split
     (1536, 24, 1, 1024, 333, True, False),  # 128-wide tiles
     (1536, 24, 4, 1000, 154, False, False),  # several waves of them
-    (64, 1, 8, 1100, 20, True, False),     # more rows than are merged: separate LayerNorms, QKV and attentions
+    (64, 1, 8, 2040, 20, True, False),     # more tokens than are merged: separate LayerNorms, QKV and attentions
 ])
 def test_block_fp32_against_float64(sd3, E, NH, B, Tx, Tc, dual, last):
     gen = torch.Generator().manual_seed(E + 7 * Tx + Tc)
