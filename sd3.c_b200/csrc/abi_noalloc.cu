@@ -109,7 +109,7 @@ int sd3_patch_embed_static(const void* latent, int io_dtype, const void* w, cons
   if (!addrs) return SD3_ERR_CUDA;
   __nv_bfloat16* scratch = addrs->scratch;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc = launch_patchify(latent, io_dtype == SD3_DTYPE_F32, scratch, 0, B, C, H, W, patch, st);
+  int rc = launch_patchify(latent, io_dtype == SD3_DTYPE_F32, scratch, false, B, C, H, W, patch, st);
   if (rc) return rc;
   GemmEpilogue e;
   e.mode = EPI_ADD_TABLE;

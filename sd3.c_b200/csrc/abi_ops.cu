@@ -123,13 +123,7 @@ int sd3_linear_f32(const float* x, const float* w, const float* bias, float* out
     set_last_error("sd3_linear_f32: bad act %d", act);
     return SD3_ERR_INVALID_ARG;
   }
-  GemmEpilogue e;
-  e.mode = act == SD3_ACT_GELU_TANH ? EPI_BIAS_GELU : EPI_BIAS;
-  e.bias = bias;
-  e.out = out;
-  e.out_f32 = 1;
-  e.ldo = N;
-  return launch_gemm_f32(x, K, w, K, M, N, K, e, S(stream));
+  return launch_gemm_f32(x, w, bias, out, M, N, K, act == SD3_ACT_GELU_TANH, S(stream));
 }
 
 int sd3_linear_gate_residual(const void* x, const void* w, const float* bias, const float* gate,
@@ -362,7 +356,7 @@ int sd3_patch_embed(const void* latent, int io_dtype, const void* w, const float
     return SD3_ERR_INVALID_ARG;
   }
   const int hp = H / patch, wp = W / patch, Kp = C * patch * patch;
-  int rc = launch_patchify(latent, io_dtype == SD3_DTYPE_F32, scratch, 0, B, C, H, W, patch,
+  int rc = launch_patchify(latent, io_dtype == SD3_DTYPE_F32, scratch, false, B, C, H, W, patch,
                            S(stream));
   if (rc) return rc;
   GemmEpilogue e;

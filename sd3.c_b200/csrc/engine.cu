@@ -899,18 +899,13 @@ int sd3_model_set_param(sd3_model* m, const char* name, const void* dev_ptr, int
       if (s.lin->w8) s.lin->w8_stale = true;
     }
     if (!rc) {
-      if (s.conv && s.lin->split) {
+      if (s.conv && s.lin->split) {  // already (out, in)
         rc = launch_split3(dev_ptr, dtype == SD3_DTYPE_F32, static_cast<bf16*>(dst), numel, st);
+      } else if (s.conv && dtype == SD3_DTYPE_F32) {
+        rc = launch_cast_f32_to_bf16(static_cast<const float*>(dev_ptr), static_cast<bf16*>(dst), numel, st);
       } else if (s.conv) {
-        if ((dtype == SD3_DTYPE_F32) == m->f32)
-          rc = check_cuda(cudaMemcpyAsync(dst, dev_ptr, numel * m->wbytes(),
-                                          cudaMemcpyDeviceToDevice, st), "conv weight copy");
-        else if (dtype == SD3_DTYPE_F32)
-          rc = launch_cast_f32_to_bf16(static_cast<const float*>(dev_ptr), static_cast<bf16*>(dst),
-                                       numel, st);
-        else
-          rc = launch_cast_bf16_to_f32(static_cast<const bf16*>(dev_ptr), static_cast<float*>(dst),
-                                       numel, st);
+        rc = check_cuda(cudaMemcpyAsync(dst, dev_ptr, numel * sizeof(bf16), cudaMemcpyDeviceToDevice, st),
+                        "conv weight copy");
       } else {
         rc = pack_linear_weight(m, dev_ptr, dtype, s.K, s.N, dst, s.lin && s.lin->split, st);
       }
@@ -1044,9 +1039,8 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   // every AdaLN vector of every block and of the final layer in one launch
   if (!m->f32 && m->ada_total % 64 == 0 && E % 64 == 0) {
     // As a tensor-core GEMM with M = batch: out (B, ada_total) = y W^T + b.  Only B
-    // of the 128 rows of each MMA carry data, but the tensor pipe has the room
-    // and TMA streams the 1.5 GB of weights at HBM speed, which the SIMT kernel
-    // (8 warps per SM at its register count) does not.
+    // of the 128 rows of each MMA carry data, but the tensor pipe has the room and TMA streams the
+    // 1.5 GB of weights at HBM speed whatever the batch (272 us); the skinny linear's time grows with it.
     SD3_TRY(launch_cast_f32_to_bf16(w.y, w.y_bf, static_cast<long>(B) * E, st));
     GemmEpilogue e;
     e.mode = EPI_BIAS;
@@ -1077,7 +1071,7 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   }
   // image stream x = patch conv + bias + position table
   {
-    SD3_TRY(launch_patchify(latent, io_f32, w.patches, m->f32 ? 3 : 0, B, c.in_channels, H, W, p, st));
+    SD3_TRY(launch_patchify(latent, io_f32, w.patches, m->f32, B, c.in_channels, H, W, p, st));
     GemmEpilogue e;
     e.mode = EPI_ADD_TABLE; e.out = w.x; e.out_f32 = 1; e.ldo = E;
     e.rows_in = Tx; e.rows_out = Tx; e.table = m->pos_store;

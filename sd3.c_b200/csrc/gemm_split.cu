@@ -82,7 +82,7 @@ struct SplitCfg {
   static_assert(NBUF % 2 == 0, "an accumulator belongs to one of the two MMA-issuing threads");
   static constexpr int TMEM_COLS = NBUF * PBN;
   static constexpr int EPI_WARPS = PBN == 64 ? 4 : 8;
-  static constexpr int CPW = 64;                     // accumulator columns per epilogue thread
+  static constexpr int CPW = 64;                     // accumulator columns per epilogue thread (split_epilogue_64)
   static constexpr int MMA2_WARP = 2 + EPI_WARPS;    // second MMA-issuing warp
   static constexpr int THREADS = 32 * (3 + EPI_WARPS);
   using Ring = OperandRing<STAGES, 2>;  // two MMA-issuing threads
@@ -416,8 +416,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
       if (!ok) break;
       if (KSPLIT == 1 && m < g.M) {
         const RowMap rm = map_row(m, g.epi);
-#pragma unroll
-        for (int c = 0; c < CPW; c += 64) split_epilogue_64<EPI, OUT>(acc + c, rm, n0 + c, g);
+        split_epilogue_64<EPI, OUT>(acc, rm, n0, g);
       }
       __syncwarp();
     }
@@ -450,8 +449,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
       const int n0 = (lt % g.tiles_n) * PBN + (ew >> 2) * CPW;
       if (m < g.M) {
         const RowMap rm = map_row(m, g.epi);
-#pragma unroll
-        for (int c = 0; c < CPW; c += 64) split_epilogue_64<EPI, OUT>(acc + c, rm, n0 + c, g);
+        split_epilogue_64<EPI, OUT>(acc, rm, n0, g);
       }
       __syncwarp();
     }

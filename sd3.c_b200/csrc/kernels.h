@@ -223,9 +223,9 @@ int launch_sinusoidal(const float* t, float* out, int B, int dim, cudaStream_t s
 int launch_pos_table(float* table, int h, int w, int E, int pmax, int base_size,
                      cudaStream_t stream);
 
-// latent (B, C, H, W) fp32/bf16 -> patches (B*h*w, C*p*p), k = c*p*p + ph*p + pw: bf16 (out_f32 = 0),
-// fp32 (1) or three bf16 planes of B*C*H*W elements (3)
-int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int B, int C, int H,
+// latent (B, C, H, W) fp32/bf16 -> patches (B*h*w, C*p*p), k = c*p*p + ph*p + pw: bf16, or
+// three bf16 planes of B*C*H*W elements
+int launch_patchify(const void* latent, int in_f32, void* out, bool out_planes, int B, int C, int H,
                     int W, int p, cudaStream_t stream);
 
 // generic conv2d (square stride, zero padding), in/out (B,C,H,W) fp32 or bf16, weights/bias fp32
@@ -252,8 +252,8 @@ int launch_transpose_split3(const void* in, int in_f32, bf16* out, int R, int C,
 int launch_rmsnorm_heads(void* x, int x_f32, long ld, long rows, int col0, int nheads, int D,
                          const float* w, float eps, cudaStream_t stream);
 
-// fp32 SIMT GEMM with the same epilogues (exact mode and odd shapes)
-int launch_gemm_f32(const float* A, long lda, const float* W /* (N,K) */, long ldw, int M, int N,
-                    int K, const GemmEpilogue& epi, cudaStream_t stream);
+// fp32 SIMT GEMM of any shape, out (M, N) = A (M, K) W (N, K)^T + bias, then GELU (tanh form) if asked for
+int launch_gemm_f32(const float* A, const float* W, const float* bias, float* out, int M, int N, int K, bool gelu,
+                    cudaStream_t stream);
 
 }  // namespace sd3

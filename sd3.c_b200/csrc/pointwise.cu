@@ -6,8 +6,8 @@
 // Reference counterparts: layernorm_forward_kernel6 (cuda/dit.cu:17-75) and
 // scale_and_shift3 (cuda/dit.cu:357-374) -> ln_modulate_kernel (one pass, both
 // modulations of a dual block at once); partial_linear_cuda launched 15x per
-// block with M = batch (cuda/dit.cu:102-354) -> skinny_linear_kernel, one
-// launch for every block's AdaLN vectors; sinusoidal_embedding
+// block with M = batch (cuda/dit.cu:102-354) -> skinny.cu and, in bf16 models, one
+// GEMM for every block's AdaLN vectors (engine.cu); sinusoidal_embedding
 // (modules.cpp:920-944); positional_embedding2D + crop
 // (modules.cpp:946-995); conv2d im2col side of PatchEmbedding
 // (modules.cpp:1037-1117); rmsnorm_key_query_kernel2 (cuda/dit.cu:384-447).
@@ -252,8 +252,8 @@ template <> __device__ __forceinline__ bf16 convert_elem<float, bf16>(float v) {
 template <> __device__ __forceinline__ float convert_elem<bf16, float>(bf16 v) { return __bfloat162float(v); }
 template <> __device__ __forceinline__ bf16 convert_elem<bf16, bf16>(bf16 v) { return v; }
 
-template <typename IT, typename OT, bool SPLIT = false>
-__global__ void patchify_kernel(const IT* latent, OT* out, int B, int C,
+template <typename IT, bool SPLIT>
+__global__ void patchify_kernel(const IT* latent, bf16* out, int B, int C,
                                 int H, int W, int p) {
   grid_dep_wait();
   grid_dep_launch();
@@ -277,7 +277,7 @@ __global__ void patchify_kernel(const IT* latent, OT* out, int B, int C,
     o[total] = static_cast<unsigned short>(m);
     o[2 * total] = static_cast<unsigned short>(l);
   } else {
-    out[idx] = convert_elem<IT, OT>(latent[src]);
+    out[idx] = convert_elem<IT, bf16>(latent[src]);
   }
 }
 
@@ -429,7 +429,7 @@ int launch_pos_table(float* table, int h, int w, int E, int pmax, int base_size,
   return after_launch("pos_table_kernel");
 }
 
-int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int B, int C, int H,
+int launch_patchify(const void* latent, int in_f32, void* out, bool out_planes, int B, int C, int H,
                     int W, int p, cudaStream_t stream) {
   if (!latent || !out || B <= 0 || C <= 0 || p <= 0 || H % p || W % p) {
     set_last_error("patchify: invalid argument");
@@ -437,18 +437,14 @@ int launch_patchify(const void* latent, int in_f32, void* out, int out_f32, int 
   }
   const long total = static_cast<long>(B) * C * H * W;
   const unsigned grid = static_cast<unsigned>((total + 255) / 256);
-  if (in_f32 && out_f32 == 3)
-    launch_dependent(patchify_kernel<float, bf16, true>, grid, 256, 0, stream, (const float*)latent, (bf16*)out, B, C, H, W, p);
-  else if (out_f32 == 3)
-    launch_dependent(patchify_kernel<bf16, bf16, true>, grid, 256, 0, stream, (const bf16*)latent, (bf16*)out, B, C, H, W, p);
-  else if (in_f32 && out_f32)
-    launch_dependent(patchify_kernel<float, float>, grid, 256, 0, stream, (const float*)latent, (float*)out, B, C, H, W, p);
+  if (in_f32 && out_planes)
+    launch_dependent(patchify_kernel<float, true>, grid, 256, 0, stream, (const float*)latent, (bf16*)out, B, C, H, W, p);
+  else if (out_planes)
+    launch_dependent(patchify_kernel<bf16, true>, grid, 256, 0, stream, (const bf16*)latent, (bf16*)out, B, C, H, W, p);
   else if (in_f32)
-    launch_dependent(patchify_kernel<float, bf16>, grid, 256, 0, stream, (const float*)latent, (bf16*)out, B, C, H, W, p);
-  else if (out_f32)
-    launch_dependent(patchify_kernel<bf16, float>, grid, 256, 0, stream, (const bf16*)latent, (float*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<float, false>, grid, 256, 0, stream, (const float*)latent, (bf16*)out, B, C, H, W, p);
   else
-    launch_dependent(patchify_kernel<bf16, bf16>, grid, 256, 0, stream, (const bf16*)latent, (bf16*)out, B, C, H, W, p);
+    launch_dependent(patchify_kernel<bf16, false>, grid, 256, 0, stream, (const bf16*)latent, (bf16*)out, B, C, H, W, p);
   return after_launch("patchify_kernel");
 }
 

@@ -1,8 +1,7 @@
-// Exact-fp32 SIMT kernels: a shared-memory tiled FFMA GEMM with the same fused
-// epilogues as the tcgen05 GEMM, and a generic attention kernel for any head
-// size up to 128.  They serve the operator-level fp32 entry points and head sizes
-// the tensor-core kernels do not cover (fp32 models: gemm_split.cu, attention_split.cu).  Speed is secondary here; the arithmetic is
-// plain fp32 FMA with fp32 accumulation.
+// Exact-fp32 SIMT kernels: a shared-memory tiled FFMA GEMM (bias, GELU), and a generic
+// attention kernel for any head size up to 128.  They serve the operator-level fp32 entry points
+// and head sizes the tensor-core kernels do not cover (fp32 models: gemm_split.cu, attention_split.cu).
+// Speed is secondary here; the arithmetic is plain fp32 FMA with fp32 accumulation.
 //
 // Reference counterparts: linear / partial_linear (modules.cpp:475-511) and
 // multihead_attention (modules.cpp:766-831).
@@ -20,49 +19,9 @@ __device__ __forceinline__ float gelu_tanh_exact(float x) {
   return 0.5f * x * (1.0f + tanhf(u));
 }
 
-template <bool OUT_F32>
-__device__ __forceinline__ void epilogue_scalar(float acc, int m, int n, int N,
-                                                const GemmEpilogue& e) {
-  int b = 0, t_in = m;
-  long orow = m;
-  if (e.rows_in > 0) {
-    b = m / e.rows_in;
-    t_in = m - b * e.rows_in;
-    orow = static_cast<long>(b) * e.rows_out + e.row_off + t_in;
-  }
-  float v = acc * e.alpha + (e.bias ? e.bias[n] : 0.f);
-  long idx = orow * e.ldo + n;
-  switch (e.mode) {
-    case EPI_BIAS_GELU:
-      v = gelu_tanh_exact(v);
-      break;
-    case EPI_GATE_RESID:
-      v = e.resid[idx] + e.gate[static_cast<long>(b) * e.gate_stride + n] * v;
-      break;
-    case EPI_ADD_TABLE:
-      v += e.table[static_cast<long>(t_in) * N + n];
-      break;
-    case EPI_UNPATCHIFY: {
-      const int p = e.up_patch, C = e.up_cin;
-      const int s = t_in % e.up_w, r = t_in / e.up_w;
-      const long Wpix = static_cast<long>(e.up_w) * p, Hpix = static_cast<long>(e.up_h) * p;
-      const int c = n % C, pw = (n / C) % p, ph = n / (C * p);
-      idx = ((static_cast<long>(b) * C + c) * Hpix + (r * p + ph)) * Wpix + (s * p + pw);
-      break;
-    }
-    default:
-      break;
-  }
-  if constexpr (OUT_F32)
-    static_cast<float*>(e.out)[idx] = v;
-  else
-    static_cast<bf16*>(e.out)[idx] = __float2bfloat16(v);
-}
-
-template <bool OUT_F32>
 __global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, int M,
-                int N, int K, const GemmEpilogue e) {
+gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                float* __restrict__ out, int M, int N, int K, int gelu) {
   __shared__ float As[SG_BK][SG_BM + 4];
   __shared__ float Ws[SG_BK][SG_BN + 4];
   const int tid = threadIdx.x;
@@ -82,8 +41,8 @@ gemm_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
     for (int j = 0; j < 4; ++j) {
       const int k = k0 + lk + j;
       const int am = m0 + lr, wn = n0 + lr;
-      As[lk + j][lr] = (am < M && k < K) ? A[static_cast<long>(am) * lda + k] : 0.f;
-      Ws[lk + j][lr] = (wn < N && k < K) ? W[static_cast<long>(wn) * ldw + k] : 0.f;
+      As[lk + j][lr] = (am < M && k < K) ? A[static_cast<long>(am) * K + k] : 0.f;
+      Ws[lk + j][lr] = (wn < N && k < K) ? W[static_cast<long>(wn) * K + k] : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -107,7 +66,10 @@ gemm_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
-      if (n < N) epilogue_scalar<OUT_F32>(acc[i][j], m, n, N, e);
+      if (n < N) {
+        const float v = acc[i][j] + (bias ? bias[n] : 0.f);
+        out[static_cast<long>(m) * N + n] = gelu ? gelu_tanh_exact(v) : v;
+      }
     }
   }
 }
@@ -205,21 +167,14 @@ int launch_attn_inst(const void* q, const void* k, const void* v, long ld, long 
 
 }  // namespace
 
-int launch_gemm_f32(const float* A, long lda, const float* W, long ldw, int M, int N, int K,
-                    const GemmEpilogue& epi, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || !A || !W || !epi.out) {
+int launch_gemm_f32(const float* A, const float* W, const float* bias, float* out, int M, int N, int K, bool gelu,
+                    cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || !A || !W || !out) {
     set_last_error("gemm_f32: invalid argument (M %d N %d K %d)", M, N, K);
     return ST_INVALID_ARG;
   }
-  if (epi.mode == EPI_GATE_RESID && (!epi.gate || !epi.resid)) {
-    set_last_error("gemm_f32: gate/residual epilogue needs gate and resid pointers");
-    return ST_INVALID_ARG;
-  }
   const dim3 grid((N + SG_BN - 1) / SG_BN, (M + SG_BM - 1) / SG_BM);
-  if (epi.out_f32)
-    gemm_f32_kernel<true><<<grid, 256, 0, stream>>>(A, lda, W, ldw, M, N, K, epi);
-  else
-    gemm_f32_kernel<false><<<grid, 256, 0, stream>>>(A, lda, W, ldw, M, N, K, epi);
+  gemm_f32_kernel<<<grid, 256, 0, stream>>>(A, W, bias, out, M, N, K, gelu ? 1 : 0);
   return after_launch("gemm_f32_kernel");
 }
 
