@@ -24,7 +24,9 @@
 // columns each; they exchange the tile's maximum through shared memory): one warp
 // per scheduler with a whole row in registers ran 2500 unrolled instructions a
 // tile, more than the instruction cache holds, at 0.3 instructions per cycle (8500 cycles a tile).
-// What bounds it: the tensor pipe, 1536 + 1680 cycles per 128 x 128 tile pair.
+// What bounds it: the chain scores -> exponentials -> products of a tile, of which the MMAs (1536 + 1680 cycles
+// per 128 x 128 tile pair) are about half: tensor pipe 43 %, issue slots 34 %, fixed latencies and polls first
+// among the stalls (1024 + 333 tokens).
 //
 // Measured against attention_simt_kernel (one warp per query, uncoalesced key rows), which this
 // replaces for fp32 models with head_dim 64: one dual block of 256 + 77 tokens 2.79 -> 0.49 ms, the

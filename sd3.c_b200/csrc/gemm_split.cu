@@ -42,10 +42,11 @@
 // MMA: tensor pipe 38 % busy); 256 x 256 tiles (3072 cycles of MMA took 4060: two stages of
 // operands, two accumulators, and an epilogue of 128 columns per thread between tiles).
 //
-// Measured, 24-block model at 512 x 512 (1024 + 333 tokens): one-CTA tiles 19.26, pairs 17.57, no cluster-scope
-// release in the accumulator's hand-back 16.8 -> 15.7 with the attention as it was then, GELU 15.5 -> 15.2,
-// 128-wide tiles only 15.3 -> 15.1 ms; the FFMA kernel and the SIMT attention took 754 ms.  One dual block of 256 + 77
-// tokens: 454, 411 (K split 381 -> 337), 338, 294 us; start 4740.
+// Measured: 24-block model at 512 x 512 (1024 + 333 tokens) 15.1 ms, one dual block of 256 + 77 tokens 295 us;
+// with FFMA GEMMs and the SIMT attention 754 ms and 4.74 ms.  What single steps gave, in the order they were made
+// (each against the commit before it; the attention changed in between): one-CTA tiles -> pairs 19.26 -> 17.57 ms
+// and 454 -> 411 us; K split 381 -> 337 us; no cluster-scope release in the accumulator's hand-back
+// 16.8 -> 15.7 ms; GELU 15.5 -> 15.2 ms; 128-wide tiles instead of 256 15.3 -> 15.1 ms.
 #include <cuda.h>
 #include <mutex>
 
@@ -92,8 +93,8 @@ struct SplitCfg {
 };
 
 // 0.5 x (1 + tanh(u)) = x / (1 + e^(-2u)),  u = sqrt(2/pi) (x + 0.044715 x^3): no cancellation for
-// negative u, two MUFU operations where tanhf takes some thirty instructions (they stood between the
-// tiles: an epilogue thread has 128 of them)
+// negative u, two MUFU operations where tanhf takes some thirty instructions (an epilogue thread
+// has 64 of them between two tiles)
 __device__ __forceinline__ float gelu_tanh_f32(float x) {
   const float t = x * fmaf(x * x, -2.0f * 1.4426950408889634f * 0.7978845608028654f * 0.044715f,
                            -2.0f * 1.4426950408889634f * 0.7978845608028654f);  // -2 u log2(e)

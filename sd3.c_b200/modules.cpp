@@ -3,8 +3,8 @@
 // denoiser forward path, running on CUDA tensors through libsd3_b200.so.
 //
 // This file is host glue only: it validates tensors, picks the precision mode
-// from the tensor dtype (float32 -> exact fp32 kernels, bfloat16 -> tcgen05
-// bf16 kernels), hands raw pointers to the C ABI (include/sd3_b200.h) on the
+// from the tensor dtype (float32 -> fp32 accuracy, operands split into bf16
+// planes; bfloat16 -> tcgen05 bf16 kernels), hands raw pointers to the C ABI (include/sd3_b200.h) on the
 // current torch stream and allocates outputs with torch.  There is no CPU
 // path: CPU tensors are rejected with an error.
 //
