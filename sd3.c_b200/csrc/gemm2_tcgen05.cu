@@ -15,13 +15,13 @@
 // 128-row half of the W tile (32 KiB instead of the 48 KiB a lone CTA needs
 // for a 128 x 256 tile); the tensor cores of both SMs read the two W halves
 // from both shared memories.  That cuts the L2 -> shared-memory traffic per
-// FLOP by a third and leaves room for a six-stage ring.  The even CTA of the
-// pair issues all MMAs, from TWO threads that take the ring's slots in turn: a
-// tcgen05.mma holds its issuing thread for about as long as it runs, so with one
-// thread the barrier test, the commit and the descriptor arithmetic of every slot
-// were idle time of the tensor pipe; now they run under the other thread's MMAs
-// (a turn counter in shared memory, bracketed by tcgen05 fences, keeps the MMAs
-// in K order).  Completion is signalled to both CTAs with
+// FLOP by a third and leaves room for a six-stage ring.  One warp of the even CTA of the
+// pair issues all MMAs, one warp of each CTA its loads.  Both stay converged and an elected lane issues:
+// descriptors and addresses then live in uniform registers.  From a branch taken by lane 0 alone an MMA took
+// 63-88 cycles to issue (a 128-wide MMA runs 64) and a slot's loads 740; elected, 33-39 and under 300.
+// Measured, lane 0 with two issuing threads that took turns -> elected lane of one warp (us, weights from
+// HBM): N = 1536, K = 6144, 589 rows 26.9 -> 20.4, 4429 rows 73.2 -> 69.1; QKV 4429 rows 59.6 -> 48.9, 13287 rows
+// 177 -> 128; GELU 4429 rows 68.9 -> 63.0.  Completion is signalled to both CTAs with
 // tcgen05.commit ... multicast::cluster.  Each CTA keeps the accumulator rows
 // of its own half of M in its own TMEM (two buffers of 256 columns) and drains
 // them through the same fused epilogues as the one-CTA kernel.
@@ -57,15 +57,16 @@ constexpr int P_RED_BYTES = 4096;
 __host__ __device__ constexpr bool pair_stages_out(int epi, bool out_f32) {
   return epi == EPI_GATE_RESID || (!out_f32 && (epi == EPI_BIAS || epi == EPI_BIAS_GELU || epi == EPI_QKV_NORM));
 }
-// Six stages of 32 KiB (eight of 24 KiB), handed over in SLOTS of two (one full/empty barrier
-// pair, one barrier test and one tcgen05.commit per slot instead of per stage: the issuing
-// thread spent ~100 of every 680 cycles of a stage on those two).
+// Six stages of 32 KiB (eight of 24 KiB), handed over in slots of one (two): a full and an empty barrier, one
+// wait and one commit each.  A stage of the wide tile is 512 cycles of MMA and single hand-overs refill the
+// ring sooner (N = 1536, K = 6144, 4429 rows: 69.1 us against 70.9 with slots of two; 13287 rows: 191 against 207);
+// one of the narrow tile is 256 cycles, less than a hand-over takes (589 rows: 24.6 us, with slots of two 20.4).
 __host__ __device__ constexpr int pair_stages(int pbn) { return pbn == 256 ? 6 : 8; }
+__host__ __device__ constexpr int pair_slot(int pbn) { return pbn == 256 ? 1 : 2; }
 __host__ __device__ constexpr int pair_red_bytes(int epi, bool out_f32) {
   return pair_stages_out(epi, out_f32) ? EPI_WARPS * P_RED_BYTES : 0;
 }
-constexpr int P_THREADS = 64 + 32 * EPI_WARPS + 32;  // + a second MMA-issuing warp
-constexpr int P_MMA2_WARP = 2 + EPI_WARPS;
+constexpr int P_THREADS = 64 + 32 * EPI_WARPS;
 __host__ __device__ constexpr int pair_smem_bytes(int epi, bool out_f32, int pbn) {
   return pair_stages(pbn) * pair_stage_bytes(pbn) + pair_red_bytes(epi, out_f32) + 256 + 1024;
 }
@@ -99,9 +100,8 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
-  volatile uint32_t* s_issued = reinterpret_cast<volatile uint32_t*>(s_abort + 1);  // slots whose MMAs have been issued
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known uniform
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const int pair = blockIdx.x >> 1;
@@ -117,7 +117,6 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       mbar_init(&tempty_bar[a], 2 * EPI_WARPS);  // epilogue warps of both CTAs (leader's copy is used)
     }
     *s_abort = 0;
-    *s_issued = 0;
     fence_barrier_init();
     prefetch_tmap(&p0.tmA);
     prefetch_tmap(&p0.tmW);
@@ -142,37 +141,46 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     grid_dep_wait();
     grid_dep_launch();
   }
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, p0.g.status};
 
   // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
-  constexpr int NSLOT = P_STAGES / 2;     // slots of two stages
-  const int KB = p0.g.k_blocks;        // the same K for all problems
-  const int KS = (KB + 1) / 2;         // slots per tile (the last may hold one stage)
+  constexpr int SLOT = pair_slot(PBN);
+  constexpr int NSLOT = P_STAGES / SLOT;
+  const int KB = p0.g.k_blocks;  // the same K for all problems
 
-  if (warp == 0 && lane == 0) {
-    // ------------------------------ TMA producer (both CTAs, one thread) ------
+  if (warp == 0) {
+    // ------------------------------ TMA producer (both CTAs, one warp) --------
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    const bool issuer = elect_one();
     constexpr int KEL = FP8 ? P_KBYTES : P_KBYTES / 2;  // K elements per stage
-    auto expect_slot = [&](int st, int ks) {
-      // all bytes of the slot (both CTAs) are credited to the leader's barrier
-      if (rank == 0) mbar_expect_tx(&full_bar[st], (KB - 2 * ks < 2 ? KB - 2 * ks : 2) * 2 * P_STAGE_BYTES);
+    const uint32_t ring = smem_u32(smem);
+    const uint32_t full_local = smem_u32(full_bar), full_leader = map_to_cta(full_local, 0);
+    // stages [kb, kb + SLOT) of a tile into slot st; all bytes of the slot (both CTAs) are credited to the
+    // leader's barrier
+    auto load_w = [&](const CUtensorMap* tmW, int st, int kb, int n0) {
+      if (rank == 0) mbar_expect_tx_at(full_local + 8 * st, min(SLOT, KB - kb) * (2 * P_STAGE_BYTES));
+#pragma unroll
+      for (int i = 0; i < SLOT; ++i)
+        if (SLOT == 1 || kb + i < KB)
+          tma_load_2d_pair_at(ring + (st * SLOT + i) * P_STAGE_BYTES + P_A_BYTES, tmW, full_leader + 8 * st,
+                              (kb + i) * KEL, n0);
     };
-    auto load_w = [&](const PairProblem& pp, int st, int ks, int n0) {
-      const uint32_t bar = map_to_cta(smem_u32(&full_bar[st]), 0);
-      for (int hs = 0; hs < (KB - 2 * ks < 2 ? KB - 2 * ks : 2); ++hs)
-        tma_load_2d_pair(smem + (2 * st + hs) * P_STAGE_BYTES + P_A_BYTES, &pp.tmW, bar, (2 * ks + hs) * KEL, n0);
+    auto load_a = [&](const CUtensorMap* tmA, int st, int kb, int m0) {
+#pragma unroll
+      for (int i = 0; i < SLOT; ++i)
+        if (SLOT == 1 || kb + i < KB)
+          tma_load_2d_pair_at(ring + (st * SLOT + i) * P_STAGE_BYTES, tmA, full_leader + 8 * st, (kb + i) * KEL, m0);
     };
     int pre = 0;  // slots of the first tile whose weights are under way before the wait
     if (p0.g.epi.w_static) {
       const PairProblem& pp = pair < end0 ? p0 : pair < end1 ? p1 : p2;
       const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
-      for (; pre < NSLOT && pre < KS; ++pre) {
-        expect_slot(pre, pre);
-        load_w(pp, pre, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF);
-      }
+      const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF;
+      for (; pre < NSLOT && pre * SLOT < KB; ++pre)
+        if (issuer) load_w(&pp.tmW, pre, pre * SLOT, n0);
     }
     grid_dep_wait();
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -180,85 +188,59 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
       const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF;
-      for (int ks = 0; ks < KS; ++ks) {
+      const CUtensorMap *tmA = &pp.tmA, *tmW = &pp.tmW;
+      for (int kb = 0; kb < KB; kb += SLOT) {
         if (pre > 0) {
           --pre;
         } else {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-          expect_slot(stage, ks);
-          load_w(pp, stage, ks, n0);
+          if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+          if (issuer) load_w(tmW, stage, kb, n0);
         }
-        const int nk = KB - 2 * ks < 2 ? KB - 2 * ks : 2;  // stages of this slot that carry data
-        const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-        for (int hs = 0; hs < nk; ++hs)
-          tma_load_2d_pair(smem + (2 * stage + hs) * P_STAGE_BYTES, &pp.tmA, bar, (2 * ks + hs) * KEL, m0);
+        if (issuer) load_a(tmA, stage, kb, m0);
         if (++stage == NSLOT) { stage = 0; phase ^= 1; }
       }
     }
-  } else if ((warp == 1 || warp == P_MMA2_WARP) && lane == 0) {
-    // ------------------------------ MMA issuers (leader only) -----------------
-    // Two threads take the slots in turn: while one issues the eight MMAs of its slot the
-    // other waits for the operands of the next one, and the commit and the barrier work of a
-    // slot run under the other thread's MMAs.  `s_issued` hands the turn over, so the MMAs
-    // reach the tensor pipe in K order.
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (leader only, one warp) --------
     if (rank == 0) {
-      const uint32_t me = warp == 1 ? 0u : 1u;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
-      uint32_t slot_no = 0;
       bool ok = true;
+      const bool issuer = elect_one();
+      const uint64_t desc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * PBN);
-        for (int ks = 0; ks < KS; ++ks) {
-          if ((slot_no & 1u) == me) {
-            if (ks == 0 && !mbar_wait(&tempty_bar[acc], acc_phase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-            if (!mbar_wait(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
-            {  // my turn: every earlier slot has been issued
-              const uint64_t t0 = global_timer_ns();
-              uint32_t it = 0;
-              while (*s_issued != slot_no) {
-                if (((++it) & 0x3ffu) == 0) {
-                  if (*wc.s_abort) { ok = false; break; }
-                  if (global_timer_ns() - t0 > SD3_WAIT_LIMIT_NS) {
-                    *wc.s_abort = 1;
-                    if (wc.g_status) atomicCAS(wc.g_status, 0, DEV_TIMEOUT_FULL);
-                    ok = false;
-                    break;
-                  }
-                }
-              }
-              if (!ok) break;
-            }
-            tc_fence_after_sync();
-            const int nk = KB - 2 * ks < 2 ? KB - 2 * ks : 2;
-            for (int hs = 0; hs < nk; ++hs) {
-              const uint32_t a_addr = smem_u32(smem + (2 * stage + hs) * P_STAGE_BYTES);
-              const uint64_t a_desc = make_smem_desc_sw128(a_addr, 16, 1024);
-              const uint64_t b_desc = make_smem_desc_sw128(a_addr + P_A_BYTES, 16, 1024);
+        if (!mbar_wait_all(&tempty_bar[acc], acc_phase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) break;
+        for (int kb = 0; kb < KB; kb += SLOT) {
+          if (!mbar_wait_all(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
+          tc_fence_after_sync();
+          if (issuer) {
+#pragma unroll
+            for (int i = 0; i < SLOT; ++i) {
+              if (SLOT > 1 && kb + i >= KB) break;
+              const uint64_t a_desc = desc0 + static_cast<uint32_t>((stage * SLOT + i) * (P_STAGE_BYTES >> 4));
+              const uint64_t b_desc = a_desc + (P_A_BYTES >> 4);
 #pragma unroll
               for (int k = 0; k < P_KBYTES / 32; ++k) {
                 const uint64_t adv = static_cast<uint64_t>((k * 32) >> 4);
                 if constexpr (FP8)
-                  mma_f8_ss_pair(d_tmem, a_desc + adv, b_desc + adv, IDESC, (ks | hs | k) != 0);
+                  mma_f8_ss_pair(d_tmem, a_desc + adv, b_desc + adv, IDESC, (kb | i | k) != 0);
                 else
-                  mma_f16_ss_pair(d_tmem, a_desc + adv, b_desc + adv, IDESC, (ks | hs | k) != 0);
+                  mma_f16_ss_pair(d_tmem, a_desc + adv, b_desc + adv, IDESC, (kb | i | k) != 0);
               }
             }
-            tc_fence_before_sync();
-            *s_issued = slot_no + 1;  // the other thread may issue the next slot
-            mma_commit_pair(&empty_bar[stage], 3);          // frees the slot in both CTAs
-            if (ks == KS - 1) mma_commit_pair(&tfull_bar[acc], 3);  // accumulator ready in both CTAs
+            mma_commit_pair(&empty_bar[stage], 3);                     // frees the slot in both CTAs
+            if (kb + SLOT >= KB) mma_commit_pair(&tfull_bar[acc], 3);  // accumulator ready in both CTAs
           }
-          ++slot_no;
           if (++stage == NSLOT) { stage = 0; phase ^= 1; }
         }
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
     }
-  } else if (warp >= 2 && warp < 2 + EPI_WARPS) {
+  } else {
     // ------------------------------ epilogue (both CTAs) ----------------------
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;

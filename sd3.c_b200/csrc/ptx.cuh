@@ -74,11 +74,10 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
+__device__ __forceinline__ void mbar_expect_tx_at(uint32_t bar_addr, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) { mbar_expect_tx_at(smem_u32(bar), bytes); }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -153,6 +152,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, c
   int ok = 1;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, w, code) ? 1 : 0;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// Bounded wait by every lane of a converged warp, with one answer for the warp.  The roles that issue TMA
+// loads and MMAs run as whole warps that stay converged and let one elected lane issue: the compiler then
+// keeps descriptors, coordinates and barrier addresses in uniform registers.  From a branch that only
+// lane 0 had taken, every tcgen05.mma took 63 to 88 cycles to issue, elected 33 to 39.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, const WaitCtx& w, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, w, code)) != 0;
 }
 
 // After an abort: give copies and MMAs already in flight a bounded time to
@@ -425,12 +432,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar_addr) {
 }
 // TMA load whose completion bytes are credited to a barrier that may live in
 // the other CTA of the pair (bar is a shared::cluster address).
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t cluster_bar_addr,
-                                                 int x, int y) {
+__device__ __forceinline__ void tma_load_2d_pair_at(uint32_t smem_dst, const void* tmap, uint32_t cluster_bar_addr,
+                                                    int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)),
+      ::"r"(smem_dst),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(cluster_bar_addr), "r"(x), "r"(y)
       : "memory");
 }
