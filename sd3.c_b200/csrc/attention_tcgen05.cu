@@ -15,10 +15,12 @@
 // The T x T score matrix never exists in memory.
 //
 // What the structure is built around (cycle-stamped traces of the issue loops):
-//  * A tcgen05.mma or tcgen05.commit holds the issuing thread 50-100 cycles and
-//    a satisfied mbarrier test about 60.  With 64-key hand-offs the single issue
-//    thread needed ~1700 cycles per 64 keys and was the bottleneck; with one
-//    hand-off per 128 keys (12 MMAs, 2 commits, 4 waits) it idles half the time.
+//  * The TMA and the MMA warp stay converged and an elected lane issues, so that descriptors,
+//    coordinates and barrier addresses live in uniform registers.  From a branch that lane 0 alone
+//    had taken, a tcgen05.mma or commit took 63-100 cycles to issue and a satisfied mbarrier test
+//    about 60; one hand-off per 128 keys (12 MMAs, 2 commits, 4 waits) dates from then.  Elected:
+//    T = 4429, batch 8, bounded 1055 -> 1029 us, batch 1 141.6 -> 133.3; T = 4096, batch 8 888 -> 843;
+//    T = 1357, batch 4 72.4 -> 67.9; online T = 16717 2261 -> 2161.
 //  * An mbarrier hop costs ~140 cycles and the completion of a committed MMA
 //    group ~240 cycles after its last cycle of math, so every dependency between
 //    the roles is given a tile of slack: a softmax warp pulls the scores of tile
@@ -285,7 +287,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_ready + 1);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known uniform
+  const int lane = threadIdx.x & 31;
   const int split = bx % a.kv_split;  // which share of the keys
   const int q0 = (bx / a.kv_split) * AT_BM;
   const int h = blockIdx.y;
@@ -318,57 +321,67 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_c
   tc_fence_after_sync();
   grid_dep_wait();
   grid_dep_launch();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, a.status};
 
   if (warp == 0) {
-    // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    // ------------------------------ TMA producer (a converged warp, one lane issues) ------
+    const bool issuer = elect_one();
+    if (issuer) {
       mbar_expect_tx(q_full, AT_TILE_BYTES);
       tma_load_3d(q_smem, &tmQKV, q_full, h * AT_D, q0, b);
-      for (int j = 0; j < nkv; ++j) {
-        const int st = j % AT_STAGES;
-        const uint32_t prev = ((j / AT_STAGES) + 1) & 1;  // parity of this stage's previous use
-        // K of tile j - STAGES is free once its scores are complete
-        if (j >= AT_STAGES && !mbar_wait(&s_full[st], prev, wc, DEV_TIMEOUT_ATTN_KV)) break;
+    }
+    for (int j = 0; j < nkv; ++j) {
+      const int st = j % AT_STAGES;
+      const uint32_t prev = ((j / AT_STAGES) + 1) & 1;  // parity of this stage's previous use
+      // K of tile j - STAGES is free once its scores are complete
+      if (j >= AT_STAGES && !mbar_wait_all(&s_full[st], prev, wc, DEV_TIMEOUT_ATTN_KV)) break;
+      if (issuer) {
         mbar_expect_tx(&k_full[st], AT_TILE_BYTES);
         tma_load_3d(k_smem + st * AT_TILE_BYTES, &tmQKV, &k_full[st], a.E + h * AT_D, (jt0 + j) * AT_BN, b);
-        // V of tile j - STAGES is free once its products are complete
-        if (j >= AT_STAGES && !mbar_wait(&pv_done[st], prev, wc, DEV_TIMEOUT_ATTN_KV)) break;
+      }
+      // V of tile j - STAGES is free once its products are complete
+      if (j >= AT_STAGES && !mbar_wait_all(&pv_done[st], prev, wc, DEV_TIMEOUT_ATTN_KV)) break;
+      if (issuer) {
         mbar_expect_tx(&v_full[st], AT_TILE_BYTES);
         tma_load_3d(v_smem + st * AT_TILE_BYTES, &tmQKV, &v_full[st], 2 * a.E + h * AT_D, (jt0 + j) * AT_BN, b);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer --------------------------------
+    // ------------------------------ MMA issuer (a converged warp, one lane issues) ------
     constexpr uint32_t IDESC_S = make_idesc(1, 1, AT_BM, AT_BN, 0, 0);  // Q K^T, both K-major, N = 128
     constexpr uint32_t IDESC_O = make_idesc(1, 1, AT_BM, AT_D, 0, 1);   // P V, V is MN-major
     const uint32_t s_tmem = tmem_base + AT_S_COL;
     const uint32_t p_tmem = tmem_base + AT_P_COL;
     const uint32_t o_tmem = tmem_base + AT_O_COL;
     const uint64_t q_desc = make_smem_desc_sw128(smem_u32(q_smem), 16, 1024);
-    if (lane == 0) {  // a single thread runs the whole issue loop
-      bool ok = mbar_wait(q_full, 0, wc, DEV_TIMEOUT_ATTN_Q);
-      // iteration j issues the scores of tile j and the products of tile j - 1
-      for (int j = 0; j <= nkv && ok; ++j) {
-        if (j < nkv) {
-          const int st = j % AT_STAGES;
-          // the softmax warps have pulled the scores of tile j - 1 into registers
-          if (j >= 1 && !mbar_wait(s_free, (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_S)) break;
-          if (!mbar_wait(&k_full[st], (j / AT_STAGES) & 1, wc, DEV_TIMEOUT_ATTN_KV)) break;
-          tc_fence_after_sync();
-          const uint64_t k_desc = make_smem_desc_sw128(smem_u32(k_smem + st * AT_TILE_BYTES), 16, 1024);
+    const uint64_t k_desc0 = make_smem_desc_sw128(smem_u32(k_smem), 16, 1024);
+    const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(v_smem), 1024, 1024);
+    const bool issuer = elect_one();
+    bool ok = mbar_wait_all(q_full, 0, wc, DEV_TIMEOUT_ATTN_Q);
+    // iteration j issues the scores of tile j and the products of tile j - 1
+    for (int j = 0; j <= nkv && ok; ++j) {
+      if (j < nkv) {
+        const int st = j % AT_STAGES;
+        // the softmax warps have pulled the scores of tile j - 1 into registers
+        if (j >= 1 && !mbar_wait_all(s_free, (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_S)) break;
+        if (!mbar_wait_all(&k_full[st], (j / AT_STAGES) & 1, wc, DEV_TIMEOUT_ATTN_KV)) break;
+        tc_fence_after_sync();
+        if (issuer) {
+          const uint64_t k_desc = k_desc0 + static_cast<uint32_t>(st * (AT_TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < AT_D / 16; ++k)
             mma_f16_ss(s_tmem, q_desc + 2 * k, k_desc + 2 * k, IDESC_S, k != 0);
           mma_commit(&s_full[st]);
         }
-        if (j >= 1) {
-          const int jj = j - 1, st = jj % AT_STAGES;
-          if (!mbar_wait(&v_full[st], (jj / AT_STAGES) & 1, wc, DEV_TIMEOUT_ATTN_KV)) break;
-          if (!mbar_wait(p_ready, jj & 1, wc, DEV_TIMEOUT_ATTN_P)) break;
-          tc_fence_after_sync();
-          const uint64_t v_desc = make_smem_desc_sw128(smem_u32(v_smem + st * AT_TILE_BYTES), 1024, 1024);
+      }
+      if (j >= 1) {
+        const int jj = j - 1, st = jj % AT_STAGES;
+        if (!mbar_wait_all(&v_full[st], (jj / AT_STAGES) & 1, wc, DEV_TIMEOUT_ATTN_KV)) break;
+        if (!mbar_wait_all(p_ready, jj & 1, wc, DEV_TIMEOUT_ATTN_P)) break;
+        tc_fence_after_sync();
+        if (issuer) {
+          const uint64_t v_desc = v_desc0 + static_cast<uint32_t>(st * (AT_TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < AT_BN / 16; ++k)  // 16 keys: 8 columns of bf16 pairs, 16 rows of V (128 B each)
             mma_f16_ts(o_tmem, p_tmem + 8 * k, v_desc + static_cast<uint64_t>((k * 16 * 128) >> 4), IDESC_O,
