@@ -1,6 +1,5 @@
 // CTA-pair variant of the tcgen05 GEMM: two CTAs (a cluster of two on
-// neighbouring SMs) cooperate on 256 x 256 (or, for problems of less than half a
-// wave of those, 256 x 128) output tiles with
+// neighbouring SMs) cooperate on 256 x 256 (or 256 x 128, where those fill the SMs better) output tiles with
 // tcgen05.mma.cta_group::2.  One launch can carry up to THREE problems of the same
 // shape class (same N, K and epilogue: the image-stream GEMM of a block, its
 // small context-stream twin and, for QKV, the second projection of a dual block);
@@ -376,18 +375,19 @@ int build_problem(PairProblem* pp, const GemmProblem& q, int operand_dtype, int 
   return ST_OK;
 }
 
-// 256-wide tiles, except for problems so small that even twice as many 128-wide tiles fit in one
-// wave of CTA pairs.  The narrow tile needs 96 bytes of operands per clock per SM at the full MMA
-// rate against 64, and its ring slots (48 KiB) are consumed in half the time of the wide tile's
-// (64 KiB) while their refill takes as long: it reaches 0.5-0.6 of the MMA rate where the wide
-// tile reaches 0.8.  Measured at 4096-4429 rows (1.3-1.5 waves of wide tiles, where wave
-// arithmetic favours the narrow ones) the wide tiles are 15-25 % faster (N = 1536, K = 6144: 72
-// against 90 us), at 2048 rows 35 %.  Only for problems of a few tiles (at most 1536 rows at N = 1536), where the
-// narrow tiles put twice as many SMs to work, do they win, by 5-8 %.
-int choose_tile_width(long tiles256, const GemmEpilogue& epi) {
-  if (!narrow_tiles_built(epi)) return 256;
+// The tile width with the least time by waves: a wave of 128-wide tiles takes 0.64 of a wave of 256-wide ones (half the
+// MMA time, but 96 bytes of operands per clock and SM where TMA brings at most 82 to 92), and the last wave's
+// epilogue, which nothing overlaps, is half as long, worth about ten 64-wide K blocks of a wide tile.  Measured, us, wide /
+// narrow (waves of each):
+//   K 1536, QKV    589 rows 15.0 / 12.9 (1, 2)   1357: 21.7 / 18.5 (2, 3)   2714: 30.3 / 33.3 (3, 6)   4429: 49.1 / 52.2 (5, 9)
+//   K 1536, GELU   333 rows 15.8 / 13.3 (1, 2)   1024: 21.0 / 19.1 (2, 3)   1357: 23.7 / 24.7 (2, 4)   4429: 61.9 / 71.7 (6, 12)
+//   K 1536, gate  2714 rows 14.5 / 14.6 (1, 2)   4429: 23.5 / 21.2 (2, 3)   5428: 26.7 / 28.8 (2, 4)
+//   K 6144, gate  2714 rows 38.6 / 43.6 (1, 2)   4429: 68.8 / 67.4 (2, 3)   5428: 75.4 / 86.9 (2, 4)
+int choose_tile_width(long tiles256, int k_blocks, const GemmEpilogue& epi) {
   const long pairs = device_sm_count() / 2;
-  return (pairs > 0 && 2 * tiles256 <= pairs) ? 128 : 256;
+  if (pairs <= 0 || !narrow_tiles_built(epi)) return 256;
+  const long wide = (tiles256 + pairs - 1) / pairs, narrow = (2 * tiles256 + pairs - 1) / pairs;
+  return 64 * narrow * k_blocks < 100 * wide * k_blocks + 1000 ? 128 : 256;
 }
 
 }  // namespace
@@ -419,7 +419,8 @@ int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int 
     }
     tiles256 += static_cast<long>((q[i].M + 255) / 256) * (N / 256);
   }
-  const int pbn = choose_tile_width(tiles256, a.epi);
+  const int kel = P_KBYTES / (fp8 ? 1 : 2);
+  const int pbn = choose_tile_width(tiles256, (K + kel - 1) / kel, a.epi);
   PairProblem p[3];
   int end[3] = {0, 0, 0}, tiles = 0;
   for (int i = 0; i < 3; ++i) {
