@@ -105,7 +105,8 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xchg + 4);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known uniform
+  const int lane = threadIdx.x & 31;
   const int q0 = (static_cast<int>(blockIdx.x) - (second ? grid0 : 0)) * AS_BM, h = blockIdx.y, b = a.b0 + blockIdx.z;
   const int T = a.T, nkv = (T + AS_BN - 1) / AS_BN;
 
@@ -135,58 +136,68 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
   tc_fence_after_sync();
   grid_dep_wait();
   grid_dep_launch();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, a.status};
 
   if (warp == 0) {
-    // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      // 64 rows from `row` of every plane (plane p of sample b is slab p * B + b); plane_bytes apart
-      auto load_rows = [&](uint8_t* dst, int plane_bytes, uint64_t* bar, int col, int row) {
-        for (int p = 0; p < 3; ++p) tma_load_3d(dst + p * plane_bytes, &tm, bar, col, row, p * a.B + b);
-      };
-      auto load_k = [&](int j) {
-        const int st = j & 1;
-        if (j >= 2 && !mbar_wait(&k_empty[st], ((j >> 1) - 1) & 1, wc, DEV_TIMEOUT_ATTN_KV)) return false;
+    // ------------------------------ TMA producer (a converged warp, one lane issues) ------
+    const bool issuer = elect_one();
+    // 64 rows from `row` of every plane (plane p of sample b is slab p * B + b); plane_bytes apart
+    auto load_rows = [&](uint8_t* dst, int plane_bytes, uint64_t* bar, int col, int row) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) tma_load_3d(dst + p * plane_bytes, &tm, bar, col, row, p * a.B + b);
+    };
+    auto load_k = [&](int j) {
+      const int st = j & 1;
+      if (j >= 2 && !mbar_wait_all(&k_empty[st], ((j >> 1) - 1) & 1, wc, DEV_TIMEOUT_ATTN_KV)) return false;
+      if (issuer) {
         mbar_expect_tx(&k_full[st], AS_TILE);
         uint8_t* d = k_smem + st * AS_TILE;
         load_rows(d, AS_PLANE, &k_full[st], a.E + h * AS_D, j * AS_BN);
         load_rows(d + AS_HPLANE, AS_PLANE, &k_full[st], a.E + h * AS_D, j * AS_BN + 64);
-        return true;
-      };
+      }
+      return true;
+    };
+    if (issuer) {
       mbar_expect_tx(q_full, AS_TILE);
       load_rows(q_smem, AS_PLANE, q_full, h * AS_D, q0);
       load_rows(q_smem + AS_HPLANE, AS_PLANE, q_full, h * AS_D, q0 + 64);
-      bool ok = load_k(0);
-      for (int j = 0; j < nkv && ok; ++j) {
-        if (j + 1 < nkv) ok = load_k(j + 1);
-        for (int hf = 0; hf < 2 && ok; ++hf) {
-          if (j >= 1 && !mbar_wait(&v_empty[hf], (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_KV)) { ok = false; break; }
+    }
+    bool ok = load_k(0);
+    for (int j = 0; j < nkv && ok; ++j) {
+      if (j + 1 < nkv) ok = load_k(j + 1);
+      for (int hf = 0; hf < 2 && ok; ++hf) {
+        if (j >= 1 && !mbar_wait_all(&v_empty[hf], (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_KV)) { ok = false; break; }
+        if (issuer) {
           mbar_expect_tx(&v_full[hf], AS_TILE / 2);
           load_rows(v_smem + hf * (AS_TILE / 2), AS_HPLANE, &v_full[hf], 2 * a.E + h * AS_D, j * AS_BN + 64 * hf);
         }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
-      constexpr uint32_t IDESC_S = make_idesc(1, 1, AS_BM, AS_BN, 0, 0);
-      constexpr uint32_t IDESC_O3 = make_idesc(1, 1, AS_BM, 192, 0, 1);  // V is MN-major
-      constexpr uint32_t IDESC_O2 = make_idesc(1, 1, AS_BM, 128, 0, 1);
-      constexpr uint32_t IDESC_O1 = make_idesc(1, 1, AS_BM, 64, 0, 1);
-      constexpr uint64_t PL = AS_PLANE >> 4;
-      constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};  // smallest products first
-      const uint32_t s_tmem = tmem_base + AS_S_COL, p_tmem = tmem_base + AS_P_COL, o_tmem = tmem_base + AS_O_COL;
-      const uint64_t q_desc = make_smem_desc_sw128(smem_u32(q_smem), 16, 1024);
-      bool ok = mbar_wait(q_full, 0, wc, DEV_TIMEOUT_ATTN_Q);
-      // iteration j issues the scores of tile j and the products of tile j - 1
-      for (int j = 0; j <= nkv && ok; ++j) {
-        if (j < nkv) {
-          const int st = j & 1;
-          if (j >= 1 && !mbar_wait(s_free, (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_S)) break;
-          if (!mbar_wait(&k_full[st], (j >> 1) & 1, wc, DEV_TIMEOUT_ATTN_KV)) break;
-          tc_fence_after_sync();
-          const uint64_t k_desc = make_smem_desc_sw128(smem_u32(k_smem + st * AS_TILE), 16, 1024);
+    // ------------------------------ MMA issuer (a converged warp, one lane issues) ------
+    constexpr uint32_t IDESC_S = make_idesc(1, 1, AS_BM, AS_BN, 0, 0);
+    constexpr uint32_t IDESC_O3 = make_idesc(1, 1, AS_BM, 192, 0, 1);  // V is MN-major
+    constexpr uint32_t IDESC_O2 = make_idesc(1, 1, AS_BM, 128, 0, 1);
+    constexpr uint32_t IDESC_O1 = make_idesc(1, 1, AS_BM, 64, 0, 1);
+    constexpr uint64_t PL = AS_PLANE >> 4;
+    constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};  // smallest products first
+    const uint32_t s_tmem = tmem_base + AS_S_COL, p_tmem = tmem_base + AS_P_COL, o_tmem = tmem_base + AS_O_COL;
+    const uint64_t q_desc = make_smem_desc_sw128(smem_u32(q_smem), 16, 1024);
+    const uint64_t k_desc0 = make_smem_desc_sw128(smem_u32(k_smem), 16, 1024);
+    // planes 8 KiB apart along N (leading-dimension offset)
+    const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(v_smem), AS_HPLANE, 1024);
+    const bool issuer = elect_one();
+    bool ok = mbar_wait_all(q_full, 0, wc, DEV_TIMEOUT_ATTN_Q);
+    // iteration j issues the scores of tile j and the products of tile j - 1
+    for (int j = 0; j <= nkv && ok; ++j) {
+      if (j < nkv) {
+        const int st = j & 1;
+        if (j >= 1 && !mbar_wait_all(s_free, (j - 1) & 1, wc, DEV_TIMEOUT_ATTN_S)) break;
+        if (!mbar_wait_all(&k_full[st], (j >> 1) & 1, wc, DEV_TIMEOUT_ATTN_KV)) break;
+        tc_fence_after_sync();
+        if (issuer) {
+          const uint64_t k_desc = k_desc0 + static_cast<uint32_t>(st * (AS_TILE >> 4));
 #pragma unroll
           for (int q = 0; q < 6; ++q)
 #pragma unroll
@@ -195,14 +206,15 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
           mma_commit(&k_empty[st]);
           mma_commit(s_full);
         }
-        if (j >= 1) {
-          const int jj = j - 1;
-          if (!mbar_wait(p_ready, jj & 1, wc, DEV_TIMEOUT_ATTN_P)) break;
-          for (int hf = 0; hf < 2; ++hf) {
-            if (!mbar_wait(&v_full[hf], jj & 1, wc, DEV_TIMEOUT_ATTN_KV)) { ok = false; break; }
-            tc_fence_after_sync();
-            // planes 8 KiB apart along N (leading-dimension offset)
-            const uint64_t v_desc = make_smem_desc_sw128(smem_u32(v_smem + hf * (AS_TILE / 2)), AS_HPLANE, 1024);
+      }
+      if (j >= 1) {
+        const int jj = j - 1;
+        if (!mbar_wait_all(p_ready, jj & 1, wc, DEV_TIMEOUT_ATTN_P)) break;
+        for (int hf = 0; hf < 2; ++hf) {
+          if (!mbar_wait_all(&v_full[hf], jj & 1, wc, DEV_TIMEOUT_ATTN_KV)) { ok = false; break; }
+          tc_fence_after_sync();
+          if (issuer) {
+            const uint64_t v_desc = v_desc0 + static_cast<uint32_t>(hf * (AS_TILE / 2 >> 4));
 #pragma unroll
             for (int k = 0; k < 4; ++k) {  // 16 keys: 8 columns of bf16 pairs, 16 rows of V (128 B each)
               const uint64_t vk = v_desc + static_cast<uint64_t>((k * 16 * 128) >> 4);
@@ -213,8 +225,8 @@ attention_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __
             }
             mma_commit(&v_empty[hf]);
           }
-          if (ok) mma_commit(pv_done);
         }
+        if (ok && issuer) mma_commit(pv_done);
       }
     }
   } else {

@@ -21,14 +21,14 @@
 // Two CTAs (a cluster on neighbouring SMs) share a 256 x PBN tile with
 // tcgen05.mma.cta_group::2 and walk tiles persistently: each CTA's warp 0 streams the
 // planes of its 128 rows of A and its half of W with TMA (3-D boxes of 64 K x rows
-// x 3 planes), two threads of the even CTA issue the 24 MMAs of every K block (blocks in turn, so the
-// barrier work of one runs under the MMAs of the other), the epilogue warps of both add
+// x 3 planes), two warps of the even CTA issue the 24 MMAs of every K block (blocks in turn, an elected lane
+// of each, see mbar_wait_all), the epilogue warps of both add
 // up the blocks and run the fused epilogue.  Four accumulators rotate, so the adds run
 // under the MMAs of the following blocks.
 //
-// A block has its own accumulator, so no order is needed between the MMAs of the two threads; but each
-// thread waits for its own blocks only, and the ring has three stages: the barriers that announce
-// landed operands are laid out by operand_ring.h so that a thread sees every phase of those it waits on.
+// A block has its own accumulator, so no order is needed between the MMAs of the two warps; but each
+// warp waits for its own blocks only, and the ring has three stages: the barriers that announce
+// landed operands are laid out by operand_ring.h so that a warp sees every phase of those it waits on.
 //
 // K split: where one wave of tiles leaves half of the SMs without work, two CTA pairs
 // (a cluster of four) share a tile, each takes half of K, and the second pair hands
@@ -42,7 +42,8 @@
 // MMA: tensor pipe 38 % busy); 256 x 256 tiles (3072 cycles of MMA took 4060: two stages of
 // operands, two accumulators, and an epilogue of 128 columns per thread between tiles).
 //
-// Measured: 24-block model at 512 x 512 (1024 + 333 tokens) 15.1 ms, one dual block of 256 + 77 tokens 295 us;
+// Measured: 24-block model at 512 x 512 (1024 + 333 tokens) 14.7 ms, one dual block of 256 + 77 tokens 291 us (15.1 and
+// 294 while lane 0 alone ran the loads and the MMAs, here and in attention_split.cu);
 // with FFMA GEMMs and the SIMT attention 754 ms and 4.74 ms.  What single steps gave, in the order they were made
 // (each against the commit before it; the attention changed in between): one-CTA tiles -> pairs 19.26 -> 17.57 ms
 // and 454 -> 411 us; K split 381 -> 337 us; no cluster-scope release in the accumulator's hand-back
@@ -255,7 +256,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + NBUF);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known uniform
   const int lane = threadIdx.x & 31;
   const uint32_t part = cluster_ctarank() >> 1;  // share of K (KSPLIT == 2)
   const uint32_t rank = cluster_ctarank() & 1;   // CTA of the pair, 0 = leader
@@ -296,7 +297,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
     grid_dep_wait();
     grid_dep_launch();
   }
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, p0.g.status};
   // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
   // K blocks of this pair (the same K for all problems)
@@ -304,15 +305,17 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
   const int KB = (KSPLIT == 2 && part == 0 ? (p0.g.k_blocks + 1) / 2 : p0.g.k_blocks) - kb0;
   float acc[CPW];  // running sums of an epilogue thread
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------
     Ring ring;
     bool ok = true;
+    const bool issuer = elect_one();
+    const uint32_t smem_at = smem_u32(smem), full_local = smem_u32(full_bar), full_leader = map_to_cta(full_local, leader);
     // the weights of a stage; all its bytes (both CTAs) are credited to the leader's barrier
-    auto load_w = [&](const SplitProblem& pp, const Ring& at, int kb, int n0) {
-      if (rank == 0) mbar_expect_tx(&full_bar[at.full], 2 * Cfg::STAGE_BYTES);
-      tma_load_3d_pair(smem + at.stage * Cfg::STAGE_BYTES + 3 * S_A_PLANE, &pp.tmW,
-                       map_to_cta(smem_u32(&full_bar[at.full]), leader), (kb0 + kb) * S_KB, n0, 0);
+    auto load_w = [&](const CUtensorMap* tmW, const Ring& at, int kb, int n0) {
+      if (rank == 0) mbar_expect_tx_at(full_local + 8 * at.full, 2 * Cfg::STAGE_BYTES);
+      tma_load_3d_pair_at(smem_at + at.stage * Cfg::STAGE_BYTES + 3 * S_A_PLANE, tmW, full_leader + 8 * at.full,
+                          (kb0 + kb) * S_KB, n0, 0);
     };
     int pre = 0;  // stages of the first tile whose weights are under way before the wait
     if (p0.g.epi.w_static) {
@@ -320,7 +323,7 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
       const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
       Ring at;
       for (; pre < STAGES && pre < KB; ++pre, at.next())
-        load_w(pp, at, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS);
+        if (issuer) load_w(&pp.tmW, at, pre, (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * Cfg::W_ROWS);
     }
     grid_dep_wait();
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -332,42 +335,46 @@ gemm_split_tcgen05_kernel(const __grid_constant__ SplitProblem p0, const __grid_
         if (pre > 0) {
           --pre;
         } else {
-          if (!mbar_wait(&empty_bar[ring.stage], ring.stage_parity ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-          load_w(pp, ring, kb, n0);
+          if (!mbar_wait_all(&empty_bar[ring.stage], ring.stage_parity ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+          if (issuer) load_w(&pp.tmW, ring, kb, n0);
         }
-        tma_load_3d_pair(smem + ring.stage * Cfg::STAGE_BYTES, &pp.tmA, map_to_cta(smem_u32(&full_bar[ring.full]), leader),
-                         (kb0 + kb) * S_KB, m0, 0);
+        if (issuer)
+          tma_load_3d_pair_at(smem_at + ring.stage * Cfg::STAGE_BYTES, &pp.tmA, full_leader + 8 * ring.full,
+                              (kb0 + kb) * S_KB, m0, 0);
         ring.next();
       }
     }
-  } else if ((warp == 1 || warp == Cfg::MMA2_WARP) && lane == 0) {
-    // ------------------------------ MMA issuers (leader only) -----------------
+  } else if (warp == 1 || warp == Cfg::MMA2_WARP) {
+    // ------------------------------ MMA issuers (leader only, two warps) ------
     if (rank == 0) {
       const int me = warp == 1 ? 0 : 1;
       Ring ring;
-      int buf = 0;  // four accumulators: a thread sees every use of its two
+      int buf = 0;  // four accumulators: a warp sees every use of its two
       uint32_t bphase = 0;
       bool ok = true;
+      const bool issuer = elect_one();
+      const uint64_t desc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         for (int kb = 0; kb < KB; ++kb) {
           if (ring.turn == me) {
-            if (!mbar_wait(&tempty_bar[buf], bphase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-            if (!mbar_wait(&full_bar[ring.full], ring.full_parity, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
+            if (!mbar_wait_all(&tempty_bar[buf], bphase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[ring.full], ring.full_parity, wc, DEV_TIMEOUT_FULL))) { ok = false; break; }
             tc_fence_after_sync();
-            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * PBN);
-            const uint32_t a_addr = smem_u32(smem + ring.stage * Cfg::STAGE_BYTES);
-            const uint64_t a0 = make_smem_desc_sw128(a_addr, 16, 1024);
-            const uint64_t w0 = make_smem_desc_sw128(a_addr + 3 * S_A_PLANE, 16, 1024);
-            constexpr uint64_t AP = S_A_PLANE >> 4, WP = Cfg::W_PLANE >> 4;
-            // (A plane, W plane), smallest products first
-            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
+            if (issuer) {
+              const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * PBN);
+              const uint64_t a0 = desc0 + static_cast<uint32_t>(ring.stage * (Cfg::STAGE_BYTES >> 4));
+              const uint64_t w0 = a0 + (3 * S_A_PLANE >> 4);
+              constexpr uint64_t AP = S_A_PLANE >> 4, WP = Cfg::W_PLANE >> 4;
+              // (A plane, W plane), smallest products first
+              constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PW[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-            for (int q = 0; q < 6; ++q)
+              for (int q = 0; q < 6; ++q)
 #pragma unroll
-              for (int k = 0; k < S_KB / 16; ++k)
-                mma_f16_ss_pair(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
-            mma_commit_pair(&empty_bar[ring.stage], pair_mask);  // frees the stage in both CTAs
-            mma_commit_pair(&tfull_bar[buf], pair_mask);    // block sum ready in both CTAs
+                for (int k = 0; k < S_KB / 16; ++k)
+                  mma_f16_ss_pair(d_tmem, a0 + PA[q] * AP + 2 * k, w0 + PW[q] * WP + 2 * k, IDESC, (q | k) != 0);
+              mma_commit_pair(&empty_bar[ring.stage], pair_mask);  // frees the stage in both CTAs
+              mma_commit_pair(&tfull_bar[buf], pair_mask);         // block sum ready in both CTAs
+            }
           }
           ring.next();
           if (++buf == NBUF) { buf = 0; bphase ^= 1; }

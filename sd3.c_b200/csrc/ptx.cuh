@@ -441,12 +441,12 @@ __device__ __forceinline__ void tma_load_2d_pair_at(uint32_t smem_dst, const voi
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(cluster_bar_addr), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, uint32_t cluster_bar_addr,
-                                                 int x, int y, int z) {
+__device__ __forceinline__ void tma_load_3d_pair_at(uint32_t smem_dst, const void* tmap, uint32_t cluster_bar_addr,
+                                                    int x, int y, int z) {
   asm volatile(
       "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)),
+      ::"r"(smem_dst),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(cluster_bar_addr), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
