@@ -8,7 +8,9 @@
 // accumulators, warps 2-5 drain the other accumulator through the fused
 // epilogue (bias / GELU-tanh / gate+residual / per-head QK-RMSNorm with token
 // re-mapping / position-table add / unpatchify), so the epilogue of tile i
-// overlaps the main loop of tile i+1.
+// overlaps the main loop of tile i+1.  Warps 0 and 1 stay converged and an elected lane issues (ptx.cuh,
+// mbar_wait_all); against loops that lane 0 ran alone: 77 x 1536 x 6144 42.9 -> 38 us, 1024 x 64 x 1536
+// 11.0 -> 8.8, 154 x 6144 x 1536 15.9 -> 15.0.
 //
 // Replaces the reference's cuBLASLt call (cuda/dit.cu:683-756 launch_linear),
 // the SGEMM used for chunked projections (cuda/dit.cu:102-354) and the
@@ -68,7 +70,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known uniform
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -94,23 +96,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   tc_fence_after_sync();
   grid_dep_wait();
   grid_dep_launch();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, g.status};
 
   const int num_tiles = g.tiles_m * g.tiles_n;
   const int KB = g.k_blocks;
 
-  if (warp == 0 && lane == 0) {
-    // ------------------------------ TMA producer (one thread) ------------------
+  if (warp == 0) {
+    // ------------------------------ TMA producer (a converged warp, one lane issues) ------
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    const bool issuer = elect_one();
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const int m0 = (tile / g.tiles_n) * BM;
       const int n0 = (tile % g.tiles_n) * BN;
       for (int kb = 0; kb < KB; ++kb) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-        {
+        if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+        if (issuer) {
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
           tma_load_2d(sa, &tmA, &full_bar[stage], kb * ELEMS_PER_STAGE, m0);
@@ -119,34 +122,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ------------------------------ MMA issuer (one thread) --------------------
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (a converged warp, one lane issues) ------
     int stage = 0;
     uint32_t phase = 0;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    bool stage_ready = false;
+    const bool issuer = elect_one();
+    const uint64_t desc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-      tc_fence_after_sync();
+      if (!mbar_wait_all(&tempty_bar[acc], acc_phase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) break;
       const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
       for (int kb = 0; kb < KB; ++kb) {
-        // readiness of this stage was tested while the previous stage's MMAs
-        // were being issued; block only if that early test failed
-        if (!stage_ready) {
-          if (!mbar_wait(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
-        }
-        int ns = stage + 1;
-        uint32_t np = phase;
-        if (ns == STAGES) { ns = 0; np ^= 1; }
-        const uint32_t next_ready = mbar_test_wait(&full_bar[ns], np);
+        if (!mbar_wait_all(&full_bar[stage], phase, wc, DEV_TIMEOUT_FULL)) { ok = false; break; }
         tc_fence_after_sync();
-        {
-          const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_STAGE_BYTES;
-          const uint64_t a_desc = make_smem_desc_sw128(a_addr, 16, 1024);
-          const uint64_t b_desc = make_smem_desc_sw128(b_addr, 16, 1024);
+        if (issuer) {
+          const uint64_t a_desc = desc0 + static_cast<uint32_t>(stage * (Cfg::STAGE_BYTES >> 4));
+          const uint64_t b_desc = a_desc + (A_STAGE_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < STAGE_K_BYTES / MMA_K_BYTES; ++k) {
             const uint64_t adv = static_cast<uint64_t>((k * MMA_K_BYTES) >> 4);
@@ -158,14 +151,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           mma_commit(&empty_bar[stage]);
           if (kb == KB - 1) mma_commit(&tfull_bar[acc]);
         }
-        stage = ns;
-        phase = np;
-        stage_ready = next_ready != 0;
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
-  } else if (warp >= 2) {
+  } else {
     // ------------------------------ epilogue ----------------------------------
     // Eight warps: warp w may read TMEM lanes [32 (w % 4), +32); warps 2-5 take
     // the first half of the tile's columns, warps 6-9 the second half.
