@@ -92,6 +92,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   constexpr int P_STAGES = pair_stages(PBN);
+  static_assert(EPI_WARPS * (PBN / 64) * P_RED_BYTES <= P_STAGES * P_STAGE_BYTES, "the last tile's boxes fit the ring");
   uint8_t* red_smem = smem + P_STAGES * P_STAGE_BYTES;  // 1024-byte aligned: stages are 32 / 24 KiB each
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + P_STAGES * P_STAGE_BYTES + pair_red_bytes(EPI, OUT_F32));
   uint64_t* empty_bar = full_bar + P_STAGES;
@@ -174,20 +175,20 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
           tma_load_2d_pair_at(ring + (st * SLOT + i) * P_STAGE_BYTES, tmA, full_leader + 8 * st, (kb + i) * KEL, m0);
     };
     int pre = 0;  // slots of the first tile whose weights are under way before the wait
-    if (p0.g.epi.w_static) {
-      const PairProblem& pp = pair < end0 ? p0 : pair < end1 ? p1 : p2;
-      const int lt = pair - (pair < end0 ? 0 : pair < end1 ? end0 : end1);
-      const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF;
-      for (; pre < NSLOT && pre * SLOT < KB; ++pre)
-        if (issuer) load_w(&pp.tmW, pre, pre * SLOT, n0);
-    }
-    grid_dep_wait();
+    bool waited = false;
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const PairProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
       const int n0 = (lt % pp.g.tiles_n) * PBN + static_cast<int>(rank) * P_BN_HALF;
       const CUtensorMap *tmA = &pp.tmA, *tmW = &pp.tmW;
+      if (!waited) {
+        if (p0.g.epi.w_static)
+          for (; pre < NSLOT && pre * SLOT < KB; ++pre)
+            if (issuer) load_w(tmW, pre, pre * SLOT, n0);
+        grid_dep_wait();
+        waited = true;
+      }
       for (int kb = 0; kb < KB; kb += SLOT) {
         if (pre > 0) {
           --pre;
@@ -255,14 +256,23 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
                              static_cast<uint32_t>(acc * PBN);
       bool drained;
+      // After the pair's last tile the operand ring is idle (its accumulator is complete, so every load has landed
+      // and every MMA has read it): each box of the epilogue gets a buffer of its own there, and none waits for the
+      // one before it to have been read.  us of a launch, before -> after: gate + residual K 1536, 589 rows 8.8 -> 8.2,
+      // 1357 rows 9.6 -> 9.3; K 6144, 589 rows 20.3 -> 19.7; GELU 1357 rows 23.5 -> 22.5, 4429 rows 61.1 -> 59.2.  (256-wide
+      // QKV tiles lose it to spilled registers: 4429 rows 47.4 -> 50.5.)
+      constexpr bool OWN_BOXES = !(EPI == EPI_QKV_NORM && PBN == 256);
+      const bool last = OWN_BOXES && tile + num_pairs >= num_tiles;
+      constexpr int BOXES = PBN / 2 / (EPI == EPI_GATE_RESID ? 32 : 64);  // of a warp and tile
+      uint8_t* box = last ? smem + (warp - 2) * (BOXES * P_RED_BYTES) : red_smem + (warp - 2) * P_RED_BYTES;
+      const int box_step = last ? P_RED_BYTES : 0;
       if constexpr (EPI == EPI_GATE_RESID)
         drained = drain_tile_gate_reduce<PBN>(t_row, m0 + quad * 32, n0, half, g, &pp.tmR, &tfull_bar[acc],
-                                              acc_phase, wc, red_smem + (warp - 2) * P_RED_BYTES);
+                                              acc_phase, wc, box, box_step);
       else
-        drained = drain_tile<PBN, EPI, OUT_F32>(
-            t_row, m0 + row, n0, half, g, &tfull_bar[acc], acc_phase, wc,
-            (pair_stages_out(EPI, OUT_F32) && g.tma_store) ? red_smem + (warp - 2) * P_RED_BYTES : nullptr,
-            &pp.tmR);
+        drained = drain_tile<PBN, EPI, OUT_F32>(t_row, m0 + row, n0, half, g, &tfull_bar[acc], acc_phase, wc,
+                                                (pair_stages_out(EPI, OUT_F32) && g.tma_store) ? box : nullptr,
+                                                &pp.tmR, box_step);
       if (!drained) break;
       tc_fence_before_sync();
       __syncwarp();

@@ -128,10 +128,11 @@ __device__ __forceinline__ RowMap map_row(int m, const GemmEpilogue& e) {
 // warp and the tensor map of the bf16 output.  With them the warp's 32 rows x 64 columns
 // leave as ONE TMA store (rows in the 128-byte swizzle, 16-byte chunk c of row r at chunk
 // c ^ (r & 7)) instead of 128 32-byte register stores; orow0 is the output row of lane 0.
+// fresh: the warp has not stored from `stage` before.
 template <int EPI, bool OUT_F32>
 __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, int n_base,
                                             const GemmArgs& g, uint8_t* stage = nullptr,
-                                            const void* tmO = nullptr, long orow0 = 0) {
+                                            const void* tmO = nullptr, long orow0 = 0, bool fresh = false) {
   const GemmEpilogue& e = g.epi;
   const int N = g.N;
   if constexpr (EPI == EPI_QKV_NORM) {
@@ -189,7 +190,7 @@ __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, in
   if constexpr (!OUT_F32 && (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_QKV_NORM)) {
     if (stage != nullptr && !e.out_e4m3) {  // warp-uniform
       const int lane = threadIdx.x & 31;
-      if (lane == 0) bulk_wait_group_read0();  // the previous store of this warp has read the buffer
+      if (lane == 0 && !fresh) bulk_wait_group_read0();  // the previous store of this warp has read the buffer
       __syncwarp();
       uint8_t* my_row = stage + lane * 128;
 #pragma unroll
@@ -244,10 +245,11 @@ __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, in
 // t_row: TMEM address of the accumulator (lane quadrant and column base applied);
 // m: global output row of this thread; n0: first output column of the tile.
 // Waits for the accumulator on tfull_bar; returns false if that wait gave up.
+// stage_step: bytes between the buffers of consecutive chunks; 0: all use the one at `stage`.
 template <int BN, int EPI, bool OUT_F32>
 __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int half, const GemmArgs& g,
                                            uint64_t* tfull_bar, uint32_t phase, const WaitCtx& wc,
-                                           uint8_t* stage = nullptr, const void* tmO = nullptr) {
+                                           uint8_t* stage = nullptr, const void* tmO = nullptr, int stage_step = 0) {
   constexpr int COLS_PER_WARP = BN / 2;
   const GemmEpilogue& e = g.epi;
   const bool valid = m < g.M;
@@ -320,7 +322,9 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
       }
       if (stage != nullptr) {
         // whole warp valid or not at all (M % 32 == 0 is a condition of this path)
-        if (valid) epilogue_64<EPI, OUT_F32>(v, rm, n_base, g, stage, tmO, rm.orow - (threadIdx.x & 31));
+        if (valid)
+          epilogue_64<EPI, OUT_F32>(v, rm, n_base, g, stage + ci * stage_step, tmO, rm.orow - (threadIdx.x & 31),
+                                    stage_step != 0);
       } else if (valid) {
         epilogue_64<EPI, OUT_F32>(v, rm, n_base, g);
       }
@@ -341,11 +345,13 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
 // sits at chunk c ^ (r & 7), which also makes the row-per-thread writes
 // conflict-free) and lane 0 issues one reduction for the box.  Requires
 // out == resid.  `stage` is 1024-byte aligned.  m_w0: first row of this warp.
+// stage_step: bytes between the buffers of consecutive boxes; 0: all use the one at
+// `stage`, each after the reduction before it has read the buffer.
 template <int BN>
 __device__ __forceinline__ bool drain_tile_gate_reduce(uint32_t t_row, int m_w0, int n0, int half,
                                                        const GemmArgs& g, const void* tmR,
                                                        uint64_t* tfull_bar, uint32_t phase,
-                                                       const WaitCtx& wc, uint8_t* stage) {
+                                                       const WaitCtx& wc, uint8_t* stage, int stage_step) {
   constexpr int CPW = BN / 2, NSUB = CPW / 32;
   const GemmEpilogue& e = g.epi;
   const int lane = threadIdx.x & 31;
@@ -353,12 +359,17 @@ __device__ __forceinline__ bool drain_tile_gate_reduce(uint32_t t_row, int m_w0,
   const int b = (m < g.M ? m : g.M - 1) / e.rows_in;
   const float* gate_row = e.gate + static_cast<long>(b) * e.gate_stride;
   const int nw = n0 + half * CPW;
-  float gg[32], bb[32];
-  load_f4_batch<8>(gate_row, nw, g.N, gg);
-  load_f4_batch<8>(e.bias, nw, g.N, bb);
+  // gate and bias are loaded ahead, those of the first boxes before the accumulator is complete: both of a 128-wide
+  // tile's; of a 256-wide one's (four boxes, unrolled) one, or the registers do not suffice
+  constexpr int AHEAD = BN == 128 ? 2 : 1;
+  float gg[AHEAD][32], bb[AHEAD][32];
+#pragma unroll
+  for (int sub = 0; sub < AHEAD; ++sub) {
+    load_f4_batch<8>(gate_row, nw + sub * 32, g.N, gg[sub]);
+    load_f4_batch<8>(e.bias, nw + sub * 32, g.N, bb[sub]);
+  }
   if (!mbar_wait_warp(tfull_bar, phase, wc, DEV_TIMEOUT_TMEM_FULL)) return false;
   tc_fence_after_sync();
-  uint8_t* my_row = stage + lane * 128;
 #pragma unroll
   for (int sub = 0; sub < NSUB; ++sub) {
     const int n_base = nw + sub * 32;
@@ -367,14 +378,16 @@ __device__ __forceinline__ bool drain_tile_gate_reduce(uint32_t t_row, int m_w0,
     tmem_wait_ld();
     float d[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) d[j] = gg[j] * fmaf(__uint_as_float(r[j]), e.alpha, bb[j]);
-    if (sub + 1 < NSUB) {
-      load_f4_batch<8>(gate_row, n_base + 32, g.N, gg);
-      load_f4_batch<8>(e.bias, n_base + 32, g.N, bb);
+    for (int j = 0; j < 32; ++j) d[j] = gg[sub % AHEAD][j] * fmaf(__uint_as_float(r[j]), e.alpha, bb[sub % AHEAD][j]);
+    if (sub + AHEAD < NSUB) {
+      load_f4_batch<8>(gate_row, n_base + 32 * AHEAD, g.N, gg[sub % AHEAD]);
+      load_f4_batch<8>(e.bias, n_base + 32 * AHEAD, g.N, bb[sub % AHEAD]);
     }
+    uint8_t* box = stage + sub * stage_step;
     // the previous reduction of this warp must have read the buffer
-    if (sub > 0 && lane == 0) bulk_wait_group_read0();
+    if (sub > 0 && stage_step == 0 && lane == 0) bulk_wait_group_read0();
     __syncwarp();
+    uint8_t* my_row = box + lane * 128;
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       *reinterpret_cast<float4*>(my_row + ((c ^ (lane & 7)) << 4)) =
@@ -382,12 +395,12 @@ __device__ __forceinline__ bool drain_tile_gate_reduce(uint32_t t_row, int m_w0,
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0 && m_w0 < g.M) {
-      tma_reduce_add_2d(tmR, stage, n_base, m_w0);
+      tma_reduce_add_2d(tmR, box, n_base, m_w0);
       bulk_commit_group();
     }
   }
   // the buffer is reused by this warp's next tile
-  if (lane == 0) bulk_wait_group_read0();
+  if (stage_step == 0 && lane == 0) bulk_wait_group_read0();
   __syncwarp();
   return true;
 }
