@@ -15,7 +15,7 @@
 //                               second QKV GEMM(x) rides in the same launch (up to MERGE_MAX_TOKENS)
 //   joint attention          -> o_c, o_x; a dual block's attention over the image tokens too
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
-//   [dual] out-proj GEMM with gate2
+//   [dual] out-proj GEMM with gate2 (up to MERGE_MAX_TOKENS in the same launch)
 //   LN+modulate(x), (c); MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual), each for x and c at once
 #include <math.h>
 #include <algorithm>
@@ -78,6 +78,7 @@ struct Workspace {
   void* a8 = nullptr;    // FP8 mode: e4m3 copy of the current GEMM's left operand
   void* attn_scratch = nullptr;  // partial results of key-split attention launches (small batches, long sequences)
   size_t attn_scratch_bytes = 0;
+  unsigned* order = nullptr;  // a dual block's two out-projections into x as one launch (GemmEpilogue::order)
   // position table cache
   float* pos = nullptr;
   int pos_h = 0, pos_w = 0;
@@ -274,6 +275,7 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
       {&w.hid_x, nTx * F * ab}, {&w.hid_c, nTc * F * ab},
       {(void**)&w.o_f32, m->f32 && m->D != 64 ? nB * T * E * 4 : 16},
       {&w.a8, m->fp8 ? (nTx > nTc ? nTx : nTc) * F : 16},
+      {(void**)&w.order, m->f32 ? 16 : gate_order_words(static_cast<long>(nTx), m->E) * sizeof(unsigned)},
       {&w.attn_scratch, 16},
   };
   // key-split attention (head_dim 64 tensor-core path): the larger need of the joint and the image-only call
@@ -535,10 +537,11 @@ bool merge_launches(int B, int Tc, int Tx) {
 }
 
 // the LayerNorms of the image and the context rows, as one launch where both write the same type
-int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st) {
+int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st,
+                unsigned* zero = nullptr, int nzero = 0) {
   if (!pc || (out_x == out_c && merge_launches(px.B, pc->T, px.T)))
-    return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
-  int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st);
+    return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st, zero, nzero);
+  int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st, zero, nzero);
   return rc ? rc : launch_ln_modulate(px, nullptr, E, 1e-6f, ms, out_x, st);
 }
 
@@ -567,12 +570,16 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const bool c8a = m->fp8 && L.c_qkv.w8, x8a = m->fp8 && L.x_qkv.w8 && (!L.dual || L.d_qkv.w8);
   const bool c8m = m->fp8 && L.c_mlp1.w8, x8m = m->fp8 && L.x_mlp1.w8;
   auto ln_out = [&](bool e4m3) { return m->f32 ? 3 : (e4m3 ? 2 : 0); };
+  // a dual block's image-only attention and out-projection beside the joint ones, or after them
+  const bool together = L.dual && m->D == 64 && merge_launches(B, Tc, Tx);
+  const bool out_together = together && !m->f32 && !L.last;
+  const size_t order_words = out_together ? gate_order_words(static_cast<long>(B) * Tx, E) : 0;
   // pre-attention LayerNorm + modulate
   {
     LnProblem px = {x, B, Tx, x_shift_a, x_scale_a, w.h_x, nullptr, nullptr, nullptr};
     if (L.dual) { px.shift2 = x_shift_2; px.scale2 = x_scale_2; px.out2 = w.h_x2; }
     const LnProblem pc = {c, B, Tc, c_shift_a, c_scale_a, w.h_c, nullptr, nullptr, nullptr};
-    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st));
+    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st, w.order, static_cast<int>(order_words)));
   }
   // QKV (context rows first, then image rows) and joint attention
   // image and context GEMMs of a kind share a launch (bf16 / FP8 modes: with head_dim 64)
@@ -581,8 +588,6 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const bool pre_j = L.c_wq_s != nullptr && L.x_wq_s != nullptr;
   const float* c_wq = pre_j ? L.c_wq_s : L.c_wq;
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
-  // a dual block's image-only attention beside the joint one, or after it
-  const bool together = L.dual && m->D == 64 && merge_launches(B, Tc, Tx);
   const bool pre_d = L.d_wq_s != nullptr;
   const float* d_wq = pre_d ? L.d_wq_s : L.d_wq;
   if (m->D == 64) {
@@ -603,7 +608,16 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const AttnCall att[2] = {{w.qkv, T, Tc, L.last ? nullptr : w.o_c, w.o_x, o8, L.joint_bound, pre_j},
                            {w.qkv2, Tx, 0, nullptr, w.o_x2, o8d, L.dual_bound, pre_d}};
   SD3_TRY(run_attention(m, att, together ? 2 : 1, B, st));
-  if (grouped && !L.last) {
+  if (out_together) {
+    // both projections into x and the context rows' one: per element of x the joint attention's part is added first,
+    // as in separate launches
+    LinearCall out[3] = {{&L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8},
+                         {&L.c_out, w.o_c, B * Tc, gate_epilogue(L.c_out, Tc, c_gate_a, ms, c), o8},
+                         {&L.d_out, w.o_x2, B * Tx, gate_epilogue(L.d_out, Tx, x_gate_2, ms, x), o8d}};
+    out[0].epi.order = out[2].epi.order = w.order;
+    out[2].epi.order_second = 1;
+    SD3_TRY(run_linear_group(m, out, 3, st));
+  } else if (grouped && !L.last) {
     SD3_TRY(run_linear_pair(m, L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8,
                             L.c_out, w.o_c, B * Tc, gate_epilogue(L.c_out, Tc, c_gate_a, ms, c), o8, st));
   } else {
@@ -615,7 +629,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
       SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
       SD3_TRY(run_attention(m, att + 1, 1, B, st));
     }
-    SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
+    if (!out_together) SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
   }
   // MLPs of both streams: LayerNorm + modulate each, then the two first linears (GELU-tanh) and
   // the two second linears (gate + residual), each pair as one grouped launch

@@ -268,7 +268,9 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       const int box_step = last ? P_RED_BYTES : 0;
       if constexpr (EPI == EPI_GATE_RESID)
         drained = drain_tile_gate_reduce<PBN>(t_row, m0 + quad * 32, n0, half, g, &pp.tmR, &tfull_bar[acc],
-                                              acc_phase, wc, box, box_step);
+                                              acc_phase, wc, box, box_step,
+                                              g.epi.order ? g.epi.order + (lt * 2 + rank) * EPI_WARPS + (warp - 2)
+                                                          : nullptr);
       else
         drained = drain_tile<PBN, EPI, OUT_F32>(t_row, m0 + row, n0, half, g, &tfull_bar[acc], acc_phase, wc,
                                                 (pair_stages_out(EPI, OUT_F32) && g.tma_store) ? box : nullptr,
@@ -416,13 +418,26 @@ bool gemm_pair_supported(int operand_dtype, int M, int N, int K, const GemmEpilo
   return operand_dtype == OPERAND_BF16;
 }
 
+// One word per pair tile of either width, CTA and epilogue warp.  Which of the words a launch uses depends on its tile
+// width, which is the same for both problems.
+size_t gate_order_words(long M, int N) {
+  return static_cast<size_t>((M + 2 * P_BM - 1) / (2 * P_BM)) * (N / 128) * 2 * EPI_WARPS;
+}
+
 // One to three problems of the same N, K, operand type and epilogue kind.
+// A tile that waits for another (GemmEpilogue::order) waits for one of an earlier problem: earlier in the list of
+// tiles that every pair walks in order, and pairs are one per SM pair of the device and started in order, so the
+// first unfinished tile never waits.
 int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
                      cudaStream_t stream) {
   const bool fp8 = operand_dtype == OPERAND_E4M3;
   const GemmProblem& a = q[0];
   long tiles256 = 0;
   for (int i = 0; i < n; ++i) {
+    if (q[i].epi.order && q[i].epi.order_second && i == 0) {
+      set_last_error("gemm_pair: the problem that adds second comes first in its launch");
+      return ST_INVALID_ARG;
+    }
     if (q[i].epi.mode != a.epi.mode || q[i].epi.out_f32 != a.epi.out_f32) {
       set_last_error("gemm_pair: grouped problems need the same epilogue kind");
       return ST_INVALID_ARG;

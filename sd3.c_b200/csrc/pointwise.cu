@@ -72,11 +72,13 @@ __device__ __forceinline__ void ln_store4(void* out, long row, long rows, int E,
 
 template <int MAXV, int OUT, bool DUAL>
 __global__ void __launch_bounds__(LN_WARPS * 32, OUT == 3 ? 3 : 4)
-ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a, int E, float eps, long mod_stride,
+ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a, unsigned* zero, int nzero, int E, float eps, long mod_stride,
                    int rpw) {
   extern __shared__ float4 ln_smem[];  // [1 + scale1 | shift1 | 1 + scale2 | shift2], E floats each
   grid_dep_wait();
   grid_dep_launch();
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<unsigned>(nzero); i += gridDim.x * blockDim.x)
+    zero[i] = 0;
   const bool second = blockIdx.x >= grid_a;
   const LnProblem& p = second ? pb : pa;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -183,7 +185,7 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
 
 template <int MAXV>
 int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
-                   cudaStream_t stream) {
+                   cudaStream_t stream, unsigned* zero, int nzero) {
   const long rows_a = static_cast<long>(a.B) * a.T, rows_b = b ? static_cast<long>(b->B) * b->T : 0;
   // rows per warp: as many as keeps at least two CTAs per SM busy
   int rpw = LN_MAX_ROWS_PER_WARP;
@@ -194,7 +196,7 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   const size_t smem = static_cast<size_t>(E) * 4 * (dual ? 4 : 2);
   const LnProblem pb = b ? *b : a;
 #define SD3_LN_LAUNCH(F32, DUALV)                                                                                    \
-  launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, E, eps,   \
+  launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero, nzero, E, eps,   \
                    mod_stride, rpw)
   if (out_f32 == 1) {
     if (dual) SD3_LN_LAUNCH(1, true); else SD3_LN_LAUNCH(1, false);
@@ -381,7 +383,7 @@ __global__ void rmsnorm_heads_kernel(XT* x, long ld, long rows, int col0, int nh
 }  // namespace
 
 int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, unsigned* zero, int nzero) {
   for (const LnProblem* p : {&a, b}) {
     if (!p) continue;
     if (!p->x || !p->out1 || !p->shift1 || !p->scale1 || p->B <= 0 || p->T <= 0 || E <= 0 || (E & 3) ||
@@ -396,7 +398,7 @@ int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps,
   }
   const int nvec = E / 4;
 #define SD3_LN_CASE(MV) \
-  if (nvec <= 32 * MV) return launch_ln_inst<MV>(a, b, E, eps, mod_stride, out_f32, stream)
+  if (nvec <= 32 * MV) return launch_ln_inst<MV>(a, b, E, eps, mod_stride, out_f32, stream, zero, nzero)
   SD3_LN_CASE(2);
   SD3_LN_CASE(6);
   SD3_LN_CASE(12);
