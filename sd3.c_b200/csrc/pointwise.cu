@@ -22,7 +22,7 @@ int device_sm_count();
 namespace {
 
 // ----------------------------------------------------------------------------
-// LayerNorm + modulate.  One warp per row, the row lives in registers.
+// LayerNorm + modulate.  One warp per row, the row lives in registers (fewer rows: one CTA per row, further down).
 // ----------------------------------------------------------------------------
 // OUT: 0 bf16, 1 fp32, 2 e4m3 (operand of an FP8 GEMM, converted as is), 3 three bf16 planes of
 // rows * E elements (operand of a split fp32 GEMM)
@@ -41,6 +41,13 @@ namespace {
 // and two of them in a row cost twice that.  The first row is requested before the
 // barrier behind the staging.  Measured (whole forward, one image): 256x256 3510 -> 3326 us,
 // 1024x1024 14.18 -> 13.96 ms.  Three CTAs per SM for the plane output, whose splits need the registers.
+constexpr int LN_ROW_QUADS = 12;  // ln_modulate_row_kernel: float4 words of a row per lane index (E up to 1536)
+// Rows of a launch (both problems) up to which it is taken, for one and for two modulations; us, kernel with staged
+// vectors / this one: one   589 rows 4.45 / 2.45, 1357 5.29 / 4.10, 2714 7.82 / 6.22, 3400 7.91 / 7.13 | 4000 8.10 / 8.35,
+//                           4429 8.34 / 8.95, 8858 17.9 / 18.4, 35432 60.6 / 68.9
+//                     two   589 rows 6.70 / 3.40, 1357 8.26 / 5.16, 2714 12.5 / 8.4, 4429 14.2 / 12.2, 8858 29.4 / 26.7,
+//                           16384 50.6 / 47.0 | 35432 97.4 / 97.4
+constexpr long LN_ROW_MAX = 3700, LN_ROW_MAX_DUAL = 32768;
 constexpr int LN_MAX_ROWS_PER_WARP = 8;
 constexpr int LN_WARPS = 8;
 
@@ -183,6 +190,72 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
   }
 }
 
+// The same for fewer rows: a CTA of four warps per row, so that the row and its modulation vectors are requested at once
+// and one memory latency is exposed, where the kernel above stages the vectors, and two modulations' take as long as the
+// row.  The sums are formed in the order of the kernel above (each lane adds its quads in order, then the lanes' tree): the
+// same bits.  Bound by latency at a thousand rows (3.2 TB/s of L2 at 1357), by L2 above (LN_ROW_MAX has the figures).
+template <int OUT, bool DUAL>
+__global__ void __launch_bounds__(128)
+ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned rows_a,
+                       unsigned* zero, int nzero, int E, float eps, long mod_stride) {
+  __shared__ float part[2][LN_ROW_QUADS][32];
+  grid_dep_wait();
+  grid_dep_launch();
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<unsigned>(nzero); i += gridDim.x * blockDim.x)
+    zero[i] = 0;
+  const bool second = blockIdx.x >= rows_a;
+  const LnProblem& p = second ? pb : pa;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nvec = E >> 2;
+  const long row = second ? blockIdx.x - rows_a : blockIdx.x, rows = static_cast<long>(p.B) * p.T;
+  const long moff = static_cast<long>(row / p.T) * mod_stride;
+  const bool dual = DUAL && p.out2 != nullptr;
+  constexpr int NV = LN_ROW_QUADS / 4;  // quads of a thread: j = NV * warp + t, elements 4 (lane + 32 j)
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 v[NV], sc1[NV], sh1[NV], sc2[DUAL ? NV : 1], sh2[DUAL ? NV : 1];
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    const int i = lane + 32 * (NV * warp + t);
+    const bool in = i < nvec;
+    v[t] = in ? *(reinterpret_cast<const float4*>(p.x + row * E) + i) : z4;
+    sc1[t] = in ? *(reinterpret_cast<const float4*>(p.scale1 + moff) + i) : z4;
+    sh1[t] = in ? *(reinterpret_cast<const float4*>(p.shift1 + moff) + i) : z4;
+    if constexpr (DUAL) {
+      sc2[t] = in && dual ? *(reinterpret_cast<const float4*>(p.scale2 + moff) + i) : z4;
+      sh2[t] = in && dual ? *(reinterpret_cast<const float4*>(p.shift2 + moff) + i) : z4;
+    }
+  }
+  auto row_sum = [&](float (&buf)[LN_ROW_QUADS][32]) {
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < LN_ROW_QUADS; ++j) s += buf[j][lane];
+    return warp_sum(s);
+  };
+#pragma unroll
+  for (int t = 0; t < NV; ++t) part[0][NV * warp + t][lane] = (v[t].x + v[t].y) + (v[t].z + v[t].w);
+  const float mean = row_sum(part[0]) / static_cast<float>(E);
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    const float a = v[t].x - mean, b = v[t].y - mean, c = v[t].z - mean, d = v[t].w - mean;
+    part[1][NV * warp + t][lane] = lane + 32 * (NV * warp + t) < nvec ? (a * a + b * b) + (c * c + d * d) : 0.f;
+  }
+  const float rstd = rsqrtf(row_sum(part[1]) / static_cast<float>(E) + eps);
+  auto modulate = [&](const float4& x, const float4& s, const float4& h) {
+    return make_float4(fmaf((x.x - mean) * rstd, s.x + 1.f, h.x), fmaf((x.y - mean) * rstd, s.y + 1.f, h.y),
+                       fmaf((x.z - mean) * rstd, s.z + 1.f, h.z), fmaf((x.w - mean) * rstd, s.w + 1.f, h.w));
+  };
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    const int i = lane + 32 * (NV * warp + t);
+    if (i >= nvec) break;
+    ln_store4<OUT>(p.out1, row, rows, E, i, modulate(v[t], sc1[t], sh1[t]));
+    if constexpr (DUAL) {
+      if (dual) ln_store4<OUT>(p.out2, row, rows, E, i, modulate(v[t], sc2[t], sh2[t]));
+    }
+  }
+}
+
 template <int MAXV>
 int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
                    cudaStream_t stream, unsigned* zero, int nzero) {
@@ -195,6 +268,27 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   const bool dual = a.out2 != nullptr || (b && b->out2 != nullptr);
   const size_t smem = static_cast<size_t>(E) * 4 * (dual ? 4 : 2);
   const LnProblem pb = b ? *b : a;
+  if (E <= 4 * 32 * LN_ROW_QUADS && rows_a + rows_b <= (dual ? LN_ROW_MAX_DUAL : LN_ROW_MAX)) {
+    const dim3 rows(static_cast<unsigned>(rows_a + rows_b));
+#define SD3_LN_ROW(F32)                                                                                                  \
+  case F32:                                                                                                              \
+    if (dual)                                                                                                            \
+      launch_dependent(ln_modulate_row_kernel<F32, true>, rows, 128, 0, stream, a, pb, static_cast<unsigned>(rows_a),    \
+                       zero, nzero, E, eps, mod_stride);                                                                 \
+    else                                                                                                                 \
+      launch_dependent(ln_modulate_row_kernel<F32, false>, rows, 128, 0, stream, a, pb, static_cast<unsigned>(rows_a),   \
+                       zero, nzero, E, eps, mod_stride);                                                                 \
+    break
+    switch (out_f32) {
+      SD3_LN_ROW(1);
+      SD3_LN_ROW(2);
+      SD3_LN_ROW(3);
+      default:
+      SD3_LN_ROW(0);
+    }
+#undef SD3_LN_ROW
+    return after_launch("ln_modulate_row_kernel");
+  }
 #define SD3_LN_LAUNCH(F32, DUALV)                                                                                    \
   launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero, nzero, E, eps,   \
                    mod_stride, rpw)
