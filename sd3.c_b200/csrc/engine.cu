@@ -1062,6 +1062,7 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
     e.out = w.mod;
     e.out_f32 = 1;
     e.ldo = m->ada_total;
+    e.w_static = 1;
     SD3_TRY(launch_gemm(w.y_bf, E, m->ada_w, E, OPERAND_BF16, B, static_cast<int>(m->ada_total), E, e,
                         m->status, st));
   } else {

@@ -23,6 +23,7 @@ struct GemmArgs {
   int tiles_m, tiles_n;
   GemmEpilogue epi;
   int wide_store;    // output rows are 32-byte aligned at every 16-column (bf16) / 8-column (f32) group
+  int a_rows;        // one-CTA kernel: rows of A that a stage loads
   int tma_store;     // CTA-pair kernel: bf16 output leaves through shared memory and a TMA store
   int* status;
 };

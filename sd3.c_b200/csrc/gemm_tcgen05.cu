@@ -94,8 +94,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  grid_dep_wait();
-  grid_dep_launch();
+  if (warp != 0) {  // the TMA producer waits after its first weight tiles
+    grid_dep_wait();
+    grid_dep_launch();
+  }
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, g.status};
 
@@ -108,17 +110,32 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     uint32_t phase = 0;
     bool ok = true;
     const bool issuer = elect_one();
+    const uint32_t stage_bytes = static_cast<uint32_t>(g.a_rows * STAGE_K_BYTES + Cfg::B_STAGE_BYTES);
+    auto load_w = [&](int st, int kb, int n0) {
+      mbar_expect_tx(&full_bar[st], stage_bytes);
+      tma_load_2d(smem + st * Cfg::STAGE_BYTES + A_STAGE_BYTES, &tmW, &full_bar[st], kb * ELEMS_PER_STAGE, n0);
+    };
+    int pre = 0;  // stages of the first tile whose weights are under way before the wait
+    bool waited = false;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const int m0 = (tile / g.tiles_n) * BM;
       const int n0 = (tile % g.tiles_n) * BN;
+      if (!waited) {
+        if (g.epi.w_static)
+          for (; pre < STAGES && pre < KB; ++pre)
+            if (issuer) load_w(pre, pre, n0);
+        grid_dep_wait();
+        waited = true;
+      }
       for (int kb = 0; kb < KB; ++kb) {
-        if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-        if (issuer) {
-          uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
-          mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
-          tma_load_2d(sa, &tmA, &full_bar[stage], kb * ELEMS_PER_STAGE, m0);
-          tma_load_2d(sa + A_STAGE_BYTES, &tmW, &full_bar[stage], kb * ELEMS_PER_STAGE, n0);
+        if (pre > 0) {
+          --pre;
+        } else {
+          if (!mbar_wait_all(&empty_bar[stage], phase ^ 1, wc, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+          if (issuer) load_w(stage, kb, n0);
         }
+        if (issuer)
+          tma_load_2d(smem + stage * Cfg::STAGE_BYTES, &tmA, &full_bar[stage], kb * ELEMS_PER_STAGE, m0);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
@@ -442,8 +459,12 @@ int launch_gemm(const void* A, long lda, const void* W, long ldw, int operand_dt
 
   g.tma_store = 0;  // register stores in the one-CTA kernel
   CUtensorMap tmA, tmW;
+  // A lone tile of rows loads the rows there are, in groups of eight: what the other rows of the MMA compute is not stored.
+  // Filling 128 rows per stage for a handful held the AdaLN GEMM (N 502272, K 1536) back; us, before -> after: one row 317 ->
+  // 220 (7.0 TB/s of weights; TMA alone reads them in 215), two 267 -> 222, eight 269 -> 228.
+  g.a_rows = M < BM ? (M + 7) / 8 * 8 : BM;
   int rc = encode_tmap_2d(&tmA, A, eb, (uint64_t)K, (uint64_t)M, (uint64_t)lda * eb,
-                          elems_per_stage, BM);
+                          elems_per_stage, g.a_rows);
   if (rc) return rc;
   rc = encode_tmap_2d(&tmW, W, eb, (uint64_t)K, (uint64_t)N, (uint64_t)ldw * eb, elems_per_stage,
                       BN);
