@@ -321,10 +321,10 @@ int launch_pair_inst(const PairProblem* p, const int* end, cudaStream_t stream) 
   return after_launch("gemm_pair_tcgen05_kernel");
 }
 
-// the block GEMM epilogues exist for both tile widths, the others for 256 only
+// the epilogues that a forward uses exist for both tile widths, the others for 256 only
 template <int EPI, bool OUT_F32, bool FP8>
 int launch_pair_width(int pbn, const PairProblem* p, const int* end, cudaStream_t stream) {
-  constexpr bool narrow_built = (EPI == EPI_GATE_RESID && OUT_F32) ||
+  constexpr bool narrow_built = (OUT_F32 && (EPI == EPI_GATE_RESID || EPI == EPI_BIAS || EPI == EPI_ADD_TABLE)) ||
                                 (!OUT_F32 && (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_QKV_NORM));
   if constexpr (narrow_built) {
     if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p, end, stream);
@@ -333,8 +333,8 @@ int launch_pair_width(int pbn, const PairProblem* p, const int* end, cudaStream_
 }
 
 bool narrow_tiles_built(const GemmEpilogue& epi) {
-  if (epi.mode == EPI_GATE_RESID) return epi.out_f32 != 0;
-  return !epi.out_f32 && (epi.mode == EPI_BIAS || epi.mode == EPI_BIAS_GELU || epi.mode == EPI_QKV_NORM);
+  if (epi.out_f32) return epi.mode == EPI_GATE_RESID || epi.mode == EPI_BIAS || epi.mode == EPI_ADD_TABLE;
+  return epi.mode == EPI_BIAS || epi.mode == EPI_BIAS_GELU || epi.mode == EPI_QKV_NORM;
 }
 
 // Tensor maps and arguments of one problem for pair tiles of width pbn.
@@ -394,6 +394,7 @@ int build_problem(PairProblem* pp, const GemmProblem& q, int operand_dtype, int 
 //   K 1536, QKV    589 rows 15.0 / 12.9 (1, 2)   1357: 21.7 / 18.5 (2, 3)   2714: 30.3 / 33.3 (3, 6)   4429: 49.1 / 52.2 (5, 9)
 //   K 1536, GELU   333 rows 15.8 / 13.3 (1, 2)   1024: 21.0 / 19.1 (2, 3)   1357: 23.7 / 24.7 (2, 4)   4429: 61.9 / 71.7 (6, 12)
 //   K 1536, gate  2714 rows 14.5 / 14.6 (1, 2)   4429: 23.5 / 21.2 (2, 3)   5428: 26.7 / 28.8 (2, 4)
+//   K 4096, fp32 output (the captions)  333 rows 24.8 / 14.9 (1, 1)   1332: 25.2 / 16.0 (1, 1)
 //   K 6144, gate  2714 rows 38.6 / 43.6 (1, 2)   4429: 68.8 / 67.4 (2, 3)   5428: 75.4 / 86.9 (2, 4)
 int choose_tile_width(long tiles256, int k_blocks, const GemmEpilogue& epi) {
   const long pairs = device_sm_count() / 2;
