@@ -47,9 +47,9 @@ using namespace gemm_detail;
 constexpr int P_BM = 128;            // rows of A per CTA (256 per pair)
 constexpr int P_KBYTES = 128;        // bytes of K per stage row (64 bf16)
 constexpr int P_A_BYTES = P_BM * P_KBYTES;
-// PBN = output columns per pair tile (256 or 128); each CTA loads PBN / 2 rows of W
+// PBN = output columns per pair tile (256, 128 or 64); each CTA loads PBN / 2 rows of W
 __host__ __device__ constexpr int pair_b_bytes(int pbn) { return (pbn / 2) * P_KBYTES; }
-__host__ __device__ constexpr int pair_stage_bytes(int pbn) { return P_A_BYTES + pair_b_bytes(pbn); }  // 32 / 24 KiB
+__host__ __device__ constexpr int pair_stage_bytes(int pbn) { return P_A_BYTES + pair_b_bytes(pbn); }  // 32 / 24 / 20 KiB
 // The epilogues that leave through shared memory (TMA reduction or TMA store) get 4 KiB per
 // epilogue warp.
 constexpr int P_RED_BYTES = 4096;
@@ -92,7 +92,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   constexpr int P_STAGES = pair_stages(PBN);
-  static_assert(EPI_WARPS * (PBN / 64) * P_RED_BYTES <= P_STAGES * P_STAGE_BYTES, "the last tile's boxes fit the ring");
+  static_assert(EPI_WARPS * ((PBN + 63) / 64) * P_RED_BYTES <= P_STAGES * P_STAGE_BYTES, "the last tile's boxes fit the ring");
   uint8_t* red_smem = smem + P_STAGES * P_STAGE_BYTES;  // 1024-byte aligned: stages are 32 / 24 KiB each
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + P_STAGES * P_STAGE_BYTES + pair_red_bytes(EPI, OUT_F32));
   uint64_t* empty_bar = full_bar + P_STAGES;
@@ -329,6 +329,9 @@ int launch_pair_width(int pbn, const PairProblem* p, const int* end, cudaStream_
   if constexpr (narrow_built) {
     if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p, end, stream);
   }
+  if constexpr (EPI == EPI_GATE_RESID) {
+    if (pbn == 64) return launch_pair_inst<EPI, OUT_F32, FP8, 64>(p, end, stream);
+  }
   return launch_pair_inst<EPI, OUT_F32, FP8, 256>(p, end, stream);
 }
 
@@ -399,6 +402,10 @@ int build_problem(PairProblem* pp, const GemmProblem& q, int operand_dtype, int 
 int choose_tile_width(long tiles256, int k_blocks, const GemmEpilogue& epi) {
   const long pairs = device_sm_count() / 2;
   if (pairs <= 0 || !narrow_tiles_built(epi)) return 256;
+  // The gate + residual GEMMs, the ones with few tiles, have 64-wide ones too, for problems that fit one wave of
+  // those.  us, 128 / 64 wide: K 6144, 256 rows 19.7 / 17.9, 333 rows 19.8 / 18.5, 700 rows 19.9 / 19.5; K 1536, 256 rows
+  // 7.7 / 7.0, 589 rows 8.2 / 8.2 (slots of four stages: 20.1 at 256 rows).
+  if (epi.mode == EPI_GATE_RESID && 4 * tiles256 <= pairs) return 64;
   const long wide = (tiles256 + pairs - 1) / pairs, narrow = (2 * tiles256 + pairs - 1) / pairs;
   return 64 * narrow * k_blocks < 100 * wide * k_blocks + 1000 ? 128 : 256;
 }
@@ -419,10 +426,10 @@ bool gemm_pair_supported(int operand_dtype, int M, int N, int K, const GemmEpilo
   return operand_dtype == OPERAND_BF16;
 }
 
-// One word per pair tile of either width, CTA and epilogue warp.  Which of the words a launch uses depends on its tile
+// One word per pair tile of any width, CTA and epilogue warp.  Which of the words a launch uses depends on its tile
 // width, which is the same for both problems.
 size_t gate_order_words(long M, int N) {
-  return static_cast<size_t>((M + 2 * P_BM - 1) / (2 * P_BM)) * (N / 128) * 2 * EPI_WARPS;
+  return static_cast<size_t>((M + 2 * P_BM - 1) / (2 * P_BM)) * (N / 64) * 2 * EPI_WARPS;
 }
 
 // One to three problems of the same N, K, operand type and epilogue kind.
