@@ -42,12 +42,13 @@ namespace {
 // barrier behind the staging.  Measured (whole forward, one image): 256x256 3510 -> 3326 us,
 // 1024x1024 14.18 -> 13.96 ms.  Three CTAs per SM for the plane output, whose splits need the registers.
 constexpr int LN_ROW_QUADS = 12;  // ln_modulate_row_kernel: float4 words of a row per lane index (E up to 1536)
-// Rows of a launch (both problems) up to which it is taken, for one and for two modulations; us, kernel with staged
-// vectors / this one: one   589 rows 4.45 / 2.45, 1357 5.29 / 4.10, 2714 7.82 / 6.22, 3400 7.91 / 7.13 | 4000 8.10 / 8.35,
-//                           4429 8.34 / 8.95, 8858 17.9 / 18.4, 35432 60.6 / 68.9
-//                     two   589 rows 6.70 / 3.40, 1357 8.26 / 5.16, 2714 12.5 / 8.4, 4429 14.2 / 12.2, 8858 29.4 / 26.7,
-//                           16384 50.6 / 47.0 | 35432 97.4 / 97.4
-constexpr long LN_ROW_MAX = 3700, LN_ROW_MAX_DUAL = 32768;
+// With one modulation it is taken with one row per CTA up to LN_ROW_MAX rows of a launch (both problems) and with several
+// above LN_ROWS_MIN, with two modulations always.  us, kernel with staged vectors / a row per CTA / several:
+//   one   589 rows 4.45 / 2.44 / 3.10   1357 5.29 / 4.14 / 4.32   2714 7.82 / 6.23 / 6.91   4429 8.34 / 8.95 / 9.64
+//         8858 17.9 / 18.4 / 17.3   13287 29.0 / - / 23.5   35432 60.6 / 68.9 / 55.2 (up to 8 rows; 64: 64.9)
+//   two   589 rows 6.70 / 3.44 / 3.06   1357 8.26 / 5.16 / 4.08   4429 14.2 / 12.2 / 8.8   13287 47.5 / 38.3 / 30.1
+//         35432 97.4 / 96.7 / 76.0 (up to 64 rows; 8: 13287 33.3, 35432 76.2)
+constexpr long LN_ROW_MAX = 3700, LN_ROWS_MIN = 8000;
 constexpr int LN_MAX_ROWS_PER_WARP = 8;
 constexpr int LN_WARPS = 8;
 
@@ -190,41 +191,50 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
   }
 }
 
-// The same for fewer rows: a CTA of four warps per row, so that the row and its modulation vectors are requested at once
-// and one memory latency is exposed, where the kernel above stages the vectors, and two modulations' take as long as the
-// row.  The sums are formed in the order of the kernel above (each lane adds its quads in order, then the lanes' tree): the
-// same bits.  Bound by latency at a thousand rows (3.2 TB/s of L2 at 1357), by L2 above (LN_ROW_MAX has the figures).
-template <int OUT, bool DUAL>
+// The same with a CTA of four warps per row: the row and its modulation vectors are requested at once and one memory latency
+// is exposed, where the kernel above stages the vectors first.  MULTI: the CTA takes per_cta consecutive rows, keeps
+// the vectors in registers (read for every row, two modulations' are four times the row's bytes, all from L2) and
+// has the next row under way while it forms one.  The sums are formed in the order of the kernel above (each lane adds its
+// quads in order, then the lanes' tree): the same bits.  Bound by latency at a thousand rows, by L2 and HBM
+// above (5.9 TB/s at 35432 rows; LN_ROW_MAX has the figures).
+template <int OUT, bool DUAL, bool MULTI>
 __global__ void __launch_bounds__(128)
-ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned rows_a,
-                       unsigned* zero, int nzero, int E, float eps, long mod_stride) {
+ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a,
+                       unsigned* zero, int nzero, int E, float eps, long mod_stride, int per_cta) {
   __shared__ float part[2][LN_ROW_QUADS][32];
   grid_dep_wait();
   grid_dep_launch();
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<unsigned>(nzero); i += gridDim.x * blockDim.x)
     zero[i] = 0;
-  const bool second = blockIdx.x >= rows_a;
+  const bool second = blockIdx.x >= grid_a;
   const LnProblem& p = second ? pb : pa;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = E >> 2;
-  const long row = second ? blockIdx.x - rows_a : blockIdx.x, rows = static_cast<long>(p.B) * p.T;
-  const long moff = static_cast<long>(row / p.T) * mod_stride;
+  const long rows = static_cast<long>(p.B) * p.T;
+  const long row0 = static_cast<long>(second ? blockIdx.x - grid_a : blockIdx.x) * (MULTI ? per_cta : 1);
+  const long row_end = !MULTI ? row0 + 1 : row0 + per_cta < rows ? row0 + per_cta : rows;
   const bool dual = DUAL && p.out2 != nullptr;
   constexpr int NV = LN_ROW_QUADS / 4;  // quads of a thread: j = NV * warp + t, elements 4 (lane + 32 j)
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 v[NV], sc1[NV], sh1[NV], sc2[DUAL ? NV : 1], sh2[DUAL ? NV : 1];
+  float4 v[NV], next[MULTI ? NV : 1], sc1[NV], sh1[NV], sc2[DUAL ? NV : 1], sh2[DUAL ? NV : 1];
+  long b_now = row0 / p.T, b_end = (b_now + 1) * p.T;  // the sample of the current row, its first row past the end
+  auto load = [&](float4* x, long row, bool mod) {
+    const long moff = b_now * mod_stride;
 #pragma unroll
-  for (int t = 0; t < NV; ++t) {
-    const int i = lane + 32 * (NV * warp + t);
-    const bool in = i < nvec;
-    v[t] = in ? *(reinterpret_cast<const float4*>(p.x + row * E) + i) : z4;
-    sc1[t] = in ? *(reinterpret_cast<const float4*>(p.scale1 + moff) + i) : z4;
-    sh1[t] = in ? *(reinterpret_cast<const float4*>(p.shift1 + moff) + i) : z4;
-    if constexpr (DUAL) {
-      sc2[t] = in && dual ? *(reinterpret_cast<const float4*>(p.scale2 + moff) + i) : z4;
-      sh2[t] = in && dual ? *(reinterpret_cast<const float4*>(p.shift2 + moff) + i) : z4;
+    for (int t = 0; t < NV; ++t) {
+      const int i = lane + 32 * (NV * warp + t);
+      const bool in = i < nvec;
+      if (x != nullptr) x[t] = in ? *(reinterpret_cast<const float4*>(p.x + row * E) + i) : z4;
+      if (!mod) continue;
+      sc1[t] = in ? *(reinterpret_cast<const float4*>(p.scale1 + moff) + i) : z4;
+      sh1[t] = in ? *(reinterpret_cast<const float4*>(p.shift1 + moff) + i) : z4;
+      if constexpr (DUAL) {
+        sc2[t] = in && dual ? *(reinterpret_cast<const float4*>(p.scale2 + moff) + i) : z4;
+        sh2[t] = in && dual ? *(reinterpret_cast<const float4*>(p.shift2 + moff) + i) : z4;
+      }
     }
-  }
+  };
+  load(v, row0, true);
   auto row_sum = [&](float (&buf)[LN_ROW_QUADS][32]) {
     __syncthreads();
     float s = 0.f;
@@ -232,26 +242,39 @@ ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_consta
     for (int j = 0; j < LN_ROW_QUADS; ++j) s += buf[j][lane];
     return warp_sum(s);
   };
+#pragma unroll 1
+  for (long row = row0; row < row_end; ++row) {
+    if constexpr (MULTI) {
+      if (row + 1 < row_end) load(next, row + 1, false);  // under way while this row is formed
+      if (row == b_end) {
+        b_end += p.T;
+        ++b_now;
+        load(nullptr, 0, true);
+      }
+    }
 #pragma unroll
-  for (int t = 0; t < NV; ++t) part[0][NV * warp + t][lane] = (v[t].x + v[t].y) + (v[t].z + v[t].w);
-  const float mean = row_sum(part[0]) / static_cast<float>(E);
+    for (int t = 0; t < NV; ++t) part[0][NV * warp + t][lane] = (v[t].x + v[t].y) + (v[t].z + v[t].w);
+    const float mean = row_sum(part[0]) / static_cast<float>(E);
 #pragma unroll
-  for (int t = 0; t < NV; ++t) {
-    const float a = v[t].x - mean, b = v[t].y - mean, c = v[t].z - mean, d = v[t].w - mean;
-    part[1][NV * warp + t][lane] = lane + 32 * (NV * warp + t) < nvec ? (a * a + b * b) + (c * c + d * d) : 0.f;
-  }
-  const float rstd = rsqrtf(row_sum(part[1]) / static_cast<float>(E) + eps);
-  auto modulate = [&](const float4& x, const float4& s, const float4& h) {
-    return make_float4(fmaf((x.x - mean) * rstd, s.x + 1.f, h.x), fmaf((x.y - mean) * rstd, s.y + 1.f, h.y),
-                       fmaf((x.z - mean) * rstd, s.z + 1.f, h.z), fmaf((x.w - mean) * rstd, s.w + 1.f, h.w));
-  };
+    for (int t = 0; t < NV; ++t) {
+      const float a = v[t].x - mean, b = v[t].y - mean, c = v[t].z - mean, d = v[t].w - mean;
+      part[1][NV * warp + t][lane] = lane + 32 * (NV * warp + t) < nvec ? (a * a + b * b) + (c * c + d * d) : 0.f;
+    }
+    const float rstd = rsqrtf(row_sum(part[1]) / static_cast<float>(E) + eps);
+    auto modulate = [&](const float4& x, const float4& s, const float4& h) {
+      return make_float4(fmaf((x.x - mean) * rstd, s.x + 1.f, h.x), fmaf((x.y - mean) * rstd, s.y + 1.f, h.y),
+                         fmaf((x.z - mean) * rstd, s.z + 1.f, h.z), fmaf((x.w - mean) * rstd, s.w + 1.f, h.w));
+    };
 #pragma unroll
-  for (int t = 0; t < NV; ++t) {
-    const int i = lane + 32 * (NV * warp + t);
-    if (i >= nvec) break;
-    ln_store4<OUT>(p.out1, row, rows, E, i, modulate(v[t], sc1[t], sh1[t]));
-    if constexpr (DUAL) {
-      if (dual) ln_store4<OUT>(p.out2, row, rows, E, i, modulate(v[t], sc2[t], sh2[t]));
+    for (int t = 0; t < NV; ++t) {
+      const int i = lane + 32 * (NV * warp + t);
+      if (i < nvec) {
+        ln_store4<OUT>(p.out1, row, rows, E, i, modulate(v[t], sc1[t], sh1[t]));
+        if constexpr (DUAL) {
+          if (dual) ln_store4<OUT>(p.out2, row, rows, E, i, modulate(v[t], sc2[t], sh2[t]));
+        }
+      }
+      if constexpr (MULTI) v[t] = next[t];
     }
   }
 }
@@ -268,16 +291,22 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   const bool dual = a.out2 != nullptr || (b && b->out2 != nullptr);
   const size_t smem = static_cast<size_t>(E) * 4 * (dual ? 4 : 2);
   const LnProblem pb = b ? *b : a;
-  if (E <= 4 * 32 * LN_ROW_QUADS && rows_a + rows_b <= (dual ? LN_ROW_MAX_DUAL : LN_ROW_MAX)) {
-    const dim3 rows(static_cast<unsigned>(rows_a + rows_b));
-#define SD3_LN_ROW(F32)                                                                                                  \
-  case F32:                                                                                                              \
-    if (dual)                                                                                                            \
-      launch_dependent(ln_modulate_row_kernel<F32, true>, rows, 128, 0, stream, a, pb, static_cast<unsigned>(rows_a),    \
-                       zero, nzero, E, eps, mod_stride);                                                                 \
-    else                                                                                                                 \
-      launch_dependent(ln_modulate_row_kernel<F32, false>, rows, 128, 0, stream, a, pb, static_cast<unsigned>(rows_a),   \
-                       zero, nzero, E, eps, mod_stride);                                                                 \
+  if (E <= 4 * 32 * LN_ROW_QUADS && (dual || rows_a + rows_b <= LN_ROW_MAX || rows_a + rows_b > LN_ROWS_MIN)) {
+    const bool multi = dual || rows_a + rows_b > LN_ROWS_MIN;
+    // rows of a CTA: as many as lets all CTAs be resident at once, up to a limit
+    const long resident = 5L * device_sm_count(), most = dual ? 64 : 8;
+    const long want = (rows_a + rows_b + resident - 1) / resident;
+    const int per = !multi ? 1 : static_cast<int>(want > most ? most : want);
+    const unsigned ga = static_cast<unsigned>((rows_a + per - 1) / per);
+    const dim3 row_ctas(ga + static_cast<unsigned>((rows_b + per - 1) / per));
+#define SD3_LN_ROW_INST(F32, DUALV, MULTIV)                                                                              \
+  launch_dependent(ln_modulate_row_kernel<F32, DUALV, MULTIV>, row_ctas, 128, 0, stream, a, pb, ga, zero, nzero, E, eps, \
+                   mod_stride, per)
+#define SD3_LN_ROW(F32)                                     \
+  case F32:                                                 \
+    if (dual) SD3_LN_ROW_INST(F32, true, true);             \
+    else if (multi) SD3_LN_ROW_INST(F32, false, true);      \
+    else SD3_LN_ROW_INST(F32, false, false);                \
     break
     switch (out_f32) {
       SD3_LN_ROW(1);
@@ -287,19 +316,26 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
       SD3_LN_ROW(0);
     }
 #undef SD3_LN_ROW
+#undef SD3_LN_ROW_INST
     return after_launch("ln_modulate_row_kernel");
   }
-#define SD3_LN_LAUNCH(F32, DUALV)                                                                                    \
-  launch_dependent(ln_modulate_kernel<MAXV, F32, DUALV>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero, nzero, E, eps,   \
-                   mod_stride, rpw)
-  if (out_f32 == 1) {
-    if (dual) SD3_LN_LAUNCH(1, true); else SD3_LN_LAUNCH(1, false);
-  } else if (out_f32 == 2) {
-    if (dual) SD3_LN_LAUNCH(2, true); else SD3_LN_LAUNCH(2, false);
-  } else if (out_f32 == 3) {
-    if (dual) SD3_LN_LAUNCH(3, true); else SD3_LN_LAUNCH(3, false);
-  } else {
-    if (dual) SD3_LN_LAUNCH(0, true); else SD3_LN_LAUNCH(0, false);
+#define SD3_LN_LAUNCH(F32)                                                                                               \
+  do {                                                                                                                   \
+    if constexpr (MAXV > LN_ROW_QUADS) {                                                                                 \
+      if (dual) {                                                                                                        \
+        launch_dependent(ln_modulate_kernel<MAXV, F32, true>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero,    \
+                         nzero, E, eps, mod_stride, rpw);                                                                \
+        break;                                                                                                           \
+      }                                                                                                                  \
+    }                                                                                                                    \
+    launch_dependent(ln_modulate_kernel<MAXV, F32, false>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero,       \
+                     nzero, E, eps, mod_stride, rpw);                                                                    \
+  } while (0)
+  switch (out_f32) {
+    case 1: SD3_LN_LAUNCH(1); break;
+    case 2: SD3_LN_LAUNCH(2); break;
+    case 3: SD3_LN_LAUNCH(3); break;
+    default: SD3_LN_LAUNCH(0);
   }
 #undef SD3_LN_LAUNCH
   return after_launch("ln_modulate_kernel");
