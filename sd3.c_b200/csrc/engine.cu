@@ -1070,7 +1070,7 @@ int sd3_dit_forward(sd3_model* m, const void* pooled, const void* captions, cons
   if (!m->f32 && m->ada_total % 64 == 0 && E % 64 == 0) {
     // As a tensor-core GEMM with M = batch: out (B, ada_total) = y W^T + b.  Only B
     // of the 128 rows of each MMA carry data, but the tensor pipe has the room and TMA streams the
-    // 1.5 GB of weights at HBM speed whatever the batch (272 us); the skinny linear's time grows with it.
+    // 1.5 GB of weights at HBM speed whatever the batch (220 us with one sample); the skinny linear's time grows with it.
     SD3_TRY(launch_cast_f32_to_bf16(w.y, w.y_bf, static_cast<long>(B) * E, st));
     GemmEpilogue e;
     e.mode = EPI_BIAS;
