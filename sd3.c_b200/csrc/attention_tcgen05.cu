@@ -38,13 +38,13 @@
 //    was 6 % slower), every eighth exponential is evaluated as a polynomial on
 //    the FMA pipe, and the multiply-subtract / row-sum pairs use the packed
 //    f32x2 instructions.
-//  * Four modes.  0: the online softmax above, for any input.  1, 2: the caller gives a bound on |q . k| (SD3.5 normalises q and k per head, so
+//  * Three instantiations.  <false, false>: the online softmax above, for any input.
+//    <true, *>: the caller gives a bound on |q . k| (SD3.5 normalises q and k per head, so
 //    64 max_d |wq_d wk_d| bounds every score whatever the input); when the exp2 argument can
 //    not exceed 80 in magnitude, P = 2^(s c) needs no running maximum at all -- no row
 //    maximum, vote, branch or rescale -- and three of every eight PAIRS of exponentials go to
-//    the FMA pipe as packed polynomials.  2: the queries were also multiplied by
-//    scale log2(e) where they were formed, so a score is its own exp2 argument.  3: as 2 for the rows whose
-//    norms bound their scores, as 0 for the others.  The kernel's
+//    the FMA pipe as packed polynomials.  <true, true>: the queries were also multiplied by
+//    scale log2(e) where they were formed, so a score is its own exp2 argument.  The kernel's
 //    time follows its instruction count (no pipe is saturated; two warps per sub-partition
 //    are bound by their own dependent-issue latency): -17 % warp instructions, -14 % time.
 //
@@ -55,10 +55,8 @@
 // rows straight into the context and image output buffers.
 #include <cuda.h>
 
-#include <algorithm>
 #include <cmath>
 #include <mutex>
-#include <type_traits>
 
 #include "kernels.h"
 #include "ptx.cuh"
@@ -101,7 +99,6 @@ struct AttnArgs {
   int kv_split;
   float* part_o;   // (B, NH, kv_split, T, 64)
   float* part_ml;  // (B, NH, kv_split, T, 2): maximum (raw score units), row sum
-  const unsigned* k_max;  // MODE 3: largest |k|^2 per (sample, head), bits of a float; null: the launch's scores are bounded
 };
 
 // O *= alpha for this thread's query row (64 fp32 columns in TMEM).  Rare (the
@@ -133,7 +130,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // exp2 on the FMA pipe: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f by a
 // degree-3 polynomial (relative error at most 8.5e-4, 2.2e-4 root mean square, below bf16 resolution: the minimax cubic,
-// 7.5e-5, changes the error of the output by less than 0.3 %), exponent added as an integer.  Inputs below -125 give a denormal-sized result.
+// 7.5e-5, changes the error of the output by less than 0.3 %), exponent added as an integer.  Inputs below -125 give a
+// denormal-sized result.
 __device__ __forceinline__ float ex2_poly(float x) {
   x = fmaxf(x, -125.0f);
   const float t = x + 12582912.0f;  // 1.5 * 2^23: the low mantissa bits now hold round(x)
@@ -253,25 +251,18 @@ __device__ __forceinline__ void exp2_pack(uint32_t (&r)[32], float c, float2& ac
   }
 }
 
-// MODE 0: online softmax.
-// MODE 1: the caller guarantees |q . k| scale log2(e) <= AT_BOUND_MAX for every query and key
+// BOUNDED: the caller guarantees |q . k| scale log2(e) <= AT_BOUND_MAX for every query and key
 // (the engine derives it from the RMSNorm weights of q and k), so 2^(s c) can neither overflow
 // nor vanish in fp32 / bf16 and the softmax needs no running maximum: no row maximum, no vote,
 // no rescaling of O; P = 2^(s c) and the row sum normalise the output exactly as before
 // (softmax is invariant to the subtracted constant).
-// MODE 2: and the queries were multiplied by scale log2(e) where they were formed
+// UNIT (bounded mode only): the queries were multiplied by scale log2(e) where they were formed
 // (the engine folds the factor into the RMSNorm weight of q), so a score is its own exp2
 // argument: one packed multiply per pair of scores less (measured: 4 % of the kernel).
-// MODE 3: queries as in mode 2, but no guarantee: the largest |k|^2 of the sample and head is known (the QKV GEMM's
-// epilogue left it), and each softmax warp compares |q| |k| of its 32 rows with AT_BOUND_MAX and takes the loop of mode 2
-// or that of mode 0.  Norm weights that spread as those of trained models do (log-normal, 0.6) leave half of the blocks
-// without a bound from the weights; of their warps 93 % are bounded by the norms.
-// With spread 0.6, forward of three 832x1216 images 34.5 -> 33.1 ms, of two 1024x1024 25.3 -> 24.3; error of the forward against
-// the fp32 model 3.82e-3 -> 3.83e-3 (mean of four, 0.2 % either way).
 // PAIR: the launch carries two attentions (a launch of one keeps its parameters at fixed places and some
 // registers fewer: 152 instead of 156 to 161).  With it and separate launches above 16384 tokens,
 // eight 1024x1024 images take 96.17 ms against 96.03 before launches were merged, 2048x2048 99.64 against 99.68.
-template <int MODE, bool PAIR>
+template <bool BOUNDED, bool UNIT, bool PAIR>
 __global__ void __launch_bounds__(AT_THREADS, 2)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
                          const __grid_constant__ AttnArgs a0, const __grid_constant__ AttnArgs a1, const int grid0) {
@@ -409,13 +400,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_c
     const uint32_t p_tmem = lane_base + AT_P_COL;
     const uint32_t o_tmem = lane_base + AT_O_COL;
     const float c = a.scale_log2e;
-    constexpr bool UNIT = MODE >= 2;
-    float m_used = 0.0f;  // running max (raw score units) the exponentials refer to
+    float m_used = BOUNDED ? 0.0f : -INFINITY;  // running max (raw score units) the exponentials refer to
     float2 l2 = make_float2(0.f, 0.f);
     bool ok = true;
-    auto softmax_tiles = [&](auto bounded) {
-    constexpr bool BOUNDED = decltype(bounded)::value;
-    m_used = BOUNDED ? 0.0f : -INFINITY;
     uint32_t pre_s = 0;  // early test of s_full for the coming tile
     uint32_t ra[32], rb[32], rc[32], rd[32];  // scores of keys 0..31, 32..63, 64..95, 96..127, then packed P
     for (int j = 0; j < nkv; ++j) {
@@ -491,34 +478,6 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_c
       tmem_wait_st();
       __syncwarp();
       mbar_arrive_lane0(p_ready, lane);
-    }
-    };
-    if constexpr (MODE == 0) {
-      softmax_tiles(std::false_type{});
-    } else if constexpr (MODE < 3) {
-      softmax_tiles(std::true_type{});
-    } else {
-      bool bounded = true;
-      if (a.k_max != nullptr) {
-        ok = mbar_wait_warp(q_full, 0, wc, DEV_TIMEOUT_ATTN_Q);
-        float q2 = 0.f;  // |q|^2 of this row (rows past T are zero); the swizzle moves 16-byte words within the row
-        const uint4* qr = reinterpret_cast<const uint4*>(q_smem + row * 128);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint4 w = qr[(i + row) & 7];
-          for (const uint32_t u : {w.x, w.y, w.z, w.w}) {
-            const float lo = __uint_as_float(u << 16), hi = __uint_as_float(u & 0xffff0000u);
-            q2 = fmaf(hi, hi, fmaf(lo, lo, q2));
-          }
-        }
-        const float k2 = __uint_as_float(a.k_max[static_cast<long>(b) * a.NH + h]);
-        // 1 % for the rounding of k to bf16; NaN and infinity compare false
-        bounded = __all_sync(0xffffffffu, 1.01f * sqrtf(q2 * k2) <= AT_BOUND_MAX) != 0;
-      }
-      if (ok) {
-        if (bounded) softmax_tiles(std::true_type{});
-        else softmax_tiles(std::false_type{});
-      }
     }
     const float l = l2.x + l2.y;
     if (ok && mbar_wait_warp(&pv_done[(nkv - 1) % AT_STAGES], ((nkv - 1) / AT_STAGES) & 1, wc, DEV_TIMEOUT_ATTN_O)) {
@@ -704,10 +663,9 @@ int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_
     std::lock_guard<std::mutex> lock(attr_mutex);
     if (!attr_done[dev]) {
       cudaError_t e = cudaSuccess;
-      for (auto kern : {attention_tcgen05_kernel<0, false>, attention_tcgen05_kernel<1, false>,
-                        attention_tcgen05_kernel<2, false>, attention_tcgen05_kernel<3, false>,
-                        attention_tcgen05_kernel<0, true>, attention_tcgen05_kernel<1, true>,
-                        attention_tcgen05_kernel<2, true>, attention_tcgen05_kernel<3, true>})
+      for (auto kern : {attention_tcgen05_kernel<false, false, false>, attention_tcgen05_kernel<true, false, false>,
+                        attention_tcgen05_kernel<true, true, false>, attention_tcgen05_kernel<false, false, true>,
+                        attention_tcgen05_kernel<true, false, true>, attention_tcgen05_kernel<true, true, true>})
         if (e == cudaSuccess)
           e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM_BYTES);
       if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(attention)");
@@ -749,8 +707,7 @@ int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_
     }
     grid[i] = qtiles * a[i].kv_split;
     const float bound_log2 = q.score_bound * fabsf(a[i].scale_log2e);
-    mode[i] = q.score_bound > 0.0f && bound_log2 <= AT_BOUND_MAX ? (unit ? 2 : 1) : unit && q.k_max ? 3 : 0;
-    a[i].k_max = mode[i] == 3 ? q.k_max : nullptr;
+    mode[i] = q.score_bound > 0.0f && bound_log2 <= AT_BOUND_MAX ? (unit ? 2 : 1) : 0;
   }
   // One launch for both where they run the same instantiation, neither splits its keys (both splits
   // would use the one scratch buffer) and the waves add up to fewer.  Measured on the forward of one image:
@@ -759,18 +716,17 @@ int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_
   const long slots = 2L * device_sm_count();
   auto waves = [&](int i) { return (static_cast<long>(grid[i]) * NH * B + slots - 1) / slots; };
   const long both = (static_cast<long>(grid[0] + grid[1]) * NH * B + slots - 1) / slots;
-  const bool one_mode = mode[0] == mode[1] || (mode[0] >= 2 && mode[1] >= 2);  // mode 3 without maxima is mode 2
-  const bool merged = n == 2 && one_mode && a[0].kv_split == 1 && a[1].kv_split == 1 &&
+  const bool merged = n == 2 && mode[0] == mode[1] && a[0].kv_split == 1 && a[1].kv_split == 1 &&
                       both < waves(0) + waves(1);
-  if (merged) mode[0] = std::max(mode[0], mode[1]);
   for (int i = 0; i < (merged ? 1 : n); ++i) {
     const int j = merged ? 1 : i;
     const dim3 g(merged ? grid[0] + grid[1] : grid[i], NH, B);
-    auto pick = [&](auto single, auto pair) { return merged ? pair : single; };
-    auto kern = mode[i] == 3   ? pick(attention_tcgen05_kernel<3, false>, attention_tcgen05_kernel<3, true>)
-                : mode[i] == 2 ? pick(attention_tcgen05_kernel<2, false>, attention_tcgen05_kernel<2, true>)
-                : mode[i] == 1 ? pick(attention_tcgen05_kernel<1, false>, attention_tcgen05_kernel<1, true>)
-                               : pick(attention_tcgen05_kernel<0, false>, attention_tcgen05_kernel<0, true>);
+    auto kern = mode[i] == 2   ? (merged ? attention_tcgen05_kernel<true, true, true>
+                                         : attention_tcgen05_kernel<true, true, false>)
+                : mode[i] == 1 ? (merged ? attention_tcgen05_kernel<true, false, true>
+                                         : attention_tcgen05_kernel<true, false, false>)
+                               : (merged ? attention_tcgen05_kernel<false, false, true>
+                                         : attention_tcgen05_kernel<false, false, false>);
     launch_dependent(kern, g, AT_THREADS, AT_SMEM_BYTES, stream, tm[i], tm[j], a[i], a[j], grid[i]);
     int rc = after_launch("attention_tcgen05_kernel");
     if (rc) return rc;

@@ -78,10 +78,7 @@ struct Workspace {
   void* a8 = nullptr;    // FP8 mode: e4m3 copy of the current GEMM's left operand
   void* attn_scratch = nullptr;  // partial results of key-split attention launches (small batches, long sequences)
   size_t attn_scratch_bytes = 0;
-  // words that a block's first LayerNorm sets to zero: the largest |k|^2 per sample and head of the joint and of the
-  // image-only attention (GemmEpilogue::k_max), then those of a dual block's two out-projections into x as one launch
-  // (GemmEpilogue::order)
-  unsigned* zeroed = nullptr;
+  unsigned* order = nullptr;  // a dual block's two out-projections into x as one launch (GemmEpilogue::order)
   // position table cache
   float* pos = nullptr;
   int pos_h = 0, pos_w = 0;
@@ -278,8 +275,7 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
       {&w.hid_x, nTx * F * ab}, {&w.hid_c, nTc * F * ab},
       {(void**)&w.o_f32, m->f32 && m->D != 64 ? nB * T * E * 4 : 16},
       {&w.a8, m->fp8 ? (nTx > nTc ? nTx : nTc) * F : 16},
-      {(void**)&w.zeroed,
-       m->f32 ? 16 : (2 * nB * m->NH + gate_order_words(static_cast<long>(nTx), m->E)) * sizeof(unsigned)},
+      {(void**)&w.order, m->f32 ? 16 : gate_order_words(static_cast<long>(nTx), m->E) * sizeof(unsigned)},
       {&w.attn_scratch, 16},
   };
   // key-split attention (head_dim 64 tensor-core path): the larger need of the joint and the image-only call
@@ -441,12 +437,9 @@ int run_qk_norm(sd3_model* m, void* qkv, int B, int T_in, int T_total, int row_o
 // QKV projection of `T_in` tokens per sample into rows [row_off, row_off+T_in)
 // of each sample of the packed (B, T_total, 3E) buffer, q/k RMSNorm included.
 int run_qkv(sd3_model* m, const Linear& L, const void* h, void* qkv, int B, int T_in, int T_total,
-            int row_off, const float* wq, const float* wk, cudaStream_t st, bool h_e4m3 = false,
-            unsigned* k_max = nullptr) {
+            int row_off, const float* wq, const float* wk, cudaStream_t st, bool h_e4m3 = false) {
   const bool norm = m->cfg.use_qk_norm && (wq || wk);
-  GemmEpilogue e = qkv_epilogue(m, qkv, B, T_in, T_total, row_off, wq, wk);
-  e.k_max = k_max;
-  int rc = run_linear(m, L, h, B * T_in, e, st, h_e4m3);
+  int rc = run_linear(m, L, h, B * T_in, qkv_epilogue(m, qkv, B, T_in, T_total, row_off, wq, wk), st, h_e4m3);
   if (rc || m->D == 64 || !norm) return rc;
   return run_qk_norm(m, qkv, B, T_in, T_total, row_off, wq, wk, st);
 }
@@ -459,7 +452,6 @@ struct AttnCall {
   bool out_e4m3;
   float score_bound;
   bool prescaled;  // q already carries scale * log2(e) (only set up for the bf16 kernel)
-  const unsigned* k_max;  // GemmEpilogue::k_max of the QKV projections, or null
 };
 
 int run_attention_simt(sd3_model* m, const void* qkv, int B, int T, int Tc, void* o_c, void* o_x, cudaStream_t st) {
@@ -488,7 +480,7 @@ int run_attention(sd3_model* m, const AttnCall* c, int n, int B, cudaStream_t st
       p[i] = {static_cast<const bf16*>(c[i].qkv), c[i].T, c[i].Tc, static_cast<bf16*>(c[i].o_c),
               static_cast<bf16*>(c[i].o_x), c[i].prescaled ? 0.0f : 1.0f / sqrtf(static_cast<float>(m->D)),
               c[i].out_e4m3 ? 1 : 0, m->ws.attn_scratch_bytes ? m->ws.attn_scratch : nullptr,
-              m->ws.attn_scratch_bytes, c[i].score_bound, c[i].k_max};
+              m->ws.attn_scratch_bytes, c[i].score_bound};
     return m->f32 ? launch_attention_split(p, n, B, m->NH, m->status, st)
                   : launch_attention_group(p, n, B, m->NH, m->status, st);
   }
@@ -581,17 +573,13 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   // a dual block's image-only attention and out-projection beside the joint ones, or after them
   const bool together = L.dual && m->D == 64 && merge_launches(B, Tc, Tx);
   const bool out_together = together && !m->f32 && !L.last;
-  unsigned* const k_max_j = w.zeroed;
-  unsigned* const k_max_d = k_max_j + static_cast<long>(B) * m->NH;
-  unsigned* const order = k_max_d + static_cast<long>(B) * m->NH;
-  const long zero_words =
-      m->f32 ? 0 : order - w.zeroed + (out_together ? static_cast<long>(gate_order_words(static_cast<long>(B) * Tx, E)) : 0);
+  const size_t order_words = out_together ? gate_order_words(static_cast<long>(B) * Tx, E) : 0;
   // pre-attention LayerNorm + modulate
   {
     LnProblem px = {x, B, Tx, x_shift_a, x_scale_a, w.h_x, nullptr, nullptr, nullptr};
     if (L.dual) { px.shift2 = x_shift_2; px.scale2 = x_scale_2; px.out2 = w.h_x2; }
     const LnProblem pc = {c, B, Tc, c_shift_a, c_scale_a, w.h_c, nullptr, nullptr, nullptr};
-    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st, w.zeroed, static_cast<int>(zero_words)));
+    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st, w.order, static_cast<int>(order_words)));
   }
   // QKV (context rows first, then image rows) and joint attention
   // image and context GEMMs of a kind share a launch (bf16 / FP8 modes: with head_dim 64)
@@ -602,17 +590,12 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   const float* x_wq = pre_j ? L.x_wq_s : L.x_wq;
   const bool pre_d = L.d_wq_s != nullptr;
   const float* d_wq = pre_d ? L.d_wq_s : L.d_wq;
-  // q pre-scaled and no bound from the norm weights: the attention looks at the norms of q and k
-  unsigned* const kj = pre_j && L.joint_bound == 0.f ? k_max_j : nullptr;
-  unsigned* const kd = pre_d && L.dual_bound == 0.f ? k_max_d : nullptr;
   if (m->D == 64) {
     // the image rows' two projections (a dual block's second one included) and the context rows'
-    LinearCall qkv[3] = {
+    const LinearCall qkv[3] = {
         {&L.x_qkv, w.h_x, B * Tx, qkv_epilogue(m, w.qkv, B, Tx, T, Tc, x_wq, L.x_wk), x8a},
         {&L.c_qkv, w.h_c, B * Tc, qkv_epilogue(m, w.qkv, B, Tc, T, 0, c_wq, L.c_wk), c8a},
         {&L.d_qkv, w.h_x2, B * Tx, qkv_epilogue(m, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk), x8a}};
-    qkv[0].epi.k_max = qkv[1].epi.k_max = kj;
-    qkv[2].epi.k_max = kd;
     SD3_TRY(run_linear_group(m, qkv, together ? 3 : 2, st));
   } else {
     SD3_TRY(run_qkv(m, L.c_qkv, w.h_c, w.qkv, B, Tc, T, 0, c_wq, L.c_wk, st, c8a));
@@ -622,8 +605,8 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   // kernel to write it (one flag for both outputs)
   const bool o8 = m->fp8 && m->D == 64 && L.x_out.w8 && (L.last || L.c_out.w8);
   const bool o8d = m->fp8 && m->D == 64 && L.d_out.w8;
-  const AttnCall att[2] = {{w.qkv, T, Tc, L.last ? nullptr : w.o_c, w.o_x, o8, L.joint_bound, pre_j, kj},
-                           {w.qkv2, Tx, 0, nullptr, w.o_x2, o8d, L.dual_bound, pre_d, kd}};
+  const AttnCall att[2] = {{w.qkv, T, Tc, L.last ? nullptr : w.o_c, w.o_x, o8, L.joint_bound, pre_j},
+                           {w.qkv2, Tx, 0, nullptr, w.o_x2, o8d, L.dual_bound, pre_d}};
   SD3_TRY(run_attention(m, att, together ? 2 : 1, B, st));
   if (out_together) {
     // both projections into x and the context rows' one: per element of x the joint attention's part is added first,
@@ -631,7 +614,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     LinearCall out[3] = {{&L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8},
                          {&L.c_out, w.o_c, B * Tc, gate_epilogue(L.c_out, Tc, c_gate_a, ms, c), o8},
                          {&L.d_out, w.o_x2, B * Tx, gate_epilogue(L.d_out, Tx, x_gate_2, ms, x), o8d}};
-    out[0].epi.order = out[2].epi.order = order;
+    out[0].epi.order = out[2].epi.order = w.order;
     out[2].epi.order_second = 1;
     SD3_TRY(run_linear_group(m, out, 3, st));
   } else if (grouped && !L.last) {
@@ -643,7 +626,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   }
   if (L.dual) {
     if (!together) {
-      SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a, kd));
+      SD3_TRY(run_qkv(m, L.d_qkv, w.h_x2, w.qkv2, B, Tx, Tx, 0, d_wq, L.d_wk, st, x8a));
       SD3_TRY(run_attention(m, att + 1, 1, B, st));
     }
     if (!out_together) SD3_TRY(run_gate_resid(m, L.d_out, w.o_x2, B, Tx, x_gate_2, ms, x, st, o8d));
@@ -721,9 +704,9 @@ int quantize_block_weights(sd3_model* m) {
 // <= D max_d |wq_d wk_d| for every query and key of an attention (context and image streams share
 // the joint attention: element-wise maxima of their weights).  1 % on top covers the bf16 rounding
 // of q and k.
-// The query norm weights also get a copy multiplied by softmax_scale * log2(e): q leaves the QKV epilogue
-// pre-scaled (one rounding to bf16, as before).  The bound is stored in those units where it is small enough
-// for the attention kernel's bounded softmax; where it is not, the kernel decides by the norms of q and k.
+// Where the bound is small enough for the attention kernel's bounded softmax, the query norm
+// weights also get a copy multiplied by softmax_scale * log2(e): q leaves the QKV epilogue
+// pre-scaled (one rounding to bf16, as before) and the bound is stored in those units.
 int compute_score_bounds(sd3_model* m) {
   for (LayerW& L : m->layers) L.joint_bound = L.dual_bound = 0.f;
   if (!m->cfg.use_qk_norm || m->f32 || m->D != 64) return ST_OK;
@@ -749,7 +732,8 @@ int compute_score_bounds(sd3_model* m) {
     for (int d = 0; d < m->D; ++d) a = std::max(a, q[d] * k[d]);
     return a;
   };
-  // the bounded softmax takes exp2 arguments of at most 80: a looser bound would not be used
+  // the bounded softmax takes exp2 arguments of at most 80: a looser bound would not be used,
+  // and then q stays unscaled and the attention keeps its running maximum
   const float c = 1.4426950408889634f / sqrtf(static_cast<float>(m->D));
   auto scaled_copy = [&](const float* w, float** dst) -> int {
     if (cudaMemcpy(h.data(), w, sizeof(float) * m->D, cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -767,9 +751,9 @@ int compute_score_bounds(sd3_model* m) {
     absmax_into(L.c_wq, q); absmax_into(L.x_wq, q);
     absmax_into(L.c_wk, k); absmax_into(L.x_wk, k);
     const float jb = 1.01f * m->D * pair_bound(q, k) * c;
-    if (ok) {
+    if (ok && jb > 0.f && jb <= 80.0f) {
       if ((rc = scaled_copy(L.c_wq, &L.c_wq_s)) || (rc = scaled_copy(L.x_wq, &L.x_wq_s))) return rc;
-      if (jb > 0.f && jb <= 80.0f) L.joint_bound = jb;
+      L.joint_bound = jb;
     } else {
       L.c_wq_s = L.x_wq_s = nullptr;  // (a buffer from an earlier finalize stays owned by the model)
     }
@@ -779,9 +763,9 @@ int compute_score_bounds(sd3_model* m) {
       absmax_into(L.d_wq, q2);
       absmax_into(L.d_wk, k2);
       const float db = 1.01f * m->D * pair_bound(q2, k2) * c;
-      if (ok) {
+      if (ok && db > 0.f && db <= 80.0f) {
         if ((rc = scaled_copy(L.d_wq, &L.d_wq_s))) return rc;
-        if (db > 0.f && db <= 80.0f) L.dual_bound = db;
+        L.dual_bound = db;
       } else {
         L.d_wq_s = nullptr;
       }

@@ -54,7 +54,7 @@ __host__ __device__ constexpr int pair_stage_bytes(int pbn) { return P_A_BYTES +
 // epilogue warp.
 constexpr int P_RED_BYTES = 4096;
 __host__ __device__ constexpr bool pair_stages_out(int epi, bool out_f32) {
-  return epi == EPI_GATE_RESID || (!out_f32 && (epi == EPI_BIAS || epi == EPI_BIAS_GELU || epi == EPI_QKV_NORM || epi == EPI_QKV_KMAX));
+  return epi == EPI_GATE_RESID || (!out_f32 && (epi == EPI_BIAS || epi == EPI_BIAS_GELU || epi == EPI_QKV_NORM));
 }
 // Six stages of 32 KiB (eight of 24 KiB), handed over in slots of one (two): a full and an empty barrier, one
 // wait and one commit each.  A stage of the wide tile is 512 cycles of MMA and single hand-overs refill the
@@ -261,7 +261,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       // one before it to have been read.  us of a launch, before -> after: gate + residual K 1536, 589 rows 8.8 -> 8.2,
       // 1357 rows 9.6 -> 9.3; K 6144, 589 rows 20.3 -> 19.7; GELU 1357 rows 23.5 -> 22.5, 4429 rows 61.1 -> 59.2.  (256-wide
       // QKV tiles lose it to spilled registers: 4429 rows 47.4 -> 50.5.)
-      constexpr bool OWN_BOXES = !((EPI == EPI_QKV_NORM || EPI == EPI_QKV_KMAX) && PBN == 256);
+      constexpr bool OWN_BOXES = !(EPI == EPI_QKV_NORM && PBN == 256);
       const bool last = OWN_BOXES && tile + num_pairs >= num_tiles;
       constexpr int BOXES = PBN / 2 / (EPI == EPI_GATE_RESID ? 32 : 64);  // of a warp and tile
       uint8_t* box = last ? smem + (warp - 2) * (BOXES * P_RED_BYTES) : red_smem + (warp - 2) * P_RED_BYTES;
@@ -325,7 +325,7 @@ int launch_pair_inst(const PairProblem* p, const int* end, cudaStream_t stream) 
 template <int EPI, bool OUT_F32, bool FP8>
 int launch_pair_width(int pbn, const PairProblem* p, const int* end, cudaStream_t stream) {
   constexpr bool narrow_built = (OUT_F32 && (EPI == EPI_GATE_RESID || EPI == EPI_BIAS || EPI == EPI_ADD_TABLE)) ||
-                                (!OUT_F32 && (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_QKV_NORM || EPI == EPI_QKV_KMAX));
+                                (!OUT_F32 && (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_QKV_NORM));
   if constexpr (narrow_built) {
     if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p, end, stream);
   }
@@ -467,23 +467,18 @@ int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int 
     end[i] = tiles;
   }
   const bool f32 = a.epi.out_f32 != 0;
-  int mode = a.epi.mode;  // of the kernel: that of the problems, or its variant where one of them asks for more
-  for (int i = 0; i < n; ++i)
-    if (q[i].epi.mode == EPI_QKV_NORM && q[i].epi.k_max && !f32) mode = EPI_QKV_KMAX;
   if (fp8) {
-    switch (mode) {
+    switch (a.epi.mode) {
       case EPI_BIAS: return launch_pair_width<EPI_BIAS, false, true>(pbn, p, end, stream);
       case EPI_BIAS_GELU: return launch_pair_width<EPI_BIAS_GELU, false, true>(pbn, p, end, stream);
       case EPI_QKV_NORM: return launch_pair_width<EPI_QKV_NORM, false, true>(pbn, p, end, stream);
-      case EPI_QKV_KMAX: return launch_pair_width<EPI_QKV_KMAX, false, true>(pbn, p, end, stream);
       case EPI_GATE_RESID: return launch_pair_width<EPI_GATE_RESID, true, true>(pbn, p, end, stream);
       default: break;
     }
     set_last_error("gemm_pair: no e4m3 instantiation for epilogue mode %d", a.epi.mode);
     return ST_UNSUPPORTED;
   }
-  switch (mode) {
-    case EPI_QKV_KMAX: return launch_pair_width<EPI_QKV_KMAX, false, false>(pbn, p, end, stream);
+  switch (a.epi.mode) {
     case EPI_BIAS:
       return f32 ? launch_pair_width<EPI_BIAS, true, false>(pbn, p, end, stream)
                  : launch_pair_width<EPI_BIAS, false, false>(pbn, p, end, stream);

@@ -129,16 +129,13 @@ __device__ __forceinline__ RowMap map_row(int m, const GemmEpilogue& e) {
 // warp and the tensor map of the bf16 output.  With them the warp's 32 rows x 64 columns
 // leave as ONE TMA store (rows in the 128-byte swizzle, 16-byte chunk c of row r at chunk
 // c ^ (r & 7)) instead of 128 32-byte register stores; orow0 is the output row of lane 0.
-// fresh: the warp has not stored from `stage` before.  one_sample: all 32 rows of the warp are here and of one sample.
-template <int EPI_, bool OUT_F32>
+// fresh: the warp has not stored from `stage` before.
+template <int EPI, bool OUT_F32>
 __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, int n_base,
-                                            const GemmArgs& g, uint8_t* stage,
-                                            const void* tmO, long orow0, bool fresh, bool one_sample) {
-  constexpr bool K_MAX = EPI_ == EPI_QKV_KMAX;
-  constexpr int EPI = K_MAX ? static_cast<int>(EPI_QKV_NORM) : EPI_;
+                                            const GemmArgs& g, uint8_t* stage = nullptr,
+                                            const void* tmO = nullptr, long orow0 = 0, bool fresh = false) {
   const GemmEpilogue& e = g.epi;
   const int N = g.N;
-  float k2 = 0.f;
   if constexpr (EPI == EPI_QKV_NORM) {
     if (e.do_norm && n_base < e.qk_cols) {
       const float* w = (n_base < (e.qk_cols >> 1)) ? e.wq : e.wk;
@@ -160,32 +157,8 @@ __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, in
       const float r = rsqrtf(((s0 + s1) + (s2 + s3)) * (1.0f / 64.0f) + e.eps);
 #pragma unroll
       for (int j = 0; j < 64; ++j) v[j] = v[j] * r * ww[j];
-      if (K_MAX && e.k_max != nullptr && n_base >= (e.qk_cols >> 1)) {
-        float q0 = 0.f, q1 = 0.f;
-#pragma unroll
-        for (int j = 0; j < 64; j += 2) {
-          q0 = fmaf(v[j], v[j], q0);
-          q1 = fmaf(v[j + 1], v[j + 1], q1);
-        }
-        k2 = q0 + q1;
-      }
     }
   }
-  // the largest |k|^2 of the sample and head (rows past M do not come here)
-  auto put_k_max = [&]() {
-    if constexpr (K_MAX) {
-      if (e.k_max != nullptr && e.do_norm && n_base < e.qk_cols && n_base >= (e.qk_cols >> 1)) {
-        const int heads = e.qk_cols >> 7, head = (n_base - (e.qk_cols >> 1)) >> 6;
-        const unsigned bits = __float_as_uint(k2);  // never negative: orders like the float; NaN above all
-        if (one_sample) {
-          const unsigned most = __reduce_max_sync(0xffffffffu, bits);
-          if ((threadIdx.x & 31) == 0) atomicMax(e.k_max + static_cast<long>(rm.b) * heads + head, most);
-        } else {
-          atomicMax(e.k_max + static_cast<long>(rm.b) * heads + head, bits);
-        }
-      }
-    }
-  };
   if constexpr (EPI == EPI_UNPATCHIFY) {
     // m = (b, r, s) over the patch grid; n = ph * (p * C) + pw * C + c
     const int p = e.up_patch, C = e.up_cin;
@@ -232,7 +205,6 @@ __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, in
         tma_store_2d(tmO, stage, n_base, static_cast<int>(orow0));
         bulk_commit_group();
       }
-      put_k_max();
       return;
     }
   }
@@ -267,7 +239,6 @@ __device__ __forceinline__ void epilogue_64(float (&v)[64], const RowMap& rm, in
       if (n < N) store8<OUT_F32>(e.out, base + gi * 8, &v[gi * 8]);
     }
   }
-  put_k_max();
 }
 
 // Drains this warp's share of one accumulator tile (rows = TMEM lanes of the
@@ -333,11 +304,6 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
     const int c_first = COLS_PER_WARP >= 64 ? half * CHUNKS : 0;
     float bb[64];
     if (active) load_f4_batch<16>(e.bias, n0 + c_first * 64, g.N, bb);
-    bool one_sample = false;
-    if constexpr (EPI == EPI_QKV_KMAX) {
-      const int first_b = __shfl_sync(0xffffffffu, rm.b, 0);
-      one_sample = __all_sync(0xffffffffu, valid && rm.b == first_b) != 0;
-    }
     if (!mbar_wait_warp(tfull_bar, phase, wc, DEV_TIMEOUT_TMEM_FULL)) return false;
     tc_fence_after_sync();
 #pragma unroll 1
@@ -355,10 +321,14 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
         v[j] = fmaf(__uint_as_float(r0[j]), e.alpha, bb[j]);
         v[32 + j] = fmaf(__uint_as_float(r1[j]), e.alpha, bb[32 + j]);
       }
-      // with a stage the whole warp is valid or not at all (M % 32 == 0 is a condition of that path)
-      if (valid)
-        epilogue_64<EPI, OUT_F32>(v, rm, n_base, g, stage ? stage + ci * stage_step : nullptr, tmO,
-                                  rm.orow - (threadIdx.x & 31), stage_step != 0, one_sample);
+      if (stage != nullptr) {
+        // whole warp valid or not at all (M % 32 == 0 is a condition of this path)
+        if (valid)
+          epilogue_64<EPI, OUT_F32>(v, rm, n_base, g, stage + ci * stage_step, tmO, rm.orow - (threadIdx.x & 31),
+                                    stage_step != 0);
+      } else if (valid) {
+        epilogue_64<EPI, OUT_F32>(v, rm, n_base, g);
+      }
       if (ci + 1 < CHUNKS) load_f4_batch<16>(e.bias, n_base + 64, g.N, bb);  // next chunk's bias
     }
   }

@@ -331,7 +331,6 @@ int dispatch_epi(const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs&
       if (!f32) break;
       return launch_inst<BN, EPI_GATE_RESID, true, FP8>(tmA, tmW, g, stream);
     case EPI_QKV_NORM:
-      if (g.epi.k_max && !f32) return launch_inst<BN, EPI_QKV_KMAX, false, FP8>(tmA, tmW, g, stream);
       return f32 ? launch_inst<BN, EPI_QKV_NORM, true, FP8>(tmA, tmW, g, stream)
                  : launch_inst<BN, EPI_QKV_NORM, false, FP8>(tmA, tmW, g, stream);
     case EPI_ADD_TABLE:

@@ -65,7 +65,6 @@ enum GemmEpi : int {
   EPI_GATE_RESID = 2,  // out = resid + gate[b, n] * (acc + bias)         (fp32 out)
   EPI_QKV_NORM = 3,    // out = per-head RMSNorm on the q and k column ranges of (acc + bias)
   EPI_ADD_TABLE = 4,   // out = acc + bias + table[m % rows_in, n]         (fp32 out)
-  EPI_QKV_KMAX = 6,    // the kernel of EPI_QKV_NORM problems with k_max (chosen by the launchers)
   EPI_UNPATCHIFY = 5,  // out[b, c, 2r+ph, 2s+pw] = acc + bias, n = ph*(p*C) + pw*C + c
 };
 
@@ -98,9 +97,6 @@ struct GemmEpilogue {
   int qk_cols = 0;
   float eps = 1e-6f;
   int do_norm = 1;
-  // optional: k_max[b * heads + head] (bits of a float, zero before the launch) becomes the largest |k|^2 of the
-  // sample's rows as written by this launch, before their rounding to bf16 (bf16 output with the fused norm)
-  unsigned* k_max = nullptr;
   // EPI_QKV_NORM, optional head-group layout (hg_groups > 1): the output is
   // (hg_groups, hg_rows, 3, E / hg_groups) -- slab g holds the q, k and v columns of the heads
   // of group g for every row -- instead of (rows, 3E); the send layout of a head all-to-all.
@@ -169,9 +165,7 @@ int launch_gemm_split(const SplitGemmProblem* q, int n, int N, int K, int* dev_s
 // shapes that fill the machine anyway): lets launches with too few CTAs split the keys of a
 // query tile over several CTAs and merge the partial results.  score_bound (optional): an upper
 // bound on |q . k| for every query and key, 0 if unknown; a bound of at most 80 / (scale log2 e)
-// lets the softmax run without a running maximum.  k_max (AttnProblem; with scale == 0 and no such
-// score_bound): the largest |k|^2 per (sample, head) as GemmEpilogue::k_max leaves it; 32 query rows at a time
-// then run without a running maximum where |q| |k| shows that they can.
+// lets the softmax run without a running maximum.
 int launch_attention_bf16(const bf16* qkv, int B, int T, int NH, int Tc, bf16* out_c, bf16* out_x,
                           float scale, int* dev_status, cudaStream_t stream, int out_e4m3 = 0,
                           void* scratch = nullptr, size_t scratch_bytes = 0, float score_bound = 0.0f);
@@ -187,7 +181,6 @@ struct AttnProblem {
   void* scratch;
   size_t scratch_bytes;
   float score_bound;
-  const unsigned* k_max = nullptr;
 };
 int launch_attention_group(const AttnProblem* p, int n, int B, int NH, int* dev_status, cudaStream_t stream);
 
