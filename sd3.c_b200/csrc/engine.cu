@@ -78,7 +78,6 @@ struct Workspace {
   void* a8 = nullptr;    // FP8 mode: e4m3 copy of the current GEMM's left operand
   void* attn_scratch = nullptr;  // partial results of key-split attention launches (small batches, long sequences)
   size_t attn_scratch_bytes = 0;
-  unsigned* order = nullptr;  // a dual block's two out-projections into x as one launch (GemmEpilogue::order)
   // position table cache
   float* pos = nullptr;
   int pos_h = 0, pos_w = 0;
@@ -275,7 +274,6 @@ int reserve_ws(sd3_model* m, int B, int Tc, int Tx) {
       {&w.hid_x, nTx * F * ab}, {&w.hid_c, nTc * F * ab},
       {(void**)&w.o_f32, m->f32 && m->D != 64 ? nB * T * E * 4 : 16},
       {&w.a8, m->fp8 ? (nTx > nTc ? nTx : nTc) * F : 16},
-      {(void**)&w.order, m->f32 ? 16 : gate_order_words(static_cast<long>(nTx), m->E) * sizeof(unsigned)},
       {&w.attn_scratch, 16},
   };
   // key-split attention (head_dim 64 tensor-core path): the larger need of the joint and the image-only call
@@ -537,11 +535,10 @@ bool merge_launches(int B, int Tc, int Tx) {
 }
 
 // the LayerNorms of the image and the context rows, as one launch where both write the same type
-int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st,
-                unsigned* zero = nullptr, int nzero = 0) {
+int run_ln_pair(const LnProblem& px, int out_x, const LnProblem* pc, int out_c, int E, long ms, cudaStream_t st) {
   if (!pc || (out_x == out_c && merge_launches(px.B, pc->T, px.T)))
-    return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st, zero, nzero);
-  int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st, zero, nzero);
+    return launch_ln_modulate(px, pc, E, 1e-6f, ms, out_x, st);
+  int rc = launch_ln_modulate(*pc, nullptr, E, 1e-6f, ms, out_c, st);
   return rc ? rc : launch_ln_modulate(px, nullptr, E, 1e-6f, ms, out_x, st);
 }
 
@@ -573,13 +570,12 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
   // a dual block's image-only attention and out-projection beside the joint ones, or after them
   const bool together = L.dual && m->D == 64 && merge_launches(B, Tc, Tx);
   const bool out_together = together && !m->f32 && !L.last;
-  const size_t order_words = out_together ? gate_order_words(static_cast<long>(B) * Tx, E) : 0;
   // pre-attention LayerNorm + modulate
   {
     LnProblem px = {x, B, Tx, x_shift_a, x_scale_a, w.h_x, nullptr, nullptr, nullptr};
     if (L.dual) { px.shift2 = x_shift_2; px.scale2 = x_scale_2; px.out2 = w.h_x2; }
     const LnProblem pc = {c, B, Tc, c_shift_a, c_scale_a, w.h_c, nullptr, nullptr, nullptr};
-    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st, w.order, static_cast<int>(order_words)));
+    SD3_TRY(run_ln_pair(px, ln_out(x8a), &pc, ln_out(c8a), E, ms, st));
   }
   // QKV (context rows first, then image rows) and joint attention
   // image and context GEMMs of a kind share a launch (bf16 / FP8 modes: with head_dim 64)
@@ -614,8 +610,7 @@ int block_body(sd3_model* m, int l, float* c, float* x, int B, int Tc, int Tx, c
     LinearCall out[3] = {{&L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8},
                          {&L.c_out, w.o_c, B * Tc, gate_epilogue(L.c_out, Tc, c_gate_a, ms, c), o8},
                          {&L.d_out, w.o_x2, B * Tx, gate_epilogue(L.d_out, Tx, x_gate_2, ms, x), o8d}};
-    out[0].epi.order = out[2].epi.order = w.order;
-    out[2].epi.order_second = 1;
+    out[2].epi.adds_after = 1;
     SD3_TRY(run_linear_group(m, out, 3, st));
   } else if (grouped && !L.last) {
     SD3_TRY(run_linear_pair(m, L.x_out, w.o_x, B * Tx, gate_epilogue(L.x_out, Tx, x_gate_a, ms, x), o8,

@@ -32,6 +32,7 @@
 
 #include "gemm_epilogue.cuh"
 #include "kernels.h"
+#include "pair_tiles.h"
 #include "ptx.cuh"
 
 namespace sd3 {
@@ -79,8 +80,7 @@ struct PairProblem {
 template <int EPI, bool OUT_F32, bool FP8, int PBN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_constant__ PairProblem p1,
-                         const __grid_constant__ PairProblem p2, const int end0, const int end1,
-                         const int num_tiles) {
+                         const __grid_constant__ PairProblem p2, const PairTiles all) {
   // M = 256 across the pair; operands bf16, or e4m3 (128 K-elements per 128-byte stage row,
   // 32 per instruction: the byte arithmetic of the stages is the same)
   constexpr uint32_t IDESC = FP8 ? make_idesc(0, 0, 2 * P_BM, PBN, 0, 0) : make_idesc(1, 1, 2 * P_BM, PBN, 0, 0);
@@ -106,6 +106,9 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
+  // tiles of 256 x PBN
+  const PairTiles tiles{all.end0, all.end1, all.end2, EPI == EPI_GATE_RESID ? all.sum : 0};
+  const int end0 = tiles.end0, end1 = tiles.end1, num_tiles = tiles.end2;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < P_STAGES; ++s) {
@@ -144,7 +147,6 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const WaitCtx wc{s_abort, p0.g.status};
 
-  // tiles of 256 x PBN: the first problem's up to end0, the second's up to end1, the third's
   constexpr int SLOT = pair_slot(PBN);
   constexpr int NSLOT = P_STAGES / SLOT;
   const int KB = p0.g.k_blocks;  // the same K for all problems
@@ -176,7 +178,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     };
     int pre = 0;  // slots of the first tile whose weights are under way before the wait
     bool waited = false;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+    for (int tile = pair; tile < num_tiles && ok; tile = tiles.next(tile, num_pairs)) {
       const PairProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
       const int m0 = (lt / pp.g.tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
@@ -210,7 +212,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       bool ok = true;
       const bool issuer = elect_one();
       const uint64_t desc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      for (int tile = pair; tile < num_tiles && ok; tile = tiles.next(tile, num_pairs)) {
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * PBN);
         if (!mbar_wait_all(&tempty_bar[acc], acc_phase ^ 1, wc, DEV_TIMEOUT_TMEM_EMPTY)) break;
         for (int kb = 0; kb < KB; kb += SLOT) {
@@ -247,7 +249,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
     const int row = quad * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+    for (int tile = pair; tile < num_tiles; tile = tiles.next(tile, num_pairs)) {
       const PairProblem& pp = tile < end0 ? p0 : tile < end1 ? p1 : p2;
       const GemmArgs& g = pp.g;
       const int lt = tile - (tile < end0 ? 0 : tile < end1 ? end0 : end1);
@@ -262,15 +264,13 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
       // 1357 rows 9.6 -> 9.3; K 6144, 589 rows 20.3 -> 19.7; GELU 1357 rows 23.5 -> 22.5, 4429 rows 61.1 -> 59.2.  (256-wide
       // QKV tiles lose it to spilled registers: 4429 rows 47.4 -> 50.5.)
       constexpr bool OWN_BOXES = !(EPI == EPI_QKV_NORM && PBN == 256);
-      const bool last = OWN_BOXES && tile + num_pairs >= num_tiles;
+      const bool last = OWN_BOXES && tiles.next(tile, num_pairs) >= num_tiles;
       constexpr int BOXES = PBN / 2 / (EPI == EPI_GATE_RESID ? 32 : 64);  // of a warp and tile
       uint8_t* box = last ? smem + (warp - 2) * (BOXES * P_RED_BYTES) : red_smem + (warp - 2) * P_RED_BYTES;
       const int box_step = last ? P_RED_BYTES : 0;
       if constexpr (EPI == EPI_GATE_RESID)
         drained = drain_tile_gate_reduce<PBN>(t_row, m0 + quad * 32, n0, half, g, &pp.tmR, &tfull_bar[acc],
-                                              acc_phase, wc, box, box_step,
-                                              g.epi.order ? g.epi.order + (lt * 2 + rank) * EPI_WARPS + (warp - 2)
-                                                          : nullptr);
+                                              acc_phase, wc, box, box_step, tiles.sum && tile >= end1);
       else
         drained = drain_tile<PBN, EPI, OUT_F32>(t_row, m0 + row, n0, half, g, &tfull_bar[acc], acc_phase, wc,
                                                 (pair_stages_out(EPI, OUT_F32) && g.tma_store) ? box : nullptr,
@@ -299,7 +299,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
 }
 
 template <int EPI, bool OUT_F32, bool FP8, int PBN>
-int launch_pair_inst(const PairProblem* p, const int* end, cudaStream_t stream) {
+int launch_pair_inst(const PairProblem* p, const PairTiles& tiles, cudaStream_t stream) {
   auto kern = gemm_pair_tcgen05_kernel<EPI, OUT_F32, FP8, PBN>;
   constexpr int SMEM = pair_smem_bytes(EPI, OUT_F32, PBN);
   static std::mutex attr_mutex;
@@ -314,25 +314,24 @@ int launch_pair_inst(const PairProblem* p, const int* end, cudaStream_t stream) 
       attr_done[dev] = true;
     }
   }
-  const int tiles = end[2];
   const int max_pairs = device_sm_count() / 2;
-  const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_dependent(kern, 2 * pairs, P_THREADS, SMEM, stream, p[0], p[1], p[2], end[0], end[1], tiles);
+  const int pairs = tiles.starts() < max_pairs ? tiles.starts() : max_pairs;
+  launch_dependent(kern, 2 * pairs, P_THREADS, SMEM, stream, p[0], p[1], p[2], tiles);
   return after_launch("gemm_pair_tcgen05_kernel");
 }
 
 // the epilogues that a forward uses exist for both tile widths, the others for 256 only
 template <int EPI, bool OUT_F32, bool FP8>
-int launch_pair_width(int pbn, const PairProblem* p, const int* end, cudaStream_t stream) {
+int launch_pair_width(int pbn, const PairProblem* p, const PairTiles& tiles, cudaStream_t stream) {
   constexpr bool narrow_built = (OUT_F32 && (EPI == EPI_GATE_RESID || EPI == EPI_BIAS || EPI == EPI_ADD_TABLE)) ||
                                 (!OUT_F32 && (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_QKV_NORM));
   if constexpr (narrow_built) {
-    if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p, end, stream);
+    if (pbn == 128) return launch_pair_inst<EPI, OUT_F32, FP8, 128>(p, tiles, stream);
   }
   if constexpr (EPI == EPI_GATE_RESID) {
-    if (pbn == 64) return launch_pair_inst<EPI, OUT_F32, FP8, 64>(p, end, stream);
+    if (pbn == 64) return launch_pair_inst<EPI, OUT_F32, FP8, 64>(p, tiles, stream);
   }
-  return launch_pair_inst<EPI, OUT_F32, FP8, 256>(p, end, stream);
+  return launch_pair_inst<EPI, OUT_F32, FP8, 256>(p, tiles, stream);
 }
 
 bool narrow_tiles_built(const GemmEpilogue& epi) {
@@ -399,14 +398,19 @@ int build_problem(PairProblem* pp, const GemmProblem& q, int operand_dtype, int 
 //   K 1536, gate  2714 rows 14.5 / 14.6 (1, 2)   4429: 23.5 / 21.2 (2, 3)   5428: 26.7 / 28.8 (2, 4)
 //   K 4096, fp32 output (the captions)  333 rows 24.8 / 14.9 (1, 1)   1332: 25.2 / 16.0 (1, 1)
 //   K 6144, gate  2714 rows 38.6 / 43.6 (1, 2)   4429: 68.8 / 67.4 (2, 3)   5428: 75.4 / 86.9 (2, 4)
-int choose_tile_width(long tiles256, int k_blocks, const GemmEpilogue& epi) {
+// after256: those of the 256-wide tiles that run after another one on the same pair (GemmEpilogue::adds_after), a wave of
+// their own.
+int choose_tile_width(long tiles256, long after256, int k_blocks, const GemmEpilogue& epi) {
   const long pairs = device_sm_count() / 2;
   if (pairs <= 0 || !narrow_tiles_built(epi)) return 256;
   // The gate + residual GEMMs, the ones with few tiles, have 64-wide ones too, for problems that fit one wave of
   // those.  us, 128 / 64 wide: K 6144, 256 rows 19.7 / 17.9, 333 rows 19.8 / 18.5, 700 rows 19.9 / 19.5; K 1536, 256 rows
   // 7.7 / 7.0, 589 rows 8.2 / 8.2 (slots of four stages: 20.1 at 256 rows).
-  if (epi.mode == EPI_GATE_RESID && 4 * tiles256 <= pairs) return 64;
-  const long wide = (tiles256 + pairs - 1) / pairs, narrow = (2 * tiles256 + pairs - 1) / pairs;
+  if (epi.mode == EPI_GATE_RESID && 4 * (tiles256 - after256) <= pairs) return 64;
+  auto waves = [&](int per256) {
+    return (per256 * (tiles256 - after256) + pairs - 1) / pairs + (per256 * after256 + pairs - 1) / pairs;
+  };
+  const long wide = waves(1), narrow = waves(2);
   return 64 * narrow * k_blocks < 100 * wide * k_blocks + 1000 ? 128 : 256;
 }
 
@@ -426,24 +430,19 @@ bool gemm_pair_supported(int operand_dtype, int M, int N, int K, const GemmEpilo
   return operand_dtype == OPERAND_BF16;
 }
 
-// One word per pair tile of any width, CTA and epilogue warp.  Which of the words a launch uses depends on its tile
-// width, which is the same for both problems.
-size_t gate_order_words(long M, int N) {
-  return static_cast<size_t>((M + 2 * P_BM - 1) / (2 * P_BM)) * (N / 64) * 2 * EPI_WARPS;
-}
-
 // One to three problems of the same N, K, operand type and epilogue kind.
-// A tile that waits for another (GemmEpilogue::order) waits for one of an earlier problem: earlier in the list of
-// tiles that every pair walks in order, and pairs are one per SM pair of the device and started in order, so the
-// first unfinished tile never waits.
 int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
                      cudaStream_t stream) {
   const bool fp8 = operand_dtype == OPERAND_E4M3;
   const GemmProblem& a = q[0];
+  // by itself such a problem is an ordinary one: it comes after the first in stream order
+  const bool sum = n > 1 && q[n - 1].epi.adds_after;
   long tiles256 = 0;
   for (int i = 0; i < n; ++i) {
-    if (q[i].epi.order && q[i].epi.order_second && i == 0) {
-      set_last_error("gemm_pair: the problem that adds second comes first in its launch");
+    if (n > 1 && q[i].epi.adds_after &&
+        (i != n - 1 || a.epi.mode != EPI_GATE_RESID || q[i].M != a.M || q[i].epi.resid != a.epi.resid ||
+         q[i].epi.ldo != a.epi.ldo)) {
+      set_last_error("gemm_pair: a problem that adds after the first has its rows and its residual, and comes last");
       return ST_INVALID_ARG;
     }
     if (q[i].epi.mode != a.epi.mode || q[i].epi.out_f32 != a.epi.out_f32) {
@@ -453,26 +452,29 @@ int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int 
     tiles256 += static_cast<long>((q[i].M + 255) / 256) * (N / 256);
   }
   const int kel = P_KBYTES / (fp8 ? 1 : 2);
-  const int pbn = choose_tile_width(tiles256, (K + kel - 1) / kel, a.epi);
+  const long after256 = sum ? static_cast<long>((a.M + 255) / 256) * (N / 256) : 0;
+  const int pbn = choose_tile_width(tiles256, after256, (K + kel - 1) / kel, a.epi);
   PairProblem p[3];
-  int end[3] = {0, 0, 0}, tiles = 0;
+  int end[3] = {0, 0, 0}, count = 0;
   for (int i = 0; i < 3; ++i) {
-    if (i < n) {
-      int rc = build_problem(&p[i], q[i], operand_dtype, N, K, pbn, dev_status);
+    const int j = sum && i == 2 ? n - 1 : i < (sum ? n - 1 : n) ? i : -1;  // one that adds after the first is the third
+    if (j >= 0) {
+      int rc = build_problem(&p[i], q[j], operand_dtype, N, K, pbn, dev_status);
       if (rc) return rc;
-      tiles += p[i].g.tiles_m * p[i].g.tiles_n;
+      count += p[i].g.tiles_m * p[i].g.tiles_n;
     } else {
       p[i] = p[0];  // no tiles
     }
-    end[i] = tiles;
+    end[i] = count;
   }
+  const PairTiles tiles{end[0], end[1], end[2], sum ? 1 : 0};
   const bool f32 = a.epi.out_f32 != 0;
   if (fp8) {
     switch (a.epi.mode) {
-      case EPI_BIAS: return launch_pair_width<EPI_BIAS, false, true>(pbn, p, end, stream);
-      case EPI_BIAS_GELU: return launch_pair_width<EPI_BIAS_GELU, false, true>(pbn, p, end, stream);
-      case EPI_QKV_NORM: return launch_pair_width<EPI_QKV_NORM, false, true>(pbn, p, end, stream);
-      case EPI_GATE_RESID: return launch_pair_width<EPI_GATE_RESID, true, true>(pbn, p, end, stream);
+      case EPI_BIAS: return launch_pair_width<EPI_BIAS, false, true>(pbn, p, tiles, stream);
+      case EPI_BIAS_GELU: return launch_pair_width<EPI_BIAS_GELU, false, true>(pbn, p, tiles, stream);
+      case EPI_QKV_NORM: return launch_pair_width<EPI_QKV_NORM, false, true>(pbn, p, tiles, stream);
+      case EPI_GATE_RESID: return launch_pair_width<EPI_GATE_RESID, true, true>(pbn, p, tiles, stream);
       default: break;
     }
     set_last_error("gemm_pair: no e4m3 instantiation for epilogue mode %d", a.epi.mode);
@@ -480,20 +482,20 @@ int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int 
   }
   switch (a.epi.mode) {
     case EPI_BIAS:
-      return f32 ? launch_pair_width<EPI_BIAS, true, false>(pbn, p, end, stream)
-                 : launch_pair_width<EPI_BIAS, false, false>(pbn, p, end, stream);
+      return f32 ? launch_pair_width<EPI_BIAS, true, false>(pbn, p, tiles, stream)
+                 : launch_pair_width<EPI_BIAS, false, false>(pbn, p, tiles, stream);
     case EPI_BIAS_GELU:
-      return f32 ? launch_pair_width<EPI_BIAS_GELU, true, false>(pbn, p, end, stream)
-                 : launch_pair_width<EPI_BIAS_GELU, false, false>(pbn, p, end, stream);
+      return f32 ? launch_pair_width<EPI_BIAS_GELU, true, false>(pbn, p, tiles, stream)
+                 : launch_pair_width<EPI_BIAS_GELU, false, false>(pbn, p, tiles, stream);
     case EPI_GATE_RESID:
       if (!f32) break;
-      return launch_pair_width<EPI_GATE_RESID, true, false>(pbn, p, end, stream);
+      return launch_pair_width<EPI_GATE_RESID, true, false>(pbn, p, tiles, stream);
     case EPI_QKV_NORM:
-      return f32 ? launch_pair_width<EPI_QKV_NORM, true, false>(pbn, p, end, stream)
-                 : launch_pair_width<EPI_QKV_NORM, false, false>(pbn, p, end, stream);
+      return f32 ? launch_pair_width<EPI_QKV_NORM, true, false>(pbn, p, tiles, stream)
+                 : launch_pair_width<EPI_QKV_NORM, false, false>(pbn, p, tiles, stream);
     case EPI_ADD_TABLE:
       if (!f32) break;
-      return launch_pair_width<EPI_ADD_TABLE, true, false>(pbn, p, end, stream);
+      return launch_pair_width<EPI_ADD_TABLE, true, false>(pbn, p, tiles, stream);
     default:
       break;
   }

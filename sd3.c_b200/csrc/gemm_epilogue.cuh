@@ -348,13 +348,14 @@ __device__ __forceinline__ bool drain_tile(uint32_t t_row, int m, int n0, int ha
 // out == resid.  `stage` is 1024-byte aligned.  m_w0: first row of this warp.
 // stage_step: bytes between the buffers of consecutive boxes; 0: all use the one at
 // `stage`, each after the reduction before it has read the buffer.
-// order: this warp's word of GemmEpilogue::order, or null.
+// after: this warp's tile before was the same rows and columns of another problem with this residual
+// (GemmEpilogue::adds_after); its reductions have to land before those of this tile.
 template <int BN>
 __device__ __forceinline__ bool drain_tile_gate_reduce(uint32_t t_row, int m_w0, int n0, int half,
                                                        const GemmArgs& g, const void* tmR,
                                                        uint64_t* tfull_bar, uint32_t phase,
                                                        const WaitCtx& wc, uint8_t* stage, int stage_step,
-                                                       unsigned* order) {
+                                                       bool after) {
   constexpr int CPW = BN / 2, NSUB = CPW / 32;
   const GemmEpilogue& e = g.epi;
   const int lane = threadIdx.x & 31;
@@ -397,22 +398,16 @@ __device__ __forceinline__ bool drain_tile_gate_reduce(uint32_t t_row, int m_w0,
           make_float4(d[4 * c], d[4 * c + 1], d[4 * c + 2], d[4 * c + 3]);
     fence_proxy_async_smem();
     __syncwarp();
-    if (sub == 0 && order != nullptr && e.order_second) {
-      int ok = 1;
-      if (lane == 0) ok = order_wait(order, wc) ? 1 : 0;
-      if (__shfl_sync(0xffffffffu, ok, 0) == 0) return false;
-    }
     if (lane == 0 && m_w0 < g.M) {
+      if (sub == 0 && after) {
+        bulk_wait_group0();
+        fence_proxy_async();
+      }
       tma_reduce_add_2d(tmR, box, n_base, m_w0);
       bulk_commit_group();
     }
   }
-  if (lane == 0) {
-    if (order != nullptr && !e.order_second)
-      order_publish(order);  // its wait covers the buffer too
-    else if (stage_step == 0)
-      bulk_wait_group_read0();  // the buffer is reused by this warp's next tile
-  }
+  if (lane == 0 && stage_step == 0) bulk_wait_group_read0();  // the buffer is reused by this warp's next tile
   __syncwarp();
   return true;
 }

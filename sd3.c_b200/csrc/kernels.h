@@ -85,11 +85,9 @@ struct GemmEpilogue {
   const float* gate = nullptr;  // gate[b * gate_stride + n]
   long gate_stride = 0;
   const float* resid = nullptr;  // same indexing as out; may alias out
-  // EPI_GATE_RESID, two problems of one launch that update the same resid: words that are zero at launch,
-  // gate_order_words(M, N) of them, shared by the two.  The problem with order_second == 0, which has to come first
-  // in the launch, adds first to every element, the other one second.
-  unsigned* order = nullptr;
-  int order_second = 0;
+  // EPI_GATE_RESID, the last problem of a grouped launch (launch_gemm_grouped): it updates the resid of the first one, and
+  // adds to every element after it, whether they share a launch (pair_tiles.h) or run one after the other.
+  int adds_after = 0;
   // EPI_QKV_NORM (head_dim 64): columns [0, qk_cols) are normalised; the first
   // half with wq, the second half with wk.  Either weight may be null (-> 1).
   const float* wq = nullptr;
@@ -136,8 +134,6 @@ struct GemmProblem {
 // covers share ONE launch (one problem's tiles run in the tail of the other's), the others get
 // their own.  Used for the image-stream GEMM of a block, its small context-stream twin and the
 // second QKV projection of a dual block.
-// Problems that update the same resid (GemmEpilogue::order) share a launch or run one after the other.
-size_t gate_order_words(long M, int N);
 int launch_gemm_grouped(const GemmProblem* q, int n, int operand_dtype, int N, int K, int* dev_status,
                         cudaStream_t stream);
 
@@ -203,7 +199,7 @@ int launch_attention_simt(const void* q, const void* k, const void* v, long ld, 
 // LayerNorm (no affine) + up to two modulations:  out_i = LN(x) * (1 + scale_i[b]) + shift_i[b]
 // x: (B*T, E) fp32.  shift/scale: [b * mod_stride + e].  out: bf16 (out_f32 = 0), fp32 (1),
 // e4m3 converted as is (2) or three bf16 planes of B*T*E elements (3, split3.cuh).  One or two
-// problems (b may be null) as one launch.  zero: nzero words that the launch also sets to zero.
+// problems (b may be null) as one launch.
 struct LnProblem {
   const float* x = nullptr;
   int B = 0, T = 0;
@@ -213,7 +209,7 @@ struct LnProblem {
   void* out2 = nullptr;
 };
 int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
-                       cudaStream_t stream, unsigned* zero = nullptr, int nzero = 0);
+                       cudaStream_t stream);
 
 // Skinny linear for M = B <= 64 rows:  out[b, n] = act_out(sum_k in[b,k] W[n,k] + bias[n] + add[b,n])
 // W is (N, K) row-major, bf16 or fp32 (w_f32).  act: 0 none, 1 SiLU.  w_static: no kernel that may

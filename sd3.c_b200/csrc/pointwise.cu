@@ -80,13 +80,11 @@ __device__ __forceinline__ void ln_store4(void* out, long row, long rows, int E,
 
 template <int MAXV, int OUT, bool DUAL>
 __global__ void __launch_bounds__(LN_WARPS * 32, OUT == 3 ? 3 : 4)
-ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a, unsigned* zero, int nzero, int E, float eps, long mod_stride,
+ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a, int E, float eps, long mod_stride,
                    int rpw) {
   extern __shared__ float4 ln_smem[];  // [1 + scale1 | shift1 | 1 + scale2 | shift2], E floats each
   grid_dep_wait();
   grid_dep_launch();
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<unsigned>(nzero); i += gridDim.x * blockDim.x)
-    zero[i] = 0;
   const bool second = blockIdx.x >= grid_a;
   const LnProblem& p = second ? pb : pa;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -200,12 +198,10 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
 template <int OUT, bool DUAL, bool MULTI>
 __global__ void __launch_bounds__(128)
 ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a,
-                       unsigned* zero, int nzero, int E, float eps, long mod_stride, int per_cta) {
+                       int E, float eps, long mod_stride, int per_cta) {
   __shared__ float part[2][LN_ROW_QUADS][32];
   grid_dep_wait();
   grid_dep_launch();
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<unsigned>(nzero); i += gridDim.x * blockDim.x)
-    zero[i] = 0;
   const bool second = blockIdx.x >= grid_a;
   const LnProblem& p = second ? pb : pa;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -281,7 +277,7 @@ ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_consta
 
 template <int MAXV>
 int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
-                   cudaStream_t stream, unsigned* zero, int nzero) {
+                   cudaStream_t stream) {
   const long rows_a = static_cast<long>(a.B) * a.T, rows_b = b ? static_cast<long>(b->B) * b->T : 0;
   // rows per warp: as many as keeps at least two CTAs per SM busy
   int rpw = LN_MAX_ROWS_PER_WARP;
@@ -300,8 +296,7 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
     const unsigned ga = static_cast<unsigned>((rows_a + per - 1) / per);
     const dim3 row_ctas(ga + static_cast<unsigned>((rows_b + per - 1) / per));
 #define SD3_LN_ROW_INST(F32, DUALV, MULTIV)                                                                              \
-  launch_dependent(ln_modulate_row_kernel<F32, DUALV, MULTIV>, row_ctas, 128, 0, stream, a, pb, ga, zero, nzero, E, eps, \
-                   mod_stride, per)
+  launch_dependent(ln_modulate_row_kernel<F32, DUALV, MULTIV>, row_ctas, 128, 0, stream, a, pb, ga, E, eps, mod_stride, per)
 #define SD3_LN_ROW(F32)                                     \
   case F32:                                                 \
     if (dual) SD3_LN_ROW_INST(F32, true, true);             \
@@ -323,13 +318,13 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   do {                                                                                                                   \
     if constexpr (MAXV > LN_ROW_QUADS) {                                                                                 \
       if (dual) {                                                                                                        \
-        launch_dependent(ln_modulate_kernel<MAXV, F32, true>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero,    \
-                         nzero, E, eps, mod_stride, rpw);                                                                \
+        launch_dependent(ln_modulate_kernel<MAXV, F32, true>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, E,       \
+                         eps, mod_stride, rpw);                                                                          \
         break;                                                                                                           \
       }                                                                                                                  \
     }                                                                                                                    \
-    launch_dependent(ln_modulate_kernel<MAXV, F32, false>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, zero,       \
-                     nzero, E, eps, mod_stride, rpw);                                                                    \
+    launch_dependent(ln_modulate_kernel<MAXV, F32, false>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, E, eps,     \
+                     mod_stride, rpw);                                                                                   \
   } while (0)
   switch (out_f32) {
     case 1: SD3_LN_LAUNCH(1); break;
@@ -513,7 +508,7 @@ __global__ void rmsnorm_heads_kernel(XT* x, long ld, long rows, int col0, int nh
 }  // namespace
 
 int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps, long mod_stride, int out_f32,
-                       cudaStream_t stream, unsigned* zero, int nzero) {
+                       cudaStream_t stream) {
   for (const LnProblem* p : {&a, b}) {
     if (!p) continue;
     if (!p->x || !p->out1 || !p->shift1 || !p->scale1 || p->B <= 0 || p->T <= 0 || E <= 0 || (E & 3) ||
@@ -528,7 +523,7 @@ int launch_ln_modulate(const LnProblem& a, const LnProblem* b, int E, float eps,
   }
   const int nvec = E / 4;
 #define SD3_LN_CASE(MV) \
-  if (nvec <= 32 * MV) return launch_ln_inst<MV>(a, b, E, eps, mod_stride, out_f32, stream, zero, nzero)
+  if (nvec <= 32 * MV) return launch_ln_inst<MV>(a, b, E, eps, mod_stride, out_f32, stream)
   SD3_LN_CASE(2);
   SD3_LN_CASE(6);
   SD3_LN_CASE(12);

@@ -23,7 +23,6 @@ enum : int {
   DEV_TIMEOUT_EMPTY = 102,      // producer waited on an smem "empty" barrier
   DEV_TIMEOUT_TMEM_FULL = 103,  // epilogue waited for an accumulator
   DEV_TIMEOUT_TMEM_EMPTY = 104, // MMA warp waited for the epilogue to drain
-  DEV_TIMEOUT_ORDER = 105,      // a reduction waited for the one before it to the same rows
   DEV_TIMEOUT_ATTN_S = 111,
   DEV_TIMEOUT_ATTN_P = 112,
   DEV_TIMEOUT_ATTN_O = 113,
@@ -71,6 +70,7 @@ __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -161,33 +161,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, c
 // lane 0 had taken, every tcgen05.mma took 63 to 88 cycles to issue, elected 33 to 39.
 __device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, const WaitCtx& w, int code) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, w, code)) != 0;
-}
-
-// Ordered reductions of two tiles of one launch into the same memory: the warp that adds first publishes when its
-// reductions have landed, the one that adds second waits (bounded) before it issues its own.  Called by one lane.
-__device__ __forceinline__ void order_publish(unsigned* flag) {
-  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  asm volatile("fence.proxy.async;" ::: "memory");
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory");
-}
-__device__ __forceinline__ bool order_wait(const unsigned* flag, const WaitCtx& w) {
-  const uint64_t t0 = global_timer_ns();
-  uint32_t it = 0;
-  while (true) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-    if (v != 0) break;
-    if (((++it) & 0x3fu) == 0) {
-      if (*w.s_abort) return false;
-      if (global_timer_ns() - t0 > SD3_WAIT_LIMIT_NS) {
-        *w.s_abort = 1;
-        if (w.g_status) atomicCAS(w.g_status, 0, DEV_TIMEOUT_ORDER);
-        return false;
-      }
-    }
-  }
-  asm volatile("fence.proxy.async;" ::: "memory");
-  return true;
 }
 
 // After an abort: give copies and MMAs already in flight a bounded time to
