@@ -12,6 +12,7 @@
 // (modules.cpp:946-995); conv2d im2col side of PatchEmbedding
 // (modules.cpp:1037-1117); rmsnorm_key_query_kernel2 (cuda/dit.cu:384-447).
 #include "kernels.h"
+#include "launch_rules.h"
 #include "ptx.cuh"
 #include "split3.cuh"
 
@@ -41,14 +42,6 @@ namespace {
 // and two of them in a row cost twice that.  The first row is requested before the
 // barrier behind the staging.  Measured (whole forward, one image): 256x256 3510 -> 3326 us,
 // 1024x1024 14.18 -> 13.96 ms.  Three CTAs per SM for the plane output, whose splits need the registers.
-constexpr int LN_ROW_QUADS = 12;  // ln_modulate_row_kernel: float4 words of a row per lane index (E up to 1536)
-// With one modulation it is taken with one row per CTA up to LN_ROW_MAX rows of a launch (both problems) and with several
-// above LN_ROWS_MIN, with two modulations always.  us, kernel with staged vectors / a row per CTA / several:
-//   one   589 rows 4.45 / 2.44 / 3.10   1357 5.29 / 4.14 / 4.32   2714 7.82 / 6.23 / 6.91   4429 8.34 / 8.95 / 9.64
-//         8858 17.9 / 18.4 / 17.3   13287 29.0 / - / 23.5   35432 60.6 / 68.9 / 55.2 (up to 8 rows; 64: 64.9)
-//   two   589 rows 6.70 / 3.44 / 3.06   1357 8.26 / 5.16 / 4.08   4429 14.2 / 12.2 / 8.8   13287 47.5 / 38.3 / 30.1
-//         35432 97.4 / 96.7 / 76.0 (up to 64 rows; 8: 13287 33.3, 35432 76.2)
-constexpr long LN_ROW_MAX = 3700, LN_ROWS_MIN = 8000;
 constexpr int LN_MAX_ROWS_PER_WARP = 8;
 constexpr int LN_WARPS = 8;
 
@@ -194,7 +187,7 @@ ln_modulate_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__
 // the vectors in registers (read for every row, two modulations' are four times the row's bytes, all from L2) and
 // has the next row under way while it forms one.  The sums are formed in the order of the kernel above (each lane adds its
 // quads in order, then the lanes' tree): the same bits.  Bound by latency at a thousand rows, by L2 and HBM
-// above (5.9 TB/s at 35432 rows; LN_ROW_MAX has the figures).
+// above (5.9 TB/s at 35432 rows).  Which sizes take it: ln_kernel (launch_rules.h), with the figures.
 template <int OUT, bool DUAL, bool MULTI>
 __global__ void __launch_bounds__(128)
 ln_modulate_row_kernel(const __grid_constant__ LnProblem pa, const __grid_constant__ LnProblem pb, const unsigned grid_a,
@@ -287,8 +280,9 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   const bool dual = a.out2 != nullptr || (b && b->out2 != nullptr);
   const size_t smem = static_cast<size_t>(E) * 4 * (dual ? 4 : 2);
   const LnProblem pb = b ? *b : a;
-  if (E <= 4 * 32 * LN_ROW_QUADS && (dual || rows_a + rows_b <= LN_ROW_MAX || rows_a + rows_b > LN_ROWS_MIN)) {
-    const bool multi = dual || rows_a + rows_b > LN_ROWS_MIN;
+  const LnKernel kind = ln_kernel(E, rows_a + rows_b, dual, device_sm_count());
+  if (kind != LN_WARP_PER_ROW) {
+    const bool multi = kind == LN_ROWS_PER_CTA;
     // rows of a CTA: as many as lets all CTAs be resident at once, up to a limit
     const long resident = 5L * device_sm_count(), most = dual ? 64 : 8;
     const long want = (rows_a + rows_b + resident - 1) / resident;
@@ -316,7 +310,7 @@ int launch_ln_inst(const LnProblem& a, const LnProblem* b, int E, float eps, lon
   }
 #define SD3_LN_LAUNCH(F32)                                                                                               \
   do {                                                                                                                   \
-    if constexpr (MAXV > LN_ROW_QUADS) {                                                                                 \
+    if constexpr (MAXV != LN_ROW_QUADS) {                                                                                \
       if (dual) {                                                                                                        \
         launch_dependent(ln_modulate_kernel<MAXV, F32, true>, grid, LN_WARPS * 32, smem, stream, a, pb, grid_a, E,       \
                          eps, mod_stride, rpw);                                                                          \
