@@ -32,6 +32,7 @@
 
 #include "gemm_epilogue.cuh"
 #include "kernels.h"
+#include "launch_rules.h"
 #include "pair_tiles.h"
 #include "ptx.cuh"
 
@@ -389,31 +390,6 @@ int build_problem(PairProblem* pp, const GemmProblem& q, int operand_dtype, int 
   return ST_OK;
 }
 
-// The tile width with the least time by waves: a wave of 128-wide tiles takes 0.64 of a wave of 256-wide ones (half the
-// MMA time, but 96 bytes of operands per clock and SM where TMA brings at most 82 to 92), and the last wave's
-// epilogue, which nothing overlaps, is half as long, worth about ten 64-wide K blocks of a wide tile.  Measured, us, wide /
-// narrow (waves of each):
-//   K 1536, QKV    589 rows 15.0 / 12.9 (1, 2)   1357: 21.7 / 18.5 (2, 3)   2714: 30.3 / 33.3 (3, 6)   4429: 49.1 / 52.2 (5, 9)
-//   K 1536, GELU   333 rows 15.8 / 13.3 (1, 2)   1024: 21.0 / 19.1 (2, 3)   1357: 23.7 / 24.7 (2, 4)   4429: 61.9 / 71.7 (6, 12)
-//   K 1536, gate  2714 rows 14.5 / 14.6 (1, 2)   4429: 23.5 / 21.2 (2, 3)   5428: 26.7 / 28.8 (2, 4)
-//   K 4096, fp32 output (the captions)  333 rows 24.8 / 14.9 (1, 1)   1332: 25.2 / 16.0 (1, 1)
-//   K 6144, gate  2714 rows 38.6 / 43.6 (1, 2)   4429: 68.8 / 67.4 (2, 3)   5428: 75.4 / 86.9 (2, 4)
-// after256: those of the 256-wide tiles that run after another one on the same pair (GemmEpilogue::adds_after), a wave of
-// their own.
-int choose_tile_width(long tiles256, long after256, int k_blocks, const GemmEpilogue& epi) {
-  const long pairs = device_sm_count() / 2;
-  if (pairs <= 0 || !narrow_tiles_built(epi)) return 256;
-  // The gate + residual GEMMs, the ones with few tiles, have 64-wide ones too, for problems that fit one wave of
-  // those.  us, 128 / 64 wide: K 6144, 256 rows 19.7 / 17.9, 333 rows 19.8 / 18.5, 700 rows 19.9 / 19.5; K 1536, 256 rows
-  // 7.7 / 7.0, 589 rows 8.2 / 8.2 (slots of four stages: 20.1 at 256 rows).
-  if (epi.mode == EPI_GATE_RESID && 4 * (tiles256 - after256) <= pairs) return 64;
-  auto waves = [&](int per256) {
-    return (per256 * (tiles256 - after256) + pairs - 1) / pairs + (per256 * after256 + pairs - 1) / pairs;
-  };
-  const long wide = waves(1), narrow = waves(2);
-  return 64 * narrow * k_blocks < 100 * wide * k_blocks + 1000 ? 128 : 256;
-}
-
 }  // namespace
 
 // Whether the CTA-pair kernel covers this problem (N a multiple of 256, enough rows to fill
@@ -451,9 +427,10 @@ int launch_gemm_pair(const GemmProblem* q, int n, int operand_dtype, int N, int 
     }
     tiles256 += static_cast<long>((q[i].M + 255) / 256) * (N / 256);
   }
-  const int kel = P_KBYTES / (fp8 ? 1 : 2);
   const long after256 = sum ? static_cast<long>((a.M + 255) / 256) * (N / 256) : 0;
-  const int pbn = choose_tile_width(tiles256, after256, (K + kel - 1) / kel, a.epi);
+  const int pbn = !narrow_tiles_built(a.epi) ? 256
+                                             : pair_tile_width(tiles256, after256, K, fp8, a.epi.mode == EPI_GATE_RESID,
+                                                               device_sm_count() / 2);
   PairProblem p[3];
   int end[3] = {0, 0, 0}, count = 0;
   for (int i = 0; i < 3; ++i) {

@@ -16,9 +16,10 @@ def rules(tmp_path_factory):
 #include <stdio.h>
 #include "launch_rules.h"
 int main() {
-  char what; long a, b, c;
-  while (scanf(" %c %ld %ld %ld", &what, &a, &b, &c) == 4)
+  char what; long a, b, c, d, e;
+  while (scanf(" %c %ld %ld %ld %ld %ld", &what, &a, &b, &c, &d, &e) == 6)
     if (what == 'n') printf("%d\\n", static_cast<int>(sd3::ln_kernel(static_cast<int>(a), b, c != 0, 148)));
+    else printf("%d\\n", sd3::pair_tile_width(a, b, static_cast<int>(c), d != 0, e != 0, 74));
 }
 """)
     subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-Werror", "-I", CSRC, str(d / "rules.cpp"), "-o", str(d / "rules")],
@@ -41,4 +42,24 @@ def test_layernorm(rules):
              (1280, 8858, 0, WARP), (1280, 9500, 0, ROWS), (1280, 35432, 1, ROWS),
              (1536, 77, 0, CTA), (1536, 3000, 0, CTA), (1536, 4429, 0, WARP), (1536, 8200, 0, ROWS), (1536, 35432, 0, ROWS),
              (1536, 589, 1, ROWS), (1536, 35432, 1, ROWS), (1540, 77, 0, WARP), (2432, 4429, 1, WARP)]
-    assert rules(["n %d %d %d" % c[:3] for c in cases]) == [c[3] for c in cases]
+    assert rules(["n %d %d %d 0 0" % c[:3] for c in cases]) == [c[3] for c in cases]
+
+
+def test_tile_width(rules):
+    def q(rows, N, K, gate, after=0, fp8=0):
+        tiles = (rows + 255) // 256 * (N // 256)
+        return "w %d %d %d %d %d" % (tiles + after, after, K, fp8, gate)
+    cases = [(q(589, 4608, 1536, 0), 128), (q(1357, 4608, 1536, 0), 128), (q(2714, 4608, 1536, 0), 256),
+             (q(4429, 4608, 1536, 0), 256), (q(1024, 6144, 1536, 0), 128), (q(1357, 6144, 1536, 0), 256),
+             (q(256, 1536, 6144, 1), 64), (q(700, 1536, 6144, 1), 64), (q(2714, 1536, 6144, 1), 256),
+             (q(4429, 1536, 6144, 1), 128), (q(5428, 1536, 6144, 1), 256), (q(4429, 1536, 1536, 1), 128),
+             (q(1332, 1536, 4096, 0), 128),
+             # few K blocks, several waves
+             (q(8192, 1024, 1024, 1), 256), (q(16384, 1024, 1024, 0), 256), (q(16384, 512, 512, 1), 256),
+             (q(8192, 1536, 512, 0), 256), (q(2714, 1024, 1024, 0), 128), (q(4096, 1536, 512, 1), 128),
+             # FP8, 576 + 333 tokens: QKV (three problems) and MLP1
+             (q(2 * 768 + 512, 4608, 1536, 0, fp8=1), 128), (q(768 + 512, 6144, 1536, 0, fp8=1), 128),
+             # a dual block's out-projections: 256 + 333, 1024 + 333 and 4096 + 333 rows
+             (q(256 + 512, 1536, 1536, 1, after=6), 64), (q(1024 + 512, 1536, 1536, 1, after=24), 128),
+             (q(4096 + 512, 1536, 1536, 1, after=96), 128)]
+    assert rules([c[0] for c in cases]) == [c[1] for c in cases]
