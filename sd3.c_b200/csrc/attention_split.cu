@@ -4,7 +4,7 @@
 // statistics, exponentials and the running output are fp32.
 //
 // One CTA owns 128 queries of one (sample, head).  Warp 0 streams the planes of
-// K (two 128-key stages) and V (two 64-key halves) with TMA; one thread of
+// K (two 128-key stages) and V (two 64-key halves) with TMA; an elected lane of
 // warp 1 issues the MMAs; eight softmax warps own half the keys of a query row
 // per thread (TMEM lane == row).  Per 128 keys:
 //   S = Q K^T   24 MMAs of N = 128, smallest products first;

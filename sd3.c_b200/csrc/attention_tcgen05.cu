@@ -5,7 +5,7 @@
 //
 // One CTA owns a 128-query tile of one (sample, head); two CTAs are resident
 // per SM (256 TMEM columns each).  Warp 0 streams K and V tiles of 128 keys with
-// TMA from the packed (B, T, 3E) q|k|v buffer; one thread of warp 1 issues the
+// TMA from the packed (B, T, 3E) q|k|v buffer; an elected lane of warp 1 issues the
 // MMAs; four softmax warps own one query row per thread (TMEM lane == row).
 // Per 128-key tile:
 //   S = Q K^T        four MMAs of N = 128 into 128 fp32 TMEM columns,

@@ -15,7 +15,7 @@
 //                               second QKV GEMM(x) rides in the same launch (up to MERGE_MAX_TOKENS)
 //   joint attention          -> o_c, o_x; a dual block's attention over the image tokens too
 //   out-proj GEMM(c), (x)     -> gate * (.) + residual fused, fp32 streams in place
-//   [dual] out-proj GEMM with gate2 (up to MERGE_MAX_TOKENS in the same launch)
+//   [dual] out-proj GEMM with gate2 (up to MERGE_MAX_TOKENS in the same launch, in bf16 and FP8)
 //   LN+modulate(x), (c); MLP1 GEMM (+GELU-tanh), MLP2 GEMM (+gate, +residual), each for x and c at once
 #include <math.h>
 #include <algorithm>

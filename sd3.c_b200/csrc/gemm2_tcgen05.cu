@@ -1,12 +1,14 @@
 // CTA-pair variant of the tcgen05 GEMM: two CTAs (a cluster of two on
-// neighbouring SMs) cooperate on 256 x 256 (or 256 x 128, where those fill the SMs better) output tiles with
-// tcgen05.mma.cta_group::2.  One launch can carry up to THREE problems of the same
+// neighbouring SMs) cooperate on 256 x 256 output tiles (256 x 128 or, for gate + residual, 256 x 64 where those fill
+// the SMs better: launch_rules.h) with tcgen05.mma.cta_group::2.  One launch can carry up to THREE problems of the same
 // shape class (same N, K and epilogue: the image-stream GEMM of a block, its
 // small context-stream twin and, for QKV, the second projection of a dual block);
 // the persistent tile loop runs one problem's tiles after the other's, so the small
 // ones ride in the tail of the large one instead of being launches of their own
 // that fill less than a wave (the third problem: forward of one 256x256 image 3284 -> 3133 us, 512x512
-// 4467 -> 4407 us, 1024x1024 unchanged).
+// 4467 -> 4407 us, 1024x1024 unchanged).  A dual block's two out-projections add to the same rows: a pair that has run
+// a tile of the first runs the third problem's tile of the same place next (pair_tiles.h; against a launch of their own,
+// 256x256 2335 -> 2311 us, 512x512 3719 -> 3690, 1024x1024 unchanged).
 //
 //   acc[m, n] = sum_k A[m, k] * W[n, k]        A: (M, K) K-major, W: (N, K) K-major
 //
@@ -19,8 +21,8 @@
 // descriptors and addresses then live in uniform registers.  From a branch taken by lane 0 alone an MMA took
 // 63-88 cycles to issue (a 128-wide MMA runs 64) and a slot's loads 740; elected, 33-39 and under 300.
 // Measured, lane 0 with two issuing threads that took turns -> elected lane of one warp (us, weights from
-// HBM): N = 1536, K = 6144, 589 rows 26.9 -> 20.4, 4429 rows 73.2 -> 69.1; QKV 4429 rows 59.6 -> 48.9, 13287 rows
-// 177 -> 128; GELU 4429 rows 68.9 -> 63.0.  Completion is signalled to both CTAs with
+// HBM): N = 1536, K = 6144, 589 rows 26.9 -> 20.0, 4429 rows 72.6 -> 68.8; QKV 4429 rows 60.9 -> 49.1, 13287 rows
+// 143 -> 123 (147 -> 130 on another box); GELU 4429 rows 68.3 -> 61.9.  Completion is signalled to both CTAs with
 // tcgen05.commit ... multicast::cluster.  Each CTA keeps the accumulator rows
 // of its own half of M in its own TMEM (two buffers of 256 columns) and drains
 // them through the same fused epilogues as the one-CTA kernel.
@@ -94,7 +96,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ PairProblem p0, const __grid_co
                                              ~static_cast<uintptr_t>(1023));
   constexpr int P_STAGES = pair_stages(PBN);
   static_assert(EPI_WARPS * ((PBN + 63) / 64) * P_RED_BYTES <= P_STAGES * P_STAGE_BYTES, "the last tile's boxes fit the ring");
-  uint8_t* red_smem = smem + P_STAGES * P_STAGE_BYTES;  // 1024-byte aligned: stages are 32 / 24 KiB each
+  uint8_t* red_smem = smem + P_STAGES * P_STAGE_BYTES;  // 1024-byte aligned: stages are 32 / 24 / 20 KiB each
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + P_STAGES * P_STAGE_BYTES + pair_red_bytes(EPI, OUT_F32));
   uint64_t* empty_bar = full_bar + P_STAGES;
   uint64_t* tfull_bar = empty_bar + P_STAGES;

@@ -81,13 +81,13 @@ struct SplitCfg {
   static constexpr int STAGE_BYTES = 3 * (S_A_PLANE + W_PLANE);  // 72 / 60 KiB
   static constexpr int STAGES = 3;                               // 216 / 180 KiB
   static constexpr int NBUF = 4;                                 // TMEM accumulators
-  static_assert(NBUF % 2 == 0, "an accumulator belongs to one of the two MMA-issuing threads");
+  static_assert(NBUF % 2 == 0, "an accumulator belongs to one of the two MMA-issuing warps");
   static constexpr int TMEM_COLS = NBUF * PBN;
   static constexpr int EPI_WARPS = PBN == 64 ? 4 : 8;
   static constexpr int CPW = 64;                     // accumulator columns per epilogue thread (split_epilogue_64)
   static constexpr int MMA2_WARP = 2 + EPI_WARPS;    // second MMA-issuing warp
   static constexpr int THREADS = 32 * (3 + EPI_WARPS);
-  using Ring = OperandRing<STAGES, 2>;  // two MMA-issuing threads
+  using Ring = OperandRing<STAGES, 2>;  // two MMA-issuing warps, an elected lane of each
   static constexpr int BAR_BYTES = (Ring::FULL_BARS + STAGES + 2 * NBUF) * 8 + 8;  // barriers, TMEM address, abort flag
   static_assert(BAR_BYTES <= 256, "barrier block");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;

@@ -299,7 +299,7 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t a_fmt, uint32_t b_fmt
 }
 
 // ----------------------------------------------------------------------------
-// tcgen05: MMA issue and commit (single thread)
+// tcgen05: MMA issue and commit (one lane)
 // ----------------------------------------------------------------------------
 // D[tmem] (+)= A[smem] * B[smem]
 __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,

@@ -438,7 +438,7 @@ class Model:
         set of tensor addresses and shapes runs the forward once eagerly (which reserves the
         workspace), captures it on the current stream and replays it; later calls only replay.
         For loops that call the denoiser on fixed device buffers (a sampler's latent buffer, a
-        serving slot): at one sample per GPU the ~270 launches of a step otherwise cost about
+        serving slot): at one sample per GPU the 180 to 270 launches of a step otherwise cost about
         2 % of it.  The tensors must stay alive and in place; a larger problem, set_param and
         reserve drop the captured graphs.  Returns `out`."""
         torch = _torch()
@@ -574,7 +574,7 @@ def sample(model, latents, cond_captions, cond_pooled, uncond_captions, uncond_p
     use_graph: record all `steps` denoiser calls and updates into one CUDA graph
     and launch that (one untimed denoiser call first sizes the workspace, which
     a stream capture must not do).  The result is bit-identical to the eager
-    loop; what it saves is the host's share of ~360 launches per step."""
+    loop; what it saves is the host's share of the 180 to 270 launches per step."""
     torch = _torch()
     n = latents.shape[0]
     dt = latents.dtype
