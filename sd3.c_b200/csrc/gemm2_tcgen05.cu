@@ -22,7 +22,7 @@
 // 63-88 cycles to issue (a 128-wide MMA runs 64) and a slot's loads 740; elected, 33-39 and under 300.
 // Measured, lane 0 with two issuing threads that took turns -> elected lane of one warp (us, weights from
 // HBM): N = 1536, K = 6144, 589 rows 26.9 -> 20.0, 4429 rows 72.6 -> 68.8; QKV 4429 rows 60.9 -> 49.1, 13287 rows
-// 143 -> 123 (147 -> 130 on another box); GELU 4429 rows 68.3 -> 61.9.  Completion is signalled to both CTAs with
+// 143 -> 123 (147 -> 130 on another GPU); GELU 4429 rows 68.3 -> 61.9.  Completion is signalled to both CTAs with
 // tcgen05.commit ... multicast::cluster.  Each CTA keeps the accumulator rows
 // of its own half of M in its own TMEM (two buffers of 256 columns) and drains
 // them through the same fused epilogues as the one-CTA kernel.
